@@ -1,78 +1,563 @@
 // The true 32-bit matrix product: C = epilogue(A[M,K] . W[N,K]^T + bias), plain FMA on
-// CUDA cores, no tensor cores and no reduced-precision mode.  Each output element is
-// accumulated by one thread over k = 0..K-1 in ascending order, so a row's result does
-// not depend on how many other rows are in the batch.
+// CUDA cores, no tensor cores and no reduced-precision mode.
+//
+// ONE order of summation for every size, so that a row's result does not depend on how many
+// other rows are in the batch nor on which of the two kernels below computes it: K is cut into
+// chunks of 32; a thread accumulates a chunk's even and its odd k's, each in ascending order, and
+// adds the two (a pair is what fma.rn.f32x2 takes: half the instructions); the chunks are cut into four runs of ceil(chunks / 4), a run's chunk sums are added
+// in ascending order, and the result is (run 0 + run 1) + (run 2 + run 3).  (Closer to the 64-bit
+// product than one chain over all of K, which was here before: 1.0e-7 against 4.9e-7 relative at
+// K = 768, 1.3e-7 against 1.0e-6 at 3,072, normal numbers.)
+//
+// gemm_f32_stream_kernel: up to eight rows a CTA, bound by the weights' way from memory.  Every
+// CTA owns a run of weight rows and requests them through a ring of shared-memory stages
+// (TMA where K is a multiple of
+// 32, else cp.async; the first of them before the kernel ahead has ended); a thread keeps its chunk of up
+// to four rows of A in registers and walks the weight rows of a stage, so an FMA costs a quarter
+// of a shared-memory operand; chunk sums meet in shared memory.  8 rows, weights from memory:
+// 2,304 x 768 6.8 us, 768 x 3,072 10.4 us, 50,257 x 768 72 us = 2.15 TB/s; the kernel before (64 x
+// 64 tiles, one CTA a tile, so 12 CTAs for 768 columns) took 177 us on average over a model's
+// products.
+//
+// gemm_f32_tile_kernel: more rows, bound by FMA issue and the shared-memory reads beside it.  Tiles of BM x BN, the four runs of K by
+// the four CTAs of a cluster (a prompt of a few hundred tokens has too few tiles for 148 SMs
+// otherwise), partial tiles added through distributed shared memory, a quarter of the rows a CTA.
+// 650 rows: 2,304 x 768 76 us, 768 x 3,072 106 us, 50,257 x 768 1.49 ms = 34 TFLOP/s (about 14
+// before).
 #include "common.cuh"
+#include "tcgen05.cuh"
+#include "tensor_map.cuh"
 
 namespace {
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
+constexpr int CH = 32;              // k's of a chunk
+constexpr int CHP = 36;             // its floats in shared memory: 16-byte reads of neighbouring
+                                    // chunks (or rows) by a quarter of a warp hit all banks once
 
-__global__ void __launch_bounds__(256)
-gemm_f32_kernel(float* __restrict__ c, const float* __restrict__ a, const float* __restrict__ w,
-                const float* __restrict__ bias, const float* __restrict__ resid, int m, int n,
-                int k, long lda, long ldw, long ldc, int act) {
-    __shared__ float as[BK][BM + 1];
-    __shared__ float ws[BK][BN + 1];
-    const int tid = threadIdx.x;
-    const int tx = tid % 16, ty = tid / 16;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    float acc[TM][TN];
+struct Args {
+    float* c;
+    const float* a;
+    const float* w;
+    const float* bias;
+    const float* resid;
+    int m, n, k;
+    long lda, ldw, ldc;
+    int act;
+    int* status;
+};
+
+using tc5::mbar_expect_tx;
+using tc5::mbar_init;
+using tc5::mbar_wait;
+using tc5::mbar_try_wait;
+using tc5::smem_u32;
+
+// copies `bytes` (0..16) and fills the rest of the 16 bytes with zeros
+__device__ __forceinline__ void cp16(uint32_t dst, const float* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp4(uint32_t dst, const float* src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// One row of `k` floats into padded chunks of shared memory by one warp (zeros beyond K;
+// a row outside the matrix, `valid` false, is left alone and `src` only has to be an address).
+template <bool VEC>
+__device__ __forceinline__ void copy_row(float* dst, const float* src, int k, int nc, int lane) {
+    const uint32_t d = smem_u32(dst);
+    if (VEC) {
+        for (int q = lane; q < nc * (CH / 4); q += 32) {
+            const int left = k - q * 4;                       // (a multiple of 4)
+            cp16(d + (uint32_t)((q >> 3) * CHP + (q & 7) * 4) * 4u, left > 0 ? src + q * 4 : src,
+                 left > 0 ? 16 : 0);
+        }
+    } else {
+        for (int i = lane; i < nc * CH; i += 32)
+            cp4(d + (uint32_t)((i >> 5) * CHP + (i & 31)) * 4u, i < k ? src + i : src, i < k ? 4 : 0);
+    }
+}
+
+// acc += a * b, both halves (each rounded once, as fmaf)
+__device__ __forceinline__ void fma2(float2& acc, float ax, float ay, float bx, float by) {
+    asm("{\n\t.reg .b64 a, b, c;\n\t"
+        "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%0, %1};\n\t"
+        "fma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
+        : "+f"(acc.x), "+f"(acc.y) : "f"(ax), "f"(ay), "f"(bx), "f"(by));
+}
+
+__device__ __forceinline__ float finish(const Args& p, float v, int row, int col) {
+    if (p.bias) v += p.bias[col];
+    v = prb_activate(v, p.act);
+    if (p.resid) v += p.resid[(size_t)row * p.ldc + col];
+    return v;
+}
+
+// ------------------------------------------------------------------------- a few rows
+constexpr int STREAM_THREADS = 256;
+constexpr int STREAM_STAGES_MAX = 6;
+
+struct StreamGeo {
+    int rows_per_cta;               // weight rows a CTA owns
+    int rows;                       // of them in a stage
+    int stages;
+    int stage_len;                  // floats of a stage
+    int nc;                         // chunks of K
+    int items, slots;               // (chunk, group of rows of A) pairs; weight rows walked side by side
+};
+
+// How the weights come: single floats or 16 bytes by cp.async (chunks padded to CHP floats), or a
+// stage at a time by TMA (K a multiple of 32; chunks of 128 bytes, their 16-byte pieces swizzled).
+enum { COPY_4 = 0, COPY_16 = 1, COPY_TMA = 2 };
+
+// {32 floats, chunks, rows} of a row-major [n, k] matrix: a copy brings `rows` whole rows, chunk
+// after chunk, 128-byte swizzle; x is always 0, so the 16-byte rule on it holds.
+int chunk_map(const float* w, int n, int k, long ldw, int rows, CUtensorMap* out) {
+    static std::unordered_map<tmap::MapKey, CUtensorMap, tmap::MapKeyHash> cache;
+    static std::mutex mu;
+    const tmap::MapKey key{w, n, k, ldw, rows};
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = cache.find(key);
+    if (it != cache.end()) {
+        *out = it->second;
+        return 0;
+    }
+    auto fn = tmap::encode_fn();
+    if (!fn) return -6;
+    cuuint64_t dims[3] = {CH, (cuuint64_t)(k / CH), (cuuint64_t)n};
+    cuuint64_t strides[2] = {CH * 4, (cuuint64_t)ldw * 4};
+    cuuint32_t box[3] = {CH, (cuuint32_t)(k / CH), (cuuint32_t)rows};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUtensorMap map;
+    if (fn(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(w), dims, strides, box, estr,
+           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return -5;
+    if (cache.size() > 8192) cache.clear();
+    cache.emplace(key, map);
+    *out = map;
+    return 0;
+}
+
+template <int MB, int COPY>
+__global__ void __launch_bounds__(STREAM_THREADS, 1)
+gemm_f32_stream_kernel(Args p, StreamGeo g, const __grid_constant__ CUtensorMap map_w) {
+    constexpr int MT = MB < 4 ? MB : 4;                       // rows of A a thread holds
+    constexpr bool VEC = COPY != COPY_4;
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    __shared__ uint64_t bars[STREAM_STAGES_MAX];
+    __shared__ int failed_word;
+    volatile int* failed = &failed_word;
+    // (the swizzle is a function of the address: stages start on 1,024 bytes)
+    float* ws = reinterpret_cast<float*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row_len = g.nc * CHP;
+    float* as = ws + (size_t)g.stages * g.stage_len;          // [MB][row_len]
+    float* part = as + MB * row_len;                          // [2][rows * MB][nc + 1]
+    const int part_len = g.rows * MB * (g.nc + 1);
+    const int n0 = blockIdx.x * g.rows_per_cta;
+    const int n1 = min(p.n, n0 + g.rows_per_cta);
+    const int m0 = blockIdx.y * MB;
+    const int n_stages = (n1 - n0 + g.rows - 1) / g.rows;
+    bool alive = true;
+    if (COPY == COPY_TMA) {
+        if (tid == 0) {
+            for (int s = 0; s < g.stages; ++s) mbar_init(smem_u32(&bars[s]), 1);
+            *failed = 0;
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        __syncthreads();
+    }
+
+    auto load_stage = [&](int s) {
+        if constexpr (COPY == COPY_TMA) {
+            if (tid == 0 && s < n_stages && alive) {
+                const uint32_t bar = smem_u32(&bars[s % g.stages]);
+                mbar_expect_tx(bar, (uint32_t)g.rows * g.nc * CH * 4);
+                asm volatile(
+                    "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+                    "[%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(ws + (size_t)(s % g.stages) * g.stage_len)),
+                    "l"(&map_w), "r"(bar), "r"(0), "r"(0), "r"(n0 + s * g.rows)
+                    : "memory");
+            }
+        } else {
+            if (s < n_stages) {
+                float* dst = ws + (size_t)(s % g.stages) * g.stage_len;
+                for (int r = warp; r < g.rows; r += STREAM_THREADS / 32) {
+                    const int n = n0 + s * g.rows + r;
+                    if (n < n1) copy_row<VEC>(dst + r * row_len, p.w + (size_t)n * p.ldw, p.k, g.nc, lane);
+                }
+            }
+            cp_commit();
+        }
+    };
+    // weights never depend on the kernel before this one; A does
+    for (int s = 0; s < g.stages; ++s) load_stage(s);
+    prb_grid_wait();
+    prb_grid_launch_dependents();
+    for (int r = warp; r < MB; r += STREAM_THREADS / 32) {
+        float* dst = as + r * row_len;
+        if (m0 + r < p.m) {
+            const float* src = p.a + (size_t)(m0 + r) * p.lda;
+            for (int i = lane * 4; i < g.nc * CH; i += 128) {
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (VEC) {
+                    if (i < p.k) v = *reinterpret_cast<const float4*>(src + i);
+                } else {
+                    if (i < p.k) v.x = src[i];
+                    if (i + 1 < p.k) v.y = src[i + 1];
+                    if (i + 2 < p.k) v.z = src[i + 2];
+                    if (i + 3 < p.k) v.w = src[i + 3];
+                }
+                *reinterpret_cast<float4*>(dst + (i >> 5) * CHP + (i & 31)) = v;
+            }
+        } else {
+            for (int i = lane * 4; i < row_len; i += 128)
+                *reinterpret_cast<float4*>(dst + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    __syncthreads();
+
+    float4 av[MT][CH / 4];
+    auto load_a = [&](int item) {
+        const int c = item % g.nc, group = item / g.nc;
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int j = 0; j < CH / 4; ++j)
+                av[i][j] = *reinterpret_cast<const float4*>(as + (group * MT + i) * row_len + c * CHP + j * 4);
+    };
+    const bool resident = g.items <= STREAM_THREADS;          // a thread keeps one item for good
+    const int my_slot = resident ? tid / g.items : 0;
+    const int first_item = resident ? tid % g.items : tid;
+    if (resident && my_slot < g.slots) load_a(first_item);
+
+    const int run = (g.nc + 3) / 4;
+    for (int s = 0; s < n_stages; ++s) {
+        if constexpr (COPY == COPY_TMA) {
+            alive = alive && mbar_wait(smem_u32(&bars[s % g.stages]), (uint32_t)(s / g.stages) & 1u, failed);
+        } else {
+            // all groups but the (stages - 1) newest have landed: stage s among them
+            switch (g.stages) {
+                case 1: cp_wait<0>(); break;
+                case 2: cp_wait<1>(); break;
+                case 3: cp_wait<2>(); break;
+                case 4: cp_wait<3>(); break;
+                case 5: cp_wait<4>(); break;
+                default: cp_wait<5>(); break;
+            }
+            __syncthreads();
+        }
+        const float* wst = ws + (size_t)(s % g.stages) * g.stage_len;
+        float* pt = part + (s & 1) * part_len;
+        const int rows = min(g.rows, n1 - (n0 + s * g.rows));
+        for (int item = first_item; item < g.items; item += STREAM_THREADS) {
+            if (my_slot >= g.slots) break;
+            if (!resident) load_a(item);
+            const int c = item % g.nc, group = item / g.nc;
+            for (int r = my_slot; r < rows; r += g.slots) {
+                const float* wr = COPY == COPY_TMA ? wst + (r * g.nc + c) * CH : wst + r * row_len + c * CHP;
+                const int swz = COPY == COPY_TMA ? (r * g.nc + c) & 7 : 0;
+                float2 acc[MT];
+#pragma unroll
+                for (int i = 0; i < MT; ++i) acc[i] = make_float2(0.0f, 0.0f);
+#pragma unroll
+                for (int j = 0; j < CH / 4; ++j) {
+                    const float4 wv = *reinterpret_cast<const float4*>(wr + (j ^ swz) * 4);
+#pragma unroll
+                    for (int i = 0; i < MT; ++i) {
+                        fma2(acc[i], av[i][j].x, av[i][j].y, wv.x, wv.y);
+                        fma2(acc[i], av[i][j].z, av[i][j].w, wv.z, wv.w);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < MT; ++i)
+                    pt[((group * MT + i) * g.rows + r) * (g.nc + 1) + c] = acc[i].x + acc[i].y;
+            }
+        }
+        __syncthreads();
+        load_stage(s + g.stages);
+        // four threads an output, a run of chunk sums each
+        for (int t0 = 0; t0 < g.rows * MB * 4; t0 += STREAM_THREADS) {
+            const int t = t0 + tid;
+            const int q = t & 3, o = t >> 2;
+            const int r = o % g.rows, i = o / g.rows;
+            float sum = 0.0f;
+            const bool live = o < g.rows * MB && r < rows && m0 + i < p.m && alive;
+            if (live) {
+                const float* src = pt + o * (g.nc + 1);
+                for (int c = q * run; c < min(g.nc, (q + 1) * run); ++c) sum += src[c];
+            }
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            if (live && q == 0) {
+                const int row = m0 + i, col = n0 + s * g.rows + r;
+                p.c[(size_t)row * p.ldc + col] = finish(p, sum, row, col);
+            }
+        }
+    }
+    if constexpr (COPY == COPY_TMA) {
+        if (tid == 0 && !alive) {
+            prb_set_status(p.status, PRB_S_WAIT_TIMEOUT, 40, blockIdx.x, blockIdx.y);
+            for (int s = 0; s < g.stages; ++s)                // (copies in flight, bounded)
+                for (uint32_t i = 0; i < (1u << 16); ++i)
+                    if (mbar_try_wait(smem_u32(&bars[s]), 0) || mbar_try_wait(smem_u32(&bars[s]), 1)) break;
+        }
+    } else {
+        cp_wait<0>();
+    }
+}
+
+// ------------------------------------------------------------------------- many rows
+constexpr int TILE_STAGES = 3;
+
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster4(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(r));
+    return v;
+}
+
+template <int BM, int BN, int TM, int TN> struct TileCfg {
+    static constexpr int THREADS = (BM / TM) * (BN / TN);
+    static constexpr int STAGE = (BM + BN) * CHP;             // floats
+    static constexpr int OUT_LD = BN + 4;
+    static constexpr size_t SMEM =
+        sizeof(float) * (size_t)(TILE_STAGES * STAGE > BM * OUT_LD ? TILE_STAGES * STAGE : BM * OUT_LD);
+};
+
+// grid (4 x column tiles, row tiles), clusters of 4 along x: CTA q sums run q of the chunks
+template <int BM, int BN, int TM, int TN, bool VEC>
+__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((BM / TM) * (BN / TN))
+gemm_f32_tile_kernel(Args p) {
+    using Cfg = TileCfg<BM, BN, TM, TN>;
+    constexpr int NT = Cfg::THREADS;
+    constexpr int TY = BM / TM, TX = BN / TN;
+    static_assert(TX % 8 == 0 && TY % 4 == 0, "a warp is 8 columns by 4 rows of threads");
+    extern __shared__ __align__(16) float smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tx = (warp % (TX / 8)) * 8 + (lane & 7);
+    const int ty = (warp / (TX / 8)) * 4 + (lane >> 3);
+    const int m0 = blockIdx.y * BM, n0 = (blockIdx.x >> 2) * BN, quarter = blockIdx.x & 3;
+    const int nc = (p.k + CH - 1) / CH, run = (nc + 3) / 4;
+    const int c0 = min(nc, quarter * run), c1 = min(nc, c0 + run);
+
+    // rows [0, BM) of a stage are A's, the next BN W's; rows outside the matrices are zeros
+    auto load_rows = [&](int c, bool weights) {
+        if (c < c1) {
+            float* st = smem + ((c - c0) % TILE_STAGES) * Cfg::STAGE + (weights ? BM * CHP : 0);
+            const float* base = weights ? p.w : p.a;
+            const long ld = weights ? p.ldw : p.lda;
+            const int first = weights ? n0 : m0, end = weights ? p.n : p.m;
+            constexpr int PER = VEC ? CH / 4 : CH;
+            const int rows = weights ? BN : BM;
+            for (int i = tid; i < rows * PER; i += NT) {
+                const int r = i / PER, e = (i % PER) * (VEC ? 4 : 1);
+                const bool in = first + r < end && c * CH + e < p.k;
+                const float* src = in ? base + (size_t)(first + r) * ld + c * CH + e : base;
+                const uint32_t dst = smem_u32(st + r * CHP + e);
+                if (VEC) cp16(dst, src, in ? 16 : 0);
+                else cp4(dst, src, in ? 4 : 0);
+            }
+        }
+    };
+    for (int s = 0; s < TILE_STAGES - 1; ++s) load_rows(c0 + s, true);
+    prb_grid_wait();
+    prb_grid_launch_dependents();
+    for (int s = 0; s < TILE_STAGES - 1; ++s) { load_rows(c0 + s, false); cp_commit(); }
+
+    float sum[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
+        for (int j = 0; j < TN; ++j) sum[i][j] = 0.0f;
 
-    for (int k0 = 0; k0 < k; k0 += BK) {
-        // 64 rows x 16 k = 1024 elements per tile, 4 per thread
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int e = tid + i * 256;
-            const int r = e / BK, kk = e % BK;
-            const int gm = m0 + r, gn = n0 + r, gk = k0 + kk;
-            as[kk][r] = (gm < m && gk < k) ? a[(size_t)gm * lda + gk] : 0.0f;
-            ws[kk][r] = (gn < n && gk < k) ? w[(size_t)gn * ldw + gk] : 0.0f;
-        }
+    for (int c = c0; c < c1; ++c) {
+        cp_wait<TILE_STAGES - 2>();
         __syncthreads();
+        load_rows(c + TILE_STAGES - 1, true);
+        load_rows(c + TILE_STAGES - 1, false);
+        cp_commit();
+        const float* st = smem + ((c - c0) % TILE_STAGES) * Cfg::STAGE;
+        const float* ap = st + ty * CHP;
+        const float* wp = st + (BM + tx) * CHP;
+        float2 acc[TM][TN];
 #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            float av[TM], wv[TN];
+        for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int i = 0; i < TM; ++i) av[i] = as[kk][ty * TM + i];
+            for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
 #pragma unroll
-            for (int j = 0; j < TN; ++j) wv[j] = ws[kk][tx * TN + j];
+        for (int e = 0; e < CH; e += 4) {
+            float4 wv[TN];
 #pragma unroll
-            for (int i = 0; i < TM; ++i)
+            for (int j = 0; j < TN; ++j) wv[j] = *reinterpret_cast<const float4*>(wp + j * TX * CHP + e);
 #pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
+            for (int i = 0; i < TM; ++i) {
+                const float4 av = *reinterpret_cast<const float4*>(ap + i * TY * CHP + e);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) fma2(acc[i][j], av.x, av.y, wv[j].x, wv[j].y);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) fma2(acc[i][j], av.z, av.w, wv[j].z, wv[j].w);
+            }
         }
-        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) sum[i][j] += acc[i][j].x + acc[i][j].y;
     }
+    cp_wait<0>();
+    __syncthreads();
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int gm = m0 + ty * TM + i;
-        if (gm >= m) continue;
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int gn = n0 + tx * TN + j;
-            if (gn >= n) continue;
-            float v = acc[i][j];
-            if (bias) v += bias[gn];
-            v = prb_activate(v, act);
-            if (resid) v += resid[(size_t)gm * ldc + gn];
-            c[(size_t)gm * ldc + gn] = v;
+        for (int j = 0; j < TN; ++j) smem[(ty + i * TY) * Cfg::OUT_LD + tx + j * TX] = sum[i][j];
+    cluster_sync_all();
+    // a quarter of the rows, four columns at a time; all remote reads are asked for at once (one
+    // after the other they cost 25 us a 128 x 128 tile, twice the tile's FMAs)
+    constexpr int PER = (BM / 4) * (BN / 4) / NT;
+    const int r0 = quarter * (BM / 4);
+    float4 v[PER][4];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int e = tid + i * NT;
+        const uint32_t at = smem_u32(smem + (r0 + e / (BN / 4)) * Cfg::OUT_LD + (e % (BN / 4)) * 4);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[i][q] = ld_cluster4(at, q);
+    }
+    const bool whole = p.ldc % 4 == 0 && ((uintptr_t)p.c) % 16 == 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int e = tid + i * NT;
+        const int row = m0 + r0 + e / (BN / 4), col = n0 + (e % (BN / 4)) * 4;
+        if (row >= p.m) continue;
+        const float4 *x = v[i];
+        const float t[4] = {(x[0].x + x[1].x) + (x[2].x + x[3].x), (x[0].y + x[1].y) + (x[2].y + x[3].y),
+                            (x[0].z + x[1].z) + (x[2].z + x[3].z), (x[0].w + x[1].w) + (x[2].w + x[3].w)};
+        float y[4];
+#pragma unroll
+        for (int d = 0; d < 4; ++d) y[d] = col + d < p.n ? finish(p, t[d], row, col + d) : 0.0f;
+        float* out = p.c + (size_t)row * p.ldc + col;
+        if (whole && col + 4 <= p.n) {
+            *reinterpret_cast<float4*>(out) = make_float4(y[0], y[1], y[2], y[3]);
+        } else {
+            for (int d = 0; d < 4; ++d)
+                if (col + d < p.n) out[d] = y[d];
         }
     }
+    __syncwarp();
+    cluster_sync_all();                                       // nobody leaves while its tile is read
+}
+
+template <int BM, int BN, int TM, int TN>
+int launch_tile(const Args& p, bool vec, cudaStream_t stream) {
+    using Cfg = TileCfg<BM, BN, TM, TN>;
+    auto kernel = vec ? gemm_f32_tile_kernel<BM, BN, TM, TN, true> : gemm_f32_tile_kernel<BM, BN, TM, TN, false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
+    if (e != cudaSuccess) return (int)e;
+    dim3 grid(4 * ((p.n + BN - 1) / BN), (p.m + BM - 1) / BM);
+    if (grid.y > 65535) return PRB_E_SIZE;
+    e = prb_launch_dependent(kernel, grid, dim3(Cfg::THREADS), Cfg::SMEM, stream, p);
+    return e == cudaSuccess ? 0 : (int)e;
+}
+
+template <int MB>
+int launch_stream(const Args& p, StreamGeo g, int copy, size_t smem, cudaStream_t stream) {
+    CUtensorMap map = {};
+    if (copy == COPY_TMA) {
+        const int rc = chunk_map(p.w, p.n, p.k, p.ldw, g.rows, &map);
+        if (rc) return rc;
+    }
+    auto kernel = copy == COPY_TMA  ? gemm_f32_stream_kernel<MB, COPY_TMA>
+                  : copy == COPY_16 ? gemm_f32_stream_kernel<MB, COPY_16>
+                                    : gemm_f32_stream_kernel<MB, COPY_4>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    dim3 grid((p.n + g.rows_per_cta - 1) / g.rows_per_cta, (p.m + MB - 1) / MB);
+    e = prb_launch_dependent(kernel, grid, dim3(STREAM_THREADS), smem, stream, p, g, map);
+    return e == cudaSuccess ? 0 : (int)e;
+}
+
+// The stream kernel's geometry for `mb` rows of A a CTA; false if it does not fit.
+bool stream_geometry(const Args& p, int mb, int copy, StreamGeo* g, size_t* smem) {
+    const size_t budget = 220 * 1024;
+    const int sms = prb_sm_count();
+    const int mt = mb < 4 ? mb : 4;
+    g->nc = (p.k + CH - 1) / CH;
+    g->items = g->nc * (mb / mt);
+    g->slots = g->items <= STREAM_THREADS ? STREAM_THREADS / g->items : 1;
+    const int groups = (p.m + mb - 1) / mb;
+    const int ctas = sms / groups > 0 ? sms / groups : 1;     // one to an SM
+    g->rows_per_cta = (p.n + ctas - 1) / ctas;
+    const size_t row = (size_t)g->nc * CHP * 4, w_row = (size_t)g->nc * (copy == COPY_TMA ? CH : CHP) * 4;
+    auto stage_bytes = [&](int rows) { return (rows * w_row + 1023) / 1024 * 1024; };
+    auto bytes = [&](int rows, int stages) {
+        return 1024 + (size_t)mb * row + stages * stage_bytes(rows) + 2ull * rows * mb * (g->nc + 1) * 4;
+    };
+    // about ten weight rows a stage (a stage costs two block barriers), at least two stages
+    // unless one holds all the CTA has; slots that have no row in a round stand idle
+    int best = 0;
+    for (int rows = 1; rows <= 12 && rows <= g->rows_per_cta; ++rows) {
+        const bool whole = rows >= g->rows_per_cta;
+        if (bytes(rows, whole ? 1 : 2) > budget) break;
+        if (rows % g->slots == 0 || best == 0 || whole || rows < g->slots) best = rows;
+    }
+    if (best == 0) return false;
+    const int wanted = (g->rows_per_cta + best - 1) / best;
+    best = (g->rows_per_cta + wanted - 1) / wanted;           // (stages of equal size)
+    g->rows = best;
+    g->stage_len = (int)(stage_bytes(best) / 4);
+    g->stages = 1;
+    while (g->stages < wanted && g->stages < STREAM_STAGES_MAX && bytes(best, g->stages + 1) <= budget)
+        ++g->stages;
+    *smem = bytes(best, g->stages);
+    return true;
 }
 }  // namespace
 
+// which: 0 the rule below; 1 the stream kernel where it fits, 2 / 3 tiles of 64 x 128, 64 x 64 (the
+// same bits from all of them).  w is read before the kernel ahead in the stream has ended: it must
+// be a tensor that no kernel of the step writes.
 PRB_API int prb_gemm_f32(float* c, const float* a, const float* w, const float* bias,
                          const float* resid, int m, int n, int k, long lda, long ldw, long ldc,
-                         int act, cudaStream_t stream) {
+                         int act, int which, int* status, cudaStream_t stream) {
     if (m <= 0 || n <= 0) return 0;
     if (k <= 0) return PRB_E_SIZE;
-    dim3 grid((n + BN - 1) / BN, (m + BM - 1) / BM);
-    if (grid.y > 65535) return PRB_E_SIZE;
-    gemm_f32_kernel<<<grid, 256, 0, stream>>>(c, a, w, bias, resid, m, n, k, lda, ldw, ldc, act);
-    PRB_LAUNCH_CHECK();
-    return 0;
+    const Args p{c, a, w, bias, resid, m, n, k, lda, ldw, ldc, act, status};
+    // 16-byte copies where every row starts on 16 bytes and K ends on them, else single floats
+    const bool vec = k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)a) % 16 == 0 &&
+                     ((uintptr_t)w) % 16 == 0;
+    // Up to 16 rows the stream kernel: 50,257 x 768 135 us against 146 as tiles, 768 x 768 5.5
+    // against 10.6; at 32 rows 263 against 147 and 17.5 against 15.6 (2,304 x 768).
+    if (which == 1 || (which == 0 && m <= 16)) {
+        StreamGeo g;
+        size_t smem;
+        int mb = m == 1 ? 1 : m == 2 ? 2 : m <= 4 ? 4 : 8;
+        const int copy = !vec ? COPY_4 : k % CH == 0 && k / CH <= 256 ? COPY_TMA : COPY_16;
+        while (mb > 1 && !stream_geometry(p, mb, copy, &g, &smem)) mb /= 2;
+        if (stream_geometry(p, mb, copy, &g, &smem) && (m + mb - 1) / mb <= 65535) {
+            switch (mb) {
+                case 1: return launch_stream<1>(p, g, copy, smem, stream);
+                case 2: return launch_stream<2>(p, g, copy, smem, stream);
+                case 4: return launch_stream<4>(p, g, copy, smem, stream);
+                default: return launch_stream<8>(p, g, copy, smem, stream);
+            }
+        }
+    }
+    if (which == 2) return launch_tile<64, 128, 8, 8>(p, vec, stream);
+    if (which == 3) return launch_tile<64, 64, 8, 4>(p, vec, stream);
+    // 64 x 128 where that leaves no SM without a CTA twice over (1.49 against 1.56 ms at 650 x 50,257
+    // x 768, 111 and 111 us at 1,000 x 2,304 x 768), else 64 x 64 (650 x 768 x 768: 28 us, tiles of
+    // 128 x 64 54 us).
+    const long big = (long)((m + 63) / 64) * ((n + 127) / 128) * 4;
+    if (big >= 2 * prb_sm_count()) return launch_tile<64, 128, 8, 8>(p, vec, stream);
+    return launch_tile<64, 64, 8, 4>(p, vec, stream);
 }

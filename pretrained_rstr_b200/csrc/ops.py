@@ -84,7 +84,7 @@ def _declare(h: ctypes.CDLL) -> None:
     h.prb_host_device_address.restype = c_void_p
     h.prb_fetch_step.argtypes = [P, P, I, I, I, P, I, P, P]
     h.prb_publish_result.argtypes = [P, P, I, P]
-    h.prb_gemm_f32.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, P]
+    h.prb_gemm_f32.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, I, P, P]
     h.prb_gemm_bf16.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, I, I, P, P]
     h.prb_gemm_bf16_scatter.argtypes = [P, P, P, P, I, I, I, L, L, L, I, I, P, P, P, I, I, I, I, I,
                                         I, P, P]
@@ -96,6 +96,9 @@ def _declare(h: ctypes.CDLL) -> None:
     h.prb_gemm_smallm_max_norm_width.argtypes = []
     h.prb_attention_generic.argtypes = [P, L, P, L, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I,
                                         I, P, P]
+    h.prb_attention_f32.argtypes = [P, L, P, L, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F,
+                                    I, P, P]
+    h.prb_attention_f32_supports.argtypes = [I, I, I]
     h.prb_attention_decode.argtypes = [P, L, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, I,
                                        P, P, I, I, P, P]
     h.prb_attention_decode_ring.argtypes = [P, L, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F,
@@ -284,7 +287,8 @@ def _declare(h: ctypes.CDLL) -> None:
     for name in ("prb_resolve_tokens", "prb_fetch_step", "prb_publish_result", "prb_embed", "prb_layernorm", "prb_bias_act", "prb_kv_append", "prb_copy_pages",
                  "prb_gemm_f32", "prb_gemm_bf16", "prb_gemm_bf16_scatter", "prb_gemm_midm",
                  "prb_gemm_midm_supports", "prb_gemm_smallm", "prb_gemm_smallm_max_rows",
-                 "prb_gemm_smallm_max_norm_width", "prb_attention_generic", "prb_attention_decode",
+                 "prb_gemm_smallm_max_norm_width", "prb_attention_generic", "prb_attention_f32",
+                 "prb_attention_f32_supports", "prb_attention_decode",
                  "prb_attention_prefill", "prb_attention_prefill_supports",
                  "prb_attention_prefill_tile", "prb_attention_prefill_tc",
                  "prb_attention_prefill_tc_supports", "prb_attention_prefill_tc_tile",
@@ -454,8 +458,11 @@ def copy_pages(storage, pairs, n_pairs, status) -> None:
                                 _p(status), _stream()), what)
 
 
-def gemm_f32(out, a, w, bias=None, resid=None, act=None) -> None:
-    """out[M,N] = act(a[M,K] . w[N,K]^T + bias) (+ resid): true 32-bit FMA."""
+def gemm_f32(out, a, w, bias=None, resid=None, act=None, kernel: int = 0, status=None) -> None:
+    """out[M,N] = act(a[M,K] . w[N,K]^T + bias) (+ resid): true 32-bit FMA, one order of
+    summation for every M.  ``w`` may be read before the kernel ahead has ended (weights, which
+    no kernel of a step writes).  ``kernel`` forces one of the kernels (1 rows of weights as a
+    stream, 2 / 3 tiles of 64 x 128, 64 x 64); left at 0 the sizes choose.  All give the same bits."""
     what = "gemm_f32"
     for name, t in (("out", out), ("a", a), ("w", w)):
         if not t.is_cuda or t.dtype != torch.float32 or t.stride(1) != 1:
@@ -471,7 +478,8 @@ def gemm_f32(out, a, w, bias=None, resid=None, act=None) -> None:
         if resid.shape != out.shape or resid.stride(0) != out.stride(0):
             raise KernelArgumentError(f"{what}: resid must have the output's shape and stride")
     _check(lib().prb_gemm_f32(_p(out), _p(a), _p(w), _p(bias), _p(resid), m, n, k, a.stride(0),
-                              w.stride(0), out.stride(0), ACT_CODES[act], _stream()), what)
+                              w.stride(0), out.stride(0), ACT_CODES[act], int(kernel), _p(status),
+                              _stream()), what)
 
 
 def gemm_bf16(out, a, w, bias=None, resid=None, act=None, tile_n: int = 0, status=None,
@@ -635,6 +643,34 @@ def attention_generic(out, q, k_pages, v_pages, block_table, seq_of_token, posit
         _p(seq_of_token), _p(positions), n_tokens, n_heads, kv_heads, head_dim, page_size,
         block_table.shape[1], num_pages, max_context, float(scale), int(window or 0),
         dtype_code(k_pages.dtype), _p(status), _stream()), what)
+
+
+def attention_f32_supports(head_dim: int, max_context: int, window) -> bool:
+    return bool(lib().prb_attention_f32_supports(int(head_dim), int(max_context), int(window or 0)))
+
+
+def attention_f32(out, q, k_pages, v_pages, block_table, seq_of_token, positions, count, n_list,
+                  n_heads, scale, window, max_context, status, tiles=None, token_list=None) -> None:
+    """True 32-bit attention of the tokens in ``tiles`` = (first token, tokens) of up to 128
+    consecutive tokens of a request each, or of the single ones in ``token_list``; ``count`` (on
+    the device) says how many of the ``n_list`` there are.  A query's result does not depend on
+    the list it came in, nor on what else is in the step."""
+    what = "attention_f32"
+    num_pages, kv_heads, page_size, head_dim = k_pages.shape
+    for name, t in (("out", out), ("q", q)):
+        if t.dtype != torch.float32 or t.stride(1) != 1 or t.shape[1] != n_heads * head_dim:
+            raise KernelArgumentError(f"{what}: {name} has the wrong type, width or inner stride")
+    for name, t in (("k_pages", k_pages), ("v_pages", v_pages)):
+        if t.dtype != torch.float32 or not t.is_contiguous():
+            raise KernelArgumentError(f"{what}: {name} must be contiguous float32")
+    for name, t in (("block_table", block_table), ("seq_of_token", seq_of_token), ("positions", positions)):
+        _need(t, torch.int32, name, what)
+    row0, rows = tiles if tiles is not None else (None, None)
+    _check(lib().prb_attention_f32(
+        _p(out), out.stride(0), _p(q), q.stride(0), _p(k_pages), _p(v_pages), _p(block_table),
+        _p(seq_of_token), _p(positions), _p(row0), _p(rows), _p(token_list), _p(count), n_list,
+        n_heads, kv_heads, head_dim, page_size, block_table.shape[1], num_pages, max_context,
+        float(scale), int(window or 0), _p(status), _stream()), what)
 
 
 _SM_COUNT = None

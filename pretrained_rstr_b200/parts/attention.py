@@ -251,7 +251,8 @@ def attend(ctx, out, q, cache: LayerCache, group, n_head: int, scale: float,
     """Attention of the step's tokens over their requests' cached keys and values.  Returns
     which kernel ran last: "ring", "split" (the split-key decode kernel) or None.
 
-    float32 runtime: the 32-bit kernel for every token.  bfloat16 runtime: prompt
+    float32 runtime: the 32-bit kernels, prompt portions in tiles of queries and single tokens by
+    themselves.  bfloat16 runtime: prompt
     portions go in tiles of up to 128 queries to a tensor-core kernel (tcgen05 for head
     size 64 and pages of a multiple of 64, else mma.sync), single tokens (decoded
     tokens, portions of a few tokens) to the split-key decode kernel; head sizes or page
@@ -261,6 +262,20 @@ def attend(ctx, out, q, cache: LayerCache, group, n_head: int, scale: float,
     fast = ctx.dtype == torch.bfloat16 and head_dim % 8 == 0 and head_dim <= 256 and \
         group.page_size >= 8 and ops.decode_split() % group.page_size == 0 and \
         ops.prefill_supports(head_dim)
+    # (decided by the model's positions, not the step's: the two 32-bit kernels add in other orders)
+    exact = ctx.dtype == torch.float32 and ops.attention_f32_supports(head_dim, ctx.max_positions, window) \
+        and cache.k.is_contiguous() and cache.v.is_contiguous()
+    if exact:
+        work = ctx.work[AttentionWork.key]
+        for name, n_max, lists in (
+                ("tiles", work.caps["tile_req"], dict(tiles=(work.arrays["tile_row0"], work.arrays["tile_rows"]))),
+                ("singles", work.caps["single_tokens"], dict(token_list=work.arrays["single_tokens"]))):
+            n = work.host_counts[name]
+            if n is None or n > 0:
+                ops.attention_f32(out, q, cache.k, cache.v, group.block_table, ctx.seq_of_token,
+                                  ctx.positions, work.counts[name], n_max if n is None else n, n_head,
+                                  scale, window, ctx.max_context, ctx.status, **lists)
+        return
     if not fast:
         ops.attention_generic(out, q, cache.k, cache.v, group.block_table, ctx.seq_of_token,
                               ctx.positions, t, n_head, scale, window, ctx.max_context, ctx.status)

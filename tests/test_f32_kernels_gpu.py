@@ -1,0 +1,96 @@
+"""The kernels of the float32 path: one order of sums whichever kernel runs, at the sizes where
+tiles, chunks and stages end."""
+import pytest
+import torch
+
+from test_kernels_gpu import _ops, _paged_case, _ref_attention
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 8, 9, 16, 17, 64, 65, 129])
+@pytest.mark.parametrize("n,k", [(1, 1), (70, 20), (130, 33), (768, 768), (257, 3072), (300, 6400),
+                                 (2304, 100), (5000, 96)])
+def test_gemm_f32_kernels_give_the_same_bits(m, n, k):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(m * 7 + n + k)
+    wide = torch.randn(m, k + 3, device="cuda", generator=g)          # rows that start off 16 bytes
+    a = wide[:, :k].contiguous()
+    w = torch.randn(n, k, device="cuda", generator=g)
+    bias = torch.randn(n, device="cuda", generator=g)
+    resid = torch.randn(m, n, device="cuda", generator=g)
+    torch.cuda.synchronize()
+    out = [torch.full((m, n), float("nan"), device="cuda") for _ in range(4)]
+    for which in range(4):
+        ops.gemm_f32(out[which], a, w, bias=bias, resid=resid, kernel=which)
+    strided = torch.full((m, n), float("nan"), device="cuda")
+    ops.gemm_f32(strided, wide[:, :k], w, bias=bias, resid=resid)
+    exact = a.double() @ w.double().t() + bias.double() + resid.double()
+    # a sum of k products in chains of at most 32 and runs of k / 128 + 2: each addition rounds
+    # by 2^-24 of the partial sum, which is at most the sum of the magnitudes
+    size = a.abs().double() @ w.abs().double().t() + bias.abs().double() + resid.abs().double()
+    assert bool(((out[0].double() - exact).abs() <= size * 2.0 ** -24 * (40 + k // 128)).all())
+    for other in out[1:] + [strided]:
+        assert torch.equal(out[0], other)
+
+
+CASES = [
+    # heads, kv heads, head size, page size, window
+    (12, 12, 64, 64, None), (4, 4, 16, 16, None), (6, 2, 64, 64, 70), (5, 1, 48, 32, 300),
+    (2, 2, 128, 128, None), (8, 4, 80, 64, 100), (3, 1, 4, 1, None), (2, 1, 100, 24, 256),
+]
+
+
+@pytest.mark.parametrize("nh,nkv,dh,ps,window", CASES)
+def test_attention_f32(nh, nkv, dh, ps, window):
+    """Tiles and single tokens against the plain reference, the same bits from both for the same
+    query; what lies behind a request's last token is poisoned."""
+    ops = _ops()
+    lengths, portions = [1, 63, 64, 65, 257, 300, 1000, 129], [1, 5, 64, 1, 17, 1, 33, 129]
+    q, k, v, table, seq, pos = _paged_case(3, nh, nkv, dh, ps, lengths, portions, torch.float32)
+    for b, n in enumerate(lengths):
+        if n % ps:
+            page = int(table[b, n // ps])
+            k[page, :, n % ps:] = float("nan")
+            v[page, :, n % ps:] = float("nan")
+    t = q.shape[0]
+    tiles, at = [], 0
+    for p in portions:
+        tiles += [(at + r, min(128, p - r)) for r in range(0, p, 128)]
+        at += p
+    ints = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")  # noqa: E731
+    row0, rows = ints([a for a, _ in tiles] + [0]), ints([b for _, b in tiles] + [0])
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    by_tile, single = torch.full_like(q, float("nan")), torch.full_like(q, float("nan"))
+    for out, n, count, lists in ((by_tile, len(tiles) + 1, ints([len(tiles)]), dict(tiles=(row0, rows))),
+                                 (single, t, ints([t]), dict(token_list=torch.arange(t, dtype=torch.int32,
+                                                                                     device="cuda")))):
+        # (bounds on the context of one and of two to eight groups of keys: another split, same bits)
+        ops.attention_f32(out, q, k, v, table, seq, pos, count, n, nh, 0.3, window, 1024, status, **lists)
+        again = torch.full_like(q, float("nan"))
+        ops.attention_f32(again, q, k, v, table, seq, pos, count, n, nh, 0.3, window, 4000, status, **lists)
+        assert torch.equal(out, again)
+    assert status.tolist() == [0, 0, 0, 0]
+    assert torch.equal(by_tile, single)
+    ref = _ref_attention(q, k, v, table, seq, pos, nh, 0.3, window)
+    assert float((by_tile - ref).abs().max()) <= 2e-5
+
+
+def test_attention_f32_records_what_is_out_of_range():
+    ops = _ops()
+    q, k, v, table, seq, pos = _paged_case(4, 2, 2, 64, 64, [100, 200], [1, 20], torch.float32)
+    table[0, 1] = -1                                       # request 0's second page is missing
+    pos[5] = 5000                                          # beyond the block table
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    one = torch.tensor([1], dtype=torch.int32, device="cuda")
+    out = torch.full_like(q, float("nan"))
+    ops.attention_f32(out, q, k, v, table, seq, pos, one, 1, 2, 0.1, None, 256, status,
+                      token_list=torch.zeros(1, dtype=torch.int32, device="cuda"))
+    assert status.tolist()[0] == 4 and bool(torch.isfinite(out[0]).all())
+    status.zero_()
+    ops.attention_f32(out, q, k, v, table, seq, pos, one, 1, 2, 0.1, None, 256, status,
+                      tiles=(one, one * 20))
+    assert status.tolist()[:3] == [2, 5, 5000] and float(out[5].abs().max()) == 0.0
+    assert bool(torch.isfinite(out[1:21]).all())
+    assert not ops.attention_f32_supports(130, 1024, None) and not ops.attention_f32_supports(62, 1024, None)
+    assert ops.attention_f32_supports(64, 1024, None)
