@@ -327,10 +327,11 @@ def attend(ctx, out, q, cache: LayerCache, group, n_head: int, scale: float,
         ring = SETTINGS.decode_ring
         if ring is None:
             ring = ops.decode_ring_prefers(n_list, n_head, ctx.max_context)
-        if ring and cap <= ops.decode_ring_max_list() and \
-                ops.decode_ring_supports(head_dim, group.page_size):
-            ws = ctx.scratch("attn_ring_ws", (ops.decode_ring_workspace(cap, n_head, head_dim),),
-                             torch.float32)
+        # (a launch takes up to 256 tokens; how many requests the engine is made for does not matter)
+        most = ops.decode_ring_max_list()
+        if ring and n_list <= most and ops.decode_ring_supports(head_dim, group.page_size):
+            ws = ctx.scratch("attn_ring_ws",
+                             (ops.decode_ring_workspace(min(cap, most), n_head, head_dim),), torch.float32)
             counters = ctx.scratch_zero("attn_decode_counters", (cap * n_head,), torch.int32)
             ops.attention_decode_ring(out, q, cache.k, cache.v, group.block_table,
                                       ctx.seq_of_token, ctx.positions, work.arrays["single_tokens"],
