@@ -377,6 +377,7 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
         if (need_pages) unit_pages(a, sh, mine);
         if (lane < stages && mine.idx >= 0 && mine.late) issue_unit(a, map_k, map_v, mine, ring0, bar0, lane);
     }
+    unsigned mine_bad = __ballot_sync(0xffffffffu, mine.bad);
     LaneUnit ahead = mine;                           // the 32 units after them, once decoded
     bool ahead_ready = false;
     int batch0 = u_begin;                            // first unit of `mine`
@@ -393,7 +394,10 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
     uint32_t qa[4][2];                               // the query as A fragments, per 16 dimensions
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) qa[ks][0] = qa[ks][1] = 0u;
-    int cur_idx = -1, cur_h = -1, cur_t = 0, cur_n_blk = 0;
+    int cur_idx = -1, cur_h = -1, cur_t = 0, cur_n_blk = 0, cur_pos = 0, cur_lo = 0, cur_blk = 0;
+    int pair_end = u_begin;                          // first unit after the current (token, head)
+    int slot = 0;
+    uint32_t parity = 0;
     int pairs_done = 0;                              // (token, head)s this warp has left behind
     bool alive = true;
 
@@ -431,37 +435,39 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
     for (int u = u_begin; u < u_end && alive; ++u) {
         if (u - batch0 >= 32) {                      // on to the next 32 units (decoded when the
             mine = ahead;                            // first of them was requested)
+            mine_bad = __ballot_sync(0xffffffffu, mine.bad);
             batch0 += 32;
             ahead_ready = false;
         }
         const int rel = u - batch0;                  // which lane decoded this unit
-        const int slot = (u - u_begin) % stages;
-        const uint32_t parity = (uint32_t)((u - u_begin) / stages) & 1u;
-        const int idx = __shfl_sync(0xffffffffu, mine.idx, rel);
-        const int h = __shfl_sync(0xffffffffu, mine.h, rel);
-        const int blk = __shfl_sync(0xffffffffu, mine.blk, rel);
-        const int pos = __shfl_sync(0xffffffffu, mine.pos, rel);
-        const int lo = __shfl_sync(0xffffffffu, mine.lo, rel);
-        const int t = __shfl_sync(0xffffffffu, mine.t, rel);
-        const int bad = __shfl_sync(0xffffffffu, mine.bad ? 1 : 0, rel);
-        if (idx != cur_idx || h != cur_h) {
+        const bool bad = (mine_bad >> rel) & 1u;
+        if (u >= pair_end) {                         // the first unit of the run or of a (token, head)
             if (cur_idx >= 0) finish_pair();
-            cur_idx = idx; cur_h = h; cur_t = t;
-            TokenSpan s{t, sh.span_b[idx], pos, 0, 0, 0};
+            cur_idx = __shfl_sync(0xffffffffu, mine.idx, rel);
+            cur_h = __shfl_sync(0xffffffffu, mine.h, rel);
+            cur_blk = __shfl_sync(0xffffffffu, mine.blk, rel);
+            cur_pos = __shfl_sync(0xffffffffu, mine.pos, rel);
+            cur_lo = __shfl_sync(0xffffffffu, mine.lo, rel);
+            cur_t = __shfl_sync(0xffffffffu, mine.t, rel);
+            TokenSpan s{cur_t, sh.span_b[cur_idx], cur_pos, 0, 0, 0};
             span_blocks(a, s);
             cur_n_blk = s.n_blk;
+            pair_end = sh.cum[cur_idx] + (cur_h + 1) * cur_n_blk;
             m = -INFINITY; l = 0.0f;
 #pragma unroll
             for (int j = 0; j < 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.0f;
             // this pair's query as A fragments: row 0 only, so only lanes 0..3 hold any of it
             const uint32_t* qp = reinterpret_cast<const uint32_t*>(
-                a.q + (size_t)t * a.q_stride + (size_t)h * DH);
+                a.q + (size_t)cur_t * a.q_stride + (size_t)cur_h * DH);
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks) {
                 qa[ks][0] = row0 ? qp[8 * ks + qd] : 0u;          // dimensions 16 ks + 2 c, + 1
                 qa[ks][1] = row0 ? qp[8 * ks + 4 + qd] : 0u;      // dimensions 16 ks + 8 + 2 c, + 1
             }
         }
+        const int idx = cur_idx, h = cur_h, t = cur_t, pos = cur_pos, lo = cur_lo, blk = cur_blk++;
+        // most units lie wholly inside what the query sees: nothing to mask there
+        const bool whole = !bad && blk * UNIT >= lo && blk * UNIT + UNIT - 1 <= pos;
         if (!mbar_wait_bounded(bar0 + 8 * slot, parity)) {
             if (lane == 0) prb_set_status(a.status, PRB_S_WAIT_TIMEOUT, 32, cta, u);
             alive = false;
@@ -469,7 +475,9 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
         }
         if (u == u_begin) RING_TRACE(4);
         const uint32_t kd = ring0 + slot * 2 * TILE, vd = kd + TILE;
+        bool wrote = false;                          // rows of the unit's tiles written from here
         if (a.k_new != nullptr && !bad && (blk + 1) * UNIT > pos - a.new_keys + 1) {
+            wrote = true;
             // rows of this unit that the step itself appended: lanes 8 j .. 8 j + 7 bring the
             // row of position pos - j, if token t - j is that position of the same request
             const int j = lane >> 3, c = lane & 7;
@@ -489,7 +497,8 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
         }
         // a masked key's values must be finite: what an earlier owner of the page left there is
         // zeroed (lane j looks after row j) before it is multiplied by a zero weight
-        {
+        if (!whole) {
+            wrote = true;
             const int key = blk * UNIT + lane;
             if (bad || key < lo || key > pos) {
 #pragma unroll
@@ -516,21 +525,31 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
                 }
             }
         }
-        // ---- softmax over the unit's keys (row 0: lanes 0..3), running maximum and sum
+        // ---- softmax over the unit's keys (row 0: lanes 0..3), running maximum and sum.  (The
+        // other lanes hold rows without a query; what they compute reaches nobody.)  A score that
+        // is not a number counts as one that is not seen.
         float um = -INFINITY;
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int key = blk * UNIT + 8 * nt + 2 * qd + e;
-                const bool seen = row0 && !bad && key >= lo && key <= pos;
-                sc[nt][e] = seen ? sc[nt][e] * a.scale : -INFINITY;
-                um = fmaxf(um, sc[nt][e]);
-            }
+            for (int e = 0; e < 2; ++e) sc[nt][e] = fmaxf(sc[nt][e] * a.scale, -INFINITY);
+        if (!whole) {
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int key = blk * UNIT + 8 * nt + 2 * qd + e;
+                    if (bad || key < lo || key > pos) sc[nt][e] = -INFINITY;
+                }
+        }
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) um = fmaxf(um, fmaxf(sc[nt][0], sc[nt][1]));
         um = fmaxf(um, __shfl_xor_sync(0xffffffffu, um, 1));
         um = fmaxf(um, __shfl_xor_sync(0xffffffffu, um, 2));
         const float m_new = fmaxf(m, um);
-        float corr = 1.0f, ps = 0.0f;
+        const float base = m_new == -INFINITY ? 0.0f : m_new;        // (nothing seen yet: weights of zero)
+        const float corr = __expf(m - base);
+        float ps = 0.0f;
         uint32_t pa[2][2];                           // the weights as A fragments, per 16 keys
         {
             float pv[4][2];
@@ -538,10 +557,9 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
             for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    pv[nt][e] = (m_new > -INFINITY && sc[nt][e] > -INFINITY) ? __expf(sc[nt][e] - m_new) : 0.0f;
+                    pv[nt][e] = __expf(sc[nt][e] - base);
                     ps += pv[nt][e];
                 }
-            if (m_new > -INFINITY) corr = (m == -INFINITY) ? 0.0f : __expf(m - m_new);
             pa[0][0] = pack_bf16(pv[0][0], pv[0][1]);
             pa[0][1] = pack_bf16(pv[1][0], pv[1][1]);
             pa[1][0] = pack_bf16(pv[2][0], pv[2][1]);
@@ -551,11 +569,13 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
         ps += __shfl_xor_sync(0xffffffffu, ps, 2);
         l = l * corr + ps;
         m = m_new;
-        __syncwarp();                                 // the zeroed value rows are in place
+        if (!whole) __syncwarp();                     // the zeroed value rows are in place
         // ---- O = O * corr + P . V: dimension tiles of 8, 16 keys a step (B fragments by
         // transposing loads from the rows of the value tile)
+        if (__any_sync(0xffffffffu, corr != 1.0f)) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { o[j][0] *= corr; o[j][1] *= corr; }
+            for (int j = 0; j < 8; ++j) { o[j][0] *= corr; o[j][1] *= corr; }
+        }
         {
             const int rr = lane & 7, mi = lane >> 3;
 #pragma unroll
@@ -576,8 +596,8 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
         // ---- the buffer is free: the unit `stages` ahead takes it
         const int nu = u + stages;
         if (nu < u_end) {
-            // (generic-proxy accesses to the buffer come before the copy engine's writes)
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            // (generic-proxy writes to the buffer come before the copy engine's)
+            if (wrote) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             if (nu - batch0 < 32) {
                 if (lane == nu - batch0) issue_unit(a, map_k, map_v, mine, ring0, bar0, slot);
             } else {
@@ -589,6 +609,7 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
                 if (lane == nu - batch0 - 32) issue_unit(a, map_k, map_v, ahead, ring0, bar0, slot);
             }
         }
+        if (++slot == stages) { slot = 0; parity ^= 1u; }
     }
     if (alive && cur_idx >= 0) finish_pair();
     if (!alive) {
