@@ -7,14 +7,17 @@
 // all of K (N = 768: 12 tiles of 64 columns), and what bounds a tile is the bytes its SM
 // takes in.  Here a cluster of S CTAs shares one tile of NB output columns: CTA r multiplies
 // the r-th part of K (A and W slices come by TMA through a ring of shared-memory stages,
-// 128-byte swizzle, mma.sync m16n8k16 with ldmatrix), keeps its partial tile in shared
-// memory, and after a cluster barrier every CTA sums, in rank order, the rows r, r + S, ...
-// of all partial tiles through distributed shared memory and runs the epilogue for them
-// (bias, activation, residual, store).  S depends on K and N only, and a row's sum is
+// 128-byte swizzle, mma.sync m16n8k16 with ldmatrix) and writes row i of its partial tile to
+// the shared memory of CTA i mod S, which after one cluster barrier sums its rows' parts in rank
+// order and runs the epilogue for them (bias, activation, residual, store).  (The parts used to
+// be read by their owner after the barrier, a remote round trip and a second barrier more:
+// 768 x 3,072 at 64 rows 8.4 -> 7.2 us in a step without dependent launch.)  S depends on K and N only, and a row's sum is
 // taken in a fixed order, so a row's result does not depend on the batch.
 // No TMA load uses cluster multicast.  Every mbarrier wait is bounded: on a timeout the
 // kernel records PRB_S_WAIT_TIMEOUT, stores nothing, waits (bounded) for its copies in
 // flight and leaves through the same cluster barriers as its peers.
+#include <mutex>
+
 #include "common.cuh"
 #include "tensor_map.cuh"
 
@@ -42,6 +45,7 @@ constexpr int WARPS = 8;
 constexpr int MROWS = 64;           // token rows of a tile (rows beyond M are zero)
 constexpr int KC = 2;               // 64-column slabs per stage
 constexpr int STAGES = 4;
+constexpr int PART_ROWS = 72;       // S * ceil(64 / S) for S up to 8, at most
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -98,16 +102,22 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void cluster_sync_all() {
+__device__ __forceinline__ void cluster_arrive() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ float ld_cluster_f32(uint32_t local_addr, int rank) {
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t local_addr, int rank) {
     uint32_t raddr;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(raddr) : "r"(local_addr), "r"(rank));
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(raddr) : "memory");
-    return v;
+    return raddr;
+}
+__device__ __forceinline__ void st_cluster_f32x2(uint32_t addr, float x, float y) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(x), "f"(y) : "memory");
+}
+__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
 struct Args {
@@ -134,14 +144,16 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
     constexpr int NT = NB / 16;                       // 8-column MMA tiles per warp: 2 or 4
     constexpr uint32_t A_BYTES = KC * MROWS * 128, W_BYTES = KC * NB * 128;
     constexpr uint32_t STAGE_BYTES = A_BYTES + W_BYTES;
-    constexpr int PP = NB + 1;                        // pitch of the partial tile (floats)
+    constexpr int PP = NB + 8;                        // pitch of a row's part (floats): rows a warp
+                                                      // writes together start 8 banks apart
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t ring = smem_u32(smem);
-    float* part = reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES);       // [64][PP]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(part + MROWS * PP + 1);
-    bars = reinterpret_cast<uint64_t*>(((uintptr_t)bars + 7) & ~(uintptr_t)7);
-    volatile int* failed = reinterpret_cast<volatile int*>(bars + 2 * STAGES);
+    // parts of this CTA's rows, [rank of the sender][row / S][PP]; 64 / S rows, rounded up
+    float* part = reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(part + PART_ROWS * PP);
+    volatile uint32_t* missing = reinterpret_cast<volatile uint32_t*>(bars + 2 * STAGES);   // [8]
+    volatile int* failed = reinterpret_cast<volatile int*>(bars + 2 * STAGES + 4);
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -154,6 +166,7 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
 
     MT_TRACE(0);
     prb_grid_launch_dependents();
+    cluster_arrive();                                 // (the peers exist: waited for before the first store to them)
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(full0 + 8 * s, 1);
@@ -229,17 +242,35 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
         }
     }
     MT_TRACE(3);
-    // ---- this CTA's partial tile -> shared memory
+    // ---- the rows of this CTA's partial tile to the CTAs that finish them
+    const int per = (MROWS + S - 1) / S;                  // rows of a CTA
+    cluster_wait();
     {
         const int g = lane >> 2, q = lane & 3;
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            const int col = nh * (NB / 2) + nt * 8 + q * 2;
-            float* p0 = part + (size_t)(mt * 16 + g) * PP + col;
-            float* p1 = part + (size_t)(mt * 16 + g + 8) * PP + col;
-            p0[0] = acc[nt][0]; p0[1] = acc[nt][1];
-            p1[0] = acc[nt][2]; p1[1] = acc[nt][3];
+        for (int half = 0; half < 2; ++half) {
+            const int row = mt * 16 + g + 8 * half;
+            if (row < a.m) {
+                const uint32_t dst = cluster_addr(
+                    smem_u32(part + (size_t)(rank * per + row / S) * PP + nh * (NB / 2) + q * 2), row % S);
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+                    st_cluster_f32x2(dst + nt * 32, acc[nt][2 * half], acc[nt][2 * half + 1]);
+            }
         }
+    }
+    // bias and residual of the outputs this thread finishes, asked for before the barrier
+    constexpr int RPP = THREADS / NB;                     // rows per pass
+    constexpr int PASSES = MROWS / RPP;                   // (S = 1; a split has 1 / S of them)
+    constexpr int AHEAD = PASSES < 4 ? PASSES : 4;
+    const int col = threadIdx.x % NB, rsub = threadIdx.x / NB;
+    const int gcol = n0 + col;
+    const float bias = (a.bias && gcol < a.n) ? a.bias[gcol] : 0.0f;
+    float res[AHEAD];
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) {
+        const int row = rank + (rsub + i * RPP) * S;
+        res[i] = (a.resid && gcol < a.n && row < a.m) ? a.resid[(size_t)row * a.ldc + gcol] : 0.0f;
     }
     __syncthreads();
     const bool bad_here = *failed != 0;
@@ -251,74 +282,112 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
             for (uint32_t w = 0; w < WAIT_LIMIT; ++w)
                 if (mbar_try_wait(bar, parity)) break;
         }
-        part[MROWS * PP] = 1.0f;                          // peers see that this part is missing
-    } else if (threadIdx.x == 0) {
-        part[MROWS * PP] = 0.0f;
     }
+    if (threadIdx.x < S)                                  // peers see whether this part is missing
+        st_cluster_u32(cluster_addr(smem_u32((const void*)(missing + rank)), threadIdx.x), bad_here ? 1u : 0u);
+    __syncwarp();
     MT_TRACE(4);
-    cluster_sync_all();                                   // every CTA's partial tile is in place
+    cluster_arrive();
+    cluster_wait();                                       // every part is in place
     MT_TRACE(5);
     // ---- rows rank, rank + S, ...: sum over the cluster in rank order, epilogue, store
     bool any_bad = false;
-    for (int r = 0; r < S; ++r) any_bad |= ld_cluster_f32(smem_u32(part + MROWS * PP), r) != 0.0f;
-    if (!any_bad) {
+    for (int r = 0; r < S; ++r) any_bad |= missing[r] != 0;
+    if (!any_bad && gcol < a.n) {
         O* out = reinterpret_cast<O*>(a.c);
-        constexpr int RPP = THREADS / NB;                 // rows per pass
-        const int col = threadIdx.x % NB, rsub = threadIdx.x / NB;
-        const int gcol = n0 + col;
-        const float bias = (a.bias && gcol < a.n) ? a.bias[gcol] : 0.0f;
-        for (int row = rank + rsub * S; row < a.m && row < MROWS; row += RPP * S) {
-            const uint32_t addr = smem_u32(part + (size_t)row * PP + col);
-            float pv[8];                                  // all requested before any is used
 #pragma unroll
-            for (int r = 0; r < 8; ++r) pv[r] = r < S ? ld_cluster_f32(addr, r) : 0.0f;
+        for (int i = 0; i < PASSES; ++i) {
+            const int local = rsub + i * RPP, row = rank + local * S;
+            if (local >= per || row >= a.m) break;
+            const float* src = part + (size_t)local * PP + col;
+            float pv[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) pv[r] = r < S ? src[(size_t)r * per * PP] : 0.0f;
             float v = 0.0f;
 #pragma unroll
             for (int r = 0; r < 8; ++r) v += pv[r];
-            if (gcol < a.n) {
-                v = prb_activate(v + bias, a.act);
-                if (a.resid) v += a.resid[(size_t)row * a.ldc + gcol];
-                out[(size_t)row * a.ldc + gcol] = prb_from_float<O>(v);
-            }
+            v = prb_activate(v + bias, a.act);
+            if (a.resid) v += i < AHEAD ? res[i < AHEAD ? i : 0] : a.resid[(size_t)row * a.ldc + gcol];
+            out[(size_t)row * a.ldc + gcol] = prb_from_float<O>(v);
         }
     }
     MT_TRACE(6);
-    cluster_sync_all();                                   // the partial tiles have been read
     MT_TRACE(7);
+}
+
+template <int NB> constexpr size_t midm_smem() {
+    return 1024 + (size_t)STAGES * KC * (MROWS + NB) * 128 + (size_t)PART_ROWS * (NB + 8) * 4 +
+           2 * STAGES * 8 + 32 + 16;
+}
+
+template <int NB, typename O> int configure_midm() {
+    static int rc = [] {
+        cudaFuncSetAttribute(gemm_midm_kernel<NB, O>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             cudaSharedmemCarveoutMaxShared);
+        return (int)cudaFuncSetAttribute(gemm_midm_kernel<NB, O>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)midm_smem<NB>());
+    }();
+    return rc;
+}
+
+template <int NB> void midm_launch(const Args& a, cudaStream_t stream, cudaLaunchConfig_t* cfg,
+                                   cudaLaunchAttribute* attr) {
+    cfg->gridDim = dim3((a.n + NB - 1) / NB, 1, a.splits);
+    cfg->blockDim = dim3(THREADS);
+    cfg->dynamicSmemBytes = midm_smem<NB>();
+    cfg->stream = stream;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = (unsigned)a.splits;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = prb_pdl_enabled() ? 1 : 0;
+    cfg->attrs = attr;
+    cfg->numAttrs = 2;
 }
 
 template <int NB, typename O>
 int launch_midm(const Args& a, const CUtensorMap& ma, const CUtensorMap& mw, cudaStream_t stream) {
-    constexpr size_t smem = 1024 + (size_t)STAGES * KC * (MROWS + NB) * 128 +
-                            (size_t)(MROWS * (NB + 1) + 2) * 4 + 16 + 2 * STAGES * 8 + 16;
-    static bool configured = false;
-    if (!configured) {
-        cudaFuncSetAttribute(gemm_midm_kernel<NB, O>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
-        cudaError_t e = cudaFuncSetAttribute(gemm_midm_kernel<NB, O>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    const int rc = configure_midm<NB, O>();
+    if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((a.n + NB - 1) / NB, 1, a.splits);
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = prb_pdl_enabled() ? 1 : 0;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = 1;
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = (unsigned)a.splits;
-    cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    midm_launch<NB>(a, stream, &cfg, attr);
     cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_midm_kernel<NB, O>, a, ma, mw);
-    if (e != cudaSuccess) return (int)e;
-    return 0;
+    return e == cudaSuccess ? 0 : (int)e;
+}
+
+// How many clusters of `splits` CTAs run at a time (asked once per device).
+template <int NB> int active_clusters(int splits) {
+    static int known[64][9] = {};
+    static std::mutex mu;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || configure_midm<NB, float>() != 0) return 1;
+    std::lock_guard<std::mutex> lock(mu);
+    if (known[dev][splits] == 0) {
+        Args a{};
+        a.n = NB;
+        a.splits = splits;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[2];
+        midm_launch<NB>(a, nullptr, &cfg, attr);
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, gemm_midm_kernel<NB, float>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        known[dev][splits] = n > 0 ? n : 1;
+    }
+    return known[dev][splits];
 }
 }  // namespace
+
+// Clusters of `splits` CTAs with tiles of `nb` columns that run at a time.
+PRB_API int prb_gemm_midm_active_clusters(int nb, int splits) {
+    if (splits < 1 || splits > 8) return 0;
+    return nb == 64 ? active_clusters<64>(splits) : active_clusters<32>(splits);
+}
 
 // 1 when the kernel takes these sizes (else the caller uses another product kernel).
 PRB_API int prb_gemm_midm_supports(int m, int n, int k) {
@@ -335,7 +404,7 @@ PRB_API int prb_gemm_midm(void* c, const void* a, const void* w, const float* bi
     if (lda % 8 != 0 || ldw % 8 != 0 || ((uintptr_t)a) % 16 != 0 || ((uintptr_t)w) % 16 != 0)
         return PRB_E_ALIGN;
     if (out_dtype != PRB_F32 && out_dtype != PRB_BF16) return PRB_E_DTYPE;
-    // Tile width and cluster size from N and K only.  All CTAs should run at once (one per
+    // Tile width and cluster size from N and K (and the device) only.  All CTAs should run at once (one per
     // SM with 64-column tiles, two with 32-column tiles); within that, the split that gives
     // an SM the fewest bytes to take in (its CTAs' slices of A and W) wins.
     const int slabs = k / 64;
@@ -349,6 +418,9 @@ PRB_API int prb_gemm_midm(void* c, const void* a, const void* w, const float* bi
         if (s > 8) s = 8;
         if (s > slabs / 2) s = slabs / 2;
         if (s < 1) s = 1;
+        // (clusters are placed inside groups of SMs whose sizes differ: 16 clusters of eight do not
+        // all run at once on 148 SMs, and a second round costs as much as the first)
+        while (s > 1 && tiles > (cand == 64 ? active_clusters<64>(s) : active_clusters<32>(s))) --s;
         const long per_cta = (long)(MROWS + cand) * 2 * ((long)k / s);
         const long ctas = (long)tiles * s;
         const long per_sm = per_cta * ((ctas + sms - 1) / sms);
