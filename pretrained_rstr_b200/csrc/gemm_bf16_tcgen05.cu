@@ -74,17 +74,26 @@ namespace {
 constexpr int BM = 128;
 constexpr int BK = 64;             // 64 bf16 = 128 bytes = one swizzle atom row
 constexpr int UMMA_K = 16;
-constexpr int GEMM_THREADS = 320;     // producer warp, MMA warp, 8 epilogue warps
+// Epilogue warps: 16 for bfloat16 tiles of 128 columns and more (four to a quarter of the tensor
+// memory's lanes; with eight, an activation's arithmetic did not hide behind the next tile: 2,193 x
+// 6,400 x 1,600 with GELU 46.1 -> 40.0 us), eight for narrower ones, which have no chunk for more
+// (137 x 3,072 x 768 in tiles of 64: 6.4 against 7.0 us), and for float32 output, where a thread
+// holds a chunk's residual values beside the next chunk's (sixteen warps leave it no registers for
+// that: 2,048 x 3,072 x 768 14.7 -> 17.4 us).
+template <typename O, int BN> constexpr int epi_warps = sizeof(O) == 4 || BN < 128 ? 8 : 16;
+template <typename O, int BN> constexpr int gemm_threads = 64 + 32 * epi_warps<O, BN>;   // + producer, MMA
+constexpr int SPLIT_THREADS = 320;     // the split-K kernel's: 8 epilogue warps
 
 using namespace tc5;
 
-template <int BN, bool PAIR = false> struct TileCfg {
+template <int BN, bool PAIR = false, int EPI = 8> struct TileCfg {
     static_assert(BN % 32 == 0 && BN >= 32 && BN <= 256, "tile width: a multiple of 32 up to 256");
     static constexpr int A_BYTES = BM * BK * 2;
     // (a CTA of a pair loads its 128 rows of A and its half of the tile's rows of W)
     static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr int STAGES = (176 * 1024) / STAGE_BYTES > 8 ? 8 : (176 * 1024) / STAGE_BYTES;
+    static constexpr int RING = (EPI > 8 ? 160 : 176) * 1024;      // (beside the epilogue's staging)
+    static constexpr int STAGES = RING / STAGE_BYTES > 8 ? 8 : RING / STAGE_BYTES;
     // two accumulators, each at a power-of-two column offset (tensor memory is allocated in
     // powers of two)
     static constexpr int ACC_STRIDE = BN <= 32 ? 32 : BN <= 64 ? 64 : BN <= 128 ? 128 : 256;
@@ -93,7 +102,7 @@ template <int BN, bool PAIR = false> struct TileCfg {
     // stages, so that it is 1024-byte aligned as the 128-byte swizzle wants)
     static constexpr int STG_BYTES = 32 * 128;
     static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 1024 /*align*/ + 256 +
-                                   (size_t)8 * STG_BYTES;
+                                   (size_t)EPI * STG_BYTES;
 };
 
 
@@ -175,18 +184,19 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
 // takes in half the bytes of W per multiply-add: the main loop of a 128 x 128 tile is bound
 // by what one SM can take in from the L2, not by its tensor core.
 template <int BN, typename O, bool PAIR>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __launch_bounds__(gemm_threads<O, BN>, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                  O* __restrict__ c, const float* __restrict__ bias,
                  const float* __restrict__ resid, int m, int n, int k, long ldc, int act,
                  int* status, Scatter sc) {
-    using Cfg = TileCfg<BN, PAIR>;
+    constexpr int EPI_WARPS = epi_warps<O, BN>;
+    using Cfg = TileCfg<BN, PAIR, EPI_WARPS>;
     extern __shared__ uint8_t smem_raw[];
     // tiles need 1024-byte alignment for the 128-byte swizzle
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* tiles = smem;
-    uint8_t* staging = smem + (size_t)Cfg::STAGES * Cfg::STAGE_BYTES;      // [8][32][128]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(staging + (size_t)8 * Cfg::STG_BYTES);
+    uint8_t* staging = smem + (size_t)Cfg::STAGES * Cfg::STAGE_BYTES;      // [EPI_WARPS][32][128]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(staging + (size_t)EPI_WARPS * Cfg::STG_BYTES);
     uint64_t* full_bar = bars;                       // [STAGES]  TMA -> MMA
     uint64_t* empty_bar = bars + Cfg::STAGES;        // [STAGES]  MMA -> TMA
     uint64_t* tfull_bar = bars + 2 * Cfg::STAGES;    // [2]       MMA -> epilogue
@@ -214,7 +224,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         for (int a = 0; a < 2; ++a) {
             mbar_init(smem_u32(&tfull_bar[a]), 1);
             // one arrival per epilogue warp (of both CTAs, on the even CTA's barrier, in a pair)
-            mbar_init(smem_u32(&tempty_bar[a]), PAIR ? 16 : 8);
+            mbar_init(smem_u32(&tempty_bar[a]), PAIR ? 2 * EPI_WARPS : EPI_WARPS);
         }
         *failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -370,7 +380,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         // columns are the same for all rows of a chunk: its bias and residual values are
         // requested a chunk ahead, before the accumulator is waited for.
         const int quarter = warp & 3;                       // TMEM lanes this warp may read
-        const int half = (warp - 2) >> 2;                   // two warps share a quarter: even / odd chunks
+        const int sub = (warp - 2) >> 2;                    // the warps of a quarter take chunks in turn
+        constexpr int STEP = EPI_WARPS / 4;
         constexpr bool F32 = sizeof(O) == 4;
         constexpr int CH = 32;                              // columns per chunk
         const bool vec_ok = ((ldc * (long)sizeof(O)) % 16 == 0) && (((uintptr_t)c) % 16 == 0) &&
@@ -436,8 +447,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             else mbar_arrive(tempty_addr[acc]);
         };
         auto tile_m0 = [&](int t) { return (t % m_tiles) * TM + rank * BM; };
-        if (walker < total_tiles && half * CH < BN) {
-            prefetch(tile_m0(walker) + quarter * 32, (walker / m_tiles) * BN + half * CH);
+        if (walker < total_tiles && sub * CH < BN) {
+            prefetch(tile_m0(walker) + quarter * 32, (walker / m_tiles) * BN + sub * CH);
             find_slots(tile_m0(walker) + quarter * 32);
         }
         for (int tile = walker; tile < total_tiles && ok; tile += walkers, ++local) {
@@ -452,21 +463,21 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             tcgen05_fence_after();
             if (warp == 2 && local == 0) GT(4);
             const int nt = tile + walkers;                  // this CTA's next tile
-            if (half * CH >= BN || n0 + half * CH >= n) {   // nothing to read for this warp
+            if (sub * CH >= BN || n0 + sub * CH >= n) {   // nothing to read for this warp
                 if (lane == 0) hand_back(acc);
-                if (nt < total_tiles && half * CH < BN)
-                    prefetch(tile_m0(nt) + quarter * 32, (nt / m_tiles) * BN + half * CH);
+                if (nt < total_tiles && sub * CH < BN)
+                    prefetch(tile_m0(nt) + quarter * 32, (nt / m_tiles) * BN + sub * CH);
                 continue;
             }
             // (the cache rows of this tile were looked up before the accumulator was waited for)
 #pragma unroll 1
-            for (int c0 = half * CH; c0 < BN; c0 += 2 * CH) {
+            for (int c0 = sub * CH; c0 < BN; c0 += STEP * CH) {
                 if (n0 + c0 >= n) break;                    // uniform across the warp
                 const int ncol = n0 + c0;
                 uint32_t r[32];
                 tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) +
                                   (uint32_t)(acc * Cfg::ACC_STRIDE + c0), r);
-                const bool last_chunk = c0 + 2 * CH >= BN || n0 + c0 + 2 * CH >= n;
+                const bool last_chunk = c0 + STEP * CH >= BN || n0 + c0 + STEP * CH >= n;
                 if (last_chunk) {
                     // this warp's last read of the accumulator: hand it back before the stores
                     tcgen05_fence_before();
@@ -487,9 +498,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     float4 r_now[F32 ? 8 : 1];
 #pragma unroll
                     for (int it = 0; it < (F32 ? 8 : 1); ++it) r_now[it] = pr[it];
-                    if (!last_chunk) prefetch(row0, ncol + 2 * CH);
+                    if (!last_chunk) prefetch(row0, ncol + STEP * CH);
                     else if (nt < total_tiles)
-                        prefetch(tile_m0(nt) + quarter * 32, (nt / m_tiles) * BN + half * CH);
+                        prefetch(tile_m0(nt) + quarter * 32, (nt / m_tiles) * BN + sub * CH);
                     const int col = ncol + rd_piece * 4;
                     // key or value columns: the page array and the offset of the lane's four
                     // columns (inside one head: head sizes are multiples of 8) within a slot
@@ -561,9 +572,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                             }
                         }
                     }
-                    if (!last_chunk) prefetch(row0, ncol + 2 * CH);
+                    if (!last_chunk) prefetch(row0, ncol + STEP * CH);
                     else if (nt < total_tiles)
-                        prefetch(tile_m0(nt) + quarter * 32, (nt / m_tiles) * BN + half * CH);
+                        prefetch(tile_m0(nt) + quarter * 32, (nt / m_tiles) * BN + sub * CH);
                 }
             }
             if (nt < total_tiles) find_slots(tile_m0(nt) + quarter * 32);
@@ -600,7 +611,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // the activation, adds the residual and stores.  A second cluster barrier keeps every CTA's
 // shared memory alive until its peers have read it.
 template <int BN, int S, typename O>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __launch_bounds__(SPLIT_THREADS, 1)
 gemm_bf16_splitk_kernel(const __grid_constant__ CUtensorMap map_a,
                         const __grid_constant__ CUtensorMap map_w, O* __restrict__ c,
                         const float* __restrict__ bias, const float* __restrict__ resid, int m,
@@ -797,7 +808,7 @@ template <int BN, typename O>
 int launch(const CUtensorMap& ma, const CUtensorMap& mw, O* c, const float* bias,
            const float* resid, int m, int n, int k, long ldc, int act, int* status,
            const Scatter& sc, cudaStream_t stream) {
-    using Cfg = TileCfg<BN>;
+    using Cfg = TileCfg<BN, false, epi_warps<O, BN>>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, O, false>,
@@ -810,7 +821,7 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mw, O* c, const float* bias
     const long tiles = (long)((n + BN - 1) / BN) * ((m + BM - 1) / BM);
     const int grid = (int)(tiles < sm_count ? tiles : sm_count);
     cudaError_t le = prb_launch_dependent(gemm_bf16_kernel<BN, O, false>, dim3(grid),
-                                          dim3(GEMM_THREADS), Cfg::SMEM, stream, ma, mw, c, bias,
+                                          dim3(gemm_threads<O, BN>), Cfg::SMEM, stream, ma, mw, c, bias,
                                           resid, m, n, k, ldc, act, status, sc);
     if (le != cudaSuccess) return (int)le;
     return 0;
@@ -821,7 +832,7 @@ template <int BN, typename O>
 int launch_pair(const CUtensorMap& ma, const CUtensorMap& mw, O* c, const float* bias,
                 const float* resid, int m, int n, int k, long ldc, int act, int* status,
                 const Scatter& sc, cudaStream_t stream) {
-    using Cfg = TileCfg<BN, true>;
+    using Cfg = TileCfg<BN, true, epi_warps<O, BN>>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, O, true>,
@@ -834,7 +845,7 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mw, O* c, const float*
     const long pairs = prb_sm_count() / 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs)));
-    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.blockDim = dim3(gemm_threads<O, BN>);
     cfg.dynamicSmemBytes = Cfg::SMEM;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -868,7 +879,7 @@ int launch_splitk(const CUtensorMap& ma, const CUtensorMap& mw, O* c, const floa
     const long tiles = (long)((n + BN - 1) / BN) * ((m + BM - 1) / BM);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(tiles * S));
-    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.blockDim = dim3(SPLIT_THREADS);
     cfg.dynamicSmemBytes = Cfg::SMEM;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -884,6 +895,42 @@ int launch_splitk(const CUtensorMap& ma, const CUtensorMap& mw, O* c, const floa
                                         resid, m, n, k, ldc, act, status);
     if (le != cudaSuccess) return (int)le;
     return 0;
+}
+
+// How many clusters of S CTAs, one to an SM, run at a time (asked once per device): clusters are
+// placed inside groups of SMs whose sizes differ, so it is less than SMs / S.
+template <int S> int ask_active_clusters() {
+    using Cfg = TileCfg<128>;
+    auto kernel = gemm_bf16_splitk_kernel<128, S, float>;
+    int n = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(S);
+    cfg.blockDim = dim3(SPLIT_THREADS);
+    cfg.dynamicSmemBytes = Cfg::SMEM;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = S;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 1;
+    }
+    return n > 0 ? n : 1;
+}
+int active_clusters(int splits) {
+    static int known[64][9] = {};
+    static std::mutex mu;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+    std::lock_guard<std::mutex> lock(mu);
+    int& n = known[dev][splits];
+    if (n == 0)
+        n = splits == 2 ? ask_active_clusters<2>() : splits == 4 ? ask_active_clusters<4>() : ask_active_clusters<8>();
+    return n;
 }
 }  // namespace
 
@@ -923,15 +970,18 @@ int gemm_bf16_entry(void* c, const void* a, const void* w, const float* bias, co
         // Few tiles and a long reduction: the k-blocks of a tile over a cluster of CTAs, which
         // costs the partial tiles' way through shared memory and two cluster barriers, while a
         // CTA finishes only its share of the tile's rows (constants fitted to measurements at
-        // 128 to 1,024 rows, N = 768 and 1,600, K = 768 to 6,400).
+        // 128 to 1,024 rows, N = 768 and 1,600, K = 768 to 6,400).  All clusters have to run at
+        // once: 280 x 768 x 3,072 as 18 clusters of eight, of which 15 fit, took 14.4 us, as 18 of
+        // four 9.0; and the exchange grows with the cluster (137 x 768 x 3,072: 128 columns by
+        // eight 8.2, 64 by four 7.4; 137 x 3,072 x 768: 128 by two 7.3, 64 unsplit 6.4).
         if (sc.kv_width == 0) {
             for (int bn = 256; bn >= 64; bn -= 64) {
                 const long tiles = mt * ((n + bn - 1) / bn);
                 for (int sp = 2; sp <= (bn > 128 ? 2 : 8); sp *= 2) {
                     const long per = (kb + sp - 1) / sp;
-                    if (tiles * sp > sms || per * (sp - 1) >= kb || per < 2) continue;
+                    if (tiles > active_clusters(sp) || per * (sp - 1) >= kb || per < 2) continue;
                     // (the partial tiles' way through shared memory grows with their width)
-                    const long exchange = bn > 128 ? 300 + 6 * bn : 700;
+                    const long exchange = bn > 128 ? 300 + 6 * bn : 700 + 100 * sp;
                     const long cost = per * (128 + bn) + 400 + exchange + per_col * bn / 2;
                     if (cost < best) { best = cost; tile_n = bn; split = sp; }
                 }
