@@ -129,6 +129,12 @@ struct Args {
     int act;
     int splits;                     // CTAs of a cluster (grid z)
     int* status;
+    // columns [q_width, q_width + kv_width) are keys, the next kv_width values of token row r: they
+    // also (only_cache: only) go to the paged cache at slots[r] (-1: none); kv_width 0: off
+    void* k_pages;
+    void* v_pages;
+    const int* slots;
+    int q_width, kv_width, head_dim, page_size, num_pages, only_cache;
 };
 
 // Address of the 16-byte piece `piece` (0..7) of row `row` in a slab of [rows][64] bfloat16
@@ -267,9 +273,12 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
     const int gcol = n0 + col;
     const float bias = (a.bias && gcol < a.n) ? a.bias[gcol] : 0.0f;
     float res[AHEAD];
+    int slot[AHEAD];
+    const bool to_cache = a.kv_width != 0 && gcol >= a.q_width && gcol < a.n;
 #pragma unroll
     for (int i = 0; i < AHEAD; ++i) {
         const int row = rank + (rsub + i * RPP) * S;
+        slot[i] = to_cache && row < a.m ? a.slots[row] : -1;
         res[i] = (a.resid && gcol < a.n && row < a.m) ? a.resid[(size_t)row * a.ldc + gcol] : 0.0f;
     }
     __syncthreads();
@@ -295,6 +304,16 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
     for (int r = 0; r < S; ++r) any_bad |= missing[r] != 0;
     if (!any_bad && gcol < a.n) {
         O* out = reinterpret_cast<O*>(a.c);
+        O* pages = nullptr;
+        int head = 0, dim = 0, kv_heads = 1;
+        if (to_cache) {
+            int cc = gcol - a.q_width;
+            pages = reinterpret_cast<O*>(cc < a.kv_width ? a.k_pages : a.v_pages);
+            if (cc >= a.kv_width) cc -= a.kv_width;
+            head = cc / a.head_dim;
+            dim = cc - head * a.head_dim;
+            kv_heads = a.kv_width / a.head_dim;
+        }
 #pragma unroll
         for (int i = 0; i < PASSES; ++i) {
             const int local = rsub + i * RPP, row = rank + local * S;
@@ -308,7 +327,18 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
             for (int r = 0; r < 8; ++r) v += pv[r];
             v = prb_activate(v + bias, a.act);
             if (a.resid) v += i < AHEAD ? res[i < AHEAD ? i : 0] : a.resid[(size_t)row * a.ldc + gcol];
-            out[(size_t)row * a.ldc + gcol] = prb_from_float<O>(v);
+            if (!to_cache || !a.only_cache) out[(size_t)row * a.ldc + gcol] = prb_from_float<O>(v);
+            if (to_cache) {
+                const int at = i < AHEAD ? slot[i < AHEAD ? i : 0] : a.slots[row];
+                if (at >= 0) {
+                    const int page = at / a.page_size;
+                    if (page >= a.num_pages)
+                        prb_set_status(a.status, PRB_S_SLOT_RANGE, row, at, a.num_pages);
+                    else
+                        pages[(((size_t)page * kv_heads + head) * a.page_size + (at - page * a.page_size)) *
+                                  a.head_dim + dim] = prb_from_float<O>(v);
+                }
+            }
         }
     }
     MT_TRACE(6);
@@ -396,14 +426,22 @@ PRB_API int prb_gemm_midm_supports(int m, int n, int k) {
 
 // a: bfloat16 [M,K]; w: bfloat16 [N,K]; c: bfloat16 or float32 [M,N] (resid float32, may
 // alias c).  M <= 64, K a multiple of 64, pitches multiples of 8 elements.
+// k_pages / v_pages / slots: the cache of the output's element type that key and value columns of a
+// fused QKV product also (only_cache: only) go to; null: none.
 PRB_API int prb_gemm_midm(void* c, const void* a, const void* w, const float* bias,
                           const float* resid, int m, int n, int k, long lda, long ldw, long ldc,
-                          int act, int out_dtype, int* status, cudaStream_t stream) {
+                          int act, int out_dtype, void* k_pages, void* v_pages, const int* slots,
+                          int q_width, int kv_width, int head_dim, int page_size, int num_pages,
+                          int only_cache, int* status, cudaStream_t stream) {
     if (m <= 0 || n <= 0) return 0;
     if (!prb_gemm_midm_supports(m, n, k)) return PRB_E_SIZE;
     if (lda % 8 != 0 || ldw % 8 != 0 || ((uintptr_t)a) % 16 != 0 || ((uintptr_t)w) % 16 != 0)
         return PRB_E_ALIGN;
     if (out_dtype != PRB_F32 && out_dtype != PRB_BF16) return PRB_E_DTYPE;
+    if (k_pages != nullptr &&
+        (v_pages == nullptr || slots == nullptr || resid != nullptr || head_dim <= 0 || kv_width <= 0 ||
+         kv_width % head_dim != 0 || page_size <= 0 || q_width < 0 || q_width + 2 * kv_width != n))
+        return PRB_E_ARG;
     // Tile width and cluster size from N and K (and the device) only.  All CTAs should run at once (one per
     // SM with 64-column tiles, two with 32-column tiles); within that, the split that gives
     // an SM the fewest bytes to take in (its CTAs' slices of A and W) wins.
@@ -430,7 +468,8 @@ PRB_API int prb_gemm_midm(void* c, const void* a, const void* w, const float* bi
     int rc = tmap::slab_map(a, m, k, lda, MROWS, KC, &ma);
     if (rc) return rc;
     if ((rc = tmap::slab_map(w, n, k, ldw, nb, KC, &mw)) != 0) return rc;
-    Args args{c, bias, resid, m, n, k, ldc, act, splits, status};
+    Args args{c, bias, resid, m, n, k, ldc, act, splits, status, k_pages, v_pages, slots, q_width,
+              k_pages != nullptr ? kv_width : 0, head_dim, page_size, num_pages, only_cache};
     if (nb == 64)
         return out_dtype == PRB_F32 ? launch_midm<64, float>(args, ma, mw, stream)
                                     : launch_midm<64, __nv_bfloat16>(args, ma, mw, stream);

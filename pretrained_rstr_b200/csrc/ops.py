@@ -88,7 +88,7 @@ def _declare(h: ctypes.CDLL) -> None:
     h.prb_gemm_bf16.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, I, I, P, P]
     h.prb_gemm_bf16_scatter.argtypes = [P, P, P, P, I, I, I, L, L, L, I, I, P, P, P, I, I, I, I, I,
                                         I, P, P]
-    h.prb_gemm_midm.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, I, P, P]
+    h.prb_gemm_midm.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, I, P, P, P, I, I, I, I, I, I, P, P]
     h.prb_gemm_midm_supports.argtypes = [I, I, I]
     h.prb_gemm_smallm.argtypes = [P, P, P, P, I, P, P, F, P, P, P, I, I, I, L, L, L, I, I,
                                   P, P, P, I, I, I, I, I, I, P, P]
@@ -535,9 +535,10 @@ def midm_supports(m: int, n: int, k: int) -> bool:
     return bool(lib().prb_gemm_midm_supports(int(m), int(n), int(k)))
 
 
-def gemm_midm(out, a, w, bias=None, resid=None, act=None, status=None) -> None:
+def gemm_midm(out, a, w, bias=None, resid=None, act=None, status=None, kv_scatter=None) -> None:
     """out[M,N] = act(a[M,K] . w[N,K]^T + bias) (+ resid) for up to 64 rows, K a multiple of
-    64: the reduction is split over a thread-block cluster (``csrc/gemm_bf16_midm.cu``)."""
+    64: the reduction is split over a thread-block cluster (``csrc/gemm_bf16_midm.cu``).
+    ``kv_scatter`` as in :func:`gemm_bf16`."""
     what = "gemm_midm"
     for name, t in (("a", a), ("w", w)):
         if not t.is_cuda or t.dtype != torch.bfloat16 or t.stride(1) != 1:
@@ -552,9 +553,22 @@ def gemm_midm(out, a, w, bias=None, resid=None, act=None, status=None) -> None:
         _need(resid, torch.float32, "resid", what)
         if resid.shape != out.shape or resid.stride(0) != out.stride(0):
             raise KernelArgumentError(f"{what}: resid must have the output's shape and stride")
+    kv = (None, None, None, 0, 0, 0, 0, 0, 0)
+    if kv_scatter is not None:
+        k_pages, v_pages, slots, q_width = kv_scatter[:4]
+        only_cache = bool(kv_scatter[4]) if len(kv_scatter) > 4 else False
+        if resid is not None:
+            raise KernelArgumentError(f"{what}: a product that scatters takes no residual")
+        if k_pages.dtype != out.dtype or v_pages.dtype != out.dtype or not k_pages.is_contiguous() \
+                or not v_pages.is_contiguous():
+            raise KernelArgumentError(f"{what}: the cache must be contiguous and of the output's type")
+        _need(slots, torch.int32, "slots", what)
+        num_pages, kv_heads, page_size, head_dim = k_pages.shape
+        kv = (_p(k_pages), _p(v_pages), _p(slots), int(q_width), kv_heads * head_dim, head_dim, page_size,
+              num_pages, int(only_cache))
     _check(lib().prb_gemm_midm(_p(out), _p(a), _p(w), _p(bias), _p(resid), m, n, k, a.stride(0),
                                w.stride(0), out.stride(0), ACT_CODES[act], dtype_code(out.dtype),
-                               _p(status), _stream()), what)
+                               *kv, _p(status), _stream()), what)
 
 
 _SMALLM = None

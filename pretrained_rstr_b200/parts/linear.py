@@ -63,16 +63,21 @@ class Linear:
             return False
         # Which kernel (measured on GPT-2 small and XL shapes): up to 16 rows
         # the weight-streaming kernel with the norm fused into it; 17 to 64 rows the cluster
-        # split-K kernel for narrow outputs and long reductions, the tensor-memory kernel for
-        # wide outputs (the register-streaming kernel where K is no multiple of 64); beyond
-        # 64 rows the tensor-memory kernel.
+        # split-K kernel for small weights, narrow outputs and long reductions, the tensor-memory
+        # kernel for wide outputs (the register-streaming kernel where K is no multiple of 64);
+        # beyond 64 rows the tensor-memory kernel.
         max_rows, max_norm = ops.smallm_limits()
-        if 16 < m <= 64 and (self.n_out <= 2048 or self.n_in >= 4 * self.n_out) and \
+        if 16 < m <= 64 and (self.n_out <= 2048 or self.n_in >= 4 * self.n_out or
+                             self.n_out * self.n_in <= 4096 * 1024) and \
                 ops.midm_supports(m, self.n_out, self.n_in):
-            # narrow outputs or long reductions at a few dozen rows: the reduction split over
-            # a thread-block cluster (measured against the other two kernels)
-            ops.gemm_midm(out, _tensor(a), self.weight, self.bias, resid, act, status=ctx.status)
-            return False
+            # a few dozen rows: the reduction split over a thread-block cluster.  Weights of up to
+            # 4 M numbers at any shape (us at 32 / 64 rows, tensor-memory kernel / this one: 2,304 x
+            # 768 10.1 / 4.6 and 10.0 / 5.3, 4,096 x 1,024 7.6 / 6.5 and 7.5 / 7.1), larger ones
+            # where the output is narrow or the reduction long (4,800 x 1,600: 10.9 / 12.6)
+            scatters = kv_scatter is not None and resid is None and kv_scatter[0].dtype == out.dtype
+            ops.gemm_midm(out, _tensor(a), self.weight, self.bias, resid, act, status=ctx.status,
+                          kv_scatter=kv_scatter if scatters else None)
+            return scatters
         if m <= max_rows and self.n_in % 8 == 0 and (m <= 16 or self.n_out <= 1024):
             if kv_scatter is not None and kv_scatter[0].dtype != out.dtype:
                 kv_scatter = None
