@@ -41,25 +41,23 @@ constexpr int DEC_WARPS = DEC_THREADS / 32;
 template <int LPK, int UB, int MIN_CTAS, bool CLUSTER>
 __global__ void __launch_bounds__(DEC_THREADS, MIN_CTAS)
 attention_decode_kernel(Args a) {
-    __shared__ Shared<DEC_WARPS> sh;
-    prb_grid_launch_dependents();
+    __shared__ Shared<DEC_WARPS, 8 * LPK, CLUSTER> sh;
     prb_grid_wait();
     unit<LPK, DEC_WARPS, UB, CLUSTER>(a, blockIdx.x, blockIdx.y, blockIdx.z, sh);
 }
 
 // The streaming variant: one more template of the same unit, with the ring in dynamic shared
 // memory (3 stages x (keys + values) x 64 positions x head_dim x 2 bytes: 48 KB at head size
-// 64, four CTAs per SM).
-template <int LPK, bool CLUSTER>
+// 64, four CTAs per SM; never as a cluster).
+template <int LPK>
 __global__ void __launch_bounds__(DEC_THREADS, 1)
 attention_decode_stream_kernel(Args a) {
     extern __shared__ __align__(128) unsigned char stream_ring[];
-    __shared__ Shared<DEC_WARPS> sh;
+    __shared__ Shared<DEC_WARPS, 8 * LPK, false> sh;
     __shared__ StreamState st;
-    prb_grid_launch_dependents();
     prb_grid_wait();
     if (threadIdx.x == 0) st.ring = stream_ring;
-    unit<LPK, DEC_WARPS, 2, CLUSTER, true>(a, blockIdx.x, blockIdx.y, blockIdx.z, sh, &st);
+    unit<LPK, DEC_WARPS, 2, false, true>(a, blockIdx.x, blockIdx.y, blockIdx.z, sh, &st);
 }
 
 // Whether the kernel may be placed on the SMs before its predecessor has ended.  Off, by
@@ -149,21 +147,18 @@ PRB_API int prb_attention_decode(void* out, long out_stride, const void* q, long
     a.max_pages = max_pages; a.num_pages = num_pages; a.scale = scale; a.window = window;
     a.workspace = workspace; a.counters = counters; a.max_splits = max_splits;
     a.split = split_keys; a.status = status;
-    // more CTAs than fit at four per SM: the leaner instance, six per SM; two to eight
-    // splits: the CTAs of a (token, head) form a cluster and merge through shared memory
+    // More CTAs than fit at four per SM: the leaner instance, six per SM.  Otherwise two to eight
+    // splits form a cluster and merge through shared memory (a layer of GPT-2 small at one request
+    // 25.0 -> 23.9 us); clusters of many CTAs wait for places side by side and lose (16 requests
+    // 37.5 us through the workspace, 40.6 as clusters; XL sizes at 8 requests 50.3 and 51.2).
     const bool many = (long)n_list * n_heads * max_splits > 4L * prb_sm_count();
-    const bool cluster = max_splits >= 2 && max_splits <= 8 && prb_decode_clusters();
+    const bool cluster = !many && max_splits >= 2 && max_splits <= MAX_CLUSTER && prb_decode_clusters();
 #define PRB_DEC(L)                                                                               \
     do {                                                                                         \
-        if (cluster)                                                                             \
-            e = many ? launch_decode(attention_decode_kernel<L, 2, 6, true>, grid, max_splits,   \
-                                     stream, a)                                                  \
-                     : launch_decode(attention_decode_kernel<L, 4, 4, true>, grid, max_splits,   \
-                                     stream, a);                                                 \
-        else                                                                                     \
-            e = many ? launch_decode(attention_decode_kernel<L, 2, 6, false>, grid, 1, stream, a) \
-                     : launch_decode(attention_decode_kernel<L, 4, 4, false>, grid, 1, stream,   \
-                                     a);                                                         \
+        if (many) e = launch_decode(attention_decode_kernel<L, 2, 6, false>, grid, 1, stream, a); \
+        else if (cluster)                                                                        \
+            e = launch_decode(attention_decode_kernel<L, 4, 4, true>, grid, max_splits, stream, a); \
+        else e = launch_decode(attention_decode_kernel<L, 4, 4, false>, grid, 1, stream, a);     \
     } while (0)
     cudaError_t e;
     // Long splits and more units than run at once: the streaming variant.
@@ -174,18 +169,17 @@ PRB_API int prb_attention_decode(void* out, long out_stride, const void* q, long
     if (use_stream) {
 #define PRB_DEC_STREAM(L)                                                                        \
     do {                                                                                         \
-        auto kern = cluster ? attention_decode_stream_kernel<L, true>                            \
-                            : attention_decode_stream_kernel<L, false>;                          \
-        static bool configured[2] = {false, false};                                              \
-        if (!configured[cluster ? 1 : 0]) {                                                      \
+        auto kern = attention_decode_stream_kernel<L>;                                           \
+        static bool configured = false;                                                          \
+        if (!configured) {                                                                       \
             cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,           \
                                  cudaSharedmemCarveoutMaxShared);                                \
             e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,          \
                                      (int)((size_t)STREAM_STAGES * 2 * STREAM_KEYS * (L * 8) * 2)); \
             if (e != cudaSuccess) return (int)e;                                                 \
-            configured[cluster ? 1 : 0] = true;                                                  \
+            configured = true;                                                                   \
         }                                                                                        \
-        e = launch_decode(kern, grid, cluster ? max_splits : 1, stream, a, ring_bytes);          \
+        e = launch_decode(kern, grid, 1, stream, a, ring_bytes);                                 \
     } while (0)
         if (pieces <= 2) PRB_DEC_STREAM(2);
         else if (pieces <= 4) PRB_DEC_STREAM(4);

@@ -211,14 +211,9 @@ class CausalAttention(Mixer):
             ops.kv_append(cache.k, cache.v, k, v, group.slots, t, ctx.status)
         o = ctx.scratch("attn_out", (ctx.token_capacity, self.q_width), dtype)[:t]
         # (the step's own keys and values lie beside the queries exactly as the cache got them)
-        last = attend(ctx, o, q, cache, group, self.n_head, self.scale, self.window,
-                      kv_new=(k, v) if cache.writes else None)
-        # After the split-key decode kernel (hundreds of small CTAs, several to an SM) the
-        # projection is launched the plain way: placed early, its CTAs take room beside them
-        # on the SMs and the pair lasts longer (measured, a layer of GPT-2 small: 30.3 -> 29.5
-        # us at 8 requests, 25.5 -> 24.1 us at one).
-        with ops.plain_launch(last == "split"):
-            self.out.forward(ctx, o, x, resid=x if accumulate else None)
+        attend(ctx, o, q, cache, group, self.n_head, self.scale, self.window,
+               kv_new=(k, v) if cache.writes else None)
+        self.out.forward(ctx, o, x, resid=x if accumulate else None)
 
 
 def prefill_key_parts(items: int, max_context: int, window: Optional[int]):
@@ -247,9 +242,8 @@ def prefill_key_parts(items: int, max_context: int, window: Optional[int]):
 
 
 def attend(ctx, out, q, cache: LayerCache, group, n_head: int, scale: float,
-           window: Optional[int], kv_new=None) -> Optional[str]:
-    """Attention of the step's tokens over their requests' cached keys and values.  Returns
-    which kernel ran last: "ring", "split" (the split-key decode kernel) or None.
+           window: Optional[int], kv_new=None) -> None:
+    """Attention of the step's tokens over their requests' cached keys and values.
 
     float32 runtime: the 32-bit kernels, prompt portions in tiles of queries and single tokens by
     themselves.  bfloat16 runtime: prompt
@@ -338,7 +332,7 @@ def attend(ctx, out, q, cache: LayerCache, group, n_head: int, scale: float,
                                       work.counts["singles"], n_list, n_head, scale, window, ws,
                                       counters, ctx.status, new_keys=AttentionWork.SINGLE_MAX_Q,
                                       max_context=ctx.max_context, kv_new=kv_new)
-            return "ring"
+            return
         split_keys, max_splits = decode_splits(n_list * n_head, ctx.max_context, group.page_size)
         # room for the shortest splits any step may choose
         splits_cap = -(-ctx.max_positions // ops.decode_split())
@@ -349,8 +343,6 @@ def attend(ctx, out, q, cache: LayerCache, group, n_head: int, scale: float,
                              ctx.positions, work.arrays["single_tokens"], work.counts["singles"],
                              n_list, n_head, scale, window, ws, counters, max_splits, ctx.status,
                              split_keys=split_keys)
-        return "split"
-    return None
 
 
 def decode_splits(pairs: int, max_context: int, page_size: int):
