@@ -267,6 +267,7 @@ __global__ void retention_step_kernel(StepArgs sa) {
     extern __shared__ __align__(16) float smem[];
     __shared__ float inv_s;
     const ScanArgs& a = sa.scan;
+    prb_grid_wait();
     prb_grid_launch_dependents();
     const int h = blockIdx.x, b = blockIdx.y;
     const int t0 = a.q_start[b], t1 = a.q_start[b + 1];
@@ -528,15 +529,19 @@ PRB_API int prb_retention_step(void* out, long out_ld, const float* proj, long l
                 freq, (const float2*)angles, rot_dims, k_scale, eps, out, out_ld, g_col};
     const size_t smem = (size_t)(2 * lanes * ni + vdim) * sizeof(float);
     const dim3 grid(heads, n_requests);
+    const bool early = (long)heads * n_requests <= 2L * prb_sm_count();
+    cudaError_t e = cudaSuccess;
+#define RET_STEP(NI, OT) \
+    e = prb_launch_maybe_early(early, retention_step_kernel<NI, OT>, grid, dim3(threads), smem, stream, sa)
     if (out_dtype == PRB_F32) {
-        if (ni == 4) retention_step_kernel<4, float><<<grid, threads, smem, stream>>>(sa);
-        else retention_step_kernel<16, float><<<grid, threads, smem, stream>>>(sa);
+        if (ni == 4) RET_STEP(4, float);
+        else RET_STEP(16, float);
     } else if (out_dtype == PRB_BF16) {
-        if (ni == 4) retention_step_kernel<4, __nv_bfloat16><<<grid, threads, smem, stream>>>(sa);
-        else retention_step_kernel<16, __nv_bfloat16><<<grid, threads, smem, stream>>>(sa);
+        if (ni == 4) RET_STEP(4, __nv_bfloat16);
+        else RET_STEP(16, __nv_bfloat16);
     } else {
         return PRB_E_DTYPE;
     }
-    PRB_LAUNCH_CHECK();
-    return 0;
+#undef RET_STEP
+    return e == cudaSuccess ? 0 : (int)e;
 }

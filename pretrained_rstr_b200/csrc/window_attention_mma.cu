@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(WD_WARPS * 32) wattn_decode_kernel(Args a) {
     constexpr int KPS = 32 / LPK;                    // value rows a step
     constexpr int STAGES = WD_STAGES;
     extern __shared__ __align__(16) float smf[];
-    prb_grid_launch_dependents();
+    prb_grid_wait();
     const int hg = a.heads / a.kv_heads;
     const int r = blockIdx.x, g = blockIdx.y;
     const int splits = gridDim.z, split = blockIdx.z;            // the cluster and this CTA's rank
@@ -607,6 +607,7 @@ __global__ void __launch_bounds__(WD_WARPS * 32) wattn_decode_kernel(Args a) {
         }
     }
     __syncthreads();
+    prb_grid_launch_dependents();                    // the next kernel may set itself up
     // the CTA's warps in warp order, then the cluster's CTAs in rank order
     for (int e = threadIdx.x; e < hg * a.vdim; e += blockDim.x) {
         const int hh = e / a.vdim, jv = e - hh * a.vdim;
@@ -729,13 +730,16 @@ PRB_API int prb_wattn_bf16(void* out, long out_ld, const float* q, const void* c
     cfg.gridDim = dim3(n_tokens, kv_heads, splits);
     cfg.blockDim = dim3(WD_WARPS * 32);
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = (unsigned)splits;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed =
+        prb_pdl_enabled() && (long long)n_tokens * kv_heads * splits <= 2LL * prb_sm_count() ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = (unsigned)splits;
     cfg.attrs = attr;
-    cfg.numAttrs = splits > 1 ? 1 : 0;
+    cfg.numAttrs = splits > 1 ? 2 : 1;
 #define WD2(HN, WN)                                                                              \
     do {                                                                                         \
         cfg.dynamicSmemBytes = decode_smem(HN, WN ? 4 : 2, hg, dim, vdim);                            \

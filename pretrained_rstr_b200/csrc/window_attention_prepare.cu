@@ -92,6 +92,7 @@ __device__ __forceinline__ void store_pair(__nv_bfloat16* p, float x, float y) {
 // in registers.  0: any size, computed again in every pass.
 template <typename C, int U>
 __global__ void __launch_bounds__(256) wattn_prepare_heads_kernel(PrepArgs a) {
+    prb_grid_wait();
     prb_grid_launch_dependents();
     const int lane = threadIdx.x & 31;
     const int per_token = a.heads + a.kv_heads;
@@ -364,7 +365,12 @@ PRB_API int prb_wattn_prepare_heads(float* q_out, void* cache, const float* proj
     const int warps = units <= 4L * prb_sm_count() ? 2 : 8;
     const unsigned blocks = (unsigned)((units + warps - 1) / warps);
     const int lane_units = (dim - rot_dims / 2 + 31) / 32;
-#define PREP1(CT, UN) wattn_prepare_heads_kernel<CT, UN><<<blocks, warps * 32, 0, stream>>>(a)
+    // (few units start while the product before them ends, as other small steps' kernels do)
+    const bool early = units <= 4L * prb_sm_count();
+    cudaError_t e = cudaSuccess;
+#define PREP1(CT, UN)                                                                            \
+    e = prb_launch_maybe_early(early, wattn_prepare_heads_kernel<CT, UN>, dim3(blocks), dim3(warps * 32), 0, \
+                               stream, a)
 #define PREP(CT)                                                                                 \
     do {                                                                                         \
         if (lane_units == 1) PREP1(CT, 1);                                                       \
@@ -377,7 +383,7 @@ PRB_API int prb_wattn_prepare_heads(float* q_out, void* cache, const float* proj
     else return PRB_E_DTYPE;
 #undef PREP
 #undef PREP1
-    PRB_LAUNCH_CHECK();
+    if (e != cudaSuccess) return (int)e;
     if (conv_q != nullptr && taps > 1 && n_requests > 0) {
         const int channels = (heads + kv_heads) * dim;
         wattn_conv_state_kernel<<<dim3((channels + 127) / 128, n_requests), 128, 0, stream>>>(a);
