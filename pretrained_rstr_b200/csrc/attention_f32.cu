@@ -451,13 +451,17 @@ int launch(K kernel, const Args& a, dim3 grid, int threads, size_t smem, cudaStr
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = grid.z;
+    // the few CTAs of a small decoding step start while the kernel before them ends
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed =
+        prb_pdl_enabled() && (long)grid.x * grid.y * grid.z <= 2L * prb_sm_count() ? 1 : 0;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     e = cudaLaunchKernelEx(&cfg, kernel, a);
     return e == cudaSuccess ? 0 : (int)e;
 }

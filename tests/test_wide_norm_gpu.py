@@ -7,7 +7,7 @@ from test_kernels_gpu import _ops
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows", [15, 16, 17, 128, 129, 300])
+@pytest.mark.parametrize("rows", [1, 15, 16, 17, 128, 129, 300])
 @pytest.mark.parametrize("width", [1024, 1028, 1600, 2044, 2048, 2052])
 @pytest.mark.parametrize("beta", [True, False])
 def test_layernorm_of_wide_rows(rows, width, beta):
