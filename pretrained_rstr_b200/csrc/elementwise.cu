@@ -85,6 +85,8 @@ layernorm_warp_kernel(elementwise::NormArgs a) {
         }
     }
     prb_grid_wait();
+    // (signalled from the top, an early norm lets its product in beside the kernel ahead: 64 requests
+    // decoding 7.31 -> 7.95 ms for 8 steps)
     prb_grid_launch_dependents();
     if (r >= a.n_rows) return;
     O* out = reinterpret_cast<O*>(a.out) + (size_t)r * a.width;
