@@ -88,6 +88,7 @@ def load_model(folder: str, dtype="bfloat16", device="cuda:0", page_size: int = 
                          strip_prefixes=arch.strip_prefixes, ignorable=arch.ignorable)
     model = arch.build(config, store, runtime)
     store.release()
+    model.settle()
     if num_pages is None:
         if max_tokens is None:
             per_request = min(config.max_positions, DEFAULT_POSITIONS)

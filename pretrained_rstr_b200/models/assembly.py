@@ -63,6 +63,15 @@ class Model:
                 elif kept[0] is not planner:
                     kept[0].absorb(planner)
 
+    def settle(self) -> None:
+        """Build what the parts would otherwise build in the first step: the matrices of products
+        that several tensors are joined into."""
+        for block in self.blocks:
+            for part in (block, block.mixer, block.feed_forward, *getattr(block.mixer, "children", ())):
+                for value in list(vars(part).values()):
+                    if hasattr(value, "settle"):
+                        value.settle()
+
     # ---------------------------------------------------------------- cache layout
     def _derive_cache_layout(self) -> None:
         # a cache is shaped by the mixer of the entry that writes it (caches are numbered by

@@ -46,7 +46,7 @@ import torch
 from ..csrc import ops
 from ..engine.batch import WorkPlanner
 from .interfaces import KVSpec, LayerCache, Mixer
-from .linear import Linear, padded_linear
+from .linear import Linear, padded_linear, settled
 from .registry import register_part
 
 
@@ -57,7 +57,7 @@ def _pad8(n: int) -> int:
 class FusedInput:
     """One matrix product for several consumers of the same input: segments of rows, each
     starting at a multiple of 8 columns of the float32 result.  Segments are added while the
-    model is built; the matrix is put together at the first use.
+    model is built; the matrix is put together when the model has been loaded (:meth:`settle`), or at the first use.
 
     Two parts that read the same input can have one product: ``a.absorb(b)`` moves b's segments
     into a; b.run then hands out the result of a's product, which has to run before it."""
@@ -109,11 +109,17 @@ class FusedInput:
                                             device=w.device))
                 at += w.shape[0] + pad
             self._linear = Linear(torch.cat(rows, dim=0), None, self.runtime)
+            settled(self._linear.weight)
             self._parts = []
             for prefix, guest in self._guests:
                 guest.cols.update({name[len(prefix):]: at for name, at in self.cols.items()
                                    if name.startswith(prefix)})
         return self._linear
+
+    def settle(self) -> None:
+        """Join the matrices now (when the model is loaded) instead of in the first step."""
+        if self.host is None and self._parts:
+            self.linear()
 
     @property
     def ahead(self) -> bool:

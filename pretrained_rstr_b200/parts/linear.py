@@ -111,6 +111,14 @@ def padded_linear(weight: torch.Tensor, runtime) -> Linear:
     return Linear(weight, None, runtime)
 
 
+def settled(weight: torch.Tensor) -> torch.Tensor:
+    """``weight`` once what computed it has ended: the products read their matrices while the kernel
+    ahead of them may still run, which must not be the one that joins a matrix together."""
+    if weight.is_cuda and not torch.cuda.is_current_stream_capturing():
+        torch.cuda.current_stream(weight.device).synchronize()
+    return weight
+
+
 class ResultProduct:
     """The matrix product a part ends with: x (+)= r . W^T + b, from a buffer of its own that the
     part fills (:meth:`buffer`, then :meth:`run`).
@@ -160,8 +168,14 @@ class ResultProduct:
             self.key += "/" + ",".join(str(int(w.shape[1])) for w, _b in self.parts)
             self._linear = Linear(torch.cat(pieces, dim=1) if len(pieces) > 1 else pieces[0], bias,
                                   self.runtime)
+            settled(self._linear.weight)
             self.parts = []
         return self._linear
+
+    def settle(self) -> None:
+        """Join the matrices now (when the model is loaded) instead of in the first step."""
+        if self.host is None:
+            self.linear()
 
     def buffer(self, ctx, t: int) -> torch.Tensor:
         """[t, columns] in the activation type: the part writes its real columns."""
