@@ -42,6 +42,7 @@ struct Args {
     int m, n, k;
     long lda, ldw, ldc;
     int act;
+    bool settled;                   // w may be read before the kernel ahead has ended
     int* status;
 };
 
@@ -465,7 +466,7 @@ int launch_tile(const Args& p, bool vec, cudaStream_t stream) {
     if (e != cudaSuccess) return (int)e;
     dim3 grid(4 * ((p.n + BN - 1) / BN), (p.m + BM - 1) / BM);
     if (grid.y > 65535) return PRB_E_SIZE;
-    e = prb_launch_dependent(kernel, grid, dim3(Cfg::THREADS), Cfg::SMEM, stream, p);
+    e = prb_launch_maybe_early(p.settled, kernel, grid, dim3(Cfg::THREADS), Cfg::SMEM, stream, p);
     return e == cudaSuccess ? 0 : (int)e;
 }
 
@@ -482,7 +483,7 @@ int launch_stream(const Args& p, StreamGeo g, int copy, size_t smem, cudaStream_
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     dim3 grid((p.n + g.rows_per_cta - 1) / g.rows_per_cta, (p.m + MB - 1) / MB);
-    e = prb_launch_dependent(kernel, grid, dim3(STREAM_THREADS), smem, stream, p, g, map);
+    e = prb_launch_maybe_early(p.settled, kernel, grid, dim3(STREAM_THREADS), smem, stream, p, g, map);
     return e == cudaSuccess ? 0 : (int)e;
 }
 
@@ -524,14 +525,14 @@ bool stream_geometry(const Args& p, int mb, int copy, StreamGeo* g, size_t* smem
 }  // namespace
 
 // which: 0 the rule below; 1 the stream kernel where it fits, 2 / 3 tiles of 64 x 128, 64 x 64 (the
-// same bits from all of them).  w is read before the kernel ahead in the stream has ended: it must
-// be a tensor that no kernel of the step writes.
+// same bits from all of them).  settled: w was written long before (by no kernel of the step), so the
+// launch may be placed, and w read, before the kernel ahead in the stream has ended.
 PRB_API int prb_gemm_f32(float* c, const float* a, const float* w, const float* bias,
                          const float* resid, int m, int n, int k, long lda, long ldw, long ldc,
-                         int act, int which, int* status, cudaStream_t stream) {
+                         int act, int which, int settled, int* status, cudaStream_t stream) {
     if (m <= 0 || n <= 0) return 0;
     if (k <= 0) return PRB_E_SIZE;
-    const Args p{c, a, w, bias, resid, m, n, k, lda, ldw, ldc, act, status};
+    const Args p{c, a, w, bias, resid, m, n, k, lda, ldw, ldc, act, settled != 0, status};
     // 16-byte copies where every row starts on 16 bytes and K ends on them, else single floats
     const bool vec = k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)a) % 16 == 0 &&
                      ((uintptr_t)w) % 16 == 0;

@@ -84,7 +84,7 @@ def _declare(h: ctypes.CDLL) -> None:
     h.prb_host_device_address.restype = c_void_p
     h.prb_fetch_step.argtypes = [P, P, I, I, I, P, I, P, P]
     h.prb_publish_result.argtypes = [P, P, I, P]
-    h.prb_gemm_f32.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, I, P, P]
+    h.prb_gemm_f32.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, I, I, P, P]
     h.prb_gemm_bf16.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, I, I, P, P]
     h.prb_gemm_bf16_scatter.argtypes = [P, P, P, P, I, I, I, L, L, L, I, I, P, P, P, I, I, I, I, I,
                                         I, P, P]
@@ -458,10 +458,11 @@ def copy_pages(storage, pairs, n_pairs, status) -> None:
                                 _p(status), _stream()), what)
 
 
-def gemm_f32(out, a, w, bias=None, resid=None, act=None, kernel: int = 0, status=None) -> None:
+def gemm_f32(out, a, w, bias=None, resid=None, act=None, kernel: int = 0, status=None,
+             settled: bool = False) -> None:
     """out[M,N] = act(a[M,K] . w[N,K]^T + bias) (+ resid): true 32-bit FMA, one order of
-    summation for every M.  ``w`` may be read before the kernel ahead has ended (weights, which
-    no kernel of a step writes).  ``kernel`` forces one of the kernels (1 rows of weights as a
+    summation for every M.  ``settled``: ``w`` was complete before the kernel ahead in the stream
+    began (a model's weights are), so it may be read while that still runs.  ``kernel`` forces one of the kernels (1 rows of weights as a
     stream, 2 / 3 tiles of 64 x 128, 64 x 64); left at 0 the sizes choose.  All give the same bits."""
     what = "gemm_f32"
     for name, t in (("out", out), ("a", a), ("w", w)):
@@ -478,8 +479,8 @@ def gemm_f32(out, a, w, bias=None, resid=None, act=None, kernel: int = 0, status
         if resid.shape != out.shape or resid.stride(0) != out.stride(0):
             raise KernelArgumentError(f"{what}: resid must have the output's shape and stride")
     _check(lib().prb_gemm_f32(_p(out), _p(a), _p(w), _p(bias), _p(resid), m, n, k, a.stride(0),
-                              w.stride(0), out.stride(0), ACT_CODES[act], int(kernel), _p(status),
-                              _stream()), what)
+                              w.stride(0), out.stride(0), ACT_CODES[act], int(kernel), int(bool(settled)),
+                              _p(status), _stream()), what)
 
 
 def gemm_bf16(out, a, w, bias=None, resid=None, act=None, tile_n: int = 0, status=None,

@@ -59,7 +59,7 @@ class Linear:
         QKV product straight to the cache; returns True when it did."""
         m = out.shape[0]
         if self.runtime.dtype == torch.float32:
-            ops.gemm_f32(out, _tensor(a), self.weight, self.bias, resid, act, status=ctx.status)
+            ops.gemm_f32(out, _tensor(a), self.weight, self.bias, resid, act, status=ctx.status, settled=True)
             return False
         # Which kernel (measured on GPT-2 small and XL shapes): up to 16 rows
         # the weight-streaming kernel with the norm fused into it; 17 to 64 rows the cluster
