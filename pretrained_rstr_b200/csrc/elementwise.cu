@@ -69,9 +69,10 @@ layernorm_warp_kernel(elementwise::NormArgs a) {
     const int r = blockIdx.x * 4 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     const int nvec = a.width / 4;
-    // gamma and beta, which no kernel writes, are asked for first, not after the statistics: the
-    // row's way through the kernel is one memory round trip long instead of two.  (With 16 pieces
-    // they would take the registers of every second warp, and come from the L1 afterwards.)
+    // gamma and beta (settled, or the launch is not early) are asked for first, not after the
+    // statistics: the row's way through the kernel is one memory round trip long instead of two.
+    // (With 16 pieces they would take the registers of every second warp, and come from the L1
+    // afterwards.)
     constexpr bool AHEAD = NV <= 8;
     const float4* g4 = reinterpret_cast<const float4*>(a.gamma);
     const float4* b4 = reinterpret_cast<const float4*>(a.beta);
@@ -138,9 +139,11 @@ layernorm_warp_kernel(elementwise::NormArgs a) {
     }
 }
 
+// settled: gamma and beta were written long before (by no kernel of the step): only then may the
+// launch start, and read them, before the kernel ahead in the stream has ended.
 PRB_API int prb_layernorm(void* out, const float* x, const float* gamma, const float* beta,
                           const int* rows, int n_rows, int n_rows_in, int width, float eps,
-                          int out_dtype, int* status, cudaStream_t stream) {
+                          int out_dtype, int settled, int* status, cudaStream_t stream) {
     if (n_rows <= 0) return 0;
     if (width <= 0 || (size_t)width * 4 > 200 * 1024) return PRB_E_SIZE;
     if (out_dtype != PRB_F32 && out_dtype != PRB_BF16) return PRB_E_DTYPE;
@@ -152,7 +155,7 @@ PRB_API int prb_layernorm(void* out, const float* x, const float* gamma, const f
     if (width % 4 == 0 && width <= 2048 && aligned) {
         const int blocks = (n_rows + 3) / 4;
         // the few rows of a decoding batch start while the product before them ends
-        const bool early = n_rows <= 128 || prb_small_ctas_early();
+        const bool early = settled && (n_rows <= 128 || prb_small_ctas_early());
         cudaError_t e;
 #define PRB_LN(OT)                                                                               \
     e = width <= 1024 ? prb_launch_maybe_early(early, layernorm_warp_kernel<OT, 8>, dim3(blocks), \

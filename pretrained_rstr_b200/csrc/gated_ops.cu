@@ -246,7 +246,7 @@ __global__ void norm_pair_kernel(NormPairArgs a) {
     const float* y = a.y + (size_t)r * a.width;
     float v[NV], xv[NV], w[NV], b[NV], w2[NV], b2[NV];
 #pragma unroll
-    for (int j = 0; j < NV; ++j) {                   // the norms' parameters: no kernel writes them
+    for (int j = 0; j < NV; ++j) {                   // the norms' parameters: settled where the launch is early
         const int i = threadIdx.x + j * blockDim.x;
         const bool in = i < a.width;
         w[j] = in ? a.w1[i] : 0.0f;
@@ -419,11 +419,13 @@ PRB_API int prb_rms_norm(void* out, float* x_out, const float* x, const float* y
     return 0;
 }
 
-// x <- x + mult * norm_1(y), then norm_2(x) or a copy of x in the activation type.
+// x <- x + mult * norm_1(y), then norm_2(x) or a copy of x in the activation type.  settled: the norms'
+// parameters were written long before (by no kernel of the step): only then may the launch start,
+// and read them, before the kernel ahead in the stream has ended.
 PRB_API int prb_norm_pair(void* out, long out_ld, float* x, const float* y, const float* w1,
                           const float* b1, const float* w2, const float* b2, int n_rows, int width,
                           int centred1, int centred2, int next, float mult, float eps1, float eps2,
-                          int out_dtype, cudaStream_t stream) {
+                          int out_dtype, int settled, cudaStream_t stream) {
     if (n_rows <= 0) return 0;
     if (width <= 0 || width > 1024 * 16) return PRB_E_SIZE;
     if (next < 0 || next > 2 || w1 == nullptr || (next != 0 && out == nullptr) || (next == 1 && w2 == nullptr))
@@ -436,7 +438,7 @@ PRB_API int prb_norm_pair(void* out, long out_ld, float* x, const float* y, cons
     if (threads < 64) threads = 64;
     // A step of few rows (one CTA an SM at most) starts while the product before it ends (with the same for
     // its neighbours, heads, gated pairs and the two mixers: six requests of Musilorn 10.61 -> 10.01 ms).
-    const bool early = n_rows <= prb_sm_count();
+    const bool early = settled && n_rows <= prb_sm_count();
     cudaError_t e = cudaSuccess;
 #define NORM_PAIR(OT)                                                                            \
     do {                                                                                         \

@@ -75,7 +75,7 @@ def require_cuda() -> None:
 def _declare(h: ctypes.CDLL) -> None:
     P, I, L, F = c_void_p, c_int, c_long, c_float
     h.prb_embed.argtypes = [P, P, P, P, P, I, I, I, I, I, P, P]
-    h.prb_layernorm.argtypes = [P, P, P, P, P, I, I, I, F, I, P, P]
+    h.prb_layernorm.argtypes = [P, P, P, P, P, I, I, I, F, I, I, P, P]
     h.prb_bias_act.argtypes = [P, P, P, P, I, I, I, I, I, P]
     h.prb_kv_append.argtypes = [P, P, P, P, L, P, I, I, I, I, I, I, P, P]
     h.prb_copy_pages.argtypes = [P, P, I, L, I, I, P, P]
@@ -140,7 +140,7 @@ def _declare(h: ctypes.CDLL) -> None:
     h.prb_gate_mul.argtypes = [P, L, P, L, P, L, I, I, I, P]
     h.prb_gate_mul.restype = c_int
     h.prb_gated_pair.argtypes = [P, L, I, P, L, I, I, I, I, F, F, F, P, L, I, I, I, P]
-    h.prb_norm_pair.argtypes = [P, L, P, P, P, P, P, P, I, I, I, I, I, F, F, F, I, P]
+    h.prb_norm_pair.argtypes = [P, L, P, P, P, P, P, P, I, I, I, I, I, F, F, F, I, I, P]
     h.prb_norm_pair.restype = c_int
     h.prb_tanh_cap.argtypes = [P, L, I, I, F, P]
     h.prb_tanh_cap.restype = c_int
@@ -392,8 +392,10 @@ def embed(out, tokens, positions, wte, wpe, status) -> None:
                            dtype_code(wte.dtype), _p(status), _stream()), what)
 
 
-def layernorm(out, x, gamma, beta, eps: float, rows=None, status=None) -> None:
-    """out[r,:] = LayerNorm(x[rows[r],:] or x[r,:]); x float32, out float32 or bfloat16."""
+def layernorm(out, x, gamma, beta, eps: float, rows=None, status=None, settled: bool = False) -> None:
+    """out[r,:] = LayerNorm(x[rows[r],:] or x[r,:]); x float32, out float32 or bfloat16.  ``settled``:
+    ``gamma`` and ``beta`` were complete before the kernel ahead in the stream began (a model's
+    parameters are), so they may be read while that still runs."""
     what = "layernorm"
     _need(x, torch.float32, "x", what)
     _need(out, None, "out", what)
@@ -408,8 +410,8 @@ def layernorm(out, x, gamma, beta, eps: float, rows=None, status=None) -> None:
     if rows is not None:
         _need(rows, torch.int32, "rows", what)
     _check(lib().prb_layernorm(_p(out), _p(x), _p(gamma), _p(beta), _p(rows), n_rows, x.shape[0],
-                               width, float(eps), dtype_code(out.dtype), _p(status), _stream()),
-           what)
+                               width, float(eps), dtype_code(out.dtype), int(bool(settled)), _p(status),
+                               _stream()), what)
 
 
 def bias_act(out, inp, bias, resid, act) -> None:
@@ -1107,11 +1109,14 @@ def gated_pair(out, inp, gate_col: int, up_col: int, n: int, out_col: int = 0, l
                                 GATED_ACT_CODES[act], dtype_code(out.dtype), _stream()), what)
 
 
-def norm_pair(x, y, mult: float, weight, bias, eps: float, centred: bool, out=None, next_norm=None) -> None:
+def norm_pair(x, y, mult: float, weight, bias, eps: float, centred: bool, out=None, next_norm=None,
+              settled: bool = False) -> None:
     """x <- x + mult * norm(y) in place (x, y float32 [T, width]; ``centred``: a layer norm with
     ``weight`` and ``bias``, else a root-mean-square norm with ``weight``), and in the same kernel,
     with ``out`` (float32 or bfloat16, rows may be further apart than width): ``next_norm`` =
-    (weight, bias or None, eps, centred) of the new x, or, without ``next_norm``, x itself."""
+    (weight, bias or None, eps, centred) of the new x, or, without ``next_norm``, x itself.
+    ``settled``: the norms' parameters were complete before the kernel ahead in the stream began (a
+    model's are), so they may be read while that still runs."""
     what = "norm_pair"
     _need(x, torch.float32, "x", what)
     _need(y, torch.float32, "y", what)
@@ -1138,7 +1143,8 @@ def norm_pair(x, y, mult: float, weight, bias, eps: float, centred: bool, out=No
     _check(lib().prb_norm_pair(_p(out), 0 if out is None else out.stride(0), _p(x), _p(y), _p(weight),
                                _p(bias), _p(w2), _p(b2), n, width, int(bool(centred)),
                                int(bool(centred2)), mode, float(mult), float(eps), float(eps2),
-                               dtype_code(x.dtype if out is None else out.dtype), _stream()), what)
+                               dtype_code(x.dtype if out is None else out.dtype), int(bool(settled)),
+                               _stream()), what)
 
 
 def tanh_cap(z, cap: float) -> None:

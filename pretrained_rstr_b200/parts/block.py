@@ -313,11 +313,11 @@ class SandwichBlock(Block):
         or a copy in the buffer it is.  True if that has been done."""
         weight, bias, eps, centred = self.norms[name].pair()
         if isinstance(reader, torch.Tensor):
-            ops.norm_pair(x, y, self.mult, weight, bias, eps, centred, out=reader)
+            ops.norm_pair(x, y, self.mult, weight, bias, eps, centred, out=reader, settled=True)
             return True
         following = getattr(reader, "pair", lambda: None)()
         ops.norm_pair(x, y, self.mult, weight, bias, eps, centred,
-                      out=None if following is None else h, next_norm=following)
+                      out=None if following is None else h, next_norm=following, settled=True)
         return following is not None
 
 

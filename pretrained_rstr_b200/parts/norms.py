@@ -26,7 +26,8 @@ class LayerNorm(Norm):
         return self.gamma, self.beta, self.eps, True
 
     def forward(self, ctx, x, out, rows=None) -> None:
-        ops.layernorm(out, x, self.gamma, self.beta, self.eps, rows=rows, status=ctx.status)
+        ops.layernorm(out, x, self.gamma, self.beta, self.eps, rows=rows, status=ctx.status,
+                      settled=True)
 
 
 def _layer_norm(params, store, runtime) -> LayerNorm:

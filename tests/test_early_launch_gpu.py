@@ -8,24 +8,62 @@ from test_kernels_gpu import _ops
 pytestmark = pytest.mark.gpu
 
 
+def _sources(g, n, k, count=8):
+    """Operands of products whose results are the [n, k] tensors to be written."""
+    return [(torch.randn(n, 640, device="cuda", generator=g), torch.randn(k, 640, device="cuda", generator=g))
+            for _ in range(count)]
+
+
+def _write(ops, out, source):
+    """out <- a product, by a kernel that lets its successor start before it has written anything."""
+    ops.gemm_f32(out, source[0], source[1], settled=True)
+
+
+def _compare(write, read, shape, sources):
+    """``read`` directly behind ``write``, for one source after the other, against the two with a
+    synchronisation between them."""
+    wants, outs = ([torch.zeros(shape, device="cuda") for _ in sources] for _ in range(2))
+    for src, want in zip(sources, wants):
+        torch.cuda.synchronize()
+        write(src)
+        torch.cuda.synchronize()
+        read(want)
+    torch.cuda.synchronize()
+    for src, out in zip(sources, outs):
+        write(src)
+        read(out)
+    for out, want in zip(outs, wants):
+        assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("m,n,k", [(8, 768, 768), (3, 2304, 100), (1, 700, 33), (65, 768, 3072), (40, 130, 33)])
 def test_gemm_f32_reads_weights_written_by_the_kernel_before_it(m, n, k):
     ops = _ops()
     g = torch.Generator(device="cuda").manual_seed(n + k)
     a = torch.randn(m, k, device="cuda", generator=g)
-    sources = [torch.randn(n, k, device="cuda", generator=g) for _ in range(8)]
-    wants = []
-    for src in sources:
-        want = torch.empty(m, n, device="cuda")
-        torch.cuda.synchronize()
-        ops.gemm_f32(want, a, src, settled=True)
-        torch.cuda.synchronize()
-        wants.append(want)
     w = torch.zeros(n, k, device="cuda")
-    outs = [torch.empty(m, n, device="cuda") for _ in sources]
-    torch.cuda.synchronize()
-    for src, out in zip(sources, outs):
-        ops.bias_act(w, src, None, None, None)
-        ops.gemm_f32(out, a, w)
-    for out, want in zip(outs, wants):
-        assert torch.equal(out, want)
+    _compare(lambda src: _write(ops, w, src), lambda out: ops.gemm_f32(out, a, w), (m, n), _sources(g, n, k))
+
+
+@pytest.mark.parametrize("rows,width", [(1, 768), (100, 1024), (20, 1600), (3, 2052)])
+def test_layernorm_reads_parameters_written_by_the_kernel_before_it(rows, width):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(rows + width)
+    x = torch.randn(rows, width, device="cuda", generator=g)
+    w = torch.zeros(2, width, device="cuda")
+    _compare(lambda src: _write(ops, w, src), lambda out: ops.layernorm(out, x, w[0], w[1], 1e-5), (rows, width),
+             _sources(g, 2, width))
+
+
+@pytest.mark.parametrize("rows,width", [(1, 768), (100, 1600), (5, 4100)])
+def test_norm_pair_reads_parameters_written_by_the_kernel_before_it(rows, width):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(rows + width)
+    y = torch.randn(rows, width, device="cuda", generator=g)
+    w = torch.zeros(4, width, device="cuda")
+
+    def read(out):                                       # (x is zero at first)
+        ops.norm_pair(out[:rows], y, 0.5, w[0], w[1], 1e-5, True, out=out[rows:],
+                      next_norm=(w[2], w[3], 1e-5, True))
+
+    _compare(lambda src: _write(ops, w, src), read, (2 * rows, width), _sources(g, 4, width))
