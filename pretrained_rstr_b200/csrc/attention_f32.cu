@@ -356,6 +356,7 @@ attention_f32_single_kernel(Args p) {
         s_row[team][x] = row;
         // the first values are asked for with the keys (the rows' addresses are all that they need)
         __syncthreads();
+        // (coherent loads: the launch may be placed while the kernel ahead still writes the step's rows)
         constexpr int VB = 32 / ND;                           // value rows in flight a thread
         float v[VB][ND];
         auto load_values = [&](int j0) {
@@ -365,7 +366,7 @@ attention_f32_single_kernel(Args p) {
 #pragma unroll
                 for (int e = 0; e < ND; ++e) {
                     const int d = x + 64 * e;
-                    v[j][e] = vrow >= 0 && d < hd ? __ldg(p.v_pages + (size_t)vrow * hd + d) : 0.0f;
+                    v[j][e] = vrow >= 0 && d < hd ? __ldcg(p.v_pages + (size_t)vrow * hd + d) : 0.0f;
                 }
             }
         };
@@ -378,7 +379,7 @@ attention_f32_single_kernel(Args p) {
                 float4 kv[16];
 #pragma unroll
                 for (int d = 0; d < 16; ++d)
-                    kv[d] = row >= 0 && d0 + d < hd / 4 ? __ldg(kr + d0 + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    kv[d] = row >= 0 && d0 + d < hd / 4 ? __ldcg(kr + d0 + d) : make_float4(0.f, 0.f, 0.f, 0.f);
                 if (d0 == 0) load_values(0);
 #pragma unroll
                 for (int d = 0; d < 16; ++d)

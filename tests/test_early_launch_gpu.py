@@ -3,7 +3,7 @@ each is launched directly behind a kernel that signals at once and then writes i
 import pytest
 import torch
 
-from test_kernels_gpu import _ops
+from test_kernels_gpu import _ops, _paged_case
 
 pytestmark = pytest.mark.gpu
 
@@ -67,3 +67,26 @@ def test_norm_pair_reads_parameters_written_by_the_kernel_before_it(rows, width)
                       next_norm=(w[2], w[3], 1e-5, True))
 
     _compare(lambda src: _write(ops, w, src), read, (2 * rows, width), _sources(g, 4, width))
+
+
+@pytest.mark.parametrize("heads,kv_heads,dh", [(12, 12, 64), (4, 1, 128), (3, 3, 20)])
+def test_attention_f32_reads_rows_written_by_the_kernel_before_it(heads, kv_heads, dh):
+    ops = _ops()
+    lengths = [250, 129, 64, 33, 7, 1]
+    q, k, v, table, seq, pos = _paged_case(5, heads, kv_heads, dh, 64, lengths, [1] * len(lengths), torch.float32)
+    t = len(lengths)
+    g = torch.Generator(device="cuda").manual_seed(dh)
+    held = torch.cat([table[b, torch.arange(n, device="cuda") // 64] * 64 + torch.arange(n, device="cuda") % 64
+                      for b, n in enumerate(lengths)]).to(torch.int32)          # every slot the requests hold
+    sources = [torch.randn(len(held), 2 * kv_heads * dh, device="cuda", generator=g) for _ in range(8)]
+    tokens, count = torch.arange(t, dtype=torch.int32, device="cuda"), torch.tensor([t], dtype=torch.int32, device="cuda")
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+
+    def write(src):
+        ops.kv_append(k, v, src[:, :kv_heads * dh], src[:, kv_heads * dh:], held, len(held), status)
+
+    def read(out):
+        ops.attention_f32(out, q, k, v, table, seq, pos, count, t, heads, 0.2, None, 256, status, token_list=tokens)
+
+    _compare(write, read, tuple(q.shape), sources)
+    assert status.tolist() == [0, 0, 0, 0]
