@@ -164,7 +164,8 @@ __global__ void gated_pair_kernel(O* __restrict__ out, long out_ld, int out_col,
 }
 
 // The same, four neighbouring columns a thread (16-byte loads; n, the columns' offsets, the
-// row pitches and the group all multiples of 4).
+// row pitches and the group all multiples of 4).  Coherent loads: the launch may be placed while the
+// kernel ahead still writes what this one reads.
 template <typename O>
 __global__ void gated_pair4_kernel(O* __restrict__ out, long out_ld, int out_col,
                                    const float* __restrict__ in, long in_ld, int gate_col, int up_col,
@@ -177,9 +178,9 @@ __global__ void gated_pair4_kernel(O* __restrict__ out, long out_ld, int out_col
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)n_rows * n4) return;
     const int t = (int)(idx / n4), i = (int)(idx - (size_t)t * n4) * 4;
-    const float4 g4 = *reinterpret_cast<const float4*>(in + (size_t)t * in_ld + gate_col + i);
-    const float4 u4 = *reinterpret_cast<const float4*>(in + (size_t)t * in_ld + up_col + i);
-    const float sc = scale ? scale[(size_t)t * scale_ld + i / group] : 1.0f;
+    const float4 g4 = __ldcg(reinterpret_cast<const float4*>(in + (size_t)t * in_ld + gate_col + i));
+    const float4 u4 = __ldcg(reinterpret_cast<const float4*>(in + (size_t)t * in_ld + up_col + i));
+    const float sc = scale ? __ldcg(scale + (size_t)t * scale_ld + i / group) : 1.0f;
     float g[4] = {g4.x, g4.y, g4.z, g4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w}, v[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {

@@ -90,3 +90,18 @@ def test_attention_f32_reads_rows_written_by_the_kernel_before_it(heads, kv_head
 
     _compare(write, read, tuple(q.shape), sources)
     assert status.tolist() == [0, 0, 0, 0]
+
+
+@pytest.mark.parametrize("rows,n", [(1, 2048), (24, 3072)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gated_pair_reads_what_the_kernel_before_it_wrote(rows, n, dtype):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    pair = torch.zeros(rows, 2 * n + 64, device="cuda")                 # gate, up, a scale for 64 columns each
+    half = torch.empty(rows, n, device="cuda", dtype=dtype)
+
+    def read(out):
+        ops.gated_pair(half, pair, 0, n, n, scale=pair[:, 2 * n:], group=64)
+        out.copy_(half)
+
+    _compare(lambda src: _write(ops, pair, src), read, (rows, n), _sources(g, rows, 2 * n + 64))
