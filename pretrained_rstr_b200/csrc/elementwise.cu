@@ -342,7 +342,7 @@ fetch_step_kernel(int* __restrict__ dev, const int* __restrict__ host, int words
                 prb_set_status(status, PRB_S_ROW_RANGE, i - tokens_at, k, n_prev);
                 x = 0;
             } else {
-                x = prev[k];
+                x = __ldcg(prev + k);      // (coherent: written while this grid was there already)
             }
         }
         dev[i] = x;

@@ -272,6 +272,7 @@ __device__ __forceinline__ float column_act(float v, int act) {
     }
 }
 
+// (coherent loads: the launch may be placed while the kernel ahead still writes `in`)
 template <typename O, bool VEC>
 __global__ void act_columns_kernel(O* __restrict__ out, long out_ld, const float* __restrict__ in, long in_ld,
                                    int n, int n_rows, int act) {
@@ -282,13 +283,13 @@ __global__ void act_columns_kernel(O* __restrict__ out, long out_ld, const float
         const int n4 = n / 4;
         if (idx >= (size_t)n_rows * n4) return;
         const int t = (int)(idx / n4), i = (int)(idx - (size_t)t * n4) * 4;
-        const float4 u = *reinterpret_cast<const float4*>(in + (size_t)t * in_ld + i);
+        const float4 u = __ldcg(reinterpret_cast<const float4*>(in + (size_t)t * in_ld + i));
         prb_store4(out + (size_t)t * out_ld + i, column_act(u.x, act), column_act(u.y, act), column_act(u.z, act),
                    column_act(u.w, act));
     } else {
         if (idx >= (size_t)n_rows * n) return;
         const int t = (int)(idx / n), i = (int)(idx - (size_t)t * n);
-        out[(size_t)t * out_ld + i] = prb_from_float<O>(column_act(in[(size_t)t * in_ld + i], act));
+        out[(size_t)t * out_ld + i] = prb_from_float<O>(column_act(__ldcg(in + (size_t)t * in_ld + i), act));
     }
 }
 }  // namespace

@@ -392,7 +392,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         uint8_t* my_stage = warp_stage + (size_t)lane * 128;         // this thread's row
         const int rd_row = lane >> 3, rd_piece = lane & 7;           // the way back: row within four, piece
         float4 pb;                                          // prefetched bias of the lane's four columns
-        float4 pr[F32 ? 8 : 1];                             // prefetched residual (float32 output)
+        float4 pr[F32 ? 8 : 1];                             // prefetched residual (float32 output; coherent
+                                                            // loads: the kernel ahead may still write it)
         auto prefetch = [&](int row0, int ncol) {
             // (pieces the fast path will not use, or that do not exist, read as zero)
             const int col = ncol + rd_piece * 4;
@@ -404,7 +405,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 for (int it = 0; it < 8; ++it) {
                     const int rr = row0 + it * 4 + rd_row;
                     pr[it] = (there && resid != nullptr && rr < m)
-                                 ? *reinterpret_cast<const float4*>(resid + (size_t)rr * ldc + col)
+                                 ? __ldcg(reinterpret_cast<const float4*>(resid + (size_t)rr * ldc + col))
                                  : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
             }
@@ -564,7 +565,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                             float x = __uint_as_float(r[j]);
                             if (bias) x += __ldg(bias + ncol + j);
                             x = epilogue_act(x, act);
-                            if (rrow) x += rrow[j];
+                            if (rrow) x += __ldcg(rrow + j);
                             crow[j] = prb_from_float<O>(x);
                             if (sc.kv_width != 0 && ncol + j >= sc.q_width) {
                                 O* dst = scatter_dst<O>(sc, ncol + j, sc.slots[row], row, status);
@@ -680,7 +681,7 @@ gemm_bf16_splitk_kernel(const __grid_constant__ CUtensorMap map_a,
             for (int i = 0; i < RPW; ++i) {
                 const int row = m0 + rank * RPC + (warp - 2) + 8 * i;
                 pre_r[i][j] = (resid && col < n && row < m && (warp - 2) + 8 * i < RPC)
-                                  ? resid[(size_t)row * ldc + col] : 0.0f;
+                                  ? __ldcg(resid + (size_t)row * ldc + col) : 0.0f;
             }
         }
     }

@@ -105,3 +105,27 @@ def test_gated_pair_reads_what_the_kernel_before_it_wrote(rows, n, dtype):
         out.copy_(half)
 
     _compare(lambda src: _write(ops, pair, src), read, (rows, n), _sources(g, rows, 2 * n + 64))
+
+
+@pytest.mark.parametrize("rows,n", [(1, 2048), (24, 3072), (5, 1030)])
+def test_act_columns_reads_what_the_kernel_before_it_wrote(rows, n):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.zeros(rows, n, device="cuda")
+    _compare(lambda src: _write(ops, x, src), lambda out: ops.act_columns(out, x), (rows, n),
+             _sources(g, rows, n))
+
+
+@pytest.mark.parametrize("m,n,k", [(300, 768, 768), (1200, 1600, 512), (130, 1027, 768), (280, 768, 3072)])
+def test_gemm_bf16_reads_the_residual_the_kernel_before_it_wrote(m, n, k):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    a = torch.randn(m, k, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(n, k, device="cuda", generator=g).to(torch.bfloat16)
+    x = torch.zeros(m, n, device="cuda")
+
+    def read(out):
+        ops.gemm_bf16(x, a, w, resid=x)
+        out.copy_(x)
+
+    _compare(lambda src: _write(ops, x, src), read, (m, n), _sources(g, m, n))
