@@ -217,7 +217,8 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
                 issued = pi + STAGES + 1;
             }
         }
-        if (alive) alive = mbar_wait(full0 + 8 * st, (uint32_t)(i / STAGES) & 1u, failed);
+        // (one answer for the warp: what follows are its instructions, not its lanes')
+        if (alive) alive = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * st, (uint32_t)(i / STAGES) & 1u, failed));
         if (i == 0) MT_TRACE(1);
         if (i == items - 1) MT_TRACE(2);
         if (alive) {
@@ -250,6 +251,7 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
     MT_TRACE(3);
     // ---- the rows of this CTA's partial tile to the CTAs that finish them
     const int per = (MROWS + S - 1) / S;                  // rows of a CTA
+    __syncwarp();
     cluster_wait();
     {
         const int g = lane >> 2, q = lane & 3;

@@ -1,0 +1,24 @@
+"""Rules of the CUDA sources that only a failure on the device would show, checked in the text."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "pretrained_rstr_b200", "csrc")
+
+
+def _code(name):
+    """A source without its comments."""
+    with open(os.path.join(CSRC, name)) as fh:
+        return re.sub(r"//[^\n]*|/\*.*?\*/", "", fh.read(), flags=re.S)
+
+
+def test_warps_meet_before_the_aligned_cluster_barrier_of_the_split_product():
+    """barrier.cluster.*.aligned wants whole warps: in the cluster split-K product a bounded wait may
+    end differently for a warp's lanes, so the answer is the warp's and the warp meets again."""
+    kernel = _code("gemm_bf16_midm.cu").split("gemm_midm_kernel(Args", 1)[1].split("midm_smem()", 1)[0]
+    assert re.search(r"alive = __all_sync\(0xffffffffu, mbar_wait\(", kernel)
+    for barrier in ("cluster_wait();", "cluster_arrive();"):
+        for before in kernel.split(barrier)[:-1]:
+            last = [line.strip() for line in before.strip().split("\n") if not line.strip().startswith("MT_TRACE")][-1]
+            assert last in ("__syncwarp();", "cluster_arrive();", "prb_grid_launch_dependents();"), last
