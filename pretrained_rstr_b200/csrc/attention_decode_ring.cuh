@@ -431,8 +431,9 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
         ++pairs_done;
     };
 
+    int u = u_begin;
 #pragma unroll 1
-    for (int u = u_begin; u < u_end && alive; ++u) {
+    for (; u < u_end; ++u) {
         if (u - batch0 >= 32) {                      // on to the next 32 units (decoded when the
             mine = ahead;                            // first of them was requested)
             mine_bad = __ballot_sync(0xffffffffu, mine.bad);
@@ -613,10 +614,10 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
     }
     if (alive && cur_idx >= 0) finish_pair();
     if (!alive) {
-        // a wait gave up: wait once more, bounded, for this warp's own copies in flight
-        for (int s = 0; s < stages; ++s)
-            for (uint32_t i = 0; i < (1u << 16); ++i)
-                if (mbar_try_wait(bar0 + 8 * s, 0) || mbar_try_wait(bar0 + 8 * s, 1)) break;
+        // the wait for unit u gave up: wait once more, bounded, for this warp's own copies in flight
+        for (int v = u; v < min(u_end, u + stages); ++v)
+            for (uint32_t i = 0; i < RING_WAIT_LIMIT; ++i)
+                if (mbar_try_wait(bar0 + 8 * ((v - u_begin) % stages), (uint32_t)((v - u_begin) / stages) & 1u)) break;
     }
     RING_TRACE(5);
     __syncthreads();                                  // every warp's edge states are in place

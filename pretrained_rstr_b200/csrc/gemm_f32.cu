@@ -163,6 +163,7 @@ gemm_f32_stream_kernel(Args p, StreamGeo g, const __grid_constant__ CUtensorMap 
     const int m0 = blockIdx.y * MB;
     const int n_stages = (n1 - n0 + g.rows - 1) / g.rows;
     bool alive = true;
+    int issued = 0;                                           // stages thread 0 has asked for
     if (COPY == COPY_TMA) {
         if (tid == 0) {
             for (int s = 0; s < g.stages; ++s) mbar_init(smem_u32(&bars[s]), 1);
@@ -183,6 +184,7 @@ gemm_f32_stream_kernel(Args p, StreamGeo g, const __grid_constant__ CUtensorMap 
                     "[%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(ws + (size_t)(s % g.stages) * g.stage_len)),
                     "l"(&map_w), "r"(bar), "r"(0), "r"(0), "r"(n0 + s * g.rows)
                     : "memory");
+                ++issued;
             }
         } else {
             if (s < n_stages) {
@@ -280,6 +282,7 @@ gemm_f32_stream_kernel(Args p, StreamGeo g, const __grid_constant__ CUtensorMap 
             }
         }
         __syncthreads();
+        if (COPY == COPY_TMA) alive = alive && !*failed;      // one thread that gave up is enough
         load_stage(s + g.stages);
         // four threads an output, a run of chunk sums each
         for (int t0 = 0; t0 < g.rows * MB * 4; t0 += STREAM_THREADS) {
@@ -303,9 +306,9 @@ gemm_f32_stream_kernel(Args p, StreamGeo g, const __grid_constant__ CUtensorMap 
     if constexpr (COPY == COPY_TMA) {
         if (tid == 0 && !alive) {
             prb_set_status(p.status, PRB_S_WAIT_TIMEOUT, 40, blockIdx.x, blockIdx.y);
-            for (int s = 0; s < g.stages; ++s)                // (copies in flight, bounded)
-                for (uint32_t i = 0; i < (1u << 16); ++i)
-                    if (mbar_try_wait(smem_u32(&bars[s]), 0) || mbar_try_wait(smem_u32(&bars[s]), 1)) break;
+            for (int s = max(0, issued - g.stages); s < issued; ++s)       // copies in flight, bounded
+                for (uint32_t i = 0; i < tc5::WAIT_LIMIT; ++i)
+                    if (mbar_try_wait(smem_u32(&bars[s % g.stages]), (uint32_t)(s / g.stages) & 1u)) break;
         }
     } else {
         cp_wait<0>();

@@ -22,3 +22,10 @@ def test_warps_meet_before_the_aligned_cluster_barrier_of_the_split_product():
         for before in kernel.split(barrier)[:-1]:
             last = [line.strip() for line in before.strip().split("\n") if not line.strip().startswith("MT_TRACE")][-1]
             assert last in ("__syncwarp();", "cluster_arrive();", "prb_grid_launch_dependents();"), last
+
+
+@pytest.mark.parametrize("name", sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))))
+def test_a_wait_names_the_phase_it_waits_for(name):
+    """A barrier answers at once for one of the two parities: a loop that takes either waits for nothing,
+    and a kernel that gave up would leave with copies on their way into its shared memory."""
+    assert not re.search(r"try_wait\([^;]*,\s*0\)\s*\|\|[^;]*try_wait\([^;]*,\s*1\)", _code(name))
