@@ -469,7 +469,8 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
         const int idx = cur_idx, h = cur_h, t = cur_t, pos = cur_pos, lo = cur_lo, blk = cur_blk++;
         // most units lie wholly inside what the query sees: nothing to mask there
         const bool whole = !bad && blk * UNIT >= lo && blk * UNIT + UNIT - 1 <= pos;
-        if (!mbar_wait_bounded(bar0 + 8 * slot, parity)) {
+        // (one answer for the warp: what follows are its instructions, not its lanes')
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar0 + 8 * slot, parity))) {
             if (lane == 0) prb_set_status(a.status, PRB_S_WAIT_TIMEOUT, 32, cta, u);
             alive = false;
             break;

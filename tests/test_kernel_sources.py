@@ -24,6 +24,12 @@ def test_warps_meet_before_the_aligned_cluster_barrier_of_the_split_product():
             assert last in ("__syncwarp();", "cluster_arrive();", "prb_grid_launch_dependents();"), last
 
 
+def test_a_warp_of_the_ring_attention_has_one_answer_to_a_wait():
+    """Its loop goes on with shuffles and matrix instructions of whole warps: a lane may not leave alone."""
+    waits = re.findall(r"if \(!(.*)mbar_wait_bounded", _code("attention_decode_ring.cuh"))
+    assert waits and all(w == "__all_sync(0xffffffffu, " for w in waits)
+
+
 @pytest.mark.parametrize("name", sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))))
 def test_a_wait_names_the_phase_it_waits_for(name):
     """A barrier answers at once for one of the two parities: a loop that takes either waits for nothing,
