@@ -174,7 +174,11 @@ attention_f32_tile_kernel(Args p) {
     for (int i = 0; i < TQ; ++i)
         if (s_pos[i] >= 0) { last = max(last, s_pos[i]); first = min(first, s_lo[i]); }
     const int g0 = last < 0 ? 0 : first / GROUP;
-    const int n_groups = last < 0 ? 0 : last / GROUP - g0 + 1;
+    int n_groups = last < 0 ? 0 : last / GROUP - g0 + 1;
+    if (n_groups > p.slots * size) {                          // not consecutive tokens: no room for their keys
+        if (tid == 0 && rank == 0) prb_set_status(p.status, PRB_S_POSITION_RANGE, row0, last, p.max_context);
+        n_groups = 0;                                         // (the same for the whole cluster; zeros are written)
+    }
     const int c_first = first / CHUNK, c_last = last / CHUNK;  // chunks anyone sees
 
     // this CTA's chunks in order: step i is chunk i % 4 of its group i / 4

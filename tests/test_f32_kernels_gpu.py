@@ -94,3 +94,28 @@ def test_attention_f32_records_what_is_out_of_range():
     assert bool(torch.isfinite(out[1:21]).all())
     assert not ops.attention_f32_supports(130, 1024, None) and not ops.attention_f32_supports(62, 1024, None)
     assert ops.attention_f32_supports(64, 1024, None)
+
+
+@pytest.mark.parametrize("window,far,context", [(70, 900, 1024), (300, 4000, 4096), (20, 260, 512), (600, 30000, 32768)])
+def test_attention_f32_refuses_a_tile_whose_tokens_are_not_consecutive(window, far, context):
+    """A windowed tile is planned for the keys that consecutive tokens see; positions further apart are
+    recorded and leave zeros, and the tile beside it is as it is alone."""
+    ops = _ops()
+    q, k, v, table, seq, pos = _paged_case(6, 2, 2, 16, 64, [context, 300], [20, 20], torch.float32)
+    pos[:20] = torch.arange(10, 30, device="cuda")
+    pos[19] = far
+    ints = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")  # noqa: E731
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    out, alone = torch.full_like(q, float("nan")), torch.full_like(q, float("nan"))
+    ops.attention_f32(alone, q, k, v, table, seq, pos, ints([1]), 1, 2, 0.3, window, context, status,
+                      tiles=(ints([20]), ints([20])))
+    assert status.tolist() == [0, 0, 0, 0]
+    ops.attention_f32(out, q, k, v, table, seq, pos, ints([2]), 2, 2, 0.3, window, context, status,
+                      tiles=(ints([0, 20]), ints([20, 20])))
+    room = -(-window // 256) + 2                                        # groups of 256 keys
+    groups = far // 256 + 1
+    if groups > -(-room // min(room, 8)) * min(room, 8):
+        assert status.tolist() == [2, 0, far, context] and float(out[:20].abs().max()) == 0.0
+    else:
+        assert status.tolist() == [0, 0, 0, 0] and bool(torch.isfinite(out[:20]).all())
+    assert torch.equal(out[20:], alone[20:])
