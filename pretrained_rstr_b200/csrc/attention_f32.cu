@@ -104,15 +104,18 @@ __device__ __forceinline__ void fma2(float& accx, float& accy, float ax, float a
         : "+f"(accx), "+f"(accy) : "f"(ax), "f"(ay), "f"(bx), "f"(by));
 }
 
-// (m, l, o) joined by a later part (mc, lc, oc); a part without a visible key changes nothing
+// (m, l, o) joined by a later part (mc, lc, oc).  A part without a visible key (no weight) changes
+// nothing; a part of keys whose scores are no numbers has no maximum either, but no sum: it makes
+// the sum none (and the result zero, as one walk over all keys does).  A part whose weight vanishes
+// beside the other contributes nothing, whatever its values are.
 template <int N>
 __device__ __forceinline__ void join(float& m, float& l, float (&o)[N], float mc, float lc, const float (&oc)[N]) {
-    if (mc == -INFINITY) return;
+    if (mc == -INFINITY && lc == 0.0f) return;
     const float mn = fmaxf(m, mc);
     const float sa = expf(m - mn), sb = expf(mc - mn);
     l = l * sa + lc * sb;
 #pragma unroll
-    for (int i = 0; i < N; ++i) o[i] = o[i] * sa + oc[i] * sb;
+    for (int i = 0; i < N; ++i) o[i] = (sa == 0.0f ? 0.0f : o[i] * sa) + (sb == 0.0f ? 0.0f : oc[i] * sb);
     m = mn;
 }
 

@@ -119,3 +119,45 @@ def test_attention_f32_refuses_a_tile_whose_tokens_are_not_consecutive(window, f
     else:
         assert status.tolist() == [0, 0, 0, 0] and bool(torch.isfinite(out[:20]).all())
     assert torch.equal(out[20:], alone[20:])
+
+
+@pytest.mark.parametrize("n", [1, 64, 65, 257, 300])
+@pytest.mark.parametrize("what", ["last key", "a chunk of keys", "query", "infinite value of no weight",
+                                  "infinite value far below", "infinite score", "lowest scores"])
+def test_attention_f32_of_values_that_are_no_numbers(n, what):
+    """What is not finite reaches a result as it does in the kernel that walks all keys at once."""
+    ops = _ops()
+    q, k, v, table, seq, pos = _paged_case(7, 2, 2, 16, 64, [n], [min(n, 40)], torch.float32)
+    at = lambda j: (int(table[0, j // 64]), slice(None), j % 64)  # noqa: E731
+    if what == "last key":
+        k[at(n - 1)] = float("nan")
+    elif what == "a chunk of keys":
+        k[int(table[0, 0])] = float("nan")
+    elif what == "query":
+        q[0, 3] = float("nan")
+    elif what == "infinite value of no weight":
+        q[:] = 1.0
+        k[at(0)] = -1e20
+        v[at(0)] = float("inf")
+    elif what == "infinite value far below":
+        q[:] = 1.0
+        k[:] = 0.0
+        k[int(table[0, 0])] = -40.0                     # (a whole chunk e^-192 below the next)
+        v[at(0)] = float("inf")
+    elif what == "infinite score":
+        q[:] = 1.0
+        k[at(n // 2)] = float("inf")
+    else:
+        q[:] = 1.0
+        k[:] = -torch.finfo(torch.float32).max
+    t = q.shape[0]
+    ints = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")  # noqa: E731
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    want = torch.empty_like(q)
+    ops.attention_generic(want, q, k, v, table, seq, pos, t, 2, 0.3, None, 512, status)
+    for lists, count in ((dict(tiles=(ints([0]), ints([t]))), 1),
+                         (dict(token_list=torch.arange(t, dtype=torch.int32, device="cuda")), t)):
+        out = torch.empty_like(q)
+        ops.attention_f32(out, q, k, v, table, seq, pos, ints([count]), count, 2, 0.3, None, 512, status, **lists)
+        assert torch.allclose(out, want, rtol=1e-5, atol=1e-6, equal_nan=True)
+    assert status.tolist() == [0, 0, 0, 0]
