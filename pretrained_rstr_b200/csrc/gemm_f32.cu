@@ -545,7 +545,8 @@ PRB_API int prb_gemm_f32(float* c, const float* a, const float* w, const float* 
         StreamGeo g;
         size_t smem;
         int mb = m == 1 ? 1 : m == 2 ? 2 : m <= 4 ? 4 : 8;
-        const int copy = !vec ? COPY_4 : k % CH == 0 && k / CH <= 256 ? COPY_TMA : COPY_16;
+        // (rows that overlap, an expanded row for one, are no tensor that a copy engine's map describes)
+        const int copy = !vec ? COPY_4 : k % CH == 0 && k / CH <= 256 && ldw >= k ? COPY_TMA : COPY_16;
         while (mb > 1 && !stream_geometry(p, mb, copy, &g, &smem)) mb /= 2;
         if (stream_geometry(p, mb, copy, &g, &smem) && (m + mb - 1) / mb <= 65535) {
             switch (mb) {

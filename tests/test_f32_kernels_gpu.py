@@ -34,6 +34,20 @@ def test_gemm_f32_kernels_give_the_same_bits(m, n, k):
         assert torch.equal(out[0], other)
 
 
+@pytest.mark.parametrize("m", [1, 7, 16, 40])
+@pytest.mark.parametrize("pitch", [0, 4, 64, 100, 132])
+def test_gemm_f32_of_weight_rows_that_overlap_or_lie_apart(m, pitch):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(pitch)
+    n, k = 300, 96
+    a = torch.randn(m, k, device="cuda", generator=g)
+    w = torch.randn(n * 132 + k, device="cuda", generator=g).as_strided((n, k), (pitch, 1))
+    out, want = (torch.full((m, n), float("nan"), device="cuda") for _ in range(2))
+    ops.gemm_f32(out, a, w)
+    ops.gemm_f32(want, a, w.clone(memory_format=torch.contiguous_format))
+    assert torch.equal(out, want)
+
+
 CASES = [
     # heads, kv heads, head size, page size, window
     (12, 12, 64, 64, None), (4, 4, 16, 16, None), (6, 2, 64, 64, 70), (5, 1, 48, 32, 300),
