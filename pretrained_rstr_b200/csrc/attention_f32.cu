@@ -450,9 +450,11 @@ attention_f32_single_kernel(Args p) {
     cluster_sync_all();
 }
 
-template <typename K>
-int launch(K kernel, const Args& a, dim3 grid, int threads, size_t smem, cudaStream_t stream) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+constexpr size_t MOST_SMEM = 220 * 1024;
+
+template <auto Kernel>
+int launch(const Args& a, dim3 grid, int threads, size_t smem, cudaStream_t stream) {
+    cudaError_t e = prb_allow_shared<Kernel>((int)MOST_SMEM);
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -470,7 +472,7 @@ int launch(K kernel, const Args& a, dim3 grid, int threads, size_t smem, cudaStr
         prb_pdl_enabled() && (long)grid.x * grid.y * grid.z <= 2L * prb_sm_count() ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    e = cudaLaunchKernelEx(&cfg, kernel, a);
+    e = cudaLaunchKernelEx(&cfg, Kernel, a);
     return e == cudaSuccess ? 0 : (int)e;
 }
 
@@ -498,7 +500,7 @@ Plan plan(int max_context, int window) {
 // 1 when the kernels take these sizes (else the caller uses prb_attention_generic).
 PRB_API int prb_attention_f32_supports(int head_dim, int max_context, int window) {
     if (head_dim < 4 || head_dim % 4 != 0 || head_dim > 128 || max_context <= 0) return 0;
-    return tile_smem(head_dim, plan(max_context, window).slots) <= 220 * 1024 ? 1 : 0;
+    return tile_smem(head_dim, plan(max_context, window).slots) <= MOST_SMEM ? 1 : 0;
 }
 
 // Attention of the step's tokens: those in tiles (`tiles` true: n_list tiles of up to 128 tokens,
@@ -525,14 +527,14 @@ PRB_API int prb_attention_f32(float* out, long out_stride, const float* q, long 
     if (tile_row0 != nullptr) {
         const size_t smem = tile_smem(head_dim, a.slots);
         dim3 grid(n_list * (128 / TQ), n_heads, z);
-        const int rc = head_dim <= 64 ? launch(attention_f32_tile_kernel<1>, a, grid, TILE_THREADS, smem, stream)
-                                      : launch(attention_f32_tile_kernel<2>, a, grid, TILE_THREADS, smem, stream);
+        const int rc = head_dim <= 64 ? launch<attention_f32_tile_kernel<1>>(a, grid, TILE_THREADS, smem, stream)
+                                      : launch<attention_f32_tile_kernel<2>>(a, grid, TILE_THREADS, smem, stream);
         if (rc) return rc;
     } else {
         const size_t smem = single_smem(head_dim, a.slots);
         dim3 grid(n_list, n_heads, z);
-        const int rc = head_dim <= 64 ? launch(attention_f32_single_kernel<1>, a, grid, THREADS, smem, stream)
-                                      : launch(attention_f32_single_kernel<2>, a, grid, THREADS, smem, stream);
+        const int rc = head_dim <= 64 ? launch<attention_f32_single_kernel<1>>(a, grid, THREADS, smem, stream)
+                                      : launch<attention_f32_single_kernel<2>>(a, grid, THREADS, smem, stream);
         if (rc) return rc;
     }
     return 0;

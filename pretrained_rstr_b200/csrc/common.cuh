@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #define PRB_API extern "C" __attribute__((visibility("default")))
 
 // argument errors (host side)
@@ -179,6 +181,19 @@ template <typename... KArgs, typename... Args>
 inline cudaError_t prb_launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block,
                                         size_t smem, cudaStream_t stream, Args... args) {
     return prb_launch_maybe_early(true, kernel, grid, block, smem, stream, args...);
+}
+
+// Lets `Kernel` ask for up to `bytes` (the same in every call) of dynamic shared memory: once per kernel
+// and device, since the call costs the host as much as a small launch.
+template <auto Kernel> inline cudaError_t prb_allow_shared(int bytes) {
+    static std::atomic<unsigned long long> done{0};              // a bit a device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 64 && ((done.load(std::memory_order_acquire) >> dev) & 1)) return cudaSuccess;
+    e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && dev < 64) done.fetch_or(1ull << dev, std::memory_order_release);
+    return e;
 }
 
 #define PRB_LAUNCH_CHECK()                               \

@@ -461,11 +461,11 @@ gemm_f32_tile_kernel(Args p) {
     cluster_sync_all();                                       // nobody leaves while its tile is read
 }
 
-template <int BM, int BN, int TM, int TN>
-int launch_tile(const Args& p, bool vec, cudaStream_t stream) {
+template <int BM, int BN, int TM, int TN, bool VEC>
+int launch_tile_by(const Args& p, cudaStream_t stream) {
     using Cfg = TileCfg<BM, BN, TM, TN>;
-    auto kernel = vec ? gemm_f32_tile_kernel<BM, BN, TM, TN, true> : gemm_f32_tile_kernel<BM, BN, TM, TN, false>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
+    constexpr auto kernel = gemm_f32_tile_kernel<BM, BN, TM, TN, VEC>;
+    cudaError_t e = prb_allow_shared<kernel>((int)Cfg::SMEM);
     if (e != cudaSuccess) return (int)e;
     dim3 grid(4 * ((p.n + BN - 1) / BN), (p.m + BM - 1) / BM);
     if (grid.y > 65535) return PRB_E_SIZE;
@@ -473,26 +473,38 @@ int launch_tile(const Args& p, bool vec, cudaStream_t stream) {
     return e == cudaSuccess ? 0 : (int)e;
 }
 
-template <int MB>
-int launch_stream(const Args& p, StreamGeo g, int copy, size_t smem, cudaStream_t stream) {
+template <int BM, int BN, int TM, int TN>
+int launch_tile(const Args& p, bool vec, cudaStream_t stream) {
+    return vec ? launch_tile_by<BM, BN, TM, TN, true>(p, stream) : launch_tile_by<BM, BN, TM, TN, false>(p, stream);
+}
+
+constexpr size_t STREAM_SMEM = 220 * 1024;                    // the most a launch of the stream kernel takes
+
+template <int MB, int COPY>
+int launch_stream_by(const Args& p, StreamGeo g, size_t smem, cudaStream_t stream) {
     CUtensorMap map = {};
-    if (copy == COPY_TMA) {
+    if (COPY == COPY_TMA) {
         const int rc = chunk_map(p.w, p.n, p.k, p.ldw, g.rows, &map);
         if (rc) return rc;
     }
-    auto kernel = copy == COPY_TMA  ? gemm_f32_stream_kernel<MB, COPY_TMA>
-                  : copy == COPY_16 ? gemm_f32_stream_kernel<MB, COPY_16>
-                                    : gemm_f32_stream_kernel<MB, COPY_4>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr auto kernel = gemm_f32_stream_kernel<MB, COPY>;
+    cudaError_t e = prb_allow_shared<kernel>((int)STREAM_SMEM);
     if (e != cudaSuccess) return (int)e;
     dim3 grid((p.n + g.rows_per_cta - 1) / g.rows_per_cta, (p.m + MB - 1) / MB);
     e = prb_launch_maybe_early(p.settled, kernel, grid, dim3(STREAM_THREADS), smem, stream, p, g, map);
     return e == cudaSuccess ? 0 : (int)e;
 }
 
+template <int MB>
+int launch_stream(const Args& p, StreamGeo g, int copy, size_t smem, cudaStream_t stream) {
+    return copy == COPY_TMA  ? launch_stream_by<MB, COPY_TMA>(p, g, smem, stream)
+           : copy == COPY_16 ? launch_stream_by<MB, COPY_16>(p, g, smem, stream)
+                             : launch_stream_by<MB, COPY_4>(p, g, smem, stream);
+}
+
 // The stream kernel's geometry for `mb` rows of A a CTA; false if it does not fit.
 bool stream_geometry(const Args& p, int mb, int copy, StreamGeo* g, size_t* smem) {
-    const size_t budget = 220 * 1024;
+    const size_t budget = STREAM_SMEM;
     const int sms = prb_sm_count();
     const int mt = mb < 4 ? mb : 4;
     g->nc = (p.k + CH - 1) / CH;

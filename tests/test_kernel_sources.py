@@ -35,3 +35,10 @@ def test_a_wait_names_the_phase_it_waits_for(name):
     """A barrier answers at once for one of the two parities: a loop that takes either waits for nothing,
     and a kernel that gave up would leave with copies on their way into its shared memory."""
     assert not re.search(r"try_wait\([^;]*,\s*0\)\s*\|\|[^;]*try_wait\([^;]*,\s*1\)", _code(name))
+
+
+@pytest.mark.parametrize("name", ["gemm_f32.cu", "attention_f32.cu"])
+def test_no_launch_sets_a_kernel_attribute(name):
+    """cudaFuncSetAttribute costs the host as much as a launch of the small kernels of a decode step."""
+    code = _code(name)
+    assert "cudaFuncSetAttribute" not in code and "prb_allow_shared<" in code
