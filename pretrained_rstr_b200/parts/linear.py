@@ -18,6 +18,27 @@ import torch
 from ..csrc import ops
 
 
+def cluster_product(m: int, n_out: int, n_in: int, sms: int) -> bool:
+    """Whether a product of ``m`` rows goes to the kernel that splits the reduction over a
+    thread-block cluster (of the tensor-memory kernel and that one).
+
+    Narrow outputs and long reductions do at 17 to 64 rows: their tiles are too few for the SMs.
+    Wide outputs do up to 32 rows, where two CTAs or more share a tile of 64 columns and the weights
+    are up to 4 M numbers.  Measured, us of norm, product and the next product together, tensor-memory
+    kernel / this one, at 17, 32, 48 and 64 rows: 2,304 x 768 14.1 / 12.7, 14.2 / 12.9, 14.8 / 13.9,
+    15.0 / 15.2; 3,072 x 768 14.8 / 14.0, 14.9 / 14.3, 15.4 / 15.7, 15.6 / 17.1; 4,096 x 1,024 17.5 /
+    17.6, 17.9 / 18.3, 18.5 / 19.4, 19.6 / 21.1; 3,840 x 1,280 (4.9 M) level up to 32 rows, 21.7 / 23.7
+    at 64; without a split 5,120 x 768 16.5 / 18.4, 16.9 / 20.1, 17.4 / 22.4, 17.6 / 24.8.  Whole decode
+    steps at 250 and 900 tokens of context, ms: GPT-2 small, 24 requests (32 rows) 0.521 / 0.500 and
+    0.647 / 0.624, 64 requests 0.588 / 0.613 and 0.885 / 0.897; medium, 24: 1.169 / 1.136 and 1.489 /
+    1.438, 48: 1.293 / 1.380 and 1.883 / 1.949."""
+    if not 16 < m <= 64:
+        return False
+    if n_out <= 2048 or n_in >= 4 * n_out:
+        return True
+    return m <= 32 and -(-n_out // 64) * 2 <= sms and n_out * n_in <= 4096 * 1024
+
+
 class Linear:
     def __init__(self, weight: torch.Tensor, bias: Optional[torch.Tensor], runtime):
         if weight.dim() != 2:
@@ -63,17 +84,12 @@ class Linear:
             return False
         # Which kernel (measured on GPT-2 small and XL shapes): up to 16 rows
         # the weight-streaming kernel with the norm fused into it; 17 to 64 rows the cluster
-        # split-K kernel for small weights, narrow outputs and long reductions, the tensor-memory
-        # kernel for wide outputs (the register-streaming kernel where K is no multiple of 64);
+        # split-K kernel where :func:`cluster_product` says so, else the tensor-memory
+        # kernel (the register-streaming kernel where K is no multiple of 64);
         # beyond 64 rows the tensor-memory kernel.
         max_rows, max_norm = ops.smallm_limits()
-        if 16 < m <= 64 and (self.n_out <= 2048 or self.n_in >= 4 * self.n_out or
-                             self.n_out * self.n_in <= 4096 * 1024) and \
+        if cluster_product(m, self.n_out, self.n_in, ops.sm_count()) and \
                 ops.midm_supports(m, self.n_out, self.n_in):
-            # a few dozen rows: the reduction split over a thread-block cluster.  Weights of up to
-            # 4 M numbers at any shape (us at 32 / 64 rows, tensor-memory kernel / this one: 2,304 x
-            # 768 10.1 / 4.6 and 10.0 / 5.3, 4,096 x 1,024 7.6 / 6.5 and 7.5 / 7.1), larger ones
-            # where the output is narrow or the reduction long (4,800 x 1,600: 10.9 / 12.6)
             scatters = kv_scatter is not None and resid is None and kv_scatter[0].dtype == out.dtype
             ops.gemm_midm(out, _tensor(a), self.weight, self.bias, resid, act, status=ctx.status,
                           kv_scatter=kv_scatter if scatters else None)
