@@ -112,27 +112,27 @@ PRB_API int prb_attention_decode_ring_max_list() { return MAX_LIST; }
 
 // Whether this kernel is the faster one for a launch of n_list tokens over contexts of up to
 // max_context keys; the split-key kernel of attention_decode.cu is the other.  Measured inside
-// whole decode steps (ms a step, split-key / ring; n_list is the capacity the step's graph
-// was made for, so 24 requests run as 32 and 48 as 64).  GPT-2 small, 12 heads: 1 request 0.372
-// / 0.364 at context 256 and 0.366 / 0.366 at 1,000; 8 requests 0.358 / 0.391 (500) and 0.417 /
-// 0.437 (1,000); 12 requests 0.540 / 0.524 and 16 requests 0.545 / 0.544 (1,000), 16 requests
-// 0.502 / 0.507 (320) and 0.561 / 0.541 (576); 32 requests 0.586 / 0.578 (250), 0.691 / 0.660
-// (320), 0.821 / 0.717 (576), 0.884 / 0.776 (1,000); 24 as 32: 0.709 / 0.726; 40: 0.875 / 0.859;
-// 48: 0.881 / 0.895; 56: 1.121 / 0.947; 64 requests 0.620 / 0.646 (250), 0.719 / 0.730 (320),
-// 0.899 / 0.858 (576), 1.140 / 0.992 (1,000).  Medium, 16 heads: 16 requests 1.360 / 1.305
-// (1,000); 32 requests 1.633 / 1.487 (250).  XL, 25 heads: 8 requests 2.55 / 2.75 (1,000); 16
-// requests 3.99 / 3.80 (1,000) and 2.80 / 2.83 (250).
+// whole decode steps, ms a step, split-key / ring, at contexts of 250, 500 and 900 tokens (n_list is
+// the capacity the step's graph was made for, so 24 requests run as 32 and 48 as 64).
+// GPT-2 small, 12 heads: 1 request 0.326 / 0.332, 0.330 / 0.334, 0.348 / 0.351; 8: 0.338 / 0.354,
+// 0.347 / 0.373, 0.390 / 0.395; 16: 0.422 / 0.453, 0.469 / 0.468, 0.537 / 0.515; 32: 0.536 / 0.523,
+// 0.607 / 0.581, 0.747 / 0.663; 64: 0.589 / 0.618, 0.782 / 0.736, 1.037 / 0.889.  Medium, 16 heads:
+// 1: 0.680 / 0.719, 0.685 / 0.724, 0.717 / 0.722; 16: 0.940 / 0.938, 1.053 / 1.071, 1.326 / 1.195; 32:
+// 1.285 / 1.181, 1.536 / 1.351, 1.696 / 1.578; 64: 1.429 / 1.303, 1.715 / 1.692, 2.246 / 2.074.  XL, 25
+// heads: 1: 1.895 / 2.029, 1.921 / 2.086, 2.068 / 2.113; 8: 1.994 / 2.161, 2.192 / 2.309, 2.493 / 2.483;
+// 16: 2.841 / 2.826, 3.190 / 3.140, 3.769 / 3.591; 32: 3.728 / 3.777, 4.479 / 4.172, 5.393 / 4.848.  An
+// engine of 320 requests, small, up to 200, 600 and 990 tokens: 65: 0.815 / 0.855, 1.120 / 1.077,
+// 1.326 / 1.213; 128: 1.209 / 1.207, 1.661 / 1.590, 1.995 / 1.837; 256: 2.434 / 2.440, 3.220 / 3.047, 3.782 /
+// 3.528.
 // The ring wins where many (token, head) pairs have long contexts (its warps stream long runs,
-// the other kernel's CTAs walk their keys one batch after the other), in the middle range at
-// every context, and at a single request with a short context (everything it reads is
-// requested before the dependency resolves and one CTA holds a whole pair).
+// the other kernel's CTAs walk their keys one batch after the other) and in the middle range at
+// nearly every context; it loses at few requests.
 PRB_API int prb_attention_decode_ring_prefers(int n_list, int n_heads, int max_context) {
     const long pairs = (long)n_list * n_heads;
     const long sms = prb_sm_count();
     if (pairs >= 4 * sms) return max_context > 512;
     if (pairs >= 2 * sms) return 1;
-    if (pairs >= sms) return n_list >= 16 && max_context > 512;
-    return pairs * 8 <= sms && max_context <= 512;
+    return pairs >= sms && n_list >= 16 && max_context > 512;
 }
 
 // Floats of workspace a launch of up to n_list tokens needs.

@@ -65,3 +65,13 @@ def test_an_engine_of_many_requests_by_either_decode_attention(tmp_path, monkeyp
     # (two layers whose attention is rounded to bfloat16 in other places)
     assert float((results[1] - results[0]).abs().max()) <= 0.1 * size
     assert float((results[2] - results[0]).abs().max()) <= 0.1 * size
+
+
+def test_few_requests_take_the_split_key_attention():
+    """A request or eight by the ring kernel: 1 to 8 % more a decode step, at every context and size."""
+    ops = _ops()
+    for heads in (12, 16, 25):
+        for context in (64, 256, 512, 1024):
+            assert not ops.decode_ring_prefers(1, heads, context)
+            assert not ops.decode_ring_prefers(8, 12, context)
+    assert ops.decode_ring_prefers(32, 12, 1024) and ops.decode_ring_prefers(256, 12, 1024)
