@@ -12,9 +12,9 @@
 //           of a 128 x 64 tile of A and a BN x 64 tile of W per pipeline stage;
 //   warp 1  allocates TMEM; one thread issues tcgen05.mma (M=128, N=BN, K=16, four per
 //           stage) and commits each stage back to the producer through an mbarrier;
-//   warps 2-9  epilogue: tcgen05.ld the accumulator (one row per thread, two warps per
-//           32-lane quarter taking alternate 32-column chunks), add bias, apply the
-//           activation, add the residual, store.
+//   the rest  epilogue, eight or sixteen warps: tcgen05.ld the accumulator (one row per thread,
+//           the two or four warps of a 32-lane quarter taking 32-column chunks in turn), add
+//           bias, apply the activation, add the residual, store.
 // Rows of A beyond M, rows of W beyond N and the K tail are zero-filled by TMA; stores
 // are masked.  K and the row pitches must be multiples of 8 elements (TMA needs 16-byte
 // strides); other sizes are refused with PRB_E_ALIGN, never computed wrongly.
@@ -77,11 +77,20 @@ constexpr int UMMA_K = 16;
 // Epilogue warps: 16 for bfloat16 tiles of 128 columns and more (four to a quarter of the tensor
 // memory's lanes; with eight, an activation's arithmetic did not hide behind the next tile: 2,193 x
 // 6,400 x 1,600 with GELU 46.1 -> 40.0 us), eight for narrower ones, which have no chunk for more
-// (137 x 3,072 x 768 in tiles of 64: 6.4 against 7.0 us), and for float32 output, where a thread
+// (137 x 3,072 x 768 in tiles of 64: 6.4 against 7.0 us), for float32 output, where a thread
 // holds a chunk's residual values beside the next chunk's (sixteen warps leave it no registers for
 // that: 2,048 x 3,072 x 768 14.7 -> 17.4 us).
-template <typename O, int BN> constexpr int epi_warps = sizeof(O) == 4 || BN < 128 ? 8 : 16;
-template <typename O, int BN> constexpr int gemm_threads = 64 + 32 * epi_warps<O, BN>;   // + producer, MMA
+template <typename O, int BN> constexpr int most_epi_warps = sizeof(O) == 4 || BN < 128 ? 8 : 16;
+// Sixteen take 16 KB of the ring, which costs tiles of 224 columns their fourth stage and pairs on 192
+// their sixth.  Without an activation to hide, the stage is worth more than the warps (us with
+// sixteen / eight: 224 columns 650 x 4,800 x 1,600 18.0 / 16.2, 2,048 x 4,800 x 1,600 40.0 / 33.7, 1,000 x
+// 3,840 x 1,280 14.7 / 14.3; pairs on 192 2,048 x 4,800 x 1,600 28.4 / 26.7, 2,193 x 5,120 x 1,280 28.7 /
+// 28.2); with one, only over a long reduction in tiles of 224 (600 x 6,400 x 1,600 with GELU 20.5 / 19.6,
+// 1,500 x 5,120 x 1,280 25.7 / 25.6, 2,193 x 4,864 x 768 24.7 / 29.4; pairs on 192 2,048 x 6,400 x 1,600
+// 38.0 / 39.7).
+template <typename O, int BN, bool PAIR>
+constexpr bool stage_before_warps = sizeof(O) == 2 && (PAIR ? BN == 192 : BN == 224);
+constexpr int gemm_threads(int epi_warps) { return 64 + 32 * epi_warps; }     // + producer, MMA
 constexpr int SPLIT_THREADS = 320;     // the split-K kernel's: 8 epilogue warps
 
 using namespace tc5;
@@ -183,13 +192,12 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
 // (tcgen05.commit ... multicast::cluster).  Each CTA finishes its own 128 rows.  A CTA thus
 // takes in half the bytes of W per multiply-add: the main loop of a 128 x 128 tile is bound
 // by what one SM can take in from the L2, not by its tensor core.
-template <int BN, typename O, bool PAIR>
-__global__ void __launch_bounds__(gemm_threads<O, BN>, 1)
+template <int BN, typename O, bool PAIR, int EPI_WARPS>
+__global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                  O* __restrict__ c, const float* __restrict__ bias,
                  const float* __restrict__ resid, int m, int n, int k, long ldc, int act,
                  int* status, Scatter sc) {
-    constexpr int EPI_WARPS = epi_warps<O, BN>;
     using Cfg = TileCfg<BN, PAIR, EPI_WARPS>;
     extern __shared__ uint8_t smem_raw[];
     // tiles need 1024-byte alignment for the 128-byte swizzle
@@ -805,14 +813,14 @@ gemm_bf16_splitk_kernel(const __grid_constant__ CUtensorMap map_a,
 // ------------------------------------------------------------------ host side
 using tmap::get_map;
 
-template <int BN, typename O>
-int launch(const CUtensorMap& ma, const CUtensorMap& mw, O* c, const float* bias,
+template <int BN, typename O, int EPI>
+int launch_as(const CUtensorMap& ma, const CUtensorMap& mw, O* c, const float* bias,
            const float* resid, int m, int n, int k, long ldc, int act, int* status,
            const Scatter& sc, cudaStream_t stream) {
-    using Cfg = TileCfg<BN, false, epi_warps<O, BN>>;
+    using Cfg = TileCfg<BN, false, EPI>;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, O, false>,
+        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, O, false, EPI>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)Cfg::SMEM);
         if (e != cudaSuccess) return (int)e;
@@ -821,22 +829,22 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mw, O* c, const float* bias
     const int sm_count = prb_sm_count();
     const long tiles = (long)((n + BN - 1) / BN) * ((m + BM - 1) / BM);
     const int grid = (int)(tiles < sm_count ? tiles : sm_count);
-    cudaError_t le = prb_launch_dependent(gemm_bf16_kernel<BN, O, false>, dim3(grid),
-                                          dim3(gemm_threads<O, BN>), Cfg::SMEM, stream, ma, mw, c, bias,
+    cudaError_t le = prb_launch_dependent(gemm_bf16_kernel<BN, O, false, EPI>, dim3(grid),
+                                          dim3(gemm_threads(EPI)), Cfg::SMEM, stream, ma, mw, c, bias,
                                           resid, m, n, k, ldc, act, status, sc);
     if (le != cudaSuccess) return (int)le;
     return 0;
 }
 
 // CTA pairs on 256 x BN tiles: clusters of two CTAs, as many as tiles or as pairs of SMs.
-template <int BN, typename O>
-int launch_pair(const CUtensorMap& ma, const CUtensorMap& mw, O* c, const float* bias,
+template <int BN, typename O, int EPI>
+int launch_pair_as(const CUtensorMap& ma, const CUtensorMap& mw, O* c, const float* bias,
                 const float* resid, int m, int n, int k, long ldc, int act, int* status,
                 const Scatter& sc, cudaStream_t stream) {
-    using Cfg = TileCfg<BN, true, epi_warps<O, BN>>;
+    using Cfg = TileCfg<BN, true, EPI>;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, O, true>,
+        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, O, true, EPI>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)Cfg::SMEM);
         if (e != cudaSuccess) return (int)e;
@@ -846,7 +854,7 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mw, O* c, const float*
     const long pairs = prb_sm_count() / 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs)));
-    cfg.blockDim = dim3(gemm_threads<O, BN>);
+    cfg.blockDim = dim3(gemm_threads(EPI));
     cfg.dynamicSmemBytes = Cfg::SMEM;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -858,10 +866,27 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mw, O* c, const float*
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_bf16_kernel<BN, O, true>, ma, mw, c, bias, resid,
+    cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_bf16_kernel<BN, O, true, EPI>, ma, mw, c, bias, resid,
                                         m, n, k, ldc, act, status, sc);
     if (le != cudaSuccess) return (int)le;
     return 0;
+}
+
+template <int BN, typename O>
+int launch(const CUtensorMap& ma, const CUtensorMap& mw, O* c, const float* bias, const float* resid, int m,
+           int n, int k, long ldc, int act, int* status, const Scatter& sc, cudaStream_t stream) {
+    if constexpr (stage_before_warps<O, BN, false>)
+        if (act == PRB_ACT_NONE || k > 1280)
+            return launch_as<BN, O, 8>(ma, mw, c, bias, resid, m, n, k, ldc, act, status, sc, stream);
+    return launch_as<BN, O, most_epi_warps<O, BN>>(ma, mw, c, bias, resid, m, n, k, ldc, act, status, sc, stream);
+}
+template <int BN, typename O>
+int launch_pair(const CUtensorMap& ma, const CUtensorMap& mw, O* c, const float* bias, const float* resid, int m,
+                int n, int k, long ldc, int act, int* status, const Scatter& sc, cudaStream_t stream) {
+    if constexpr (stage_before_warps<O, BN, true>)
+        if (act == PRB_ACT_NONE)
+            return launch_pair_as<BN, O, 8>(ma, mw, c, bias, resid, m, n, k, ldc, act, status, sc, stream);
+    return launch_pair_as<BN, O, most_epi_warps<O, BN>>(ma, mw, c, bias, resid, m, n, k, ldc, act, status, sc, stream);
 }
 
 template <int BN, int S, typename O>

@@ -40,3 +40,24 @@ def test_gemm_midm_scatters_keys_and_values_to_the_cache(m, heads, kv_heads, dh,
     assert status.tolist() == [0, 0, 0, 0]
     with pytest.raises(ops.KernelArgumentError):
         ops.gemm_midm(torch.zeros(m, n, device="cuda"), a, w, kv_scatter=(k3, v3, slots, q_width))
+
+
+@pytest.mark.parametrize("tile_n,pair", [(224, False), (192, True)])
+@pytest.mark.parametrize("m,n,k", [(129, 230, 64), (300, 1000, 1280), (257, 449, 1288), (650, 4800, 1600)])
+@pytest.mark.parametrize("act", [None, "gelu"])
+def test_gemm_bf16_with_eight_or_sixteen_epilogue_warps(tile_n, pair, m, n, k, act):
+    """The tiles whose epilogue has eight warps or sixteen, by activation and reduction."""
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    a = torch.randn(m, k, device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn(n, k, device="cuda", generator=g) / k ** 0.5).to(torch.bfloat16)
+    bias = torch.randn(n, device="cuda", generator=g)
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    out = torch.full((m, n + 8 - n % 8), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.gemm_bf16(out[:, :n], a, w, bias=bias, act=act, tile_n=tile_n, pair=pair, status=status)
+    ref = a.double() @ w.double().t() + bias.double()
+    if act:
+        ref = torch.nn.functional.gelu(ref)
+    # bfloat16 rounds once (2^-9 of the value); the 32-bit sum of k products of size 1 / sqrt(k)
+    assert bool(((out[:, :n].double() - ref).abs() <= 2.0 ** -8 * ref.abs().clamp(min=0.25)).all())
+    assert bool(torch.isnan(out[:, n:]).all()) and status.tolist() == [0, 0, 0, 0]
