@@ -81,9 +81,10 @@ def test_attention_f32(nh, nkv, dh, ps, window):
                                                                                      device="cuda")))):
         # (bounds on the context of one and of two to eight groups of keys: another split, same bits)
         ops.attention_f32(out, q, k, v, table, seq, pos, count, n, nh, 0.3, window, 1024, status, **lists)
-        again = torch.full_like(q, float("nan"))
-        ops.attention_f32(again, q, k, v, table, seq, pos, count, n, nh, 0.3, window, 4000, status, **lists)
-        assert torch.equal(out, again)
+        for bound in [4000] + ([window, window + 1] if window else []):   # (windowed: positions lie behind it)
+            again = torch.full_like(q, float("nan"))
+            ops.attention_f32(again, q, k, v, table, seq, pos, count, n, nh, 0.3, window, bound, status, **lists)
+            assert torch.equal(out, again)
     assert status.tolist() == [0, 0, 0, 0]
     assert torch.equal(by_tile, single)
     ref = _ref_attention(q, k, v, table, seq, pos, nh, 0.3, window)
@@ -126,9 +127,9 @@ def test_attention_f32_refuses_a_tile_whose_tokens_are_not_consecutive(window, f
     assert status.tolist() == [0, 0, 0, 0]
     ops.attention_f32(out, q, k, v, table, seq, pos, ints([2]), 2, 2, 0.3, window, context, status,
                       tiles=(ints([0, 20]), ints([20, 20])))
-    room = -(-window // 256) + 2                                        # groups of 256 keys
-    groups = far // 256 + 1
-    if groups > -(-room // min(room, 8)) * min(room, 8):
+    room = (window + 31 + 254) // 256 + 1                # groups of 256 keys that 32 tokens' windows touch
+    ctas = min(room, 8, context // 256)
+    if far // 256 + 1 > -(-room // ctas) * ctas:
         assert status.tolist() == [2, 0, far, context] and float(out[:20].abs().max()) == 0.0
     else:
         assert status.tolist() == [0, 0, 0, 0] and bool(torch.isfinite(out[:20]).all())
