@@ -415,12 +415,6 @@ template <int NB> int active_clusters(int splits) {
 }
 }  // namespace
 
-// Clusters of `splits` CTAs with tiles of `nb` columns that run at a time.
-PRB_API int prb_gemm_midm_active_clusters(int nb, int splits) {
-    if (splits < 1 || splits > 8) return 0;
-    return nb == 64 ? active_clusters<64>(splits) : active_clusters<32>(splits);
-}
-
 // 1 when the kernel takes these sizes (else the caller uses another product kernel).
 PRB_API int prb_gemm_midm_supports(int m, int n, int k) {
     return m >= 1 && m <= MROWS && n >= 1 && k >= 64 && k % 64 == 0 ? 1 : 0;
