@@ -2,9 +2,9 @@
 // split into fixed ranges of absolute positions so that a single token still fills the
 // GPU, partial results merged in split order.
 //
-// Grid (token list, head, split).  Split s owns positions [s*SPLIT, (s+1)*SPLIT), a
-// multiple of the page size, so what a split sums and in which order depends only on
-// the token's own visible range [lo, pos], never on the batch.  Each warp takes the
+// Grid (token list, head, split).  Split s owns positions [s * split, (s + 1) * split), split a
+// multiple of SPLIT keys and of the page size that the launch chooses, so what a split sums and in
+// which order depends on the token's own visible range [lo, pos] and that choice alone.  Each warp takes the
 // keys of the split in turn, 32/LPK keys per load (LPK lanes share one key row, 16 bytes
 // each), keeps a running maximum and sum (online softmax, float32) and accumulates
 // weighted values; warps are merged through shared memory, splits through a float32
@@ -99,12 +99,12 @@ cudaError_t launch_decode(K kernel, dim3 grid, int cluster_z, cudaStream_t strea
 PRB_API int prb_attention_decode_split() { return SPLIT; }
 PRB_API int prb_attention_decode_max_split_pages() { return MAX_SPLIT_PAGES; }
 
-// Switch (for measurements): 0 = splits always merge through the workspace.
 // Switch (for measurements): -1 = the streaming variant where it is chosen, 0 = never,
 // 1 = wherever it applies.
 static int g_decode_stream = -1;
 static int prb_decode_stream() { return g_decode_stream; }
 PRB_API void prb_attention_decode_set_stream(int mode) { g_decode_stream = mode; }
+// Switch (for measurements): 0 = splits always merge through the workspace.
 static int g_decode_clusters = 1;
 static int prb_decode_clusters() { return g_decode_clusters; }
 PRB_API void prb_attention_decode_set_clusters(int on) { g_decode_clusters = on ? 1 : 0; }

@@ -154,9 +154,9 @@ __device__ __forceinline__ void st_first_cta(float* local, float v) {
 
 // The cluster's first CTA merges the splits s_first..s_last in split order from its own shared
 // memory, where their CTAs have written (maximum, sum, weighted values); the arithmetic is that
-// of the workspace merge.  (It used to read them from the other CTAs' shared memory one after the
-// other, 24 remote round trips for eight splits and a second cluster barrier: a layer of GPT-2 small 24.7
-// -> 23.9 us at one request, 30.3 -> 29.1 at eight.)
+// of the workspace merge.  (Reading them from the other CTAs' shared memory one after the other is 24
+// remote round trips for eight splits and a second cluster barrier: a layer of GPT-2 small 24.7 us
+// at one request and 30.3 at eight, 23.9 and 29.1 so.)
 template <int NW, int DH>
 __device__ __forceinline__ void merge_cluster(const Args& a, int t, int h, int s_first, int s_last,
                                               const Shared<NW, DH, true>& sh) {

@@ -19,10 +19,13 @@
 //   attention_f32_single_kernel  one query; four teams of 64 threads take a chunk each, straight
 //                                from memory (a thread a key, then a thread a dimension): what
 //                                counts is that a group's 128 KB are requested at once
-// One thread block a (token, head) walking all keys with a thread a key, which came before,
-// bounded both: 8 requests left most SMs idle, and a prompt read every key again for each query.
-// 8 requests of about 100 tokens, 12 heads: 44 -> 8.5 us a launch (a chain of look-ups: list, place
-// of the token, page, keys, values); prompts of 650 tokens together: 376 -> 94 us.
+// With one thread block a (token, head) that walks all keys (attention_generic.cu) 8 requests leave
+// most SMs idle, and a prompt reads every key again for each query.  8 requests of about 100 tokens,
+// 12 heads: 8.5 us a launch (a chain of look-ups: list, place of the token, page, keys, values), 44
+// that way; prompts of 650 tokens together 94 us, 376 that way.  Contexts or prompts of some 20
+// tokens are where that way is the faster one (12 heads: 64 requests of 10 tokens 7.6 us, here 19.0; a
+// prompt of 17 8.3 and 18.3): a group's CTA takes its rounds whatever it holds, and the order of sums
+// has to be the same for all of a model's steps.
 #include "common.cuh"
 
 namespace {

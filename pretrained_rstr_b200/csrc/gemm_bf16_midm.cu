@@ -9,10 +9,11 @@
 // the r-th part of K (A and W slices come by TMA through a ring of shared-memory stages,
 // 128-byte swizzle, mma.sync m16n8k16 with ldmatrix) and writes row i of its partial tile to
 // the shared memory of CTA i mod S, which after one cluster barrier sums its rows' parts in rank
-// order and runs the epilogue for them (bias, activation, residual, store).  (The parts used to
-// be read by their owner after the barrier, a remote round trip and a second barrier more:
-// 768 x 3,072 at 64 rows 8.4 -> 7.2 us in a step without dependent launch.)  S depends on K and N only, and a row's sum is
-// taken in a fixed order, so a row's result does not depend on the batch.
+// order and runs the epilogue for them (bias, activation, residual, store).  (Parts that their owner
+// reads after the barrier cost a remote round trip and a second barrier more: 768 x 3,072 at 64 rows
+// 8.4 us in a step without dependent launch, 7.2 so.)  S depends on K, N and how many clusters the
+// device runs at a time, and a row's sum is taken in a fixed order, so a row's result does not depend
+// on the batch.
 // No TMA load uses cluster multicast.  Every mbarrier wait is bounded: on a timeout the
 // kernel records PRB_S_WAIT_TIMEOUT, stores nothing, waits (bounded) for its copies in
 // flight and leaves through the same cluster barriers as its peers.

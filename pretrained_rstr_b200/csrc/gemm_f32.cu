@@ -4,26 +4,28 @@
 // ONE order of summation for every size, so that a row's result does not depend on how many
 // other rows are in the batch nor on which of the two kernels below computes it: K is cut into
 // chunks of 32; a thread accumulates a chunk's even and its odd k's, each in ascending order, and
-// adds the two (a pair is what fma.rn.f32x2 takes: half the instructions); the chunks are cut into four runs of ceil(chunks / 4), a run's chunk sums are added
-// in ascending order, and the result is (run 0 + run 1) + (run 2 + run 3).  (Closer to the 64-bit
-// product than one chain over all of K, which was here before: 1.0e-7 against 4.9e-7 relative at
-// K = 768, 1.3e-7 against 1.0e-6 at 3,072, normal numbers.)
+// adds the two (a pair is what fma.rn.f32x2 takes: half the instructions); the chunks are cut into
+// four runs of ceil(chunks / 4), a run's chunk sums are added in ascending order, and the result is
+// (run 0 + run 1) + (run 2 + run 3).  (Closer to the 64-bit product than one chain over all of K:
+// 1.0e-7 against 4.9e-7 relative at K = 768, 1.3e-7 against 1.0e-6 at 3,072, normal numbers.)
 //
-// gemm_f32_stream_kernel: up to eight rows a CTA, bound by the weights' way from memory.  Every
-// CTA owns a run of weight rows and requests them through a ring of shared-memory stages
-// (TMA where K is a multiple of
-// 32, else cp.async; the first of them before the kernel ahead has ended); a thread keeps its chunk of up
-// to four rows of A in registers and walks the weight rows of a stage, so an FMA costs a quarter
-// of a shared-memory operand; chunk sums meet in shared memory.  8 rows, weights from memory:
-// 2,304 x 768 6.8 us, 768 x 3,072 10.4 us, 50,257 x 768 72 us = 2.15 TB/s; the kernel before (64 x
-// 64 tiles, one CTA a tile, so 12 CTAs for 768 columns) took 177 us on average over a model's
-// products.
+// gemm_f32_stream_kernel: up to eight rows a CTA (9 to 16 rows are two groups of CTAs, which read the
+// weights each), bound by the weights' way from memory.  Every CTA owns a run of weight rows and
+// requests them through a ring of shared-memory stages (TMA where K is a multiple of 32, else
+// cp.async; the first of them, where the caller says that the weights are settled, before the kernel
+// ahead has ended); a thread keeps its chunk of up to four rows of A in registers and walks the
+// weight rows of a stage, so an FMA costs a quarter of a shared-memory operand; chunk sums meet in
+// shared memory.  8 rows, weights from memory: 2,304 x 768 6.8 us, 768 x 3,072 10.4 us, 50,257 x 768
+// 72 us = 2.15 TB/s; one CTA a tile of 64 x 64 (12 CTAs for 768 columns) takes 177 us on average over
+// a model's products.
 //
-// gemm_f32_tile_kernel: more rows, bound by FMA issue and the shared-memory reads beside it.  Tiles of BM x BN, the four runs of K by
-// the four CTAs of a cluster (a prompt of a few hundred tokens has too few tiles for 148 SMs
-// otherwise), partial tiles added through distributed shared memory, a quarter of the rows a CTA.
-// 650 rows: 2,304 x 768 76 us, 768 x 3,072 106 us, 50,257 x 768 1.49 ms = 34 TFLOP/s (about 14
-// before).
+// gemm_f32_tile_kernel: more rows.  Tiles of BM x BN, the four runs of K by the four CTAs of a cluster
+// (a prompt of a few hundred tokens has too few tiles for 148 SMs otherwise), partial tiles added
+// through distributed shared memory, a quarter of the rows a CTA.  650 rows: 2,304 x 768 76 us, 768 x
+// 3,072 106 us, 50,257 x 768 1.49 ms = 34 TFLOP/s; one CTA a tile over all of K 14 TFLOP/s.  What bounds
+// it: 255 registers leave two CTAs of four warps an SM, whose schedulers issue in 42 % of the cycles
+// (an instruction every 4.35 cycles a warp: 1.2 of fixed latency, 0.5 for the FMA pipe, 0.4 for shared
+// memory); neither the FMA units nor shared memory are half busy (counters at 650 x 2,304 x 768).
 #include "common.cuh"
 #include "tcgen05.cuh"
 #include "tensor_map.cuh"
