@@ -541,7 +541,8 @@ def midm_supports(m: int, n: int, k: int) -> bool:
 def gemm_midm(out, a, w, bias=None, resid=None, act=None, status=None, kv_scatter=None) -> None:
     """out[M,N] = act(a[M,K] . w[N,K]^T + bias) (+ resid) for up to 64 rows, K a multiple of
     64: the reduction is split over a thread-block cluster (``csrc/gemm_bf16_midm.cu``).
-    ``kv_scatter`` as in :func:`gemm_bf16`."""
+    ``kv_scatter`` as in :func:`gemm_bf16`.  ``w`` may be read while the kernel ahead in the stream
+    still runs: it has to be complete before that began, as a model's weights are."""
     what = "gemm_midm"
     for name, t in (("a", a), ("w", w)):
         if not t.is_cuda or t.dtype != torch.bfloat16 or t.stride(1) != 1:
@@ -595,7 +596,9 @@ def gemm_smallm(out, w, a=None, norm_input=None, gamma=None, beta=None, eps=0.0,
     of X is the norm of row norm_rows[t] of ``norm_input`` (an index outside it gives a zero
     row and is recorded in ``status``).  ``kv_scatter`` = (k_pages, v_pages,
     slots, q_width): the product is a fused QKV projection; its key and value columns are also
-    written to the paged cache (same element type as ``out``) at each token's slot."""
+    written to the paged cache (same element type as ``out``) at each token's slot.  ``w``, ``gamma``
+    and ``beta`` may be read while the kernel ahead in the stream still runs: they have to be
+    complete before that began, as a model's are."""
     what = "gemm_smallm"
     if not w.is_cuda or w.dtype != torch.bfloat16 or w.stride(1) != 1:
         raise KernelArgumentError(f"{what}: w must be bfloat16 on CUDA with unit inner stride")
