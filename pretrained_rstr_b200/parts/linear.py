@@ -88,7 +88,7 @@ class Linear:
         # kernel (the register-streaming kernel where K is no multiple of 64);
         # beyond 64 rows the tensor-memory kernel.
         max_rows, max_norm = ops.smallm_limits()
-        if cluster_product(m, self.n_out, self.n_in, ops.sm_count()) and \
+        if 16 < m <= 64 and cluster_product(m, self.n_out, self.n_in, ops.sm_count()) and \
                 ops.midm_supports(m, self.n_out, self.n_in):
             scatters = kv_scatter is not None and resid is None and kv_scatter[0].dtype == out.dtype
             ops.gemm_midm(out, _tensor(a), self.weight, self.bias, resid, act, status=ctx.status,
