@@ -66,13 +66,18 @@ attention_decode_ring_kernel(RingArgs a, const __grid_constant__ CUtensorMap map
     prb_grid_launch_dependents();                   // the next kernel may set itself up
     const uint32_t ring_base = (smem_addr(ring_raw) + 1023u) & ~1023u;
     if (threadIdx.x < RING_WARPS) sh.bars_valid[threadIdx.x] = 0;
+    if (threadIdx.x == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
+    }
     plan(a, sh);
     RING_TRACE(1);
-    early(a, &map_k, &map_v, sh, ring_base, (int)gridDim.x, (int)blockIdx.x);
+    LaneUnit mine;
+    const Run run = early(a, &map_k, &map_v, sh, ring_base, (int)gridDim.x, (int)blockIdx.x, mine);
     RING_TRACE(2);
     prb_grid_wait();
     RING_TRACE(3);
-    late(a, &map_k, &map_v, sh, ring_base, (int)gridDim.x, (int)blockIdx.x);
+    late(a, &map_k, &map_v, sh, ring_base, (int)blockIdx.x, run, mine);
 }
 
 int launch_ring(const RingArgs& a, const CUtensorMap& mk, const CUtensorMap& mv, int grid, int warps,

@@ -8,7 +8,10 @@
 //            (depends only on what was on the device before the step began);
 //   early()  every warp works out its run of units and requests as many of them as it has ring
 //            buffers, except units that hold rows the step itself writes when those rows are
-//            not handed over beside the queries (also independent of the step's kernels);
+//            not handed over beside the queries (also independent of the step's kernels).  Where
+//            the product ahead leaves no room beside it, plan() and early() are waited for: their
+//            look-ups are in parallel where they can be, their divisions are of 32 bits and the
+//            tensor maps are asked for first.
 //   late()   after the dependency has resolved: queries, the step's own rows, scores, values,
 //            the merge inside the CTA and across CTAs.
 #pragma once
@@ -28,6 +31,7 @@ constexpr int ROW = DH * 2;                   // bytes of a row
 constexpr int TILE = UNIT * ROW;              // bytes of a unit's keys (and of its values)
 constexpr int MAX_LIST = 256;                 // most single tokens of a launch
 constexpr int MAX_STAGES = 4;
+constexpr int MERGE = 6;                      // CTAs' states a merging warp asks for at once
 constexpr int PART = DH + 4;                  // floats of a partial state: values, maximum, sum
 constexpr uint32_t RING_WAIT_LIMIT = 1u << 22;
 
@@ -66,7 +70,6 @@ struct Shared {
     int n;                          // places of the token list in use
     int warp_tot[RING_WARPS];
     unsigned long long bars[RING_WARPS * MAX_STAGES];
-    unsigned bad_mask[RING_WARPS];  // units (of a warp's first 32) with a page outside the pool
     int bars_valid[RING_WARPS];     // barriers of each warp that hold a valid object (0 at first:
                                     // whoever owns this struct clears it once, before early())
     // what a warp leaves for the merge: the state of the first and of the last (token, head)
@@ -148,13 +151,13 @@ __device__ __forceinline__ void span_blocks(const RingArgs& a, TokenSpan& s) {
     s.first_blk = s.lo / UNIT;
     s.n_blk = s.pos / UNIT - s.first_blk + 1;
 }
-__device__ __forceinline__ TokenSpan token_span(const RingArgs& a, int idx, int n) {
+__device__ __forceinline__ TokenSpan token_span(const RingArgs& a, int t, bool on) {
     TokenSpan s{-1, -1, 0, 0, 0, 0};
-    if (idx >= n) return s;
-    s.t = a.token_list ? a.token_list[idx] : idx;
+    if (!on) return s;
+    s.t = t;
     s.b = a.seq_of_token[s.t];
+    s.pos = a.positions[s.t];                    // (asked for beside the request)
     if (s.b < 0) return s;
-    s.pos = a.positions[s.t];
     if (s.pos < 0 || s.pos >= a.max_pages * a.page_size) {
         prb_set_status(a.status, PRB_S_POSITION_RANGE, s.t, s.pos, 0);
         s.b = -1;
@@ -178,15 +181,26 @@ __device__ __forceinline__ void merge_into(Partial& acc, float m2, float l2, flo
     acc.m = mn;
 }
 
+// Counts this CTA in among those of a (token, head); returns how many came before it.
+__device__ __forceinline__ int count_in(int* counter) {
+    int before;
+    asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
+    return before;
+}
+
 // ---- plan: units per token and their running sum.  Ends with a barrier of the CTA.
 RING_FN void plan(const RingArgs& a, Shared& sh) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_warps = (int)blockDim.x >> 5;
+    // the list's entries are asked for beside their count; those beyond it are not looked at
+    auto listed = [&](int i) { return a.token_list != nullptr && i < a.n_list ? a.token_list[i] : i; };
+    int t = listed((int)threadIdx.x);
     int n = a.n_list;
     if (a.token_count != nullptr) n = min(n, *a.token_count);
     int run = 0;
     for (int base = 0; base < n; base += (int)blockDim.x) {
-        const TokenSpan s = token_span(a, base + (int)threadIdx.x, n);
+        if (base > 0) t = listed(base + (int)threadIdx.x);
+        const TokenSpan s = token_span(a, t, base + (int)threadIdx.x < n);
         if (base + (int)threadIdx.x < n) {
             sh.span_t[base + threadIdx.x] = s.t;
             sh.span_b[base + threadIdx.x] = s.b;
@@ -223,21 +237,21 @@ RING_FN void plan(const RingArgs& a, Shared& sh) {
 // a (token, head) are mostly warps of one CTA.  With few units the runs are a unit long and
 // only `wpc` warps of every CTA have one, so that the work is spread over all SMs.
 struct Run {
-    long per, wpc, gw;
+    unsigned per, wpc;
     int u_begin, u_end;
 };
 RING_FN Run my_run(const Shared& sh, int n_ctas, int cta) {
-    const int warp = threadIdx.x >> 5, n_warps = (int)blockDim.x >> 5;
+    const unsigned warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     Run r;
-    const long total_units = sh.cum[sh.n];
-    const long workers = (long)n_ctas * n_warps;
-    r.per = total_units > 0 ? (total_units + workers - 1) / workers : 1;
-    const long busy = (total_units + r.per - 1) / r.per;         // workers that have a run
-    r.wpc = min((long)n_warps, max(1L, (busy + n_ctas - 1) / (long)n_ctas));
-    r.gw = (long)cta * r.wpc + warp;
-    const bool has_run = warp < r.wpc && r.gw < busy;
-    r.u_begin = has_run ? (int)(r.gw * r.per) : 0;
-    r.u_end = has_run ? (int)min(total_units, r.gw * r.per + r.per) : 0;
+    const unsigned total_units = (unsigned)sh.cum[sh.n];
+    const unsigned workers = (unsigned)n_ctas * n_warps;
+    r.per = max(1u, (total_units + workers - 1) / workers);
+    const unsigned busy = (total_units + r.per - 1) / r.per;     // workers that have a run
+    r.wpc = min(n_warps, max(1u, (busy + (unsigned)n_ctas - 1) / (unsigned)n_ctas));
+    const unsigned gw = (unsigned)cta * r.wpc + warp;
+    const bool has_run = warp < r.wpc && gw < busy;
+    r.u_begin = has_run ? (int)(gw * r.per) : 0;
+    r.u_end = has_run ? (int)min(total_units, gw * r.per + r.per) : 0;
     return r;
 }
 
@@ -267,10 +281,10 @@ RING_FN LaneUnit decode_unit(const RingArgs& a, const Shared& sh, int u, int u_e
     }
     TokenSpan s{sh.span_t[lo_i], sh.span_b[lo_i], sh.span_pos[lo_i], 0, 0, 0};
     span_blocks(a, s);
-    const int r = u - sh.cum[lo_i];
+    const unsigned r = (unsigned)(u - sh.cum[lo_i]);
     lu.idx = lo_i;
-    lu.h = r / s.n_blk;
-    lu.blk = s.first_blk + r % s.n_blk;
+    lu.h = (int)(r / (unsigned)s.n_blk);
+    lu.blk = s.first_blk + (int)r - lu.h * s.n_blk;
     lu.pos = s.pos; lu.lo = s.lo; lu.t = s.t;
     lu.late = a.k_new == nullptr && lu.blk * UNIT + UNIT > s.pos - a.new_keys + 1;
     return lu;
@@ -329,10 +343,10 @@ __device__ __forceinline__ uint32_t warp_ring(uint32_t ring_base, int stages) {
 }
 
 // ---- early: request what does not depend on the step's kernels.  `n_ctas`, `cta`: how many
-// CTAs share the launch and which one this is.
-RING_FN void early(const RingArgs& a, const CUtensorMap* map_k,
+// CTAs share the launch and which one this is.  Returns the warp's run and in `mine` the lanes' units.
+RING_FN Run early(const RingArgs& a, const CUtensorMap* map_k,
                                       const CUtensorMap* map_v, Shared& sh, uint32_t ring_base,
-                                      int n_ctas, int cta) {
+                                      int n_ctas, int cta, LaneUnit& mine) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int stages = a.stages;
     if (lane == 0) {
@@ -347,36 +361,26 @@ RING_FN void early(const RingArgs& a, const CUtensorMap* map_k,
     const Run r = my_run(sh, n_ctas, cta);
     const uint32_t ring0 = warp_ring(ring_base, stages);
     const uint32_t bar0 = smem_addr(&sh.bars[warp * MAX_STAGES]);
-    LaneUnit mine = decode_unit(a, sh, r.u_begin + lane, r.u_end);
-    if (lane < stages) unit_pages(a, sh, mine);
-    const unsigned bad = __ballot_sync(0xffffffffu, mine.bad);
-    if (lane == 0) sh.bad_mask[warp] = bad;
+    mine = decode_unit(a, sh, r.u_begin + lane, r.u_end);
+    unit_pages(a, sh, mine);
     if (lane < stages && mine.idx >= 0 && !mine.late) issue_unit(a, map_k, map_v, mine, ring0, bar0, lane);
+    return r;
 }
 
 // ---- late: everything that needs the step's queries (and its own keys and values).
 RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
                                      const CUtensorMap* map_v, Shared& sh, uint32_t ring_base,
-                                     int n_ctas, int cta) {
+                                     int cta, const Run& r, LaneUnit& mine) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_warps = (int)blockDim.x >> 5;
     const int stages = a.stages;
-    const Run r = my_run(sh, n_ctas, cta);
     const int u_begin = r.u_begin, u_end = r.u_end;
     const uint32_t ring0 = warp_ring(ring_base, stages);
     const uint32_t bar0 = smem_addr(&sh.bars[warp * MAX_STAGES]);
     const int hpg = a.n_heads / a.kv_heads;          // query heads per key/value head
-    auto cta_of = [&](long u) { return (u / r.per) / r.wpc; };   // the CTA whose warps hold unit u
+    auto cta_of = [&](int u) { return (int)((unsigned)u / r.per / r.wpc); };   // whose warps hold unit u
 
-    // the lanes' units again (from shared memory), the pages of those still to be requested
-    LaneUnit mine = decode_unit(a, sh, u_begin + lane, u_end);
-    {
-        const unsigned bad = sh.bad_mask[warp];
-        if (lane < stages) mine.bad = (bad >> lane) & 1u;
-        const bool need_pages = mine.idx >= 0 && (lane >= stages || mine.late);
-        if (need_pages) unit_pages(a, sh, mine);
-        if (lane < stages && mine.idx >= 0 && mine.late) issue_unit(a, map_k, map_v, mine, ring0, bar0, lane);
-    }
+    if (lane < stages && mine.idx >= 0 && mine.late) issue_unit(a, map_k, map_v, mine, ring0, bar0, lane);
     unsigned mine_bad = __ballot_sync(0xffffffffu, mine.bad);
     LaneUnit ahead = mine;                           // the 32 units after them, once decoded
     bool ahead_ready = false;
@@ -396,6 +400,9 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
     for (int ks = 0; ks < 4; ++ks) qa[ks][0] = qa[ks][1] = 0u;
     int cur_idx = -1, cur_h = -1, cur_t = 0, cur_n_blk = 0, cur_pos = 0, cur_lo = 0, cur_blk = 0;
     int pair_end = u_begin;                          // first unit after the current (token, head)
+    // a row of the step's own keys and values (an eighth of it a lane): which, and where it belongs
+    uint4 own_k = make_uint4(0, 0, 0, 0), own_v = own_k;
+    int own_key = -1;
     int slot = 0;
     uint32_t parity = 0;
     int pairs_done = 0;                              // (token, head)s this warp has left behind
@@ -405,7 +412,7 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
     // in this warp's run it is written out; otherwise it is left in shared memory for the merge
     // (only the first and the last (token, head) of a run can be shared with other warps).
     auto finish_pair = [&]() {
-        const long p_u0 = (long)sh.cum[cur_idx] + (long)cur_h * cur_n_blk, p_u1 = p_u0 + cur_n_blk;
+        const int p_u0 = sh.cum[cur_idx] + cur_h * cur_n_blk, p_u1 = p_u0 + cur_n_blk;
         if (p_u0 >= u_begin && p_u1 <= u_end) {
             const float inv = l > 0.0f ? 1.0f / l : 0.0f;
             __nv_bfloat16* head_out = a.out + (size_t)cur_t * a.out_stride + (size_t)cur_h * DH;
@@ -465,8 +472,25 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
                 qa[ks][0] = row0 ? qp[8 * ks + qd] : 0u;          // dimensions 16 ks + 2 c, + 1
                 qa[ks][1] = row0 ? qp[8 * ks + 4 + qd] : 0u;      // dimensions 16 ks + 8 + 2 c, + 1
             }
+            // rows that the step itself appended: lanes 8 j .. 8 j + 7 bring the row of position
+            // pos - j, if token t - j is that position of the same request (asked for now, beside the
+            // query, and put in when their unit has landed)
+            own_key = -1;
+            if (a.k_new != nullptr) {
+                const int j = lane >> 3, c = lane & 7;
+                const int key = cur_pos - j;
+                const int src = cur_idx - j;         // its place in the token list
+                if (j < a.new_keys && key >= cur_blk * UNIT && key >= cur_lo && src >= 0 &&
+                    (key / UNIT - cur_blk) < u_end - u && sh.span_t[src] == cur_t - j &&
+                    sh.span_b[src] == sh.span_b[cur_idx] && sh.span_pos[src] == key) {
+                    own_key = key;
+                    const size_t off = (size_t)(cur_t - j) * a.kv_stride + (size_t)(cur_h / hpg) * DH + c * 8;
+                    own_k = *reinterpret_cast<const uint4*>(a.k_new + off);
+                    own_v = *reinterpret_cast<const uint4*>(a.v_new + off);
+                }
+            }
         }
-        const int idx = cur_idx, h = cur_h, t = cur_t, pos = cur_pos, lo = cur_lo, blk = cur_blk++;
+        const int pos = cur_pos, lo = cur_lo, blk = cur_blk++;
         // most units lie wholly inside what the query sees: nothing to mask there
         const bool whole = !bad && blk * UNIT >= lo && blk * UNIT + UNIT - 1 <= pos;
         // (one answer for the warp: what follows are its instructions, not its lanes')
@@ -480,20 +504,11 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
         bool wrote = false;                          // rows of the unit's tiles written from here
         if (a.k_new != nullptr && !bad && (blk + 1) * UNIT > pos - a.new_keys + 1) {
             wrote = true;
-            // rows of this unit that the step itself appended: lanes 8 j .. 8 j + 7 bring the
-            // row of position pos - j, if token t - j is that position of the same request
-            const int j = lane >> 3, c = lane & 7;
-            const int key = pos - j;
-            const int src = idx - j;                 // its place in the token list
-            if (j < a.new_keys && key >= blk * UNIT && key < (blk + 1) * UNIT && key >= lo && src >= 0 &&
-                sh.span_t[src] == t - j && sh.span_b[src] == sh.span_b[idx] && sh.span_pos[src] == key) {
-                const int hk = h / hpg, rr = key - blk * UNIT;
-                const size_t off = (size_t)(t - j) * a.kv_stride + (size_t)hk * DH + c * 8;
-                const uint4 kk = *reinterpret_cast<const uint4*>(a.k_new + off);
-                const uint4 vv = *reinterpret_cast<const uint4*>(a.v_new + off);
+            if (own_key >= 0 && own_key / UNIT == blk) {
+                const int rr = own_key - blk * UNIT, c = lane & 7;
                 const uint32_t dst = (uint32_t)rr * ROW + (uint32_t)((c ^ (rr & 7)) << 4);
-                asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(kd + dst), "r"(kk.x), "r"(kk.y), "r"(kk.z), "r"(kk.w) : "memory");
-                asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(vd + dst), "r"(vv.x), "r"(vv.y), "r"(vv.z), "r"(vv.w) : "memory");
+                asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(kd + dst), "r"(own_k.x), "r"(own_k.y), "r"(own_k.z), "r"(own_k.w) : "memory");
+                asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(vd + dst), "r"(own_v.x), "r"(own_v.y), "r"(own_v.z), "r"(own_v.w) : "memory");
             }
             __syncwarp();
         }
@@ -624,39 +639,38 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
     __syncthreads();                                  // every warp's edge states are in place
 
     // ---- merge.  The edge states of the CTA's warps, in warp order, form chains of the same
-    // (token, head); the warp that holds a chain's first state merges it.  A chain that is the
+    // (token, head); the warp that holds a chain's first state merges it: lane 2 w + e looks at state e
+    // of warp w, so that the maximum and the weights of all of them take one round.  A chain that is the
     // whole (token, head) is written out; otherwise it goes to the workspace, and the last CTA
     // of that (token, head) to arrive merges the CTAs' states in CTA order.
+    const int state_w = lane >> 1, state_e = lane & 1;
+    const int state_pair = state_w < n_warps ? sh.edge_pair[state_w][state_e] : -1;
 #pragma unroll 1
     for (int e = 0; e < 2; ++e) {
-        const int pair = sh.edge_pair[warp][e];
+        const int pair = __shfl_sync(0xffffffffu, state_pair, 2 * warp + e);
         if (pair < 0) continue;
-        bool first = true;                            // no earlier state of this pair in the CTA?
-        if (e == 1 && sh.edge_pair[warp][0] == pair) first = false;
-        if (first && warp > 0 && (sh.edge_pair[warp - 1][1] == pair ||
-                                  (sh.edge_pair[warp - 1][1] < 0 && sh.edge_pair[warp - 1][0] == pair)))
-            first = false;
-        if (!first) continue;
-        Partial acc{-INFINITY, 0.0f, 0.0f, 0.0f};
-        bool go = true;
-#pragma unroll 1
-        for (int w = warp; w < n_warps && go; ++w)
-#pragma unroll 1
-            for (int e2 = (w == warp ? e : 0); e2 < 2; ++e2) {
-                if (sh.edge_pair[w][e2] != pair) {
-                    // a warp's second slot may be empty (its run was one (token, head) long)
-                    if (sh.edge_pair[w][e2] < 0 && e2 == 1) continue;
-                    go = false;
-                    break;
-                }
-                const float* st = sh.edge_state[w][e2];
-                merge_into(acc, st[DH], st[DH + 1], st[2 * lane], st[2 * lane + 1]);
-            }
+        const unsigned chain = __ballot_sync(0xffffffffu, state_pair == pair);
+        if (__ffs(chain) - 1 != 2 * warp + e) continue;      // an earlier state of this pair in the CTA
+        const bool in = state_pair == pair;
+        const float sm = in ? sh.edge_state[state_w][state_e][DH] : -INFINITY;
+        const float sl = in ? sh.edge_state[state_w][state_e][DH + 1] : 0.0f;
+        Partial acc;
+        acc.m = prb_warp_max(sm);
+        const float sc = sm == -INFINITY ? 0.0f : __expf(sm - acc.m);
+        acc.l = prb_warp_sum(sl * sc);
+        acc.o0 = acc.o1 = 0.0f;
+        for (unsigned left = chain; left != 0; left &= left - 1) {
+            const int at = __ffs(left) - 1;
+            const float c = __shfl_sync(0xffffffffu, sc, at);
+            const float2 v = *reinterpret_cast<const float2*>(&sh.edge_state[at >> 1][at & 1][2 * lane]);
+            acc.o0 += v.x * c;
+            acc.o1 += v.y * c;
+        }
         const int idx = pair / a.n_heads, h = pair - idx * a.n_heads;
         TokenSpan s{sh.span_t[idx], sh.span_b[idx], sh.span_pos[idx], 0, 0, 0};
         span_blocks(a, s);
-        const long p_u0 = (long)sh.cum[idx] + (long)h * s.n_blk, p_u1 = p_u0 + s.n_blk;
-        const long fc = cta_of(p_u0), lc = cta_of(p_u1 - 1);
+        const int p_u0 = sh.cum[idx] + h * s.n_blk, p_u1 = p_u0 + s.n_blk;
+        const int fc = cta_of(p_u0), lc = cta_of(p_u1 - 1);
         __nv_bfloat16* dst = a.out + (size_t)s.t * a.out_stride + (size_t)h * DH + 2 * lane;
         if (fc == lc) {
             const float inv = acc.l > 0.0f ? 1.0f / acc.l : 0.0f;
@@ -666,28 +680,28 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
         float* part = a.workspace + (size_t)(cta + pair) * PART;
         *reinterpret_cast<float2*>(part + 2 * lane) = make_float2(acc.o0, acc.o1);
         if (lane == 0) { part[DH] = acc.m; part[DH + 1] = acc.l; }
-        __threadfence();
         __syncwarp();
         int last = 0;
-        if (lane == 0) last = atomicAdd(&a.counters[pair], 1) == (int)(lc - fc) ? 1 : 0;
+        // (released: the warp's stores above come before the count; acquired: the others' are seen)
+        if (lane == 0) last = count_in(&a.counters[pair]) == lc - fc ? 1 : 0;
         last = __shfl_sync(0xffffffffu, last, 0);
         if (!last) continue;
-        __threadfence();
+        __syncwarp();
         // the CTAs' states in CTA order (= block order); all loads first, then the sums
         Partial tot{-INFINITY, 0.0f, 0.0f, 0.0f};
 #pragma unroll 1
-        for (long c0 = fc; c0 <= lc; c0 += 4) {
-            float pm[4], pl[4];
-            float2 po[4];
+        for (int c0 = fc; c0 <= lc; c0 += MERGE) {
+            float pm[MERGE], pl[MERGE];
+            float2 po[MERGE];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < MERGE; ++j) {
                 const float* pw = a.workspace + (size_t)(min(c0 + j, lc) + pair) * PART;
                 pm[j] = __ldcg(pw + DH);
                 pl[j] = __ldcg(pw + DH + 1);
                 po[j] = __ldcg(reinterpret_cast<const float2*>(pw + 2 * lane));
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+            for (int j = 0; j < MERGE; ++j)
                 if (c0 + j <= lc) merge_into(tot, pm[j], pl[j], po[j].x, po[j].y);
         }
         const float inv = tot.l > 0.0f ? 1.0f / tot.l : 0.0f;
