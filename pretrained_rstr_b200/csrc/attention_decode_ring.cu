@@ -137,7 +137,7 @@ PRB_API int prb_attention_decode_ring_prefers(int n_list, int n_heads, int max_c
     const long sms = prb_sm_count();
     if (pairs >= 4 * sms) return max_context > 512;
     if (pairs >= 2 * sms) return 1;
-    return pairs >= sms && n_list >= 16 && max_context > 512;
+    return pairs >= sms && max_context > 512;
 }
 
 // Floats of workspace a launch of up to n_list tokens needs.

@@ -78,13 +78,17 @@ constexpr int MAX_STAGES = 8;
 constexpr int MAX_CTAS_PER_SM = 2;
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
 
-// How a launch cuts its work: every CTA takes the strips blockIdx.x + j * grid, each strip
-// in `chunks` pieces of `kc` K elements (kc / 64 slabs of 64), which go round a ring of
-// `stages` shared-memory buffers, so that the copies of the next pieces (of this strip and
-// the next) are in flight while a piece is multiplied.  One TMA copy brings the 16 weight
-// rows of a piece, one more the tokens' activations; a slab lands as [rows][64] with the
-// 128-byte swizzle.
+constexpr int STREAM_THREADS = THREADS + 32;
+constexpr int MIN_HEIGHT = 8;        // rows of W in the lowest strip
+
+// How a launch cuts its work: a strip is `height` (at most 16) rows of W; every CTA takes the strips
+// blockIdx.x + j * grid, each strip in `chunks` pieces of `kc` K elements (kc / 64 slabs of 64), which
+// go round a ring of `stages` shared-memory buffers, so that the copies of the next pieces (of this
+// strip and the next) are in flight while a piece is multiplied.  One TMA copy brings a piece's
+// weight rows, one more the tokens' activations; a slab lands as [rows][64] with the 128-byte swizzle.
 struct Geometry {
+    int height;
+    int strips, per;    // strips of the matrix; the most a CTA has
     int kc, chunks, stages;
     int early;      // ring buffers whose weight copies start before the previous kernel is done
 };
@@ -95,25 +99,35 @@ struct Plan {
 };
 
 // Tuning knobs (0 = the built-in choice): K elements per piece, CTAs per SM, ring depth,
-// shared-memory budget of a CTA in KB.
-int g_tune[5] = {0, 0, 0, 0, 0};   // [4]: ring buffers filled before the wait on the previous kernel
+// shared-memory budget of a CTA in KB, ring buffers filled before the wait on the previous kernel
+// (negative: none), height of a strip.
+int g_tune[6] = {0, 0, 0, 0, 0, 0};
 
 inline int sm_count() { return prb_sm_count(); }
 
-__host__ __device__ inline size_t stage_size(int mp, bool ln, int kc) {
-    return (size_t)(kc / 64) * (ROWS * 128 + (ln ? 0 : mp * 128));
+// bytes of a piece's weight rows (its tokens start on a swizzle atom behind them) and of the piece
+__host__ __device__ inline uint32_t weight_bytes(int height, int kc) {
+    return ((uint32_t)(kc / 64) * height * 128 + 1023u) & ~1023u;
+}
+__host__ __device__ inline uint32_t stage_size(int mp, bool ln, int height, int kc) {
+    return weight_bytes(height, kc) + (ln ? 0u : (uint32_t)(kc / 64) * mp * 128);
 }
 
 inline Plan make_plan(int mt, bool ln, int n, int k) {
     const int mp = 8 * mt;
-    const size_t fixed = (size_t)WARPS * ROWS * mp * sizeof(float) + 256 + 1024 +
+    const size_t fixed = (size_t)2 * WARPS * ROWS * mp * sizeof(float) + 256 + 1024 +
                          (ln ? (size_t)mp * norm_pitch(k) * 2 + (size_t)2 * k * sizeof(float) : 0);
     const size_t sm_bytes = 224 * 1024;                // shared memory of an SM that CTAs can share
     Plan p;
     Geometry& g = p.geo;
-    const int strips = (n + ROWS - 1) / ROWS;
     const int sms = sm_count();
     const int max_stages = g_tune[2] > 0 && g_tune[2] < MAX_STAGES ? g_tune[2] : MAX_STAGES;
+    auto spread = [&](int height, int slots) {         // the strips dealt out evenly
+        g.height = height;
+        g.strips = (n + height - 1) / height;
+        g.per = (g.strips + slots - 1) / slots;
+        p.grid = (g.strips + g.per - 1) / g.per;
+    };
     // Pieces as large as possible (a whole strip when a copy can hold it); as many CTAs per
     // SM as still leaves each a ring of two pieces (or all its work), because what limits a
     // short streaming kernel is the bytes in flight; the strips are then dealt out evenly.
@@ -124,19 +138,18 @@ inline Plan make_plan(int mt, bool ln, int n, int k) {
         if (g.kc > k) g.kc = k;
         if (g.kc > 64 * 256) continue;                 // a copy takes at most 256 slabs
         g.chunks = (k + g.kc - 1) / g.kc;
-        const size_t stage = stage_size(mp, ln, g.kc);
         for (int per_sm = (g_tune[1] > 0 ? g_tune[1] : MAX_CTAS_PER_SM); per_sm >= 1; --per_sm) {
             size_t budget = g_tune[3] > 0 ? (size_t)g_tune[3] * 1024 : sm_bytes / per_sm - 1024;
             if (budget > 216 * 1024) budget = 216 * 1024;    // a CTA's own limit
-            if (fixed + stage > budget) continue;
+            if (fixed + stage_size(mp, ln, ROWS, g.kc) > budget) continue;
             const int slots = sms * per_sm;
-            const int per = (strips + slots - 1) / slots;
-            const int items = g.chunks * per;
+            spread(g_tune[5] > 0 ? g_tune[5] : ROWS, slots);
+            const size_t stage = stage_size(mp, ln, g.height, g.kc);
+            const int items = g.chunks * g.per;
             int fit = (int)((budget - fixed) / stage);
             if (fit > max_stages) fit = max_stages;
             g.stages = fit < items ? fit : items;
             if (g.stages < items && g.stages < 2 && !(g_tune[0] > 0 && per_sm == 1)) continue;
-            p.grid = (strips + per - 1) / per;
             p.smem = fixed + (size_t)g.stages * stage;
             return p;
         }
@@ -146,9 +159,8 @@ inline Plan make_plan(int mt, bool ln, int n, int k) {
     g.kc = 64;
     g.chunks = k / 64;
     g.stages = 1;
-    const int per = (strips + sms - 1) / sms;
-    p.grid = (strips + per - 1) / per;
-    p.smem = fixed + stage_size(mp, ln, 64);
+    spread(ROWS, sms);
+    p.smem = fixed + stage_size(mp, ln, ROWS, 64);
     return p;
 }
 // How many ring buffers' weight copies start before the wait on the previous kernel.  All of
@@ -158,7 +170,7 @@ inline Plan make_plan(int mt, bool ln, int n, int k) {
 // rows (three strips a CTA) takes 9.7 us instead of 11.0 us, its qkv 9.1 instead of 9.9 us.
 inline Plan finish_plan(Plan p, bool ln) {
     p.geo.early = ln ? 1 : p.geo.stages;
-    if (g_tune[4] > 0 && g_tune[4] < p.geo.stages) p.geo.early = g_tune[4];
+    if (g_tune[4] > 0) p.geo.early = g_tune[4];                  // (the kernel takes no more than there are)
     if (g_tune[4] < 0) p.geo.early = 0;
     return p;
 }
@@ -203,6 +215,17 @@ __device__ __forceinline__ void tma_load_slabs(uint32_t dst, const CUtensorMap* 
         "[%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
         "l"(map), "r"(bar), "r"(0), "r"(row), "r"(slab)
         : "memory");
+}
+// the ninth warp waits here until the eight others have normed the rows
+__device__ __forceinline__ void norm_done_arrive() {
+    asm volatile("bar.arrive 2, %0;" ::"n"(STREAM_THREADS) : "memory");
+}
+__device__ __forceinline__ void norm_done_wait() {
+    asm volatile("bar.sync 2, %0;" ::"n"(STREAM_THREADS) : "memory");
+}
+// a barrier of the warps that multiply
+__device__ __forceinline__ void compute_barrier() {
+    asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
 }
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     uint4 v;
@@ -265,38 +288,37 @@ __device__ __forceinline__ void norm_rows_staged(const Args& a, __nv_bfloat16* x
         for (int r = 0; r < R; ++r)
             if (xrow[r] != nullptr) norm_row_any(xrow[r], dst[r], gb, k, a.beta != nullptr, a.eps, a.uncentred == 0);
     }
-    __syncthreads();
+    compute_barrier();
 }
 
 
+// Nine warps: eight multiply, the ninth requests the copies.
 template <int MT, bool LN, typename O>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(STREAM_THREADS, 2)
 gemm_stream_kernel(Args a, Geometry geo, const __grid_constant__ CUtensorMap map_w,
                    const __grid_constant__ CUtensorMap map_x) {
     constexpr int MP = 8 * MT;
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    float* red = reinterpret_cast<float*>(smem_raw);                         // [8][16][MP]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(red + WARPS * ROWS * MP);    // full[], empty[]
+    float* red = reinterpret_cast<float*>(smem_raw);                         // [2][8][16][MP]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(red + 2 * WARPS * ROWS * MP);    // full[], empty[]
     volatile int* failed = reinterpret_cast<volatile int*>(bars + 2 * MAX_STAGES);
     uint8_t* after = reinterpret_cast<uint8_t*>(bars) + 256;
     float* gb = reinterpret_cast<float*>(after);                             // LN only: gamma, beta
     __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(after + (LN ? (size_t)2 * a.k * 4 : 0));
     uint8_t* ring = reinterpret_cast<uint8_t*>(xs) + (LN ? (size_t)MP * a.xs_pitch * 2 : 0);
     const uint32_t stage_base = (smem_u32(ring) + 1023u) & ~1023u;            // swizzle atoms
-    const uint32_t slabs = (uint32_t)geo.kc / 64;
-    const uint32_t w_bytes = slabs * ROWS * 128, x_bytes = LN ? 0u : slabs * MP * 128;
-    const uint32_t stage_bytes = w_bytes + x_bytes;
+    const int height = geo.height;
+    const uint32_t w_bytes = weight_bytes(height, geo.kc);
+    const uint32_t stage_bytes = stage_size(MP, LN, height, geo.kc);
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + MAX_STAGES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane >> 2, q = lane & 3;
-    const int k = a.k, m = a.m, n = a.n;
-    const int strips = (n + ROWS - 1) / ROWS;
-    const int mine = (strips - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // my strips
-    const int items = mine * geo.chunks;
+    const int m = a.m, n = a.n;
+    // strips blockIdx.x, blockIdx.x + grid, .. of geo.strips
+    const int mine = geo.per - ((int)blockIdx.x + (geo.per - 1) * (int)gridDim.x >= geo.strips ? 1 : 0);
 
     TRACE(0);
-    if constexpr (LN) {
+    if (LN && warp < WARPS) {
         // the norm's parameters come first: they are needed early and are not in any cache
         const uint32_t gdst = smem_u32(gb);
         for (int i = threadIdx.x; i < a.k / 4; i += THREADS) {
@@ -304,7 +326,7 @@ gemm_stream_kernel(Args a, Geometry geo, const __grid_constant__ CUtensorMap map
             if (a.beta) cp_async16(gdst + (a.k + i * 4) * 4, a.beta + i * 4);
         }
     }
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == THREADS) {
         for (int s = 0; s < geo.stages; ++s) {
             mbar_init(full0 + 8 * s, 1);
             mbar_init(empty0 + 8 * s, WARPS);
@@ -314,46 +336,79 @@ gemm_stream_kernel(Args a, Geometry geo, const __grid_constant__ CUtensorMap map
     }
     __syncthreads();
 
-    // item i = (my strip i / chunks, piece i % chunks) -> ring buffer i % stages
-    auto issue_weights = [&](int i) {
-        const int st = i % geo.stages;
-        const int n0 = ((int)blockIdx.x + (i / geo.chunks) * (int)gridDim.x) * ROWS;
-        mbar_expect_tx(full0 + 8 * st, stage_bytes);
-        tma_load_slabs(stage_base + st * stage_bytes, &map_w, full0 + 8 * st, n0,
-                       (i % geo.chunks) * (int)slabs);
-    };
-    auto issue_tokens = [&](int i) {
-        if constexpr (!LN) {
-            const int st = i % geo.stages;
-            tma_load_slabs(stage_base + st * stage_bytes + w_bytes, &map_x, full0 + 8 * st, 0,
-                           (i % geo.chunks) * (int)slabs);
+    if (warp == WARPS) {
+        // ---- the copies: pieces in the order they are multiplied, round the ring
+        const int slabs = geo.kc / 64, items = mine * geo.chunks;
+        const uint32_t copied = (uint32_t)slabs * (uint32_t)(height + (LN ? 0 : MP)) * 128;
+        int issued = 0, stage = 0, row = (int)blockIdx.x * height, c = 0;
+        auto weights = [&]() {
+            if (lane == 0) {
+                mbar_expect_tx(full0 + 8 * stage, copied);
+                tma_load_slabs(stage_base + stage * stage_bytes, &map_w, full0 + 8 * stage, row, c * slabs);
+            }
+        };
+        auto tokens = [&](int to, int piece) {
+            if (!LN && lane == 0)
+                tma_load_slabs(stage_base + to * stage_bytes + w_bytes, &map_x, full0 + 8 * to, 0, piece * slabs);
+        };
+        auto next = [&]() {
+            ++issued;
+            if (++stage == geo.stages) stage = 0;
+            if (++c == geo.chunks) { c = 0; row += (int)gridDim.x * height; }
+        };
+        // The weights do not depend on the previous kernel; everything else does.
+        const int first = min(geo.stages, items), early = min(geo.early, first);
+        while (issued < early) { weights(); next(); }
+        prb_grid_wait();
+        prb_grid_launch_dependents();
+        for (int i = 0, piece = 0; i < early; ++i) {
+            tokens(i, piece);
+            if (++piece == geo.chunks) piece = 0;
         }
-    };
-    // The weights do not depend on the previous kernel; everything else does.
-    const int first = min(geo.stages, items), early = min(geo.early, first);
-    if (threadIdx.x == 0)
-        for (int i = 0; i < early; ++i) issue_weights(i);
+        if constexpr (LN) norm_done_wait();            // (the rows' loads go before the weights that follow)
+        uint32_t parity = 0;
+        while (issued < items) {
+            // (a warp has one answer to a wait)
+            if (issued >= geo.stages &&
+                !__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * stage, parity, failed)))
+                break;
+            weights();
+            tokens(stage, c);
+            next();
+            if (issued > geo.stages && stage == 0) parity ^= 1u;
+        }
+        __syncthreads();                               // the other warps are done
+        if (*failed && lane == 0) {
+            // A wait gave up.  Record it; copies already started must land before the CTA's
+            // shared memory is given back.
+            prb_set_status(a.status, PRB_S_WAIT_TIMEOUT, blockIdx.x, 0, 0);
+            for (int i = max(0, issued - geo.stages); i < issued; ++i) {
+                const uint32_t bar = full0 + 8 * (i % geo.stages);
+                const uint32_t phase = (uint32_t)(i / geo.stages) & 1u;
+                for (uint32_t w = 0; w < WAIT_LIMIT; ++w)
+                    if (mbar_try_wait(bar, phase)) break;
+            }
+        }
+        return;
+    }
+
     prb_grid_wait();
     // The next kernel may start its own copies from here on.  (From the top of the kernel its weights
     // were asked for beside this one's: four products of a GPT-2 small layer 15.0 us at one request
     // and 15.7 at eight, 14.6 and 15.1 from here; after the last copy has landed 14.9 and 15.5.)
     prb_grid_launch_dependents();
-    if (threadIdx.x == 0)
-        for (int i = 0; i < early; ++i) issue_tokens(i);
     TRACE(1);
     if constexpr (LN) {
         cp_async_wait_all();
-        __syncthreads();
+        compute_barrier();
         TRACE(2);
         norm_rows_staged<MT>(a, xs, gb);
+        norm_done_arrive();
     }
-    if (threadIdx.x == 0)
-        for (int i = early; i < first; ++i) {
-            issue_weights(i);
-            issue_tokens(i);
-        }
     TRACE(4);
 
+    const int g = lane >> 2, q = lane & 3;
+    O* out = reinterpret_cast<O*>(a.out);
     // Four accumulators per token group (first / second MMA of a step, even / odd turn of
     // the warp) keep the MMAs independent of one another; they are added in a fixed order.
     float acc[MT][4][4];
@@ -361,85 +416,74 @@ gemm_stream_kernel(Args a, Geometry geo, const __grid_constant__ CUtensorMap map
     for (int i = 0; i < MT; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.0f;
-    int issued = first;                            // items whose copies were started (thread 0)
     bool alive = true;
-    O* out = reinterpret_cast<O*>(a.out);
-    // this thread's 16-byte pieces of a slab row: logical piece 4 * (step & 1) + q of rows g,
-    // g + 8 (and of token rows g, g + 8), swizzled with the row
-    const uint32_t row_off = (uint32_t)g * 128;
+    // (rows the strip does not have repeat its last one: their sums go nowhere)
+    const int wr0 = min(g, height - 1), wr1 = min(g + 8, height - 1);
     // the epilogue's element of this thread (ROWS * MP <= THREADS): its bias and residual are
     // fetched when a strip begins
     const int e_tok = threadIdx.x / ROWS, e_r = threadIdx.x % ROWS;
-    float e_bias = 0.0f, e_resid = 0.0f;
-    for (int i = 0; i < items; ++i) {
-        const int st = i % geo.stages;
-        const int c = i % geo.chunks;
-        if (c == 0) {
-            const int col = ((int)blockIdx.x + (i / geo.chunks) * (int)gridDim.x) * ROWS + e_r;
-            // plain loads from addresses that are always valid (a word of shared memory when
-            // there is nothing to fetch): nothing waits for them before the epilogue
-            const bool mine_e = e_tok < m && col < n;
-            const float* bp = (a.bias && mine_e) ? a.bias + col : red;
-            const float* rp = (a.resid && mine_e) ? a.resid + (size_t)e_tok * a.ldc + col : red;
-            e_bias = *bp;
-            e_resid = *rp;
-        }
-        // refill the buffer of the item before, once every warp has released it
-        if (alive && threadIdx.x == 0 && i >= 1 && i - 1 + geo.stages < items) {
-            const int pi = i - 1;
-            if (mbar_wait(empty0 + 8 * (pi % geo.stages), (uint32_t)(pi / geo.stages) & 1u, failed)) {
-                issue_weights(pi + geo.stages);
-                issue_tokens(pi + geo.stages);
-                issued = pi + geo.stages + 1;
-            }
-        }
-        // After a wait gave up nothing more is multiplied or stored, but every warp still
-        // walks all items so that the CTA's barriers stay matched.
-        if (i == 0) TRACE(3);
-        if (alive) alive = mbar_wait(full0 + 8 * st, (uint32_t)(i / geo.stages) & 1u, failed);
-        if (i == 0) TRACE(5);
-        const int k0 = c * geo.kc;
-        const int steps = min(geo.kc, k - k0) / KSTEP;
-        const uint32_t wbase = stage_base + st * stage_bytes;
-        const uint32_t xbase = wbase + w_bytes;
-        auto one_step = [&](int s, int turn) {
-            const uint32_t piece = (uint32_t)(((4 * (s & 1) + q) ^ g) << 4);
-            const uint32_t wslab = wbase + (uint32_t)(s >> 1) * (ROWS * 128) + row_off + piece;
-            const uint4 wa = lds128(wslab), wb = lds128(wslab + 8 * 128);
+    int stage = 0, col = (int)blockIdx.x * height + e_r;
+    uint32_t parity = 0;
+    for (int strip = 0; strip < mine; ++strip, col += (int)gridDim.x * height) {
+        const bool mine_e = threadIdx.x < ROWS * MP && e_tok < m && e_r < height && col < n;
+        // plain loads from addresses that are always valid (a word of shared memory when
+        // there is nothing to fetch): nothing waits for them before the epilogue
+        const float* bp = (a.bias && mine_e) ? a.bias + col : red;
+        const float* rp = (a.resid && mine_e) ? a.resid + (size_t)e_tok * a.ldc + col : red;
+        const float e_bias = *bp, e_resid = *rp;
+        for (int c = 0; c < geo.chunks; ++c) {
+            // After a wait gave up nothing more is multiplied or stored, but every warp still
+            // walks all pieces so that the barriers stay matched.
+            if (strip == 0 && c == 0) TRACE(3);
+            if (alive) alive = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * stage, parity, failed));
+            if (strip == 0 && c == 0) TRACE(5);
+            const int k0 = c * geo.kc;
+            const int steps = min(geo.kc, a.k - k0) / KSTEP;
+            const uint32_t wbase = stage_base + stage * stage_bytes;
+            const uint32_t xbase = wbase + w_bytes;
+            // this thread's 16-byte pieces of a slab row: logical piece 4 * (step & 1) + q of rows g,
+            // g + 8 (and of token rows g, g + 8), swizzled with the row
+            auto one_step = [&](int s, int turn) {
+                const uint32_t slab = (uint32_t)(s >> 1), piece = (uint32_t)(4 * (s & 1) + q);
+                const uint32_t r0 = slab * height + wr0, r1 = slab * height + wr1;
+                const uint4 wa = lds128(wbase + r0 * 128 + ((piece ^ (r0 & 7)) << 4));
+                const uint4 wb = lds128(wbase + r1 * 128 + ((piece ^ (r1 & 7)) << 4));
 #pragma unroll
-            for (int nt = 0; nt < MT; ++nt) {
-                uint4 xv;
-                if constexpr (LN) {
-                    xv = *reinterpret_cast<const uint4*>(xs + (size_t)(nt * 8 + g) * a.xs_pitch + k0 +
-                                                         s * KSTEP + q * 8);
-                } else {
-                    xv = lds128(xbase + (uint32_t)(s >> 1) * (MP * 128) + nt * 8 * 128 + row_off + piece);
+                for (int nt = 0; nt < MT; ++nt) {
+                    uint4 xv;
+                    if constexpr (LN) {
+                        xv = *reinterpret_cast<const uint4*>(xs + (size_t)(nt * 8 + g) * a.xs_pitch + k0 +
+                                                             s * KSTEP + q * 8);
+                    } else {
+                        xv = lds128(xbase + (slab * MP + nt * 8 + g) * 128 + ((piece ^ g) << 4));
+                    }
+                    // elements 0..3 of each load feed the first MMA, 4..7 the second
+                    mma16816(acc[nt][2 * turn], wa.x, wb.x, wa.y, wb.y, xv.x, xv.y);
+                    mma16816(acc[nt][2 * turn + 1], wa.z, wb.z, wa.w, wb.w, xv.z, xv.w);
                 }
-                // elements 0..3 of each load feed the first MMA, 4..7 the second
-                mma16816(acc[nt][2 * turn], wa.x, wb.x, wa.y, wb.y, xv.x, xv.y);
-                mma16816(acc[nt][2 * turn + 1], wa.z, wb.z, wa.w, wb.w, xv.z, xv.w);
+            };
+            if (alive) {
+                int s = warp;
+                for (; s + WARPS < steps; s += 2 * WARPS) {
+                    one_step(s, 0);
+                    one_step(s + WARPS, 1);
+                }
+                if (s < steps) one_step(s, 0);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(empty0 + 8 * stage);
             }
-        };
-        if (alive) {
-            int s = warp;
-            for (; s + WARPS < steps; s += 2 * WARPS) {
-                one_step(s, 0);
-                one_step(s + WARPS, 1);
-            }
-            if (s < steps) one_step(s, 0);
+            if (++stage == geo.stages) { stage = 0; parity ^= 1u; }
         }
-        if (alive && i + geo.stages < items) {     // the buffer will be used again
-            __syncwarp();
-            if (lane == 0) mbar_arrive(empty0 + 8 * st);
-        }
-        if (c != geo.chunks - 1) continue;
-        if (i == geo.chunks - 1) TRACE(6);
+        if (strip == 0) TRACE(6);
 
-        // ---- the strip is complete: add the warps' partial sums in warp order
+        // ---- the strip is complete: add the warps' partial sums in warp order.  (Two places for them
+        // in turn: who writes the next strip's has passed this strip's barrier, and who writes the one
+        // after that has passed the next.)
         // acc[nt][0,1]: feature g, tokens nt*8 + q*2 + {0,1}; acc[nt][2,3]: feature g + 8
+        float* sums = red + (strip & 1) * WARPS * ROWS * MP;
 #pragma unroll
         for (int nt = 0; nt < MT; ++nt) {
-            float* base = red + ((size_t)warp * ROWS) * MP + nt * 8 + q * 2;
+            float* base = sums + ((size_t)warp * ROWS) * MP + nt * 8 + q * 2;
             float sum[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -451,14 +495,12 @@ gemm_stream_kernel(Args a, Geometry geo, const __grid_constant__ CUtensorMap map
             base[(size_t)(g + 8) * MP] = sum[2];
             base[(size_t)(g + 8) * MP + 1] = sum[3];
         }
-        __syncthreads();
-        const int n0 = ((int)blockIdx.x + (i / geo.chunks) * (int)gridDim.x) * ROWS;
-        const int col = n0 + e_r;
-        if (!*failed && threadIdx.x < ROWS * MP && e_tok < m && col < n) {
+        compute_barrier();
+        if (!*failed && mine_e) {
             const int tok = e_tok, r = e_r;            // consecutive threads: consecutive features
             float v = 0.0f;
 #pragma unroll
-            for (int wv = 0; wv < WARPS; ++wv) v += red[((size_t)wv * ROWS + r) * MP + tok];
+            for (int wv = 0; wv < WARPS; ++wv) v += sums[((size_t)wv * ROWS + r) * MP + tok];
             if (a.bias) v += e_bias;
             v = prb_activate(v, a.act);
             if (a.resid) v += e_resid;
@@ -482,23 +524,9 @@ gemm_stream_kernel(Args a, Geometry geo, const __grid_constant__ CUtensorMap map
                 }
             }
         }
-        __syncthreads();                           // `red` is free for the next strip
     }
     __syncthreads();
     TRACE(7);
-    if (*failed) {
-        // A wait gave up.  Record it; copies already started must land before the CTA's
-        // shared memory is given back.
-        if (threadIdx.x == 0) {
-            prb_set_status(a.status, PRB_S_WAIT_TIMEOUT, blockIdx.x, 0, 0);
-            for (int i = max(0, issued - geo.stages); i < issued; ++i) {
-                const uint32_t bar = full0 + 8 * (i % geo.stages);
-                const uint32_t parity = (uint32_t)(i / geo.stages) & 1u;
-                for (uint32_t w = 0; w < WAIT_LIMIT; ++w)
-                    if (mbar_try_wait(bar, parity)) break;
-            }
-        }
-    }
 }
 
 // Sizes this kernel takes; anything else goes to the register-prefetch kernel.
@@ -514,7 +542,7 @@ int launch_stream(Args a, cudaStream_t stream) {
     if (p.smem > 220 * 1024) return PRB_E_SIZE;
     CUtensorMap map_w, map_x;
     const int slabs = p.geo.kc / 64;
-    int rc = tmap::slab_map(a.w, a.n, a.k, a.ldw, ROWS, slabs, &map_w);
+    int rc = tmap::slab_map(a.w, a.n, a.k, a.ldw, p.geo.height, slabs, &map_w);
     if (rc) return rc;
     if (LN) map_x = map_w;
     else if ((rc = tmap::slab_map(a.x, a.m, a.k, a.ldx, MP, slabs, &map_x)) != 0) return rc;
@@ -532,7 +560,7 @@ int launch_stream(Args a, cudaStream_t stream) {
         if (e != cudaSuccess) return (int)e;
         configured = p.smem;
     }
-    cudaError_t e = prb_launch_dependent(gemm_stream_kernel<MT, LN, O>, dim3(p.grid), dim3(THREADS),
+    cudaError_t e = prb_launch_dependent(gemm_stream_kernel<MT, LN, O>, dim3(p.grid), dim3(STREAM_THREADS),
                                          p.smem, stream, a, p.geo, map_w, map_x);
     if (e != cudaSuccess) return (int)e;
     return 0;
@@ -557,9 +585,10 @@ PRB_API int prb_gemm_smallm_trace(unsigned long long* host, int n) {
     return (int)cudaMemcpyFromSymbol(host, stream::g_trace, sizeof(unsigned long long) * n);
 }
 #endif
-PRB_API int prb_gemm_smallm_tune(int kc, int ctas_per_sm, int stages, int budget_kb, int early) {
+PRB_API int prb_gemm_smallm_tune(int kc, int ctas_per_sm, int stages, int budget_kb, int early, int height) {
+    if (height != 0 && (height < stream::MIN_HEIGHT || height > ROWS)) return PRB_E_SIZE;
     stream::g_tune[0] = kc; stream::g_tune[1] = ctas_per_sm;
-    stream::g_tune[2] = stages; stream::g_tune[3] = budget_kb; stream::g_tune[4] = early;
+    stream::g_tune[2] = stages; stream::g_tune[3] = budget_kb; stream::g_tune[4] = early; stream::g_tune[5] = height;
     return 0;
 }
 PRB_API int prb_gemm_smallm_max_norm_width() { return LN_MAX_K; }
