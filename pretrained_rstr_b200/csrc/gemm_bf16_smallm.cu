@@ -79,15 +79,15 @@ constexpr int MAX_CTAS_PER_SM = 2;
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
 
 constexpr int STREAM_THREADS = THREADS + 32;
-constexpr int MIN_HEIGHT = 8;        // rows of W in the lowest strip
 
-// How a launch cuts its work: a strip is `height` (at most 16) rows of W; every CTA takes the strips
-// blockIdx.x + j * grid, each strip in `chunks` pieces of `kc` K elements (kc / 64 slabs of 64), which
-// go round a ring of `stages` shared-memory buffers, so that the copies of the next pieces (of this
-// strip and the next) are in flight while a piece is multiplied.  One TMA copy brings a piece's
-// weight rows, one more the tokens' activations; a slab lands as [rows][64] with the 128-byte swizzle.
+// How a launch cuts its work: every CTA takes the strips blockIdx.x + j * grid, each strip
+// in `chunks` pieces of `kc` K elements (kc / 64 slabs of 64), which go round a ring of
+// `stages` shared-memory buffers, so that the copies of the next pieces (of this strip and
+// the next) are in flight while a piece is multiplied.  One TMA copy brings the 16 weight
+// rows of a piece, one more the tokens' activations; a slab lands as [rows][64] with the
+// 128-byte swizzle.  (Strips of 8 to 14 rows, so that every SM has the same number of rows, are
+// slower at every width: 768 columns of the vocabulary 17.2 us as 16, 18.7 as 14, 20.3 as 11 rows.)
 struct Geometry {
-    int height;
     int strips, per;    // strips of the matrix; the most a CTA has
     int kc, chunks, stages;
     int early;      // ring buffers whose weight copies start before the previous kernel is done
@@ -100,17 +100,13 @@ struct Plan {
 
 // Tuning knobs (0 = the built-in choice): K elements per piece, CTAs per SM, ring depth,
 // shared-memory budget of a CTA in KB, ring buffers filled before the wait on the previous kernel
-// (negative: none), height of a strip.
-int g_tune[6] = {0, 0, 0, 0, 0, 0};
+// (negative: none).
+int g_tune[5] = {0, 0, 0, 0, 0};
 
 inline int sm_count() { return prb_sm_count(); }
 
-// bytes of a piece's weight rows (its tokens start on a swizzle atom behind them) and of the piece
-__host__ __device__ inline uint32_t weight_bytes(int height, int kc) {
-    return ((uint32_t)(kc / 64) * height * 128 + 1023u) & ~1023u;
-}
-__host__ __device__ inline uint32_t stage_size(int mp, bool ln, int height, int kc) {
-    return weight_bytes(height, kc) + (ln ? 0u : (uint32_t)(kc / 64) * mp * 128);
+__host__ __device__ inline size_t stage_size(int mp, bool ln, int kc) {
+    return (size_t)(kc / 64) * (ROWS * 128 + (ln ? 0 : mp * 128));
 }
 
 inline Plan make_plan(int mt, bool ln, int n, int k) {
@@ -122,9 +118,8 @@ inline Plan make_plan(int mt, bool ln, int n, int k) {
     Geometry& g = p.geo;
     const int sms = sm_count();
     const int max_stages = g_tune[2] > 0 && g_tune[2] < MAX_STAGES ? g_tune[2] : MAX_STAGES;
-    auto spread = [&](int height, int slots) {         // the strips dealt out evenly
-        g.height = height;
-        g.strips = (n + height - 1) / height;
+    auto spread = [&](int slots) {                     // the strips dealt out evenly
+        g.strips = (n + ROWS - 1) / ROWS;
         g.per = (g.strips + slots - 1) / slots;
         p.grid = (g.strips + g.per - 1) / g.per;
     };
@@ -141,10 +136,9 @@ inline Plan make_plan(int mt, bool ln, int n, int k) {
         for (int per_sm = (g_tune[1] > 0 ? g_tune[1] : MAX_CTAS_PER_SM); per_sm >= 1; --per_sm) {
             size_t budget = g_tune[3] > 0 ? (size_t)g_tune[3] * 1024 : sm_bytes / per_sm - 1024;
             if (budget > 216 * 1024) budget = 216 * 1024;    // a CTA's own limit
-            if (fixed + stage_size(mp, ln, ROWS, g.kc) > budget) continue;
-            const int slots = sms * per_sm;
-            spread(g_tune[5] > 0 ? g_tune[5] : ROWS, slots);
-            const size_t stage = stage_size(mp, ln, g.height, g.kc);
+            const size_t stage = stage_size(mp, ln, g.kc);
+            if (fixed + stage > budget) continue;
+            spread(sms * per_sm);
             const int items = g.chunks * g.per;
             int fit = (int)((budget - fixed) / stage);
             if (fit > max_stages) fit = max_stages;
@@ -159,18 +153,19 @@ inline Plan make_plan(int mt, bool ln, int n, int k) {
     g.kc = 64;
     g.chunks = k / 64;
     g.stages = 1;
-    spread(ROWS, sms);
-    p.smem = fixed + stage_size(mp, ln, ROWS, 64);
+    spread(sms);
+    p.smem = fixed + stage_size(mp, ln, 64);
     return p;
 }
 // How many ring buffers' weight copies start before the wait on the previous kernel.  All of
 // them, except with the norm fused: the norm's own loads (every CTA reads the same rows) then
 // come back behind whatever weights the SM has in flight, and nothing is multiplied before
-// the norm is done.  With one buffer before and the others after the norm, GPT-2 XL's fc at 8
-// rows (three strips a CTA) takes 9.7 us instead of 11.0 us, its qkv 9.1 instead of 9.9 us.
+// the norm is done.  With two buffers before and the others after the norm the four products of a
+// layer take 26.2 us at 8 rows of 1,600 columns (one: 26.7, all: 26.9) and 21.0 of 1,280 (21.5, 21.2),
+// the vocabulary 16.5 at 768 (17.2, 16.8) and 31.2 at 1,600 (31.8, 31.9).
 inline Plan finish_plan(Plan p, bool ln) {
-    p.geo.early = ln ? 1 : p.geo.stages;
-    if (g_tune[4] > 0) p.geo.early = g_tune[4];                  // (the kernel takes no more than there are)
+    p.geo.early = ln ? 2 : p.geo.stages;                          // (the kernel takes no more than there are)
+    if (g_tune[4] > 0) p.geo.early = g_tune[4];
     if (g_tune[4] < 0) p.geo.early = 0;
     return p;
 }
@@ -292,7 +287,11 @@ __device__ __forceinline__ void norm_rows_staged(const Args& a, __nv_bfloat16* x
 }
 
 
-// Nine warps: eight multiply, the ninth requests the copies.
+// Nine warps: eight multiply, the ninth requests the copies.  What bounds a CTA of many strips is what a
+// strip costs besides its bytes: with the copies requested by a thread of the eight, quotients and
+// remainders of run-time counts in every piece and two barriers a strip that was about 0.95 us.  8 rows,
+// before and now: the vocabulary of 768 columns 23.5 -> 16.5 us, of 1,600 43.3 -> 31.2; the four products
+// of a layer 29.8 -> 26.2 at 1,600 columns, 17.8 -> 16.4 at 1,024.
 template <int MT, bool LN, typename O>
 __global__ void __launch_bounds__(STREAM_THREADS, 2)
 gemm_stream_kernel(Args a, Geometry geo, const __grid_constant__ CUtensorMap map_w,
@@ -307,9 +306,8 @@ gemm_stream_kernel(Args a, Geometry geo, const __grid_constant__ CUtensorMap map
     __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(after + (LN ? (size_t)2 * a.k * 4 : 0));
     uint8_t* ring = reinterpret_cast<uint8_t*>(xs) + (LN ? (size_t)MP * a.xs_pitch * 2 : 0);
     const uint32_t stage_base = (smem_u32(ring) + 1023u) & ~1023u;            // swizzle atoms
-    const int height = geo.height;
-    const uint32_t w_bytes = weight_bytes(height, geo.kc);
-    const uint32_t stage_bytes = stage_size(MP, LN, height, geo.kc);
+    const uint32_t w_bytes = (uint32_t)(geo.kc / 64) * ROWS * 128;
+    const uint32_t stage_bytes = (uint32_t)stage_size(MP, LN, geo.kc);
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + MAX_STAGES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -339,11 +337,10 @@ gemm_stream_kernel(Args a, Geometry geo, const __grid_constant__ CUtensorMap map
     if (warp == WARPS) {
         // ---- the copies: pieces in the order they are multiplied, round the ring
         const int slabs = geo.kc / 64, items = mine * geo.chunks;
-        const uint32_t copied = (uint32_t)slabs * (uint32_t)(height + (LN ? 0 : MP)) * 128;
-        int issued = 0, stage = 0, row = (int)blockIdx.x * height, c = 0;
+        int issued = 0, stage = 0, row = (int)blockIdx.x * ROWS, c = 0;
         auto weights = [&]() {
             if (lane == 0) {
-                mbar_expect_tx(full0 + 8 * stage, copied);
+                mbar_expect_tx(full0 + 8 * stage, stage_bytes);
                 tma_load_slabs(stage_base + stage * stage_bytes, &map_w, full0 + 8 * stage, row, c * slabs);
             }
         };
@@ -354,7 +351,7 @@ gemm_stream_kernel(Args a, Geometry geo, const __grid_constant__ CUtensorMap map
         auto next = [&]() {
             ++issued;
             if (++stage == geo.stages) stage = 0;
-            if (++c == geo.chunks) { c = 0; row += (int)gridDim.x * height; }
+            if (++c == geo.chunks) { c = 0; row += (int)gridDim.x * ROWS; }
         };
         // The weights do not depend on the previous kernel; everything else does.
         const int first = min(geo.stages, items), early = min(geo.early, first);
@@ -417,15 +414,13 @@ gemm_stream_kernel(Args a, Geometry geo, const __grid_constant__ CUtensorMap map
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.0f;
     bool alive = true;
-    // (rows the strip does not have repeat its last one: their sums go nowhere)
-    const int wr0 = min(g, height - 1), wr1 = min(g + 8, height - 1);
     // the epilogue's element of this thread (ROWS * MP <= THREADS): its bias and residual are
     // fetched when a strip begins
     const int e_tok = threadIdx.x / ROWS, e_r = threadIdx.x % ROWS;
-    int stage = 0, col = (int)blockIdx.x * height + e_r;
+    int stage = 0, col = (int)blockIdx.x * ROWS + e_r;
     uint32_t parity = 0;
-    for (int strip = 0; strip < mine; ++strip, col += (int)gridDim.x * height) {
-        const bool mine_e = threadIdx.x < ROWS * MP && e_tok < m && e_r < height && col < n;
+    for (int strip = 0; strip < mine; ++strip, col += (int)gridDim.x * ROWS) {
+        const bool mine_e = threadIdx.x < ROWS * MP && e_tok < m && col < n;
         // plain loads from addresses that are always valid (a word of shared memory when
         // there is nothing to fetch): nothing waits for them before the epilogue
         const float* bp = (a.bias && mine_e) ? a.bias + col : red;
@@ -444,10 +439,9 @@ gemm_stream_kernel(Args a, Geometry geo, const __grid_constant__ CUtensorMap map
             // this thread's 16-byte pieces of a slab row: logical piece 4 * (step & 1) + q of rows g,
             // g + 8 (and of token rows g, g + 8), swizzled with the row
             auto one_step = [&](int s, int turn) {
-                const uint32_t slab = (uint32_t)(s >> 1), piece = (uint32_t)(4 * (s & 1) + q);
-                const uint32_t r0 = slab * height + wr0, r1 = slab * height + wr1;
-                const uint4 wa = lds128(wbase + r0 * 128 + ((piece ^ (r0 & 7)) << 4));
-                const uint4 wb = lds128(wbase + r1 * 128 + ((piece ^ (r1 & 7)) << 4));
+                const uint32_t slab = (uint32_t)(s >> 1), piece = (uint32_t)(((4 * (s & 1) + q) ^ g) << 4);
+                const uint32_t wslab = wbase + (slab * ROWS + g) * 128 + piece;
+                const uint4 wa = lds128(wslab), wb = lds128(wslab + 8 * 128);
 #pragma unroll
                 for (int nt = 0; nt < MT; ++nt) {
                     uint4 xv;
@@ -455,7 +449,7 @@ gemm_stream_kernel(Args a, Geometry geo, const __grid_constant__ CUtensorMap map
                         xv = *reinterpret_cast<const uint4*>(xs + (size_t)(nt * 8 + g) * a.xs_pitch + k0 +
                                                              s * KSTEP + q * 8);
                     } else {
-                        xv = lds128(xbase + (slab * MP + nt * 8 + g) * 128 + ((piece ^ g) << 4));
+                        xv = lds128(xbase + (slab * MP + nt * 8 + g) * 128 + piece);
                     }
                     // elements 0..3 of each load feed the first MMA, 4..7 the second
                     mma16816(acc[nt][2 * turn], wa.x, wb.x, wa.y, wb.y, xv.x, xv.y);
@@ -542,7 +536,7 @@ int launch_stream(Args a, cudaStream_t stream) {
     if (p.smem > 220 * 1024) return PRB_E_SIZE;
     CUtensorMap map_w, map_x;
     const int slabs = p.geo.kc / 64;
-    int rc = tmap::slab_map(a.w, a.n, a.k, a.ldw, p.geo.height, slabs, &map_w);
+    int rc = tmap::slab_map(a.w, a.n, a.k, a.ldw, ROWS, slabs, &map_w);
     if (rc) return rc;
     if (LN) map_x = map_w;
     else if ((rc = tmap::slab_map(a.x, a.m, a.k, a.ldx, MP, slabs, &map_x)) != 0) return rc;
@@ -585,10 +579,9 @@ PRB_API int prb_gemm_smallm_trace(unsigned long long* host, int n) {
     return (int)cudaMemcpyFromSymbol(host, stream::g_trace, sizeof(unsigned long long) * n);
 }
 #endif
-PRB_API int prb_gemm_smallm_tune(int kc, int ctas_per_sm, int stages, int budget_kb, int early, int height) {
-    if (height != 0 && (height < stream::MIN_HEIGHT || height > ROWS)) return PRB_E_SIZE;
+PRB_API int prb_gemm_smallm_tune(int kc, int ctas_per_sm, int stages, int budget_kb, int early) {
     stream::g_tune[0] = kc; stream::g_tune[1] = ctas_per_sm;
-    stream::g_tune[2] = stages; stream::g_tune[3] = budget_kb; stream::g_tune[4] = early; stream::g_tune[5] = height;
+    stream::g_tune[2] = stages; stream::g_tune[3] = budget_kb; stream::g_tune[4] = early;
     return 0;
 }
 PRB_API int prb_gemm_smallm_max_norm_width() { return LN_MAX_K; }
