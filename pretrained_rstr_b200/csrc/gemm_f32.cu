@@ -318,7 +318,37 @@ gemm_f32_stream_kernel(Args p, StreamGeo g, const __grid_constant__ CUtensorMap 
 }
 
 // ------------------------------------------------------------------------- many rows
-constexpr int TILE_STAGES = 3;
+int g_tile_runs = 0;                // (for measurements: 1, 2 or 4 runs a CTA; 0: the rule below)
+constexpr int TILE_STAGES = 2;      // (a chunk's FMAs take several times its copies' way)
+
+// {32 floats, rows} of a row-major [rows, k] matrix, 128-byte swizzle, zeros beyond both; x is a
+// multiple of 32 floats, so the 16-byte rule on it holds.
+int tile_map(const float* t, int rows, int k, long ld, int box_rows, CUtensorMap* out) {
+    static std::unordered_map<tmap::SlabKey, CUtensorMap, tmap::SlabKeyHash> cache;
+    static std::mutex mu;
+    const tmap::SlabKey key{t, rows, k, ld, box_rows, 1};
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = cache.find(key);
+    if (it != cache.end()) {
+        *out = it->second;
+        return 0;
+    }
+    auto fn = tmap::encode_fn();
+    if (!fn) return -6;
+    cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+    cuuint32_t box[2] = {CH, (cuuint32_t)box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    CUtensorMap map;
+    if (fn(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(t), dims, strides, box, estr,
+           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return -5;
+    if (cache.size() > 8192) cache.clear();
+    cache.emplace(key, map);
+    *out = map;
+    return 0;
+}
 
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -332,152 +362,271 @@ __device__ __forceinline__ float4 ld_cluster4(uint32_t addr, uint32_t rank) {
                  : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(r));
     return v;
 }
+// two neighbouring floats as fma.rn.f32x2 takes them, four of them by one read of shared memory
+typedef unsigned long long pair_t;
+__device__ __forceinline__ void fma_pairs(pair_t& acc, pair_t a, pair_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float add_pair(pair_t v) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+    return x + y;
+}
 
-template <int BM, int BN, int TM, int TN> struct TileCfg {
+// RUNS: runs of K a CTA takes (the others of the four are its cluster's)
+template <int BM, int BN, int TM, int TN, int RUNS> struct TileCfg {
     static constexpr int THREADS = (BM / TM) * (BN / TN);
-    static constexpr int STAGE = (BM + BN) * CHP;             // floats
+    static constexpr int STAGE = (BM + BN) * CH;              // floats
+    static constexpr int HELD = RUNS / 2;                     // runs' sums set aside
     static constexpr int OUT_LD = BN + 4;
-    static constexpr size_t SMEM =
-        sizeof(float) * (size_t)(TILE_STAGES * STAGE > BM * OUT_LD ? TILE_STAGES * STAGE : BM * OUT_LD);
+    static constexpr int RING = TILE_STAGES * STAGE > BM * OUT_LD ? TILE_STAGES * STAGE : BM * OUT_LD;
+    static constexpr size_t SMEM = 1024 + sizeof(float) * ((size_t)RING + (size_t)HELD * BM * BN);
 };
 
-// grid (4 x column tiles, row tiles), clusters of 4 along x: CTA q sums run q of the chunks
-template <int BM, int BN, int TM, int TN, bool VEC>
-__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((BM / TM) * (BN / TN))
-gemm_f32_tile_kernel(Args p) {
-    using Cfg = TileCfg<BM, BN, TM, TN>;
-    constexpr int NT = Cfg::THREADS;
+// grid (cluster x column tiles, row tiles), clusters of 4 / RUNS along x: CTA q sums runs RUNS * q ..
+template <int BM, int BN, int TM, int TN, int COPY, int RUNS>
+__global__ void __cluster_dims__(4 / RUNS, 1, 1) __launch_bounds__((BM / TM) * (BN / TN), TM * TN <= 32 ? 3 : 2)
+gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w) {
+    using Cfg = TileCfg<BM, BN, TM, TN, RUNS>;
+    constexpr int NT = Cfg::THREADS, CL = 4 / RUNS;
     constexpr int TY = BM / TM, TX = BN / TN;
-    static_assert(TX % 8 == 0 && TY % 4 == 0, "a warp is 8 columns by 4 rows of threads");
-    extern __shared__ __align__(16) float smem[];
+    static_assert(TX % 8 == 0 && TY % 8 == 0, "a warp is 8 columns by 4 rows of threads; a thread's rows share a swizzle");
+    extern __shared__ __align__(16) uint8_t tile_raw[];
+    __shared__ uint64_t bars[TILE_STAGES];
+    __shared__ int failed_word;
+    volatile int* failed = &failed_word;
+    float* smem = reinterpret_cast<float*>(((uintptr_t)tile_raw + 1023) & ~(uintptr_t)1023);
+    float* held = smem + Cfg::RING;                           // [HELD][TM * TN][NT]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tx = (warp % (TX / 8)) * 8 + (lane & 7);
     const int ty = (warp / (TX / 8)) * 4 + (lane >> 3);
-    const int m0 = blockIdx.y * BM, n0 = (blockIdx.x >> 2) * BN, quarter = blockIdx.x & 3;
+    const int part = blockIdx.x % CL;
+    const int m0 = blockIdx.y * BM, n0 = (blockIdx.x / CL) * BN;
     const int nc = (p.k + CH - 1) / CH, run = (nc + 3) / 4;
-    const int c0 = min(nc, quarter * run), c1 = min(nc, c0 + run);
+    const int c0 = min(nc, part * RUNS * run), c1 = min(nc, c0 + RUNS * run);
+    if (COPY == COPY_TMA && tid == 0) {
+        for (int s = 0; s < TILE_STAGES; ++s) mbar_init(smem_u32(&bars[s]), 1);
+        *failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
 
-    // rows [0, BM) of a stage are A's, the next BN W's; rows outside the matrices are zeros
+    // rows [0, BM) of a stage are A's, the next BN W's; rows outside the matrices are zeros.  A row is
+    // a chunk of 128 bytes, its 16-byte pieces swizzled with the row.
     auto load_rows = [&](int c, bool weights) {
-        if (c < c1) {
-            float* st = smem + ((c - c0) % TILE_STAGES) * Cfg::STAGE + (weights ? BM * CHP : 0);
+        if (c >= c1) return;
+        const int s = (c - c0) % TILE_STAGES;
+        float* st = smem + s * Cfg::STAGE + (weights ? BM * CH : 0);
+        if constexpr (COPY == COPY_TMA) {
+            if (tid == 0) {
+                const uint32_t bar = smem_u32(&bars[s]);
+                if (weights) mbar_expect_tx(bar, Cfg::STAGE * 4);
+                asm volatile(
+                    "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+                    "[%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(st)),
+                    "l"(weights ? &map_w : &map_a), "r"(bar), "r"(c * CH), "r"(weights ? n0 : m0)
+                    : "memory");
+            }
+        } else {
             const float* base = weights ? p.w : p.a;
             const long ld = weights ? p.ldw : p.lda;
             const int first = weights ? n0 : m0, end = weights ? p.n : p.m;
-            constexpr int PER = VEC ? CH / 4 : CH;
+            constexpr int PER = COPY == COPY_16 ? CH / 4 : CH;
             const int rows = weights ? BN : BM;
             for (int i = tid; i < rows * PER; i += NT) {
-                const int r = i / PER, e = (i % PER) * (VEC ? 4 : 1);
+                const int r = i / PER, e = (i % PER) * (CH / PER);
                 const bool in = first + r < end && c * CH + e < p.k;
                 const float* src = in ? base + (size_t)(first + r) * ld + c * CH + e : base;
-                const uint32_t dst = smem_u32(st + r * CHP + e);
-                if (VEC) cp16(dst, src, in ? 16 : 0);
+                const uint32_t dst = smem_u32(st + r * CH + (((e >> 2) ^ (r & 7)) << 2) + (e & 3));
+                if (COPY == COPY_16) cp16(dst, src, in ? 16 : 0);
                 else cp4(dst, src, in ? 4 : 0);
             }
         }
     };
-    for (int s = 0; s < TILE_STAGES - 1; ++s) load_rows(c0 + s, true);
+    if (COPY == COPY_TMA) __syncthreads();
+    for (int s = 0; s < TILE_STAGES; ++s) load_rows(c0 + s, true);
     prb_grid_wait();
     prb_grid_launch_dependents();
-    for (int s = 0; s < TILE_STAGES - 1; ++s) { load_rows(c0 + s, false); cp_commit(); }
+    for (int s = 0; s < TILE_STAGES; ++s) {
+        load_rows(c0 + s, false);
+        if (COPY != COPY_TMA) cp_commit();
+    }
 
     float sum[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) sum[i][j] = 0.0f;
-
-    for (int c = c0; c < c1; ++c) {
-        cp_wait<TILE_STAGES - 2>();
-        __syncthreads();
-        load_rows(c + TILE_STAGES - 1, true);
-        load_rows(c + TILE_STAGES - 1, false);
-        cp_commit();
-        const float* st = smem + ((c - c0) % TILE_STAGES) * Cfg::STAGE;
-        const float* ap = st + ty * CHP;
-        const float* wp = st + (BM + tx) * CHP;
-        float2 acc[TM][TN];
+    const uint32_t sw_a = (uint32_t)(ty & 7), sw_w = (uint32_t)(tx & 7);
+    bool alive = true;
+    int c = c0;
+#pragma unroll 1
+    for (int r = 0; r < RUNS; ++r) {
+        const int end = min(c1, c0 + (r + 1) * run);
+#pragma unroll 1
+        for (; c < end; ++c) {
+            const int s = (c - c0) % TILE_STAGES;
+            if constexpr (COPY == COPY_TMA) {
+                if (alive) alive = mbar_wait(smem_u32(&bars[s]), (uint32_t)((c - c0) / TILE_STAGES) & 1u, failed);
+            } else {
+                cp_wait<TILE_STAGES - 1>();
+                __syncthreads();
+            }
+            const float* ap = smem + s * Cfg::STAGE + ty * CH;
+            const float* wp = smem + s * Cfg::STAGE + (BM + tx) * CH;
+            pair_t acc[TM][TN];
 #pragma unroll
-        for (int i = 0; i < TM; ++i)
+            for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+                for (int j = 0; j < TN; ++j) acc[i][j] = 0;
 #pragma unroll
-        for (int e = 0; e < CH; e += 4) {
-            float4 wv[TN];
+            for (uint32_t e = 0; e < CH / 4; ++e) {
+                const float *ea = ap + ((e ^ sw_a) << 2), *ew = wp + ((e ^ sw_w) << 2);
+                ulonglong2 wv[TN];
 #pragma unroll
-            for (int j = 0; j < TN; ++j) wv[j] = *reinterpret_cast<const float4*>(wp + j * TX * CHP + e);
+                for (int j = 0; j < TN; ++j) wv[j] = *reinterpret_cast<const ulonglong2*>(ew + j * TX * CH);
 #pragma unroll
-            for (int i = 0; i < TM; ++i) {
-                const float4 av = *reinterpret_cast<const float4*>(ap + i * TY * CHP + e);
+                for (int i = 0; i < TM; ++i) {
+                    const ulonglong2 av = *reinterpret_cast<const ulonglong2*>(ea + i * TY * CH);
 #pragma unroll
-                for (int j = 0; j < TN; ++j) fma2(acc[i][j], av.x, av.y, wv[j].x, wv[j].y);
+                    for (int j = 0; j < TN; ++j) fma_pairs(acc[i][j], av.x, wv[j].x);
 #pragma unroll
-                for (int j = 0; j < TN; ++j) fma2(acc[i][j], av.z, av.w, wv[j].z, wv[j].w);
+                    for (int j = 0; j < TN; ++j) fma_pairs(acc[i][j], av.y, wv[j].y);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) sum[i][j] += add_pair(acc[i][j]);
+            __syncthreads();                                  // the stage has been read
+            load_rows(c + TILE_STAGES, true);
+            load_rows(c + TILE_STAGES, false);
+            if (COPY != COPY_TMA) cp_commit();
+        }
+        // two runs are added, then the two sums of two
+        if constexpr (RUNS > 1) {
+            float* mine = held + (RUNS == 4 && r == 2 ? BM * BN : 0) + tid;
+            if (RUNS == 4 && r == 1) {
+#pragma unroll
+                for (int i = 0; i < TM * TN; ++i) mine[i * NT] = mine[i * NT] + sum[i / TN][i % TN];
+            } else if ((r & 1) == 0) {
+#pragma unroll
+                for (int i = 0; i < TM * TN; ++i) mine[i * NT] = sum[i / TN][i % TN];
+            } else {
+                float* second = held + (RUNS == 4 ? BM * BN : 0) + tid;
+#pragma unroll
+                for (int i = 0; i < TM * TN; ++i) {
+                    float t = second[i * NT] + sum[i / TN][i % TN];
+                    if (RUNS == 4) t = held[i * NT + tid] + t;
+                    sum[i / TN][i % TN] = t;
+                }
+            }
+            if (r < RUNS - 1) {
+#pragma unroll
+                for (int i = 0; i < TM * TN; ++i) sum[i / TN][i % TN] = 0.0f;
             }
         }
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TN; ++j) sum[i][j] += acc[i][j].x + acc[i][j].y;
     }
-    cp_wait<0>();
+    if (COPY != COPY_TMA) {
+        cp_wait<0>();
+    } else if (!alive && tid == 0) {
+        prb_set_status(p.status, PRB_S_WAIT_TIMEOUT, 41, blockIdx.x, blockIdx.y);
+        for (int i = max(c0, c1 - TILE_STAGES); i < c1; ++i)  // the last copies, bounded
+            for (uint32_t w = 0; w < tc5::WAIT_LIMIT; ++w)
+                if (mbar_try_wait(smem_u32(&bars[(i - c0) % TILE_STAGES]), (uint32_t)((i - c0) / TILE_STAGES) & 1u)) break;
+    }
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) smem[(ty + i * TY) * Cfg::OUT_LD + tx + j * TX] = sum[i][j];
-    cluster_sync_all();
-    // a quarter of the rows, four columns at a time; all remote reads are asked for at once (one
+    if (CL > 1) cluster_sync_all();
+    else __syncthreads();
+    // a part of the rows, four columns at a time; all remote reads are asked for at once (one
     // after the other they cost 25 us a 128 x 128 tile, twice the tile's FMAs)
-    constexpr int PER = (BM / 4) * (BN / 4) / NT;
-    const int r0 = quarter * (BM / 4);
-    float4 v[PER][4];
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        const int e = tid + i * NT;
-        const uint32_t at = smem_u32(smem + (r0 + e / (BN / 4)) * Cfg::OUT_LD + (e % (BN / 4)) * 4);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) v[i][q] = ld_cluster4(at, q);
-    }
+    constexpr int ROWS = BM / CL, PER = ROWS * (BN / 4) / NT, AT_ONCE = PER < 4 ? PER : 4;
+    static_assert(ROWS * (BN / 4) % NT == 0 && PER % AT_ONCE == 0, "whole rounds");
+    const int r0 = part * ROWS;
     const bool whole = p.ldc % 4 == 0 && ((uintptr_t)p.c) % 16 == 0;
 #pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        const int e = tid + i * NT;
-        const int row = m0 + r0 + e / (BN / 4), col = n0 + (e % (BN / 4)) * 4;
-        if (row >= p.m) continue;
-        const float4 *x = v[i];
-        const float t[4] = {(x[0].x + x[1].x) + (x[2].x + x[3].x), (x[0].y + x[1].y) + (x[2].y + x[3].y),
-                            (x[0].z + x[1].z) + (x[2].z + x[3].z), (x[0].w + x[1].w) + (x[2].w + x[3].w)};
-        float y[4];
+    for (int i0 = 0; i0 < PER; i0 += AT_ONCE) {
+        float4 v[AT_ONCE][CL];
 #pragma unroll
-        for (int d = 0; d < 4; ++d) y[d] = col + d < p.n ? finish(p, t[d], row, col + d) : 0.0f;
-        float* out = p.c + (size_t)row * p.ldc + col;
-        if (whole && col + 4 <= p.n) {
-            *reinterpret_cast<float4*>(out) = make_float4(y[0], y[1], y[2], y[3]);
-        } else {
-            for (int d = 0; d < 4; ++d)
-                if (col + d < p.n) out[d] = y[d];
+        for (int i = 0; i < AT_ONCE; ++i) {
+            const int e = tid + (i0 + i) * NT;
+            const float* at = smem + (r0 + e / (BN / 4)) * Cfg::OUT_LD + (e % (BN / 4)) * 4;
+#pragma unroll
+            for (int q = 0; q < CL; ++q)
+                v[i][q] = CL > 1 ? ld_cluster4(smem_u32(at), q) : *reinterpret_cast<const float4*>(at);
+        }
+#pragma unroll
+        for (int i = 0; i < AT_ONCE; ++i) {
+            const int e = tid + (i0 + i) * NT;
+            const int row = m0 + r0 + e / (BN / 4), col = n0 + (e % (BN / 4)) * 4;
+            if (row >= p.m || !alive) continue;
+            float4 x = v[i][0];
+            if constexpr (CL == 2) {
+                x = make_float4(x.x + v[i][1].x, x.y + v[i][1].y, x.z + v[i][1].z, x.w + v[i][1].w);
+            } else if constexpr (CL == 4) {
+                const float4 y = v[i][1], z = v[i][2], w = v[i][3];
+                x = make_float4((x.x + y.x) + (z.x + w.x), (x.y + y.y) + (z.y + w.y),
+                                (x.z + y.z) + (z.z + w.z), (x.w + y.w) + (z.w + w.w));
+            }
+            const float t[4] = {x.x, x.y, x.z, x.w};
+            float y[4];
+#pragma unroll
+            for (int d = 0; d < 4; ++d) y[d] = col + d < p.n ? finish(p, t[d], row, col + d) : 0.0f;
+            float* out = p.c + (size_t)row * p.ldc + col;
+            if (whole && col + 4 <= p.n) {
+                *reinterpret_cast<float4*>(out) = make_float4(y[0], y[1], y[2], y[3]);
+            } else {
+                for (int d = 0; d < 4; ++d)
+                    if (col + d < p.n) out[d] = y[d];
+            }
         }
     }
-    __syncwarp();
-    cluster_sync_all();                                       // nobody leaves while its tile is read
+    if (CL > 1) {
+        __syncwarp();
+        cluster_sync_all();                                   // nobody leaves while its tile is read
+    }
 }
 
-template <int BM, int BN, int TM, int TN, bool VEC>
+template <int BM, int BN, int TM, int TN, int COPY, int RUNS>
 int launch_tile_by(const Args& p, cudaStream_t stream) {
-    using Cfg = TileCfg<BM, BN, TM, TN>;
-    constexpr auto kernel = gemm_f32_tile_kernel<BM, BN, TM, TN, VEC>;
+    using Cfg = TileCfg<BM, BN, TM, TN, RUNS>;
+    CUtensorMap map_a = {}, map_w = {};
+    if (COPY == COPY_TMA) {
+        int rc = tile_map(p.a, p.m, p.k, p.lda, BM, &map_a);
+        if (rc == 0) rc = tile_map(p.w, p.n, p.k, p.ldw, BN, &map_w);
+        if (rc) return rc;
+    }
+    constexpr auto kernel = gemm_f32_tile_kernel<BM, BN, TM, TN, COPY, RUNS>;
     cudaError_t e = prb_allow_shared<kernel>((int)Cfg::SMEM);
     if (e != cudaSuccess) return (int)e;
-    dim3 grid(4 * ((p.n + BN - 1) / BN), (p.m + BM - 1) / BM);
+    dim3 grid((4 / RUNS) * ((p.n + BN - 1) / BN), (p.m + BM - 1) / BM);
     if (grid.y > 65535) return PRB_E_SIZE;
-    e = prb_launch_maybe_early(p.settled, kernel, grid, dim3(Cfg::THREADS), Cfg::SMEM, stream, p);
+    e = prb_launch_maybe_early(p.settled, kernel, grid, dim3(Cfg::THREADS), Cfg::SMEM, stream, p, map_a, map_w);
     return e == cudaSuccess ? 0 : (int)e;
 }
 
-template <int BM, int BN, int TM, int TN>
-int launch_tile(const Args& p, bool vec, cudaStream_t stream) {
-    return vec ? launch_tile_by<BM, BN, TM, TN, true>(p, stream) : launch_tile_by<BM, BN, TM, TN, false>(p, stream);
+template <int BM, int BN, int TM, int TN, int RUNS>
+int launch_tile(const Args& p, int copy, cudaStream_t stream) {
+    return copy == COPY_TMA  ? launch_tile_by<BM, BN, TM, TN, COPY_TMA, RUNS>(p, stream)
+           : copy == COPY_16 ? launch_tile_by<BM, BN, TM, TN, COPY_16, 1>(p, stream)
+                             : launch_tile_by<BM, BN, TM, TN, COPY_4, 1>(p, stream);
+}
+// Runs a CTA takes, of tiles of 64 x 128.
+int tile_runs(long tiles, int k) {
+    if (g_tile_runs > 0) return g_tile_runs;
+    const int run = ((k + CH - 1) / CH + 3) / 4;
+    const long slots = 2L * prb_sm_count();
+    int best = 1;
+    double least = 0.0;
+    for (int runs = 1; runs <= 4; runs *= 2) {
+        const double t = (double)((tiles * (4 / runs) + slots - 1) / slots) * (runs * run + 1.5);
+        if (runs == 1 || t < least) { least = t; best = runs; }
+    }
+    return best;
 }
 
 constexpr size_t STREAM_SMEM = 220 * 1024;                    // the most a launch of the stream kernel takes
@@ -571,12 +720,21 @@ PRB_API int prb_gemm_f32(float* c, const float* a, const float* w, const float* 
             }
         }
     }
-    if (which == 2) return launch_tile<64, 128, 8, 8>(p, vec, stream);
-    if (which == 3) return launch_tile<64, 64, 8, 4>(p, vec, stream);
+    // (rows that overlap are no tensor that a copy engine's map describes)
+    const int tiled = !vec ? COPY_4 : ldw >= k && lda >= k ? COPY_TMA : COPY_16;
     // 64 x 128 where that leaves no SM without a CTA twice over (1.49 against 1.56 ms at 650 x 50,257
     // x 768, 111 and 111 us at 1,000 x 2,304 x 768), else 64 x 64 (650 x 768 x 768: 28 us, tiles of
     // 128 x 64 54 us).
-    const long big = (long)((m + 63) / 64) * ((n + 127) / 128) * 4;
-    if (big >= 2 * prb_sm_count()) return launch_tile<64, 128, 8, 8>(p, vec, stream);
-    return launch_tile<64, 64, 8, 4>(p, vec, stream);
+    const long big = (long)((m + 63) / 64) * ((n + 127) / 128);
+    if (which == 3 || (which != 2 && big * 4 < 2 * prb_sm_count())) return launch_tile<64, 64, 8, 4, 1>(p, tiled, stream);
+    switch (tile_runs(big, k)) {
+        case 1: return launch_tile<64, 128, 8, 8, 1>(p, tiled, stream);
+        case 2: return launch_tile<64, 128, 8, 8, 2>(p, tiled, stream);
+        default: return launch_tile<64, 128, 8, 8, 4>(p, tiled, stream);
+    }
+}
+PRB_API int prb_gemm_f32_tune(int runs) {
+    if (runs != 0 && runs != 1 && runs != 2 && runs != 4) return PRB_E_SIZE;
+    g_tile_runs = runs;
+    return 0;
 }

@@ -92,8 +92,9 @@ class ModelRunner:
         self.graph_max_tokens = runtime.max_batched_tokens
         self._graphs: Dict[tuple, tuple] = {}
         self._seen: Dict[tuple, int] = {}
-        self._pairs_host = torch.empty((runtime.max_requests, 2), dtype=torch.int32,
-                                       pin_memory=True)
+        # (one for each staging buffer and group: a step's page copies are queued like the rest of it)
+        self._pairs_hosts = [[torch.empty((runtime.max_requests, 2), dtype=torch.int32, pin_memory=True)
+                              for _ in range(self.n_groups)] for _ in range(2)]
         self._pairs_dev = torch.zeros((runtime.max_requests, 2), dtype=torch.int32,
                                       device=self.device)
         self.scratch = ScratchPool(self.device)
@@ -350,15 +351,20 @@ class ModelRunner:
                 ops.resolve_tokens(ctx.tokens, ctx.n_tokens, self.tokens_out, self.status)
         self._host_events[ctx.staging_turn].record()
         self.last_h2d_bytes = words * 4
+        if not ctx.copies:
+            return
         for g in range(self.n_groups):
             pairs = [(src, dst) for (gg, src, dst) in ctx.copies if gg == g]
-            for i in range(0, len(pairs), self._pairs_host.shape[0]):
-                chunk = pairs[i:i + self._pairs_host.shape[0]]
-                self._pairs_host[:len(chunk)] = torch.tensor(chunk, dtype=torch.int32)
-                self._pairs_dev[:len(chunk)].copy_(self._pairs_host[:len(chunk)], non_blocking=True)
+            host = self._pairs_hosts[ctx.staging_turn][g]
+            for i in range(0, len(pairs), host.shape[0]):
+                if i > 0:                            # the pinned buffer is used again within the step
+                    torch.cuda.current_stream().synchronize()
+                chunk = pairs[i:i + host.shape[0]]
+                host[:len(chunk)] = torch.tensor(chunk, dtype=torch.int32)
+                self._pairs_dev[:len(chunk)].copy_(host[:len(chunk)], non_blocking=True)
                 self.storage.copy_pages(g, self._pairs_dev, len(chunk), self.status)
-                torch.cuda.current_stream().synchronize()      # pinned pairs buffer is reused
                 self.counters["cow_copies"] += len(chunk)
+        self._host_events[ctx.staging_turn].record()     # who takes this staging buffer next waits for these too
 
     def commit(self, entries: Sequence[Entry]) -> None:
         for e in entries:
