@@ -201,11 +201,20 @@ gemm_f32_stream_kernel(Args p, StreamGeo g, const __grid_constant__ CUtensorMap 
     };
     // weights never depend on the kernel before this one; A does
     for (int s = 0; s < g.stages; ++s) load_stage(s);
+    const bool resident = g.items <= STREAM_THREADS;          // a thread keeps one item for good
+    const int my_slot = resident ? tid / g.items : 0;
+    const int first_item = resident ? tid - my_slot * g.items : tid;
+    // the sum this thread finishes in the first round of a stage: a run of output (row of A, weight row)
+    const int fin_q = tid & 3, fin_i = (tid >> 2) / g.rows, fin_r = (tid >> 2) - fin_i * g.rows;
     prb_grid_wait();
     prb_grid_launch_dependents();
     for (int r = warp; r < MB; r += STREAM_THREADS / 32) {
         float* dst = as + r * row_len;
-        if (m0 + r < p.m) {
+        if (COPY == COPY_TMA && m0 + r < p.m) {
+            // (all of the row at once: loaded and stored a few pieces at a time, 3,072 columns took
+            // six round trips to the L2)
+            copy_row<true>(dst, p.a + (size_t)(m0 + r) * p.lda, p.k, g.nc, lane);
+        } else if (m0 + r < p.m) {
             const float* src = p.a + (size_t)(m0 + r) * p.lda;
             for (int i = lane * 4; i < g.nc * CH; i += 128) {
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -224,6 +233,10 @@ gemm_f32_stream_kernel(Args p, StreamGeo g, const __grid_constant__ CUtensorMap 
                 *reinterpret_cast<float4*>(dst + i) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }
+    if (COPY == COPY_TMA) {
+        cp_commit();
+        cp_wait<0>();
+    }
     __syncthreads();
 
     float4 av[MT][CH / 4];
@@ -235,13 +248,15 @@ gemm_f32_stream_kernel(Args p, StreamGeo g, const __grid_constant__ CUtensorMap 
             for (int j = 0; j < CH / 4; ++j)
                 av[i][j] = *reinterpret_cast<const float4*>(as + (group * MT + i) * row_len + c * CHP + j * 4);
     };
-    const bool resident = g.items <= STREAM_THREADS;          // a thread keeps one item for good
-    const int my_slot = resident ? tid / g.items : 0;
-    const int first_item = resident ? tid % g.items : tid;
     if (resident && my_slot < g.slots) load_a(first_item);
 
     const int run = (g.nc + 3) / 4;
     for (int s = 0; s < n_stages; ++s) {
+        // what the first round's sums are finished with is asked for before the stage is waited for
+        const int fin_row = m0 + fin_i, fin_col = n0 + s * g.rows + fin_r;
+        const bool fin = fin_q == 0 && fin_i < MB && fin_row < p.m && fin_r < min(g.rows, n1 - (n0 + s * g.rows));
+        const float fin_bias = fin && p.bias ? p.bias[fin_col] : 0.0f;
+        const float fin_resid = fin && p.resid ? p.resid[(size_t)fin_row * p.ldc + fin_col] : 0.0f;
         if constexpr (COPY == COPY_TMA) {
             alive = alive && mbar_wait(smem_u32(&bars[s % g.stages]), (uint32_t)(s / g.stages) & 1u, failed);
         } else {
@@ -290,7 +305,7 @@ gemm_f32_stream_kernel(Args p, StreamGeo g, const __grid_constant__ CUtensorMap 
         for (int t0 = 0; t0 < g.rows * MB * 4; t0 += STREAM_THREADS) {
             const int t = t0 + tid;
             const int q = t & 3, o = t >> 2;
-            const int r = o % g.rows, i = o / g.rows;
+            const int i = t0 == 0 ? fin_i : o / g.rows, r = t0 == 0 ? fin_r : o - i * g.rows;
             float sum = 0.0f;
             const bool live = o < g.rows * MB && r < rows && m0 + i < p.m && alive;
             if (live) {
@@ -301,7 +316,16 @@ gemm_f32_stream_kernel(Args p, StreamGeo g, const __grid_constant__ CUtensorMap 
             sum += __shfl_xor_sync(0xffffffffu, sum, 2);
             if (live && q == 0) {
                 const int row = m0 + i, col = n0 + s * g.rows + r;
-                p.c[(size_t)row * p.ldc + col] = finish(p, sum, row, col);
+                float v;
+                if (t0 == 0) {
+                    v = sum;
+                    if (p.bias) v += fin_bias;
+                    v = prb_activate(v, p.act);
+                    if (p.resid) v += fin_resid;
+                } else {
+                    v = finish(p, sum, row, col);
+                }
+                p.c[(size_t)row * p.ldc + col] = v;
             }
         }
     }
