@@ -168,7 +168,8 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
     const int rank = blockIdx.z, S = a.splits;
     // this CTA's part of K, in slabs of 64
     const int slabs = a.k / 64;
-    const int slab_lo = (int)((long)slabs * rank / S), slab_hi = (int)((long)slabs * (rank + 1) / S);
+    const int slab_lo = (int)((unsigned)(slabs * rank) / (unsigned)S);
+    const int slab_hi = (int)((unsigned)(slabs * (rank + 1)) / (unsigned)S);
     const int items = (slab_hi - slab_lo + KC - 1) / KC;
 
     MT_TRACE(0);
@@ -197,6 +198,30 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
     const int first = min(STAGES, items);
     if (threadIdx.x == 0)
         for (int i = 0; i < first; ++i) issue_w(i);
+    // What takes quotients of run-time counts is worked out before the wait, not between the last
+    // multiplication and the store: where this warp's rows go, and where a column lies in the cache.
+    const int per = (int)((unsigned)(MROWS + S - 1) / (unsigned)S);      // rows of a CTA
+    uint32_t part_dst[2];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const unsigned row = (warp & 3) * 16 + (lane >> 2) + 8 * half, to = row / (unsigned)S;
+        part_dst[half] = cluster_addr(
+            smem_u32(part + (size_t)(rank * per + (int)to) * PP + (warp >> 2) * (NB / 2) + (lane & 3) * 2),
+            row - to * S);
+    }
+    const int col = threadIdx.x % NB, rsub = threadIdx.x / NB;
+    const int gcol = n0 + col;
+    const bool to_cache = a.kv_width != 0 && gcol >= a.q_width && gcol < a.n;
+    O* column = nullptr;                              // this column in page 0, place 0
+    long page_len = 0;                                // elements of a page
+    if (to_cache) {
+        unsigned cc = (unsigned)(gcol - a.q_width);
+        column = reinterpret_cast<O*>(cc < (unsigned)a.kv_width ? a.k_pages : a.v_pages);
+        if (cc >= (unsigned)a.kv_width) cc -= a.kv_width;
+        const unsigned head = cc / (unsigned)a.head_dim, dim = cc - head * a.head_dim;
+        page_len = (long)a.kv_width * a.page_size;
+        column += (long)head * a.page_size * a.head_dim + dim;
+    }
     prb_grid_wait();
     if (threadIdx.x == 0)
         for (int i = 0; i < first; ++i) issue_a(i);
@@ -251,20 +276,17 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
     }
     MT_TRACE(3);
     // ---- the rows of this CTA's partial tile to the CTAs that finish them
-    const int per = (MROWS + S - 1) / S;                  // rows of a CTA
     __syncwarp();
     cluster_wait();
     {
-        const int g = lane >> 2, q = lane & 3;
+        const int g = lane >> 2;
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const int row = mt * 16 + g + 8 * half;
             if (row < a.m) {
-                const uint32_t dst = cluster_addr(
-                    smem_u32(part + (size_t)(rank * per + row / S) * PP + nh * (NB / 2) + q * 2), row % S);
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt)
-                    st_cluster_f32x2(dst + nt * 32, acc[nt][2 * half], acc[nt][2 * half + 1]);
+                    st_cluster_f32x2(part_dst[half] + nt * 32, acc[nt][2 * half], acc[nt][2 * half + 1]);
             }
         }
     }
@@ -272,16 +294,23 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
     constexpr int RPP = THREADS / NB;                     // rows per pass
     constexpr int PASSES = MROWS / RPP;                   // (S = 1; a split has 1 / S of them)
     constexpr int AHEAD = PASSES < 4 ? PASSES : 4;
-    const int col = threadIdx.x % NB, rsub = threadIdx.x / NB;
-    const int gcol = n0 + col;
     const float bias = (a.bias && gcol < a.n) ? a.bias[gcol] : 0.0f;
     float res[AHEAD];
-    int slot[AHEAD];
-    const bool to_cache = a.kv_width != 0 && gcol >= a.q_width && gcol < a.n;
+    O* place[AHEAD];                                      // in the cache, or null
+    auto cache_place = [&](int row) -> O* {
+        const int at = to_cache && row < a.m ? a.slots[row] : -1;
+        if (at < 0) return nullptr;
+        const int page = (int)((unsigned)at / (unsigned)a.page_size);
+        if (page >= a.num_pages) {
+            prb_set_status(a.status, PRB_S_SLOT_RANGE, row, at, a.num_pages);
+            return nullptr;
+        }
+        return column + page * page_len + (long)(at - page * a.page_size) * a.head_dim;
+    };
 #pragma unroll
     for (int i = 0; i < AHEAD; ++i) {
         const int row = rank + (rsub + i * RPP) * S;
-        slot[i] = to_cache && row < a.m ? a.slots[row] : -1;
+        place[i] = rsub + i * RPP < per ? cache_place(row) : nullptr;
         res[i] = (a.resid && gcol < a.n && row < a.m) ? a.resid[(size_t)row * a.ldc + gcol] : 0.0f;
     }
     __syncthreads();
@@ -307,16 +336,6 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
     for (int r = 0; r < S; ++r) any_bad |= missing[r] != 0;
     if (!any_bad && gcol < a.n) {
         O* out = reinterpret_cast<O*>(a.c);
-        O* pages = nullptr;
-        int head = 0, dim = 0, kv_heads = 1;
-        if (to_cache) {
-            int cc = gcol - a.q_width;
-            pages = reinterpret_cast<O*>(cc < a.kv_width ? a.k_pages : a.v_pages);
-            if (cc >= a.kv_width) cc -= a.kv_width;
-            head = cc / a.head_dim;
-            dim = cc - head * a.head_dim;
-            kv_heads = a.kv_width / a.head_dim;
-        }
 #pragma unroll
         for (int i = 0; i < PASSES; ++i) {
             const int local = rsub + i * RPP, row = rank + local * S;
@@ -332,15 +351,8 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
             if (a.resid) v += i < AHEAD ? res[i < AHEAD ? i : 0] : a.resid[(size_t)row * a.ldc + gcol];
             if (!to_cache || !a.only_cache) out[(size_t)row * a.ldc + gcol] = prb_from_float<O>(v);
             if (to_cache) {
-                const int at = i < AHEAD ? slot[i < AHEAD ? i : 0] : a.slots[row];
-                if (at >= 0) {
-                    const int page = at / a.page_size;
-                    if (page >= a.num_pages)
-                        prb_set_status(a.status, PRB_S_SLOT_RANGE, row, at, a.num_pages);
-                    else
-                        pages[(((size_t)page * kv_heads + head) * a.page_size + (at - page * a.page_size)) *
-                                  a.head_dim + dim] = prb_from_float<O>(v);
-                }
+                O* at = i < AHEAD ? place[i < AHEAD ? i : 0] : cache_place(row);
+                if (at != nullptr) *at = prb_from_float<O>(v);
             }
         }
     }
