@@ -174,6 +174,7 @@ PRB_API int prb_attention_decode_ring(void* out, long out_stride, const void* q,
     a.block_table = block_table; a.seq_of_token = seq_of_token; a.positions = positions;
     a.token_list = token_list; a.token_count = token_count;
     a.n_list = n_list; a.n_heads = n_heads; a.kv_heads = kv_heads; a.page_size = page_size;
+    a.hpg = n_heads / kv_heads;
     a.max_pages = max_pages; a.num_pages = num_pages; a.scale = scale; a.window = window;
     a.k_new = (const __nv_bfloat16*)k_new; a.v_new = (const __nv_bfloat16*)v_new; a.kv_stride = kv_stride;
     a.new_keys = new_keys; a.workspace = workspace; a.counters = counters; a.status = status;

@@ -46,6 +46,7 @@ struct RingArgs {
     const int* token_list;
     const int* token_count;
     int n_list, n_heads, kv_heads, page_size, max_pages, num_pages;
+    int hpg;                        // query heads per key/value head
     float scale;
     int window;
     int new_keys;                   // a token's last `new_keys` visible positions may have been
@@ -262,7 +263,8 @@ struct LaneUnit {
     bool late;                  // holds rows the step itself may have written (and they are not
                                 // handed over beside the queries)
     bool bad;                   // a page of it lies outside the pool
-    int pages[4];               // its pages (one when the page holds 32 keys or more)
+    int first[4];               // where its pages' rows start in the cache seen as rows of 64 numbers
+                                // (one when the page holds 32 keys or more)
     int rows;                   // rows to copy: up to the end of the last page it touches
 };
 // Which unit it is: from shared memory only.
@@ -272,7 +274,7 @@ RING_FN LaneUnit decode_unit(const RingArgs& a, const Shared& sh, int u, int u_e
     lu.h = lu.blk = lu.pos = lu.lo = lu.t = 0;
     lu.late = lu.bad = false;
     lu.rows = 0;
-    lu.pages[0] = lu.pages[1] = lu.pages[2] = lu.pages[3] = -1;
+    lu.first[0] = lu.first[1] = lu.first[2] = lu.first[3] = 0;
     if (u >= u_end) return lu;
     int lo_i = 0, hi_i = sh.n;                       // largest idx with cum[idx] <= u
     while (hi_i - lo_i > 1) {
@@ -289,27 +291,30 @@ RING_FN LaneUnit decode_unit(const RingArgs& a, const Shared& sh, int u, int u_e
     lu.late = a.k_new == nullptr && lu.blk * UNIT + UNIT > s.pos - a.new_keys + 1;
     return lu;
 }
-// Its pages, from the block table.
+// Its rows, by the block table (worked out with the look-up, so that nothing but the copies is left to
+// the lane that requests them).
 RING_FN void unit_pages(const RingArgs& a, const Shared& sh, LaneUnit& lu) {
     if (lu.idx < 0) return;
-    const int k0 = lu.blk * UNIT;
-    const int last_key = min(k0 + UNIT - 1, lu.pos);
-    const int* table = a.block_table + (size_t)sh.span_b[lu.idx] * a.max_pages;
-    if (a.page_size >= UNIT) {
-        lu.pages[0] = table[k0 / a.page_size];
+    const unsigned k0 = (unsigned)lu.blk * UNIT, page_size = (unsigned)a.page_size;
+    const unsigned slot = k0 / page_size, off = k0 - slot * page_size;
+    const int* table = a.block_table + (size_t)sh.span_b[lu.idx] * a.max_pages + slot;
+    const int hk = a.hpg == 1 ? lu.h : (int)((unsigned)lu.h / (unsigned)a.hpg);
+    const int page0 = table[0];
+    if (page_size >= UNIT) {
         lu.rows = UNIT;
-        if (lu.pages[0] < 0 || lu.pages[0] >= a.num_pages) lu.bad = true;
+        if (page0 < 0 || page0 >= a.num_pages) lu.bad = true;
+        lu.first[0] = (page0 * a.kv_heads + hk) * a.page_size + (int)off;
     } else {
-        const int fit = UNIT / a.page_size;          // 2 or 4 pages to a unit
-        const int used = (last_key - k0) / a.page_size + 1;
+        const int used = (min((int)k0 + UNIT - 1, lu.pos) - (int)k0) / a.page_size + 1;   // of 2 or 4 pages to a unit
         lu.rows = used * a.page_size;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            lu.pages[i] = (i < fit && i < used) ? table[k0 / a.page_size + i] : -1;
-            if (i < used && (lu.pages[i] < 0 || lu.pages[i] >= a.num_pages)) lu.bad = true;
+            const int page = i == 0 ? page0 : i < used ? table[i] : 0;
+            if (page < 0 || page >= a.num_pages) lu.bad = true;
+            lu.first[i] = (page * a.kv_heads + hk) * a.page_size;
         }
     }
-    if (lu.bad) prb_set_status(a.status, PRB_S_PAGE_RANGE, lu.t, k0, lu.pages[0]);
+    if (lu.bad) prb_set_status(a.status, PRB_S_PAGE_RANGE, lu.t, (int)k0, page0);
 }
 // This lane starts the copies of its unit into ring buffer `slot` of its warp.
 RING_FN void issue_unit(const RingArgs& a, const CUtensorMap* map_k,
@@ -321,18 +326,16 @@ RING_FN void issue_unit(const RingArgs& a, const CUtensorMap* map_k,
         return;
     }
     const uint32_t kd = ring0 + slot * 2 * TILE, vd = kd + TILE;
-    const int hk = lu.h / (a.n_heads / a.kv_heads);
     mbar_expect_tx(bar, 2u * lu.rows * ROW);
     if (a.page_size >= UNIT) {
-        const int row = (lu.pages[0] * a.kv_heads + hk) * a.page_size + (lu.blk * UNIT) % a.page_size;
-        tma_rows(kd, map_k, bar, row);
-        tma_rows(vd, map_v, bar, row);
+        tma_rows(kd, map_k, bar, lu.first[0]);
+        tma_rows(vd, map_v, bar, lu.first[0]);
     } else {
-        const int used = lu.rows / a.page_size;
-        for (int i = 0; i < used; ++i) {
-            const int row = (lu.pages[i] * a.kv_heads + hk) * a.page_size;
-            tma_rows(kd + i * a.page_size * ROW, map_k, bar, row);
-            tma_rows(vd + i * a.page_size * ROW, map_v, bar, row);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (i * a.page_size >= lu.rows) break;
+            tma_rows(kd + i * a.page_size * ROW, map_k, bar, lu.first[i]);
+            tma_rows(vd + i * a.page_size * ROW, map_v, bar, lu.first[i]);
         }
     }
 }
@@ -377,7 +380,6 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
     const int u_begin = r.u_begin, u_end = r.u_end;
     const uint32_t ring0 = warp_ring(ring_base, stages);
     const uint32_t bar0 = smem_addr(&sh.bars[warp * MAX_STAGES]);
-    const int hpg = a.n_heads / a.kv_heads;          // query heads per key/value head
     auto cta_of = [&](int u) { return (int)((unsigned)u / r.per / r.wpc); };   // whose warps hold unit u
 
     if (lane < stages && mine.idx >= 0 && mine.late) issue_unit(a, map_k, map_v, mine, ring0, bar0, lane);
@@ -484,7 +486,7 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
                     (key / UNIT - cur_blk) < u_end - u && sh.span_t[src] == cur_t - j &&
                     sh.span_b[src] == sh.span_b[cur_idx] && sh.span_pos[src] == key) {
                     own_key = key;
-                    const size_t off = (size_t)(cur_t - j) * a.kv_stride + (size_t)(cur_h / hpg) * DH + c * 8;
+                    const size_t off = (size_t)(cur_t - j) * a.kv_stride + (size_t)((unsigned)cur_h / (unsigned)a.hpg) * DH + c * 8;
                     own_k = *reinterpret_cast<const uint4*>(a.k_new + off);
                     own_v = *reinterpret_cast<const uint4*>(a.v_new + off);
                 }
