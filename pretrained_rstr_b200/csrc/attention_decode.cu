@@ -147,6 +147,8 @@ PRB_API int prb_attention_decode(void* out, long out_stride, const void* q, long
     a.max_pages = max_pages; a.num_pages = num_pages; a.scale = scale; a.window = window;
     a.workspace = workspace; a.counters = counters; a.max_splits = max_splits;
     a.split = split_keys; a.status = status;
+    a.page_shift = __builtin_ctz((unsigned)page_size);         // (it divides SPLIT, a power of two)
+    a.hpg = n_heads / kv_heads;
     // More CTAs than fit at four per SM: the leaner instance, six per SM.  Otherwise two to eight
     // splits form a cluster and merge through shared memory (a layer of GPT-2 small at one request
     // 25.0 -> 23.9 us); clusters of many CTAs wait for places side by side and lose (16 requests

@@ -50,6 +50,8 @@ struct Args {
     int* counters;
     int max_splits;
     int split;                      // keys per split: a multiple of SPLIT
+    int page_shift;                 // page_size is 1 << page_shift (it divides SPLIT): no quotient a key
+    int hpg;                        // query heads per key/value head
     int* status;
 };
 
@@ -208,17 +210,17 @@ __device__ __forceinline__ void unit(const Args& a, int idx, int h, int s,
     constexpr int KPW = 32 / LPK;                 // keys per warp per load
 
     DEC_TRACE(0);
-    if (a.token_count != nullptr && idx >= *a.token_count) return;
+    // (the list's entry is asked for beside the count, the position beside the request)
     const int t = a.token_list ? a.token_list[idx] : idx;
-    const int b = a.seq_of_token[t];
+    if (a.token_count != nullptr && idx >= *a.token_count) return;
+    const int b = a.seq_of_token[t], pos = a.positions[t];
     if (b < 0) return;
-    const int pos = a.positions[t];
     if (pos < 0 || pos >= a.max_pages * a.page_size) {
         if (threadIdx.x == 0 && s == 0) prb_set_status(a.status, PRB_S_POSITION_RANGE, t, pos, 0);
         return;
     }
     const int lo = (a.window > 0 && pos - a.window + 1 > 0) ? pos - a.window + 1 : 0;
-    const int s_first = lo / a.split, s_last = pos / a.split;
+    const int s_first = (int)((unsigned)lo / (unsigned)a.split), s_last = (int)((unsigned)pos / (unsigned)a.split);
     if (s_last >= a.max_splits) {                   // the launch does not cover this context
         if (threadIdx.x == 0 && s == 0) prb_set_status(a.status, PRB_S_POSITION_RANGE, t, pos, a.max_splits);
         return;
@@ -243,7 +245,7 @@ __device__ __forceinline__ void unit(const Args& a, int idx, int h, int s,
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = lane % LPK;                   // which 16-byte piece of the row
     const int kslot = lane / LPK;                 // which key of the warp's load
-    const int hk = h / (a.n_heads / a.kv_heads);
+    const int hk = a.hpg == 1 ? h : (int)((unsigned)h / (unsigned)a.hpg);
     const int* table = a.block_table + (size_t)b * a.max_pages;
     const bool piece_ok = sub * 8 < a.head_dim;
 
@@ -267,8 +269,9 @@ __device__ __forceinline__ void unit(const Args& a, int idx, int h, int s,
     for (int i = 0; i < 8; ++i) acc[i] = 0.0f;
 
     // page ids of this split, once
-    const int first_page = (s * a.split) / a.page_size;
-    for (int i = threadIdx.x; i < a.split / a.page_size; i += (NW * 32))
+    const int shift = a.page_shift, in_page = a.page_size - 1;
+    const int first_page = (s * a.split) >> shift;
+    for (int i = threadIdx.x; i < a.split >> shift; i += (NW * 32))
         sh_pages[i] = (first_page + i < a.max_pages) ? table[first_page + i] : -1;
     if constexpr (STREAM) {
         if (threadIdx.x == 0) {
@@ -300,14 +303,14 @@ __device__ __forceinline__ void unit(const Args& a, int idx, int h, int s,
             bt.k[u] = make_uint4(0, 0, 0, 0);
             bt.v[u] = make_uint4(0, 0, 0, 0);
             if (j < k_end) {
-                const int page = sh_pages[j / a.page_size - first_page];
+                const int page = sh_pages[(j >> shift) - first_page];
                 if (page < 0 || page >= a.num_pages) {
                     prb_set_status(a.status, PRB_S_PAGE_RANGE, t, j, page);
                 } else {
                     bt.ok[u] = true;
                     if (piece_ok) {
                         const size_t row =
-                            (((size_t)page * a.kv_heads + hk) * a.page_size + (j % a.page_size)) *
+                            (((size_t)page * a.kv_heads + hk) * a.page_size + (j & in_page)) *
                                 a.head_dim + sub * 8;
                         bt.k[u] = *reinterpret_cast<const uint4*>(a.k_pages + row);
                         bt.v[u] = *reinterpret_cast<const uint4*>(a.v_pages + row);
@@ -357,8 +360,8 @@ __device__ __forceinline__ void unit(const Args& a, int idx, int h, int s,
             const int cnt = min(STREAM_KEYS, k_end - j0);
             const uint32_t fb = st_smem(&stream->full[st]);
             bool bad = false;
-            for (int j = j0; j < j0 + cnt; j += a.page_size - j % a.page_size) {
-                const int page = sh_pages[j / a.page_size - first_page];
+            for (int j = j0; j < j0 + cnt; j += a.page_size - (j & in_page)) {
+                const int page = sh_pages[(j >> shift) - first_page];
                 if (page < 0 || page >= a.num_pages) {
                     prb_set_status(a.status, PRB_S_PAGE_RANGE, t, j, page);
                     bad = true;
@@ -372,9 +375,9 @@ __device__ __forceinline__ void unit(const Args& a, int idx, int h, int s,
             st_mbar_expect_tx(fb, 2u * cnt * row_bytes);
             const uint32_t kd = ring + st * stage_bytes, vd = kd + STREAM_KEYS * row_bytes;
             for (int j = j0; j < j0 + cnt;) {
-                const int off = j % a.page_size;
+                const int off = j & in_page;
                 const int n = min(a.page_size - off, j0 + cnt - j);
-                const int page = sh_pages[j / a.page_size - first_page];
+                const int page = sh_pages[(j >> shift) - first_page];
                 const size_t row = (((size_t)page * a.kv_heads + hk) * a.page_size + off) * a.head_dim;
                 st_bulk_copy(kd + (j - j0) * row_bytes, a.k_pages + row, n * row_bytes, fb);
                 st_bulk_copy(vd + (j - j0) * row_bytes, a.v_pages + row, n * row_bytes, fb);
