@@ -342,8 +342,7 @@ gemm_f32_stream_kernel(Args p, StreamGeo g, const __grid_constant__ CUtensorMap 
 }
 
 // ------------------------------------------------------------------------- many rows
-int g_tile_runs = 0;                // (for measurements: 1, 2 or 4 runs a CTA; 0: the rule below)
-constexpr int TILE_STAGES = 2;      // (a chunk's FMAs take several times its copies' way)
+int g_tile_runs = 0;                // (for measurements: 1 or 2 runs a CTA of 64 x 128; 0: the rule below)
 
 // {32 floats, rows} of a row-major [rows, k] matrix, 128-byte swizzle, zeros beyond both; x is a
 // multiple of 32 floats, so the 16-byte rule on it holds.
@@ -401,9 +400,10 @@ __device__ __forceinline__ float add_pair(pair_t v) {
 template <int BM, int BN, int TM, int TN, int RUNS> struct TileCfg {
     static constexpr int THREADS = (BM / TM) * (BN / TN);
     static constexpr int STAGE = (BM + BN) * CH;              // floats
-    static constexpr int HELD = RUNS / 2;                     // runs' sums set aside
+    static constexpr int STAGES = BN > 64 ? 2 : 4;            // (of 24 KB: a chunk's FMAs take several times its copies' way)
+    static constexpr int HELD = RUNS - 1;                     // runs' sums set aside
     static constexpr int OUT_LD = BN + 4;
-    static constexpr int RING = TILE_STAGES * STAGE > BM * OUT_LD ? TILE_STAGES * STAGE : BM * OUT_LD;
+    static constexpr int RING = STAGES * STAGE > BM * OUT_LD ? STAGES * STAGE : BM * OUT_LD;
     static constexpr size_t SMEM = 1024 + sizeof(float) * ((size_t)RING + (size_t)HELD * BM * BN);
 };
 
@@ -412,7 +412,8 @@ template <int BM, int BN, int TM, int TN, int COPY, int RUNS>
 __global__ void __cluster_dims__(4 / RUNS, 1, 1) __launch_bounds__((BM / TM) * (BN / TN), TM * TN <= 32 ? 3 : 2)
 gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w) {
     using Cfg = TileCfg<BM, BN, TM, TN, RUNS>;
-    constexpr int NT = Cfg::THREADS, CL = 4 / RUNS;
+    constexpr int NT = Cfg::THREADS, CL = 4 / RUNS, TILE_STAGES = Cfg::STAGES;
+    static_assert(RUNS == 1 || RUNS == 2, "one run or two");
     constexpr int TY = BM / TM, TX = BN / TN;
     static_assert(TX % 8 == 0 && TY % 8 == 0, "a warp is 8 columns by 4 rows of threads; a thread's rows share a swizzle");
     extern __shared__ __align__(16) uint8_t tile_raw[];
@@ -420,7 +421,7 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
     __shared__ int failed_word;
     volatile int* failed = &failed_word;
     float* smem = reinterpret_cast<float*>(((uintptr_t)tile_raw + 1023) & ~(uintptr_t)1023);
-    float* held = smem + Cfg::RING;                           // [HELD][TM * TN][NT]
+    float* held = smem + Cfg::RING;                           // [TM * TN][NT]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tx = (warp % (TX / 8)) * 8 + (lane & 7);
     const int ty = (warp / (TX / 8)) * 4 + (lane >> 3);
@@ -528,26 +529,16 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
             if (COPY != COPY_TMA) cp_commit();
         }
         // two runs are added, then the two sums of two
-        if constexpr (RUNS > 1) {
-            float* mine = held + (RUNS == 4 && r == 2 ? BM * BN : 0) + tid;
-            if (RUNS == 4 && r == 1) {
+        if constexpr (RUNS == 2) {
+            float* mine = held + tid;
 #pragma unroll
-                for (int i = 0; i < TM * TN; ++i) mine[i * NT] = mine[i * NT] + sum[i / TN][i % TN];
-            } else if ((r & 1) == 0) {
-#pragma unroll
-                for (int i = 0; i < TM * TN; ++i) mine[i * NT] = sum[i / TN][i % TN];
-            } else {
-                float* second = held + (RUNS == 4 ? BM * BN : 0) + tid;
-#pragma unroll
-                for (int i = 0; i < TM * TN; ++i) {
-                    float t = second[i * NT] + sum[i / TN][i % TN];
-                    if (RUNS == 4) t = held[i * NT + tid] + t;
-                    sum[i / TN][i % TN] = t;
+            for (int i = 0; i < TM * TN; ++i) {
+                if (r == 0) {
+                    mine[i * NT] = sum[i / TN][i % TN];
+                    sum[i / TN][i % TN] = 0.0f;
+                } else {
+                    sum[i / TN][i % TN] = mine[i * NT] + sum[i / TN][i % TN];
                 }
-            }
-            if (r < RUNS - 1) {
-#pragma unroll
-                for (int i = 0; i < TM * TN; ++i) sum[i / TN][i % TN] = 0.0f;
             }
         }
     }
@@ -564,8 +555,7 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
     for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) smem[(ty + i * TY) * Cfg::OUT_LD + tx + j * TX] = sum[i][j];
-    if (CL > 1) cluster_sync_all();
-    else __syncthreads();
+    cluster_sync_all();
     // a part of the rows, four columns at a time; all remote reads are asked for at once (one
     // after the other they cost 25 us a 128 x 128 tile, twice the tile's FMAs)
     constexpr int ROWS = BM / CL, PER = ROWS * (BN / 4) / NT, AT_ONCE = PER < 4 ? PER : 4;
@@ -578,10 +568,9 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
 #pragma unroll
         for (int i = 0; i < AT_ONCE; ++i) {
             const int e = tid + (i0 + i) * NT;
-            const float* at = smem + (r0 + e / (BN / 4)) * Cfg::OUT_LD + (e % (BN / 4)) * 4;
+            const uint32_t at = smem_u32(smem + (r0 + e / (BN / 4)) * Cfg::OUT_LD + (e % (BN / 4)) * 4);
 #pragma unroll
-            for (int q = 0; q < CL; ++q)
-                v[i][q] = CL > 1 ? ld_cluster4(smem_u32(at), q) : *reinterpret_cast<const float4*>(at);
+            for (int q = 0; q < CL; ++q) v[i][q] = ld_cluster4(at, q);
         }
 #pragma unroll
         for (int i = 0; i < AT_ONCE; ++i) {
@@ -591,7 +580,7 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
             float4 x = v[i][0];
             if constexpr (CL == 2) {
                 x = make_float4(x.x + v[i][1].x, x.y + v[i][1].y, x.z + v[i][1].z, x.w + v[i][1].w);
-            } else if constexpr (CL == 4) {
+            } else {
                 const float4 y = v[i][1], z = v[i][2], w = v[i][3];
                 x = make_float4((x.x + y.x) + (z.x + w.x), (x.y + y.y) + (z.y + w.y),
                                 (x.z + y.z) + (z.z + w.z), (x.w + y.w) + (z.w + w.w));
@@ -609,10 +598,8 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
             }
         }
     }
-    if (CL > 1) {
-        __syncwarp();
-        cluster_sync_all();                                   // nobody leaves while its tile is read
-    }
+    __syncwarp();
+    cluster_sync_all();                                       // nobody leaves while its tile is read
 }
 
 template <int BM, int BN, int TM, int TN, int COPY, int RUNS>
@@ -639,18 +626,20 @@ int launch_tile(const Args& p, int copy, cudaStream_t stream) {
            : copy == COPY_16 ? launch_tile_by<BM, BN, TM, TN, COPY_16, 1>(p, stream)
                              : launch_tile_by<BM, BN, TM, TN, COPY_4, 1>(p, stream);
 }
-// Runs a CTA takes, of tiles of 64 x 128.
+// Runs a CTA of 64 x 128 takes.  Two halve what a tile costs besides its FMAs (first copies, parts
+// through the cluster, about one and a half chunks' time) but leave half as many CTAs to deal out: the rule counts rounds
+// of two CTAs an SM, the last one cheaper where an SM has one CTA alone.  One run / two, us: 690 x 50,257 x
+// 768 1,465 / 1,304, 1,000 x 2,304 110 / 95, 690 x 3,072 98 / 95; 300 x 2,304 41 / 50, 1,000 x 768 41 / 50.
+// (All four runs in a CTA leave room for one an SM: 1,831.)
 int tile_runs(long tiles, int k) {
     if (g_tile_runs > 0) return g_tile_runs;
     const int run = ((k + CH - 1) / CH + 3) / 4;
-    const long slots = 2L * prb_sm_count();
-    int best = 1;
-    double least = 0.0;
-    for (int runs = 1; runs <= 4; runs *= 2) {
-        const double t = (double)((tiles * (4 / runs) + slots - 1) / slots) * (runs * run + 1.5);
-        if (runs == 1 || t < least) { least = t; best = runs; }
-    }
-    return best;
+    const long sms = prb_sm_count(), slots = 2 * sms;
+    auto rounds = [&](int runs) {
+        const long ctas = tiles * (4 / runs), rest = ctas % slots;
+        return ((double)(ctas / slots) + (rest == 0 ? 0.0 : rest <= sms ? 0.6 : 1.0)) * (runs * run + 1.5);
+    };
+    return rounds(2) < rounds(1) ? 2 : 1;
 }
 
 constexpr size_t STREAM_SMEM = 220 * 1024;                    // the most a launch of the stream kernel takes
@@ -746,19 +735,15 @@ PRB_API int prb_gemm_f32(float* c, const float* a, const float* w, const float* 
     }
     // (rows that overlap are no tensor that a copy engine's map describes)
     const int tiled = !vec ? COPY_4 : ldw >= k && lda >= k ? COPY_TMA : COPY_16;
-    // 64 x 128 where that leaves no SM without a CTA twice over (1.49 against 1.56 ms at 650 x 50,257
-    // x 768, 111 and 111 us at 1,000 x 2,304 x 768), else 64 x 64 (650 x 768 x 768: 28 us, tiles of
-    // 128 x 64 54 us).
+    // 64 x 128 where that gives most SMs two CTAs (690 x 768 x 768 28 us against 33, 690 x 768 x 3,072
+    // 91 against 109), else 64 x 64 (300 x 768 x 768 21 us against 23, 300 x 768 x 3,072 72 against 74).
     const long big = (long)((m + 63) / 64) * ((n + 127) / 128);
-    if (which == 3 || (which != 2 && big * 4 < 2 * prb_sm_count())) return launch_tile<64, 64, 8, 4, 1>(p, tiled, stream);
-    switch (tile_runs(big, k)) {
-        case 1: return launch_tile<64, 128, 8, 8, 1>(p, tiled, stream);
-        case 2: return launch_tile<64, 128, 8, 8, 2>(p, tiled, stream);
-        default: return launch_tile<64, 128, 8, 8, 4>(p, tiled, stream);
-    }
+    if (which == 3 || (which != 2 && big * 8 < 3 * prb_sm_count())) return launch_tile<64, 64, 8, 4, 1>(p, tiled, stream);
+    return tile_runs(big, k) == 2 ? launch_tile<64, 128, 8, 8, 2>(p, tiled, stream)
+                                  : launch_tile<64, 128, 8, 8, 1>(p, tiled, stream);
 }
 PRB_API int prb_gemm_f32_tune(int runs) {
-    if (runs != 0 && runs != 1 && runs != 2 && runs != 4) return PRB_E_SIZE;
+    if (runs < 0 || runs > 2) return PRB_E_SIZE;
     g_tile_runs = runs;
     return 0;
 }
