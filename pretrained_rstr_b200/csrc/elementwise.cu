@@ -59,37 +59,12 @@ __global__ void layernorm_kernel(elementwise::NormArgs a) {
     elementwise::layernorm_row<O>(a, blockIdx.x, row, scratch);
 }
 
-// Rows that fit a warp's registers (width <= 1024 with NV = 8 pieces a lane, <= 2048 with 16; a
-// multiple of 4): one warp per row, four rows per CTA, 16-byte loads, statistics by shuffles only.
-// Same two-pass formula.  Bound by the row's one way from memory; a block a row with its row in
-// shared memory and four block barriers took 12.0 us at 2,193 x 1,600 (21 MB), this 9.2.
-template <typename O, int NV>
-__global__ void __launch_bounds__(128)
-layernorm_warp_kernel(elementwise::NormArgs a) {
-    const int r = blockIdx.x * 4 + (threadIdx.x >> 5);
+// Row r by one warp, in its registers: 16-byte loads, statistics by shuffles only, two passes.  gamma and
+// beta give the parameters of the lane's i-th piece, columns 4 idx ..
+template <typename O, int NV, typename G, typename B>
+__device__ __forceinline__ void norm_row_of_warp(const elementwise::NormArgs& a, int r, const G& gamma, const B& beta) {
     const int lane = threadIdx.x & 31;
     const int nvec = a.width / 4;
-    // gamma and beta (settled, or the launch is not early) are asked for first, not after the
-    // statistics: the row's way through the kernel is one memory round trip long instead of two.
-    // (With 16 pieces they would take the registers of every second warp, and come from the L1
-    // afterwards.)
-    constexpr bool AHEAD = NV <= 8;
-    const float4* g4 = reinterpret_cast<const float4*>(a.gamma);
-    const float4* b4 = reinterpret_cast<const float4*>(a.beta);
-    float4 g[AHEAD ? NV : 1], b[AHEAD ? NV : 1];
-    if constexpr (AHEAD) {
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const int idx = lane + 32 * i;
-            g[i] = idx < nvec ? __ldg(g4 + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
-            b[i] = (idx < nvec && a.beta) ? __ldg(b4 + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    }
-    prb_grid_wait();
-    // (signalled from the top, an early norm lets its product in beside the kernel ahead: 64 requests
-    // decoding 7.31 -> 7.95 ms for 8 steps)
-    prb_grid_launch_dependents();
-    if (r >= a.n_rows) return;
     O* out = reinterpret_cast<O*>(a.out) + (size_t)r * a.width;
     const int src = a.rows ? a.rows[r] : r;
     if (src < 0 || src >= a.n_rows_in) {
@@ -122,8 +97,7 @@ layernorm_warp_kernel(elementwise::NormArgs a) {
     for (int i = 0; i < NV; ++i) {
         const int idx = lane + 32 * i;
         if (idx < nvec) {
-            const float4 gv = AHEAD ? g[AHEAD ? i : 0] : __ldg(g4 + idx);
-            const float4 bv = AHEAD ? b[AHEAD ? i : 0] : a.beta ? __ldg(b4 + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 gv = gamma(idx, i), bv = beta(idx, i);
             const float y0 = (v[i].x - mean) * inv * gv.x + bv.x, y1 = (v[i].y - mean) * inv * gv.y + bv.y;
             const float y2 = (v[i].z - mean) * inv * gv.z + bv.z, y3 = (v[i].w - mean) * inv * gv.w + bv.w;
             if constexpr (sizeof(O) == 4) {
@@ -137,6 +111,70 @@ layernorm_warp_kernel(elementwise::NormArgs a) {
             }
         }
     }
+}
+
+// Rows that fit a warp's registers (width <= 1024 with NV = 8 pieces a lane, <= 2048 with 16; a
+// multiple of 4): one warp per row, four rows per CTA, 16-byte loads, statistics by shuffles only.
+// Same two-pass formula.  Bound by the row's one way from memory; a block a row with its row in
+// shared memory and four block barriers took 12.0 us at 2,193 x 1,600 (21 MB), this 9.2.
+template <typename O, int NV>
+__global__ void __launch_bounds__(128)
+layernorm_warp_kernel(elementwise::NormArgs a) {
+    const int r = blockIdx.x * 4 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    const int nvec = a.width / 4;
+    // gamma and beta (settled, or the launch is not early) are asked for first, not after the
+    // statistics: the row's way through the kernel is one memory round trip long instead of two.
+    // (With 16 pieces they would take the registers of every second warp, and come from the L1
+    // afterwards.)
+    constexpr bool AHEAD = NV <= 8;
+    const float4* g4 = reinterpret_cast<const float4*>(a.gamma);
+    const float4* b4 = reinterpret_cast<const float4*>(a.beta);
+    float4 g[AHEAD ? NV : 1], b[AHEAD ? NV : 1];
+    if constexpr (AHEAD) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int idx = lane + 32 * i;
+            g[i] = idx < nvec ? __ldg(g4 + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
+            b[i] = (idx < nvec && a.beta) ? __ldg(b4 + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    prb_grid_wait();
+    // (signalled from the top, an early norm lets its product in beside the kernel ahead: 64 requests
+    // decoding 7.31 -> 7.95 ms for 8 steps)
+    prb_grid_launch_dependents();
+    if (r >= a.n_rows) return;
+    norm_row_of_warp<O, NV>(
+        a, r, [&](int idx, int i) { return AHEAD ? g[AHEAD ? i : 0] : __ldg(g4 + idx); },
+        [&](int idx, int i) {
+            return AHEAD ? b[AHEAD ? i : 0] : a.beta ? __ldg(b4 + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
+        });
+}
+
+// The same for the rows of a prompt (more than 128): one CTA of sixteen warps an SM, a row a warp at a
+// time.  What bounds such a launch is not its bytes (3 us of 9.5 at 2,193 x 1,600) but its way: the start
+// behind the product ahead, one memory round trip, the parameters, the stores.  Many CTAs of four warps
+// cannot be placed early (they crowd on the SMs that the product leaves first); one an SM can: its
+// shared memory, more than half of an SM's, keeps a second one away.  It brings gamma and beta there while
+// the product ends.
+constexpr int ROWS_THREADS = 512;
+constexpr int ROWS_SMEM = 116 * 1024;
+template <typename O, int NV>
+__global__ void __launch_bounds__(ROWS_THREADS, 1)
+layernorm_rows_kernel(elementwise::NormArgs a) {
+    extern __shared__ __align__(16) float norm_gb[];               // gamma, beta
+    const int lane = threadIdx.x & 31, nvec = a.width / 4;
+    float4* gb = reinterpret_cast<float4*>(norm_gb);
+    for (int i = threadIdx.x; i < nvec; i += ROWS_THREADS) {
+        gb[i] = __ldg(reinterpret_cast<const float4*>(a.gamma) + i);
+        gb[nvec + i] = a.beta ? __ldg(reinterpret_cast<const float4*>(a.beta) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    prb_grid_wait();
+    prb_grid_launch_dependents();
+    __syncthreads();
+    for (long r = (long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; r < a.n_rows; r += (ROWS_THREADS / 32) * (long)gridDim.x)
+        norm_row_of_warp<O, NV>(a, (int)r, [&](int idx, int) { return gb[idx]; },
+                                [&](int idx, int) { return gb[nvec + idx]; });
 }
 
 // settled: gamma and beta were written long before (by no kernel of the step): only then may the
@@ -153,10 +191,29 @@ PRB_API int prb_layernorm(void* out, const float* x, const float* gamma, const f
     // (also one row: 2.6 us against 3.7 of the block-a-row kernel, and a row's bits do not depend on
     // how many there are)
     if (width % 4 == 0 && width <= 2048 && aligned) {
-        const int blocks = (n_rows + 3) / 4;
-        // the few rows of a decoding batch start while the product before them ends
-        const bool early = settled && (n_rows <= 128 || prb_small_ctas_early());
         cudaError_t e;
+        if (n_rows > 128) {
+#define PRB_LN_ROWS(OT, NV)                                                                        \
+    do {                                                                                           \
+        constexpr auto kernel = layernorm_rows_kernel<OT, NV>;                                     \
+        e = prb_allow_shared<kernel>(ROWS_SMEM);                                                   \
+        if (e == cudaSuccess)                                                                      \
+            e = prb_launch_maybe_early(settled != 0, kernel, dim3(n_rows < prb_sm_count() ? n_rows : prb_sm_count()), \
+                                       dim3(ROWS_THREADS), ROWS_SMEM, stream, a);                  \
+    } while (0)
+            if (out_dtype == PRB_F32) {
+                if (width <= 1024) PRB_LN_ROWS(float, 8);
+                else PRB_LN_ROWS(float, 16);
+            } else {
+                if (width <= 1024) PRB_LN_ROWS(__nv_bfloat16, 8);
+                else PRB_LN_ROWS(__nv_bfloat16, 16);
+            }
+#undef PRB_LN_ROWS
+            return e == cudaSuccess ? 0 : (int)e;
+        }
+        // the few rows of a decoding batch start while the product before them ends
+        const int blocks = (n_rows + 3) / 4;
+        const bool early = settled != 0;
 #define PRB_LN(OT)                                                                               \
     e = width <= 1024 ? prb_launch_maybe_early(early, layernorm_warp_kernel<OT, 8>, dim3(blocks), \
                                                dim3(128), 0, stream, a)                          \

@@ -1,0 +1,85 @@
+"""Kernels whose work is dealt out by the sizes of a launch, at the sizes where that turns: strips and
+pieces of the weight-streaming product, runs of K of the 32-bit tiles, rows of the norm."""
+import pytest
+import torch
+
+from test_kernels_gpu import _ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
+@pytest.mark.parametrize("n,k", [(16, 64), (4736, 64), (4737, 128), (9473, 768), (50257, 768), (2368, 2048),
+                                 (300, 6400), (4800, 1600)])
+@pytest.mark.parametrize("norm", [False, True])
+def test_weight_streaming_product_of_many_strips(m, n, k, norm):
+    """One strip a CTA, a second one for some, many; a ring that is used again; pieces of a strip."""
+    ops = _ops()
+    if norm and k > ops.smallm_limits()[1]:
+        pytest.skip("too wide for the fused norm")
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    w = (torch.randn(n, k, device="cuda", generator=g) * 0.1).to(torch.bfloat16)
+    bias = torch.randn(n, device="cuda", generator=g)
+    out = torch.full((m, n), float("nan"), device="cuda")
+    if norm:
+        x = torch.randn(m, k, device="cuda", generator=g) * 2.0 + 0.5
+        gamma, beta = torch.rand(k, device="cuda", generator=g) + 0.5, torch.randn(k, device="cuda", generator=g)
+        ops.gemm_smallm(out, w, norm_input=x, gamma=gamma, beta=beta, eps=1e-6, bias=bias)
+        a = torch.nn.functional.layer_norm(x, (k,), gamma, beta, 1e-6).to(torch.bfloat16)
+    else:
+        a = (torch.randn(m, k, device="cuda", generator=g) * 0.5).to(torch.bfloat16)
+        resid = torch.randn(m, n, device="cuda", generator=g)
+        out.copy_(resid)
+        ops.gemm_smallm(out, w, a=a, bias=bias, resid=out)
+        bias = bias + resid
+    ref = a.float() @ w.float().t() + bias
+    # without the norm only the order of 32-bit sums differs; a normed number may round to the other
+    # of two neighbouring bfloat16 numbers (2^-8 of it) in either
+    tol = 3e-2 if norm else 2e-4
+    assert float((out - ref).abs().max()) <= tol * max(1.0, float(ref.abs().max()))
+
+
+@pytest.mark.parametrize("m,n,k", [(17, 1, 1), (64, 128, 32), (65, 129, 128), (129, 257, 132), (100, 300, 260),
+                                   (130, 512, 768)])
+def test_float32_tiles_of_one_and_of_two_runs_a_cta_give_the_same_bits(m, n, k):
+    """Also with runs of K that are empty, and with rows that no copy engine's map describes."""
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randn(m, k, device="cuda", generator=g)
+    wide = torch.randn(n, k + 1, device="cuda", generator=g)
+    resid = torch.randn(m, n, device="cuda", generator=g)
+    out = []
+    try:
+        for runs in (1, 2):
+            assert ops.lib().prb_gemm_f32_tune(runs) == 0
+            for w in (wide[:, :k].contiguous(), wide[:, :k]):
+                out.append(torch.full((m, n), float("nan"), device="cuda"))
+                ops.gemm_f32(out[-1], a, w, resid=resid, kernel=2)
+    finally:
+        ops.lib().prb_gemm_f32_tune(0)
+    few = torch.full((m, n), float("nan"), device="cuda")
+    for i in range(0, m, 16):
+        ops.gemm_f32(few[i:i + 16], a[i:i + 16], wide[:, :k].contiguous(), resid=resid[i:i + 16].contiguous())
+    for other in out[1:] + [few]:
+        assert torch.equal(out[0], other)
+
+
+@pytest.mark.parametrize("rows", [128, 129, 149, 2368, 2369, 5000])
+@pytest.mark.parametrize("width", [4, 768, 1024, 1028, 1600, 2048])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_norm_of_many_rows(rows, width, dtype):
+    """More than 128 rows by the kernel of a CTA an SM: the same bits as a few at a time, and right."""
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(rows + width)
+    x = torch.randn(rows, width, device="cuda", generator=g) * 3.0 + 1.0
+    gamma, beta = torch.randn(width, device="cuda", generator=g), torch.randn(width, device="cuda", generator=g)
+    out = torch.full((rows, width), float("nan"), device="cuda", dtype=dtype)
+    few = torch.full_like(out, float("nan"))
+    ops.layernorm(out, x, gamma, beta, 1e-5)
+    for i in range(0, rows, 100):
+        ops.layernorm(few[i:i + 100], x[i:i + 100], gamma, beta, 1e-5)
+    assert torch.equal(out, few)
+    ref = torch.nn.functional.layer_norm(x.double(), (width,), gamma.double(), beta.double(), 1e-5)
+    # 32-bit statistics of rows around 1: a few roundings of 2^-24 of numbers up to 3, or bfloat16's own
+    tol = 1e-5 if dtype == torch.float32 else 2.0 ** -8
+    assert bool(((out.double() - ref).abs() <= tol * (1.0 + ref.abs())).all())
