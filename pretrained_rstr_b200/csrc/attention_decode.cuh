@@ -50,7 +50,9 @@ struct Args {
     int* counters;
     int max_splits;
     int split;                      // keys per split: a multiple of SPLIT
-    int page_shift;                 // page_size is 1 << page_shift (it divides SPLIT): no quotient a key
+    int page_shift;                 // page_size is 1 << page_shift (it divides SPLIT): no quotient a key.
+                                    // (With one, and the look-ups one after the other, 16 steps of GPT-2 small
+                                    // took 4.73 ms at one request and 5.63 at eight; 4.52 and 5.43 so.)
     int hpg;                        // query heads per key/value head
     int* status;
 };

@@ -116,7 +116,8 @@ PRB_API int prb_attention_decode_ring_supports(int head_dim, int page_size) {
 PRB_API int prb_attention_decode_ring_max_list() { return MAX_LIST; }
 
 // Whether this kernel is the faster one for a launch of n_list tokens over contexts of up to
-// max_context keys; the split-key kernel of attention_decode.cu is the other.  Measured inside
+// max_context keys; the split-key kernel of attention_decode.cu is the other.  Measured (with the
+// look-ups and the merge of both as they were) inside
 // whole decode steps, ms a step, split-key / ring, at contexts of 250, 500 and 900 tokens (n_list is
 // the capacity the step's graph was made for, so 24 requests run as 32 and 48 as 64).
 // GPT-2 small, 12 heads: 1 request 0.326 / 0.332, 0.330 / 0.334, 0.348 / 0.351; 8: 0.338 / 0.354,
@@ -131,7 +132,9 @@ PRB_API int prb_attention_decode_ring_max_list() { return MAX_LIST; }
 // 3.528.
 // The ring wins where many (token, head) pairs have long contexts (its warps stream long runs,
 // the other kernel's CTAs walk their keys one batch after the other) and in the middle range at
-// nearly every context; it loses at few requests.
+// nearly every context; it loses at few requests.  Since its look-ups go side by side and its merge takes one
+// round, also at 8 requests of XL with more than 512 keys (450 to 900 tokens: 4 steps 9.82 ms by the
+// split-key kernel, 9.38 by this one), while 8 requests of GPT-2 small are level (16 steps 6.08 and 6.08).
 PRB_API int prb_attention_decode_ring_prefers(int n_list, int n_heads, int max_context) {
     const long pairs = (long)n_list * n_heads;
     const long sms = prb_sm_count();

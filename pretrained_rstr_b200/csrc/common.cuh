@@ -152,11 +152,11 @@ int prb_pdl_enabled();
 // that sizes a grid or counts waves takes the number from here.
 int prb_sm_count();
 
-// Kernels of many small CTAs (a prompt's norms, the attention kernels but the ring) are not placed
+// Kernels of many small CTAs (the attention kernels but the ring) are not placed
 // early: their CTAs would fill the few SMs that the predecessor leaves free, several to an SM, instead
 // of spreading over all of them when it has ended, and then run at the pace of those SMs (measured: a
 // prompt step of 256 to 1,024 tokens is 6 % slower with them placed early).  With no more than a CTA
-// or two an SM they are: norms of up to 128 rows, the 32-bit attention and products of a small step,
+// or two an SM they are: the norms, the 32-bit attention and products of a small step,
 // the small kernels of Musilorn's decode step (each says so where it is launched).  They still
 // call prb_grid_launch_dependents(), so that a successor of one CTA per SM sets itself up
 // while they run.  prb_small_ctas_early() is the switch for measurements.

@@ -156,7 +156,8 @@ layernorm_warp_kernel(elementwise::NormArgs a) {
 // behind the product ahead, one memory round trip, the parameters, the stores.  Many CTAs of four warps
 // cannot be placed early (they crowd on the SMs that the product leaves first); one an SM can: its
 // shared memory, more than half of an SM's, keeps a second one away.  It brings gamma and beta there while
-// the product ends.
+// the product ends.  Prompts of 2,193 tokens of GPT-2 XL (96 norms) 8.19 -> 7.89 ms, one of 137 tokens of
+// GPT-2 small (24) 0.532 -> 0.526.
 constexpr int ROWS_THREADS = 512;
 constexpr int ROWS_SMEM = 116 * 1024;
 template <typename O, int NV>

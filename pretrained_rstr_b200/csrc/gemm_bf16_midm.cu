@@ -200,6 +200,7 @@ gemm_midm_kernel(Args a, const __grid_constant__ CUtensorMap map_a,
         for (int i = 0; i < first; ++i) issue_w(i);
     // What takes quotients of run-time counts is worked out before the wait, not between the last
     // multiplication and the store: where this warp's rows go, and where a column lies in the cache.
+    // (23 rows: 1,024 x 4,096 7.8 -> 7.05 us, 3,072 x 1,024 7.0 -> 6.3; 64 rows: 768 x 3,072 6.4 -> 5.9.)
     const int per = (int)((unsigned)(MROWS + S - 1) / (unsigned)S);      // rows of a CTA
     uint32_t part_dst[2];
 #pragma unroll

@@ -15,17 +15,19 @@
 // cp.async; the first of them, where the caller says that the weights are settled, before the kernel
 // ahead has ended); a thread keeps its chunk of up to four rows of A in registers and walks the
 // weight rows of a stage, so an FMA costs a quarter of a shared-memory operand; chunk sums meet in
-// shared memory.  8 rows, weights from memory: 2,304 x 768 6.8 us, 768 x 3,072 10.4 us, 50,257 x 768
-// 72 us = 2.15 TB/s; one CTA a tile of 64 x 64 (12 CTAs for 768 columns) takes 177 us on average over
-// a model's products.
+// shared memory.  The rows of A come by asynchronous copies, all at once, and what the sums are finished
+// with (quotients of run-time counts, bias, residual) is there before them: 8 rows, 2,304 x 768 7.1 -> 6.1 us,
+// 768 x 768 5.1 -> 4.3, 3,072 x 768 8.6 -> 7.6, 768 x 3,072 10.4 -> 8.3, 50,257 x 768 84 -> 77 us = 2.0 TB/s; one
+// CTA a tile of 64 x 64 (12 CTAs for 768 columns) takes 177 us on average over a model's products.
 //
-// gemm_f32_tile_kernel: more rows.  Tiles of BM x BN, the four runs of K by the four CTAs of a cluster
-// (a prompt of a few hundred tokens has too few tiles for 148 SMs otherwise), partial tiles added
-// through distributed shared memory, a quarter of the rows a CTA.  650 rows: 2,304 x 768 76 us, 768 x
-// 3,072 106 us, 50,257 x 768 1.49 ms = 34 TFLOP/s; one CTA a tile over all of K 14 TFLOP/s.  What bounds
-// it: 255 registers leave two CTAs of four warps an SM, whose schedulers issue in 42 % of the cycles
-// (an instruction every 4.35 cycles a warp: 1.2 of fixed latency, 0.5 for the FMA pipe, 0.4 for shared
-// memory); neither the FMA units nor shared memory are half busy (counters at 650 x 2,304 x 768).
+// gemm_f32_tile_kernel: more rows.  Tiles of BM x BN, the four runs of K by the CTAs of a cluster, one or
+// two each (a prompt of a few hundred tokens has too few tiles for 148 SMs otherwise), partial tiles added
+// through distributed shared memory, a part of the rows a CTA.  Stages come by TMA where the rows allow
+// it; a chunk's row is 128 bytes, its 16-byte pieces swizzled.  690 rows: 2,304 x 768 77 -> 75 us, 3,072 x 768
+// 101 -> 95, 768 x 768 31 -> 28, 768 x 3,072 106 -> 91, 50,257 x 768 1.50 -> 1.31 ms = 41 TFLOP/s; one CTA a tile
+// over all of K 14 TFLOP/s.  What bounds it: the FMA loop.  fma.rn.f32x2 of operands in three registers
+// runs at 57 TFLOP/s (72 with two), 8 x 8 outputs a thread read 16 bytes of shared memory for 8 of them,
+// which is the most that shared memory gives, and 255 registers leave two warps a scheduler to overlap the two.
 #include "common.cuh"
 #include "tcgen05.cuh"
 #include "tensor_map.cuh"
@@ -430,6 +432,8 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
     const int nc = (p.k + CH - 1) / CH, run = (nc + 3) / 4;
     const int c0 = min(nc, part * RUNS * run), c1 = min(nc, c0 + RUNS * run);
     if (COPY == COPY_TMA && tid == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
         for (int s = 0; s < TILE_STAGES; ++s) mbar_init(smem_u32(&bars[s]), 1);
         *failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -735,10 +739,13 @@ PRB_API int prb_gemm_f32(float* c, const float* a, const float* w, const float* 
     }
     // (rows that overlap are no tensor that a copy engine's map describes)
     const int tiled = !vec ? COPY_4 : ldw >= k && lda >= k ? COPY_TMA : COPY_16;
-    // 64 x 128 where that gives most SMs two CTAs (690 x 768 x 768 28 us against 33, 690 x 768 x 3,072
-    // 91 against 109), else 64 x 64 (300 x 768 x 768 21 us against 23, 300 x 768 x 3,072 72 against 74).
-    const long big = (long)((m + 63) / 64) * ((n + 127) / 128);
-    if (which == 3 || (which != 2 && big * 8 < 3 * prb_sm_count())) return launch_tile<64, 64, 8, 4, 1>(p, tiled, stream);
+    // 64 x 128 where that leaves no SM without a CTA twice over, or nearly two an SM in one round of
+    // clusters (66 tiles: 690 x 768 x 768 28 us against 33, 690 x 768 x 3,072 91 against 109; 72 tiles take a
+    // second round: 137 x 3,072 x 768 39.5 against 36); else 64 x 64 (30 tiles: 300 x 768 x 768 21 us
+    // against 23, 300 x 768 x 3,072 72 against 74).
+    const long big = (long)((m + 63) / 64) * ((n + 127) / 128), sms = prb_sm_count();
+    const bool wide = big * 2 >= sms || (big * 8 >= 3 * sms && big * 20 <= 9 * sms);
+    if (which == 3 || (which != 2 && !wide)) return launch_tile<64, 64, 8, 4, 1>(p, tiled, stream);
     return tile_runs(big, k) == 2 ? launch_tile<64, 128, 8, 8, 2>(p, tiled, stream)
                                   : launch_tile<64, 128, 8, 8, 1>(p, tiled, stream);
 }
