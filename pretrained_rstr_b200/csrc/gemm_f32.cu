@@ -48,7 +48,30 @@ struct Args {
     int act;
     bool settled;                   // w may be read before the kernel ahead has ended
     int* status;
+    // Columns of a fused QKV product that also go to the paged cache ([q_width, q_width + kv_width) are
+    // keys, the next kv_width values); kv_width == 0: none.
+    float* k_pages;                 // [pages][kv heads][page_size][head_dim]
+    float* v_pages;
+    const int* slots;               // cache slot of each row, -1 = none
+    int q_width, kv_width, head_dim, page_size, num_pages;
 };
+
+// Where (row, col) also goes in the cache, or null.
+__device__ __forceinline__ float* cache_place(const Args& p, int row, int col) {
+    if (p.kv_width == 0 || col < p.q_width) return nullptr;
+    const int slot = p.slots[row];
+    if (slot < 0) return nullptr;
+    const unsigned page = (unsigned)slot / (unsigned)p.page_size, off = (unsigned)slot - page * p.page_size;
+    if ((int)page >= p.num_pages) {
+        prb_set_status(p.status, PRB_S_SLOT_RANGE, row, slot, p.num_pages);
+        return nullptr;
+    }
+    unsigned c = (unsigned)(col - p.q_width);
+    float* pages = c < (unsigned)p.kv_width ? p.k_pages : p.v_pages;
+    if (c >= (unsigned)p.kv_width) c -= p.kv_width;
+    const unsigned h = c / (unsigned)p.head_dim, d = c - h * p.head_dim;
+    return pages + (size_t)page * p.kv_width * p.page_size + ((size_t)h * p.page_size + off) * p.head_dim + d;
+}
 
 using tc5::mbar_expect_tx;
 using tc5::mbar_init;
@@ -259,6 +282,7 @@ gemm_f32_stream_kernel(Args p, StreamGeo g, const __grid_constant__ CUtensorMap 
         const bool fin = fin_q == 0 && fin_i < MB && fin_row < p.m && fin_r < min(g.rows, n1 - (n0 + s * g.rows));
         const float fin_bias = fin && p.bias ? p.bias[fin_col] : 0.0f;
         const float fin_resid = fin && p.resid ? p.resid[(size_t)fin_row * p.ldc + fin_col] : 0.0f;
+        float* const fin_cache = fin ? cache_place(p, fin_row, fin_col) : nullptr;
         if constexpr (COPY == COPY_TMA) {
             alive = alive && mbar_wait(smem_u32(&bars[s % g.stages]), (uint32_t)(s / g.stages) & 1u, failed);
         } else {
@@ -328,6 +352,8 @@ gemm_f32_stream_kernel(Args p, StreamGeo g, const __grid_constant__ CUtensorMap 
                     v = finish(p, sum, row, col);
                 }
                 p.c[(size_t)row * p.ldc + col] = v;
+                float* const cached = t0 == 0 ? fin_cache : cache_place(p, row, col);
+                if (cached != nullptr) *cached = v;
             }
         }
     }
@@ -600,6 +626,18 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
                 for (int d = 0; d < 4; ++d)
                     if (col + d < p.n) out[d] = y[d];
             }
+            if (p.kv_width != 0 && col + 4 > p.q_width) {
+                if (p.q_width % 4 == 0 && p.head_dim % 4 == 0 && ((uintptr_t)p.k_pages | (uintptr_t)p.v_pages) % 16 == 0) {
+                    // (four columns of one head)
+                    float* const cached = col < p.n ? cache_place(p, row, col) : nullptr;
+                    if (cached != nullptr) *reinterpret_cast<float4*>(cached) = make_float4(y[0], y[1], y[2], y[3]);
+                } else {
+                    for (int d = 0; d < 4; ++d) {
+                        float* const cached = col + d < p.n ? cache_place(p, row, col + d) : nullptr;
+                        if (cached != nullptr) *cached = y[d];
+                    }
+                }
+            }
         }
     }
     __syncwarp();
@@ -710,12 +748,20 @@ bool stream_geometry(const Args& p, int mb, int copy, StreamGeo* g, size_t* smem
 // which: 0 the rule below; 1 the stream kernel where it fits, 2 / 3 tiles of 64 x 128, 64 x 64 (the
 // same bits from all of them).  settled: w was written long before (by no kernel of the step), so the
 // launch may be placed, and w read, before the kernel ahead in the stream has ended.
+// kv_width > 0: the product is a fused QKV projection, whose key and value columns also go to the paged
+// cache (float32, contiguous) at slots[row]: the append behind a decode step's product was 2.8 us a layer.
 PRB_API int prb_gemm_f32(float* c, const float* a, const float* w, const float* bias,
                          const float* resid, int m, int n, int k, long lda, long ldw, long ldc,
-                         int act, int which, int settled, int* status, cudaStream_t stream) {
+                         int act, int which, int settled, float* k_pages, float* v_pages,
+                         const int* slots, int q_width, int kv_width, int head_dim, int page_size,
+                         int num_pages, int* status, cudaStream_t stream) {
     if (m <= 0 || n <= 0) return 0;
     if (k <= 0) return PRB_E_SIZE;
-    const Args p{c, a, w, bias, resid, m, n, k, lda, ldw, ldc, act, settled != 0, status};
+    if (kv_width != 0 && (kv_width < 0 || head_dim <= 0 || kv_width % head_dim != 0 || page_size <= 0 || q_width < 0 ||
+                          q_width + 2 * kv_width != n || k_pages == nullptr || v_pages == nullptr || slots == nullptr))
+        return PRB_E_ARG;
+    const Args p{c, a, w, bias, resid, m, n, k, lda, ldw, ldc, act, settled != 0, status,
+                 k_pages, v_pages, slots, q_width, kv_width, head_dim, page_size, num_pages};
     // 16-byte copies where every row starts on 16 bytes and K ends on them, else single floats
     const bool vec = k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)a) % 16 == 0 &&
                      ((uintptr_t)w) % 16 == 0;

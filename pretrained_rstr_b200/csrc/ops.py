@@ -84,7 +84,8 @@ def _declare(h: ctypes.CDLL) -> None:
     h.prb_host_device_address.restype = c_void_p
     h.prb_fetch_step.argtypes = [P, P, I, I, I, P, I, P, P]
     h.prb_publish_result.argtypes = [P, P, I, P]
-    h.prb_gemm_f32.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, I, I, P, P]
+    h.prb_gemm_f32.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, I, I, P, P, P, I, I, I, I, I,
+                                       P, P]
     h.prb_gemm_bf16.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, I, I, P, P]
     h.prb_gemm_bf16_scatter.argtypes = [P, P, P, P, I, I, I, L, L, L, I, I, P, P, P, I, I, I, I, I,
                                         I, P, P]
@@ -461,9 +462,10 @@ def copy_pages(storage, pairs, n_pairs, status) -> None:
 
 
 def gemm_f32(out, a, w, bias=None, resid=None, act=None, kernel: int = 0, status=None,
-             settled: bool = False) -> None:
+             settled: bool = False, kv_scatter=None) -> None:
     """out[M,N] = act(a[M,K] . w[N,K]^T + bias) (+ resid): true 32-bit FMA, one order of
-    summation for every M.  ``settled``: ``w`` was complete before the kernel ahead in the stream
+    summation for every M.  ``kv_scatter`` = (k_pages, v_pages, slots, q_width): the key and value columns
+    of a fused QKV product also go to the paged cache (float32, contiguous) at each row's slot.  ``settled``: ``w`` was complete before the kernel ahead in the stream
     began (a model's weights are), so it may be read while that still runs.  ``kernel`` forces one of the kernels (1 rows of weights as a
     stream, 2 / 3 tiles of 64 x 128, 64 x 64); left at 0 the sizes choose.  All give the same bits."""
     what = "gemm_f32"
@@ -480,9 +482,18 @@ def gemm_f32(out, a, w, bias=None, resid=None, act=None, kernel: int = 0, status
         _need(resid, torch.float32, "resid", what)
         if resid.shape != out.shape or resid.stride(0) != out.stride(0):
             raise KernelArgumentError(f"{what}: resid must have the output's shape and stride")
-    _check(lib().prb_gemm_f32(_p(out), _p(a), _p(w), _p(bias), _p(resid), m, n, k, a.stride(0),
-                              w.stride(0), out.stride(0), ACT_CODES[act], int(kernel), int(bool(settled)),
-                              _p(status), _stream()), what)
+    kv = (None, None, None, 0, 0, 0, 0, 0)
+    if kv_scatter is not None:
+        k_pages, v_pages, slots, q_width = kv_scatter[:4]
+        num_pages, kv_heads, page_size, head_dim = k_pages.shape
+        if k_pages.dtype != torch.float32 or v_pages.dtype != torch.float32 or slots.dtype != torch.int32 or \
+                not k_pages.is_contiguous() or not v_pages.is_contiguous() or slots.numel() < m or \
+                q_width + 2 * kv_heads * head_dim != n:
+            raise KernelArgumentError(f"{what}: cache type or widths do not fit the product")
+        kv = (_p(k_pages), _p(v_pages), _p(slots), q_width, kv_heads * head_dim, head_dim, page_size, num_pages)
+    _check(lib().prb_gemm_f32(
+        _p(out), _p(a), _p(w), _p(bias), _p(resid), m, n, k, a.stride(0), w.stride(0), out.stride(0),
+        ACT_CODES[act], int(kernel), int(bool(settled)), *kv, _p(status), _stream()), what)
 
 
 def gemm_bf16(out, a, w, bias=None, resid=None, act=None, tile_n: int = 0, status=None,

@@ -80,8 +80,12 @@ class Linear:
         QKV product straight to the cache; returns True when it did."""
         m = out.shape[0]
         if self.runtime.dtype == torch.float32:
-            ops.gemm_f32(out, _tensor(a), self.weight, self.bias, resid, act, status=ctx.status, settled=True)
-            return False
+            if kv_scatter is not None and (resid is not None or not kv_scatter[0].is_contiguous() or
+                                           not kv_scatter[1].is_contiguous()):
+                kv_scatter = None
+            ops.gemm_f32(out, _tensor(a), self.weight, self.bias, resid, act, status=ctx.status, settled=True,
+                         kv_scatter=kv_scatter)
+            return kv_scatter is not None
         # Which kernel (measured on GPT-2 small and XL shapes): up to 16 rows
         # the weight-streaming kernel with the norm fused into it; 17 to 64 rows the cluster
         # split-K kernel where :func:`cluster_product` says so, else the tensor-memory

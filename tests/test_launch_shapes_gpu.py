@@ -83,3 +83,30 @@ def test_norm_of_many_rows(rows, width, dtype):
     # 32-bit statistics of rows around 1: a few roundings of 2^-24 of numbers up to 3, or bfloat16's own
     tol = 1e-5 if dtype == torch.float32 else 2.0 ** -8
     assert bool(((out.double() - ref).abs() <= tol * (1.0 + ref.abs())).all())
+
+
+@pytest.mark.parametrize("m", [1, 8, 13, 40, 130])
+@pytest.mark.parametrize("heads,kv_heads,dh,ps", [(6, 3, 64, 16), (2, 1, 20, 24), (3, 3, 7, 1), (12, 12, 64, 64)])
+def test_float32_product_scatters_keys_and_values(m, heads, kv_heads, dh, ps):
+    """The key and value columns of a fused QKV product reach the cache as the append kernel brings them."""
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(m + dh)
+    q_width, kv_width, k = heads * dh, kv_heads * dh, 96
+    n, pages = q_width + 2 * kv_width, 2 + 140 // ps
+    a, w = torch.randn(m, k, device="cuda", generator=g), torch.randn(n, k, device="cuda", generator=g)
+    bias = torch.randn(n, device="cuda", generator=g)
+    slots = torch.randperm(pages * ps, generator=torch.Generator().manual_seed(m))[:m].to(torch.int32)
+    slots[m // 2] = -1
+    slots = slots.cuda()
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    cache = [torch.zeros(pages, kv_heads, ps, dh, device="cuda") for _ in range(4)]
+    out = [torch.full((m, n), float("nan"), device="cuda") for _ in range(2)]
+    ops.gemm_f32(out[0], a, w, bias=bias, status=status, kv_scatter=(cache[0], cache[1], slots, q_width))
+    ops.gemm_f32(out[1], a, w, bias=bias)
+    ops.kv_append(cache[2], cache[3], out[1][:, q_width:q_width + kv_width], out[1][:, q_width + kv_width:], slots,
+                  m, status)
+    assert torch.equal(out[0], out[1]) and torch.equal(cache[0], cache[2]) and torch.equal(cache[1], cache[3])
+    assert status.tolist() == [0, 0, 0, 0]
+    slots[0] = pages * ps                                  # a slot outside the pool is recorded, not written
+    ops.gemm_f32(out[0], a, w, bias=bias, status=status, kv_scatter=(cache[0], cache[1], slots, q_width))
+    assert status.tolist()[0] == 3
