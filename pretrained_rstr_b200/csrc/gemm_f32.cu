@@ -48,8 +48,8 @@ struct Args {
     int act;
     bool settled;                   // w may be read before the kernel ahead has ended
     int* status;
-    // Columns of a fused QKV product that also go to the paged cache ([q_width, q_width + kv_width) are
-    // keys, the next kv_width values); kv_width == 0: none.
+    // The stream kernel only: columns of a fused QKV product that also go to the paged cache ([q_width,
+    // q_width + kv_width) are keys, the next kv_width values); kv_width == 0: none.
     float* k_pages;                 // [pages][kv heads][page_size][head_dim]
     float* v_pages;
     const int* slots;               // cache slot of each row, -1 = none
@@ -626,18 +626,6 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
                 for (int d = 0; d < 4; ++d)
                     if (col + d < p.n) out[d] = y[d];
             }
-            if (p.kv_width != 0 && col + 4 > p.q_width) {
-                if (p.q_width % 4 == 0 && p.head_dim % 4 == 0 && ((uintptr_t)p.k_pages | (uintptr_t)p.v_pages) % 16 == 0) {
-                    // (four columns of one head)
-                    float* const cached = col < p.n ? cache_place(p, row, col) : nullptr;
-                    if (cached != nullptr) *reinterpret_cast<float4*>(cached) = make_float4(y[0], y[1], y[2], y[3]);
-                } else {
-                    for (int d = 0; d < 4; ++d) {
-                        float* const cached = col + d < p.n ? cache_place(p, row, col + d) : nullptr;
-                        if (cached != nullptr) *cached = y[d];
-                    }
-                }
-            }
         }
     }
     __syncwarp();
@@ -748,8 +736,10 @@ bool stream_geometry(const Args& p, int mb, int copy, StreamGeo* g, size_t* smem
 // which: 0 the rule below; 1 the stream kernel where it fits, 2 / 3 tiles of 64 x 128, 64 x 64 (the
 // same bits from all of them).  settled: w was written long before (by no kernel of the step), so the
 // launch may be placed, and w read, before the kernel ahead in the stream has ended.
-// kv_width > 0: the product is a fused QKV projection, whose key and value columns also go to the paged
-// cache (float32, contiguous) at slots[row]: the append behind a decode step's product was 2.8 us a layer.
+// kv_width > 0 (up to 16 rows that the stream kernel takes, else refused): the product is a fused QKV
+// projection, whose key and value columns also go to the paged cache (float32, contiguous) at slots[row]: 8
+// requests generating 24 tokens 19.2 -> 19.0 ms.  (In the tiles' epilogue it cost more than the append
+// behind them: three prompts of 301 tokens 7.36 -> 7.49 ms.)
 PRB_API int prb_gemm_f32(float* c, const float* a, const float* w, const float* bias,
                          const float* resid, int m, int n, int k, long lda, long ldw, long ldc,
                          int act, int which, int settled, float* k_pages, float* v_pages,
@@ -783,6 +773,7 @@ PRB_API int prb_gemm_f32(float* c, const float* a, const float* w, const float* 
             }
         }
     }
+    if (kv_width != 0) return PRB_E_SIZE;
     // (rows that overlap are no tensor that a copy engine's map describes)
     const int tiled = !vec ? COPY_4 : ldw >= k && lda >= k ? COPY_TMA : COPY_16;
     // 64 x 128 where that leaves no SM without a CTA twice over, or nearly two an SM in one round of

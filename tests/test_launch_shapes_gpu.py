@@ -85,7 +85,7 @@ def test_norm_of_many_rows(rows, width, dtype):
     assert bool(((out.double() - ref).abs() <= tol * (1.0 + ref.abs())).all())
 
 
-@pytest.mark.parametrize("m", [1, 8, 13, 40, 130])
+@pytest.mark.parametrize("m", [1, 4, 8, 13, 16])
 @pytest.mark.parametrize("heads,kv_heads,dh,ps", [(6, 3, 64, 16), (2, 1, 20, 24), (3, 3, 7, 1), (12, 12, 64, 64)])
 def test_float32_product_scatters_keys_and_values(m, heads, kv_heads, dh, ps):
     """The key and value columns of a fused QKV product reach the cache as the append kernel brings them."""
@@ -110,3 +110,7 @@ def test_float32_product_scatters_keys_and_values(m, heads, kv_heads, dh, ps):
     slots[0] = pages * ps                                  # a slot outside the pool is recorded, not written
     ops.gemm_f32(out[0], a, w, bias=bias, status=status, kv_scatter=(cache[0], cache[1], slots, q_width))
     assert status.tolist()[0] == 3
+    many = torch.zeros(17, k, device="cuda")               # more rows than the kernel that does it takes
+    with pytest.raises(ops.KernelArgumentError, match="size"):
+        ops.gemm_f32(torch.zeros(17, n, device="cuda"), many, w,
+                     kv_scatter=(cache[0], cache[1], torch.zeros(17, dtype=torch.int32, device="cuda"), q_width))
