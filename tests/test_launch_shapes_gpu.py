@@ -114,3 +114,10 @@ def test_float32_product_scatters_keys_and_values(m, heads, kv_heads, dh, ps):
     with pytest.raises(ops.KernelArgumentError, match="size"):
         ops.gemm_f32(torch.zeros(17, n, device="cuda"), many, w,
                      kv_scatter=(cache[0], cache[1], torch.zeros(17, dtype=torch.int32, device="cuda"), q_width))
+
+
+def test_which_decode_attention_a_launch_of_few_requests_takes():
+    """From a (token, head) an SM and more than 512 keys the ring kernel, however few the requests."""
+    ops = _ops()
+    assert ops.decode_ring_prefers(8, 25, 1024) and ops.decode_ring_prefers(16, 12, 1024)
+    assert not ops.decode_ring_prefers(8, 25, 512) and not ops.decode_ring_prefers(8, 16, 1024)
