@@ -26,8 +26,8 @@
 // it; a chunk's row is 128 bytes, its 16-byte pieces swizzled.  690 rows: 2,304 x 768 77 -> 75 us, 3,072 x 768
 // 101 -> 95, 768 x 768 31 -> 28, 768 x 3,072 106 -> 91, 50,257 x 768 1.50 -> 1.31 ms = 41 TFLOP/s; one CTA a tile
 // over all of K 14 TFLOP/s.  What bounds it: the FMA loop.  fma.rn.f32x2 of operands in three registers
-// runs at 57 TFLOP/s (72 with two), 8 x 8 outputs a thread read 16 bytes of shared memory for 8 of them,
-// which is the most that shared memory gives, and 255 registers leave two warps a scheduler to overlap the two.
+// runs at 57 TFLOP/s (72 with two); 255 registers leave two warps a scheduler, which cover neither its
+// latency nor that of shared memory whole (counters at 690 x 3,072 x 768: issue slots 38 %, shared memory 59 %).
 #include "common.cuh"
 #include "tcgen05.cuh"
 #include "tensor_map.cuh"
