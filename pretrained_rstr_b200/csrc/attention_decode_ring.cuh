@@ -175,13 +175,21 @@ __device__ __forceinline__ TokenSpan token_span(const RingArgs& a, int t, bool o
 struct Partial {
     float m, l, o0, o1;
 };
-__device__ __forceinline__ void merge_into(Partial& acc, float m2, float l2, float a0, float a1) {
-    const float mn = fmaxf(acc.m, m2);
-    const float c1 = (acc.m == -INFINITY) ? 0.0f : __expf(acc.m - mn);
-    const float c2 = (m2 == -INFINITY) ? 0.0f : __expf(m2 - mn);
+// What the sum so far (maximum `m`) and the state added to it (`m2`) are scaled by; mn: the larger maximum.
+__device__ __forceinline__ void merge_weights(float m, float m2, float mn, float& c1, float& c2) {
+    c1 = (m == -INFINITY) ? 0.0f : __expf(m - mn);
+    c2 = (m2 == -INFINITY) ? 0.0f : __expf(m2 - mn);
+}
+__device__ __forceinline__ void merge_by(Partial& acc, float c1, float c2, float l2, float a0, float a1) {
     acc.l = acc.l * c1 + l2 * c2;
     acc.o0 = acc.o0 * c1 + a0 * c2;
     acc.o1 = acc.o1 * c1 + a1 * c2;
+}
+__device__ __forceinline__ void merge_into(Partial& acc, float m2, float l2, float a0, float a1) {
+    const float mn = fmaxf(acc.m, m2);
+    float c1, c2;
+    merge_weights(acc.m, m2, mn, c1, c2);
+    merge_by(acc, c1, c2, l2, a0, a1);
     acc.m = mn;
 }
 
@@ -645,7 +653,9 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
 
     // ---- merge.  The edge states of the CTA's warps, in warp order, form chains of the same
     // (token, head); the warp that holds a chain's first state merges it: lane 2 w + e looks at state e
-    // of warp w, so that the maximum and the weights of all of them take one round.  A chain that is the
+    // of warp w, so that the maxima and the weights of all of them take one round; the sums then follow one
+    // another in the chain's order, as those of the CTAs' states do: how many warps of a CTA or CTAs share a
+    // (token, head) does not change its bits.  A chain that is the
     // whole (token, head) is written out; otherwise it goes to the workspace, and the last CTA
     // of that (token, head) to arrive merges the CTAs' states in CTA order.
     const int state_w = lane >> 1, state_e = lane & 1;
@@ -659,17 +669,23 @@ RING_FN void late(const RingArgs& a, const CUtensorMap* map_k,
         const bool in = state_pair == pair;
         const float sm = in ? sh.edge_state[state_w][state_e][DH] : -INFINITY;
         const float sl = in ? sh.edge_state[state_w][state_e][DH + 1] : 0.0f;
-        Partial acc;
-        acc.m = prb_warp_max(sm);
-        const float sc = sm == -INFINITY ? 0.0f : __expf(sm - acc.m);
-        acc.l = prb_warp_sum(sl * sc);
-        acc.o0 = acc.o1 = 0.0f;
+        float upto = sm;                                     // the maximum of the states up to the lane's
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto = fmaxf(upto, v);
+        }
+        float before = __shfl_up_sync(0xffffffffu, upto, 1);
+        if (lane == 0) before = -INFINITY;
+        float c1, c2;
+        merge_weights(before, sm, upto, c1, c2);
+        Partial acc{-INFINITY, 0.0f, 0.0f, 0.0f};
         for (unsigned left = chain; left != 0; left &= left - 1) {
             const int at = __ffs(left) - 1;
-            const float c = __shfl_sync(0xffffffffu, sc, at);
             const float2 v = *reinterpret_cast<const float2*>(&sh.edge_state[at >> 1][at & 1][2 * lane]);
-            acc.o0 += v.x * c;
-            acc.o1 += v.y * c;
+            acc.m = __shfl_sync(0xffffffffu, upto, at);
+            merge_by(acc, __shfl_sync(0xffffffffu, c1, at), __shfl_sync(0xffffffffu, c2, at),
+                     __shfl_sync(0xffffffffu, sl, at), v.x, v.y);
         }
         const int idx = pair / a.n_heads, h = pair - idx * a.n_heads;
         TokenSpan s{sh.span_t[idx], sh.span_b[idx], sh.span_pos[idx], 0, 0, 0};

@@ -44,6 +44,30 @@ def test_ring_attention_of_long_token_lists(t, nh, nkv, ps, window):
     assert status.tolist() == [0, 0, 0, 0]
 
 
+@pytest.mark.parametrize("blocks", [2, 5, 8])
+def test_ring_attention_merges_in_one_order(blocks):
+    """Blocks of 32 keys, a warp each: in the warps of one CTA where a token an SM is asked for, in a CTA each
+    where few are.  Either way their states are merged in the keys' order: the same bits."""
+    ops = _ops()
+    sms = min(ops.sm_count(), ops.decode_ring_max_list())
+    few = max(1, sms // blocks)
+    _q, k, v, table, seq, pos = _paged_case(blocks, 1, 1, 64, 64, [32 * blocks - i % 32 for i in range(sms)],
+                                            [1] * sms, torch.bfloat16)
+    ws = torch.zeros(ops.decode_ring_workspace(sms, 1, 64), device="cuda")
+    counters = torch.zeros(sms, dtype=torch.int32, device="cuda")
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    for seed in range(40):
+        q = torch.randn(sms, 64, generator=torch.Generator().manual_seed(seed)).to(torch.bfloat16).cuda()
+        many, apart = torch.full_like(q, float("nan")), torch.full_like(q, float("nan"))
+        ops.attention_decode_ring(many, q, k, v, table, seq, pos, None, None, sms, 1, 0.2, None, ws, counters, status)
+        for first in range(0, sms, few):
+            tokens = torch.arange(first, min(sms, first + few), dtype=torch.int32, device="cuda")
+            ops.attention_decode_ring(apart, q, k, v, table, seq, pos, tokens, None, len(tokens), 1, 0.2, None, ws,
+                                      counters, status)
+        assert torch.equal(many, apart)
+    assert status.tolist() == [0, 0, 0, 0] and int(counters.abs().sum()) == 0
+
+
 @pytest.mark.parametrize("requests,context", [(100, 600), (130, 70)])
 def test_an_engine_of_many_requests_by_either_decode_attention(tmp_path, monkeypatch, requests, context):
     cfg = GPT2Config.from_dict(dict(n_layer=2, n_embd=256, n_head=4, n_inner=512, vocab_size=512, n_positions=1024))
