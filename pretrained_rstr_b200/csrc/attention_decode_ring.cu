@@ -132,15 +132,17 @@ PRB_API int prb_attention_decode_ring_max_list() { return MAX_LIST; }
 // 3.528.
 // The ring wins where many (token, head) pairs have long contexts (its warps stream long runs,
 // the other kernel's CTAs walk their keys one batch after the other) and in the middle range at
-// nearly every context; it loses at few requests.  Since its look-ups go side by side and its merge takes one
-// round, also at 8 requests of XL with more than 512 keys (450 to 900 tokens: 4 steps 9.82 ms by the
-// split-key kernel, 9.38 by this one), while 8 requests of GPT-2 small are level (16 steps 6.08 and 6.08).
+// nearly every context; it loses at few requests.
+// Fewer than 16 tokens of one or two (token, head) pairs an SM stay with the split-key kernel, also where
+// this one has become the faster (8 requests of XL at 450 to 900 tokens): that one multiplies the values
+// by 32-bit weights, this one rounds the weights to bfloat16 for its matrix instructions, and the line
+// between them moves no launch from the former to the latter.
 PRB_API int prb_attention_decode_ring_prefers(int n_list, int n_heads, int max_context) {
     const long pairs = (long)n_list * n_heads;
     const long sms = prb_sm_count();
     if (pairs >= 4 * sms) return max_context > 512;
     if (pairs >= 2 * sms) return 1;
-    return pairs >= sms && max_context > 512;
+    return pairs >= sms && n_list >= 16 && max_context > 512;
 }
 
 // Floats of workspace a launch of up to n_list tokens needs.

@@ -116,8 +116,13 @@ def test_float32_product_scatters_keys_and_values(m, heads, kv_heads, dh, ps):
                      kv_scatter=(cache[0], cache[1], torch.zeros(17, dtype=torch.int32, device="cuda"), q_width))
 
 
-def test_which_decode_attention_a_launch_of_few_requests_takes():
-    """From a (token, head) an SM and more than 512 keys the ring kernel, however few the requests."""
+@pytest.mark.parametrize("heads", [20, 25, 32])
+def test_a_few_requests_keep_32_bit_weights(heads):
+    """Fewer than 16 tokens of up to two (token, head) pairs an SM stay with the kernel that multiplies the values
+    by 32-bit weights; the other one rounds them to bfloat16."""
     ops = _ops()
-    assert ops.decode_ring_prefers(8, 25, 1024) and ops.decode_ring_prefers(16, 12, 1024)
-    assert not ops.decode_ring_prefers(8, 25, 512) and not ops.decode_ring_prefers(8, 16, 1024)
+    for tokens in range(1, 16):
+        for context in (256, 512, 768, 1024):
+            if tokens * heads < 2 * ops.sm_count():
+                assert not ops.decode_ring_prefers(tokens, heads, context)
+    assert ops.decode_ring_prefers(16, 12, 1024) and not ops.decode_ring_prefers(16, 12, 512)
