@@ -413,6 +413,13 @@ __device__ __forceinline__ float4 ld_cluster4(uint32_t addr, uint32_t rank) {
                  : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(r));
     return v;
 }
+__device__ __forceinline__ int ld_cluster1(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    int v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(r) : "memory");
+    return v;
+}
 // two neighbouring floats as fma.rn.f32x2 takes them, four of them by one read of shared memory
 typedef unsigned long long pair_t;
 __device__ __forceinline__ void fma_pairs(pair_t& acc, pair_t a, pair_t b) {
@@ -466,6 +473,8 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
 
+    bool alive = true;
+    int asked = c0;                                           // chunks before it thread 0 has asked for
     // rows [0, BM) of a stage are A's, the next BN W's; rows outside the matrices are zeros.  A row is
     // a chunk of 128 bytes, its 16-byte pieces swizzled with the row.
     auto load_rows = [&](int c, bool weights) {
@@ -473,9 +482,14 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
         const int s = (c - c0) % TILE_STAGES;
         float* st = smem + s * Cfg::STAGE + (weights ? BM * CH : 0);
         if constexpr (COPY == COPY_TMA) {
-            if (tid == 0) {
+            // (after a wait that gave up, of whichever thread, nothing more is asked for: the stage's copy may
+            // still be on its way)
+            if (tid == 0 && !*failed) {
                 const uint32_t bar = smem_u32(&bars[s]);
-                if (weights) mbar_expect_tx(bar, Cfg::STAGE * 4);
+                if (weights) {
+                    mbar_expect_tx(bar, Cfg::STAGE * 4);
+                    asked = c + 1;
+                }
                 asm volatile(
                     "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
                     "[%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(st)),
@@ -513,7 +527,6 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
 #pragma unroll
         for (int j = 0; j < TN; ++j) sum[i][j] = 0.0f;
     const uint32_t sw_a = (uint32_t)(ty & 7), sw_w = (uint32_t)(tx & 7);
-    bool alive = true;
     int c = c0;
 #pragma unroll 1
     for (int r = 0; r < RUNS; ++r) {
@@ -574,9 +587,9 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
     }
     if (COPY != COPY_TMA) {
         cp_wait<0>();
-    } else if (!alive && tid == 0) {
+    } else if (tid == 0 && *failed) {                         // (the last chunk's barrier is behind every wait)
         prb_set_status(p.status, PRB_S_WAIT_TIMEOUT, 41, blockIdx.x, blockIdx.y);
-        for (int i = max(c0, c1 - TILE_STAGES); i < c1; ++i)  // the last copies, bounded
+        for (int i = max(c0, asked - TILE_STAGES); i < asked; ++i)       // copies in flight, bounded
             for (uint32_t w = 0; w < tc5::WAIT_LIMIT; ++w)
                 if (mbar_try_wait(smem_u32(&bars[(i - c0) % TILE_STAGES]), (uint32_t)((i - c0) / TILE_STAGES) & 1u)) break;
     }
@@ -601,6 +614,13 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
             const uint32_t at = smem_u32(smem + (r0 + e / (BN / 4)) * Cfg::OUT_LD + (e % (BN / 4)) * 4);
 #pragma unroll
             for (int q = 0; q < CL; ++q) v[i][q] = ld_cluster4(at, q);
+        }
+        // a partial tile that a CTA of the cluster gave up on is in nobody's sums
+        if (COPY == COPY_TMA && i0 == 0) {
+            int any = 0;
+#pragma unroll
+            for (int q = 0; q < CL; ++q) any |= ld_cluster1(smem_u32(&failed_word), q);
+            alive = any == 0;
         }
 #pragma unroll
         for (int i = 0; i < AT_ONCE; ++i) {
