@@ -95,6 +95,7 @@ struct Geometry {
 struct Plan {
     Geometry geo;
     int grid;
+    int sets;       // places for a strip's sums: 2, taken in turn, save a barrier a strip
     size_t smem;
 };
 
@@ -111,8 +112,8 @@ __host__ __device__ inline size_t stage_size(int mp, bool ln, int kc) {
 
 inline Plan make_plan(int mt, bool ln, int n, int k) {
     const int mp = 8 * mt;
-    const size_t fixed = (size_t)2 * WARPS * ROWS * mp * sizeof(float) + 256 + 1024 +
-                         (ln ? (size_t)mp * norm_pitch(k) * 2 + (size_t)2 * k * sizeof(float) : 0);
+    const size_t set = (size_t)WARPS * ROWS * mp * sizeof(float);
+    const size_t fixed = 256 + 1024 + (ln ? (size_t)mp * norm_pitch(k) * 2 + (size_t)2 * k * sizeof(float) : 0);
     const size_t sm_bytes = 224 * 1024;                // shared memory of an SM that CTAs can share
     Plan p;
     Geometry& g = p.geo;
@@ -126,6 +127,9 @@ inline Plan make_plan(int mt, bool ln, int n, int k) {
     // Pieces as large as possible (a whole strip when a copy can hold it); as many CTAs per
     // SM as still leaves each a ring of two pieces (or all its work), because what limits a
     // short streaming kernel is the bytes in flight; the strips are then dealt out evenly.
+    // A second set of sums (4 or 8 KB) where it costs neither the SM a CTA nor a strip its one piece.
+    // (16 rows, weights from memory, with it / without: 3,072 x 1,600 5.57 / 4.31 us, 50,257 x 768 29.8 / 22.3,
+    // 50,257 x 1,600 44.8 / 41.1, 1,600 x 1,600 3.20 / 3.01.)
     const int cand[] = {k, 2048, 1024, 512, 256, 128, 64};
     for (int c = 0; c < 7; ++c) {
         g.kc = cand[c];
@@ -137,24 +141,27 @@ inline Plan make_plan(int mt, bool ln, int n, int k) {
             size_t budget = g_tune[3] > 0 ? (size_t)g_tune[3] * 1024 : sm_bytes / per_sm - 1024;
             if (budget > 216 * 1024) budget = 216 * 1024;    // a CTA's own limit
             const size_t stage = stage_size(mp, ln, g.kc);
-            if (fixed + stage > budget) continue;
             spread(sms * per_sm);
             const int items = g.chunks * g.per;
-            int fit = (int)((budget - fixed) / stage);
-            if (fit > max_stages) fit = max_stages;
-            g.stages = fit < items ? fit : items;
-            if (g.stages < items && g.stages < 2 && !(g_tune[0] > 0 && per_sm == 1)) continue;
-            p.smem = fixed + (size_t)g.stages * stage;
-            return p;
+            for (p.sets = 2; p.sets >= 1; --p.sets) {
+                const size_t taken = fixed + p.sets * set;
+                if (taken + stage > budget) continue;
+                int fit = (int)((budget - taken) / stage);
+                if (fit > max_stages) fit = max_stages;
+                g.stages = fit < items ? fit : items;
+                if (g.stages < items && g.stages < 2 && !(g_tune[0] > 0 && per_sm == 1)) continue;
+                p.smem = taken + (size_t)g.stages * stage;
+                return p;
+            }
         }
         if (g_tune[0] > 0) break;
     }
     // nothing fits (a very wide K with many rows): smallest pieces, one CTA per SM
     g.kc = 64;
     g.chunks = k / 64;
-    g.stages = 1;
+    g.stages = p.sets = 1;
     spread(sms);
-    p.smem = fixed + stage_size(mp, ln, 64);
+    p.smem = fixed + set + stage_size(mp, ln, 64);
     return p;
 }
 // How many ring buffers' weight copies start before the wait on the previous kernel.  All of
@@ -292,14 +299,14 @@ __device__ __forceinline__ void norm_rows_staged(const Args& a, __nv_bfloat16* x
 // remainders of run-time counts in every piece and two barriers a strip that was about 0.95 us.  8 rows,
 // before and now: the vocabulary of 768 columns 23.5 -> 16.5 us, of 1,600 43.3 -> 31.2; the four products
 // of a layer 29.8 -> 26.2 at 1,600 columns, 17.8 -> 16.4 at 1,024.
-template <int MT, bool LN, typename O>
+template <int MT, bool LN, typename O, int SETS>
 __global__ void __launch_bounds__(STREAM_THREADS, 2)
 gemm_stream_kernel(Args a, Geometry geo, const __grid_constant__ CUtensorMap map_w,
                    const __grid_constant__ CUtensorMap map_x) {
     constexpr int MP = 8 * MT;
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    float* red = reinterpret_cast<float*>(smem_raw);                         // [2][8][16][MP]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(red + 2 * WARPS * ROWS * MP);    // full[], empty[]
+    float* red = reinterpret_cast<float*>(smem_raw);                         // [SETS][8][16][MP]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(red + SETS * WARPS * ROWS * MP);    // full[], empty[]
     volatile int* failed = reinterpret_cast<volatile int*>(bars + 2 * MAX_STAGES);
     uint8_t* after = reinterpret_cast<uint8_t*>(bars) + 256;
     float* gb = reinterpret_cast<float*>(after);                             // LN only: gamma, beta
@@ -472,9 +479,10 @@ gemm_stream_kernel(Args a, Geometry geo, const __grid_constant__ CUtensorMap map
 
         // ---- the strip is complete: add the warps' partial sums in warp order.  (Two places for them
         // in turn: who writes the next strip's has passed this strip's barrier, and who writes the one
-        // after that has passed the next.)
+        // after that has passed the next.  With one place a second barrier stands before the next strip's.)
         // acc[nt][0,1]: feature g, tokens nt*8 + q*2 + {0,1}; acc[nt][2,3]: feature g + 8
-        float* sums = red + (strip & 1) * WARPS * ROWS * MP;
+        if (SETS == 1 && strip > 0) compute_barrier();         // the last strip's have been read
+        float* sums = red + (strip & (SETS - 1)) * WARPS * ROWS * MP;
 #pragma unroll
         for (int nt = 0; nt < MT; ++nt) {
             float* base = sums + ((size_t)warp * ROWS) * MP + nt * 8 + q * 2;
@@ -528,12 +536,10 @@ inline bool takes(const Args& a) {
     return a.m <= 16 && a.k % 64 == 0 && a.ldw % 8 == 0 && (a.xf != nullptr || a.ldx % 8 == 0);
 }
 
-template <int MT, bool LN, typename O>
-int launch_stream(Args a, cudaStream_t stream) {
+template <int MT, bool LN, typename O, int SETS>
+int launch_stream_by(const Args& a, const Plan& p, cudaStream_t stream) {
     constexpr int MP = 8 * MT;
-    a.xs_pitch = LN ? norm_pitch(a.k) : a.k;
-    const Plan p = finish_plan(make_plan(MT, LN, a.n, a.k), LN);
-    if (p.smem > 220 * 1024) return PRB_E_SIZE;
+    constexpr auto kernel = gemm_stream_kernel<MT, LN, O, SETS>;
     CUtensorMap map_w, map_x;
     const int slabs = p.geo.kc / 64;
     int rc = tmap::slab_map(a.w, a.n, a.k, a.ldw, ROWS, slabs, &map_w);
@@ -542,22 +548,27 @@ int launch_stream(Args a, cudaStream_t stream) {
     else if ((rc = tmap::slab_map(a.x, a.m, a.k, a.ldx, MP, slabs, &map_x)) != 0) return rc;
     static bool carved = false;
     if (!carved) {      // several CTAs per SM need the large shared-memory carve-out
-        cudaFuncSetAttribute(gemm_stream_kernel<MT, LN, O>,
-                             cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         carved = true;
     }
     static size_t configured = 0;
     if (p.smem > 48 * 1024 && p.smem > configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_stream_kernel<MT, LN, O>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
         if (e != cudaSuccess) return (int)e;
         configured = p.smem;
     }
-    cudaError_t e = prb_launch_dependent(gemm_stream_kernel<MT, LN, O>, dim3(p.grid), dim3(STREAM_THREADS),
-                                         p.smem, stream, a, p.geo, map_w, map_x);
+    cudaError_t e = prb_launch_dependent(kernel, dim3(p.grid), dim3(STREAM_THREADS), p.smem, stream, a, p.geo, map_w,
+                                         map_x);
     if (e != cudaSuccess) return (int)e;
     return 0;
+}
+
+template <int MT, bool LN, typename O>
+int launch_stream(Args a, cudaStream_t stream) {
+    a.xs_pitch = LN ? norm_pitch(a.k) : a.k;
+    const Plan p = finish_plan(make_plan(MT, LN, a.n, a.k), LN);
+    if (p.smem > 220 * 1024) return PRB_E_SIZE;
+    return p.sets == 2 ? launch_stream_by<MT, LN, O, 2>(a, p, stream) : launch_stream_by<MT, LN, O, 1>(a, p, stream);
 }
 }  // namespace stream
 
@@ -582,6 +593,15 @@ PRB_API int prb_gemm_smallm_trace(unsigned long long* host, int n) {
 PRB_API int prb_gemm_smallm_tune(int kc, int ctas_per_sm, int stages, int budget_kb, int early) {
     stream::g_tune[0] = kc; stream::g_tune[1] = ctas_per_sm;
     stream::g_tune[2] = stages; stream::g_tune[3] = budget_kb; stream::g_tune[4] = early;
+    return 0;
+}
+// How a product of m <= 16 rows is cut, with or without the norm: CTAs, pieces of K, places for a strip's sums.
+PRB_API int prb_gemm_smallm_plan(int m, int norm, int n, int k, int* ctas, int* pieces, int* sets) {
+    if (m < 1 || m > 16 || n <= 0 || k <= 0 || k % 64 != 0) return PRB_E_SIZE;
+    const stream::Plan p = stream::make_plan(m <= 8 ? 1 : 2, norm != 0, n, k);
+    *ctas = p.grid;
+    *pieces = p.geo.chunks;
+    *sets = p.sets;
     return 0;
 }
 PRB_API int prb_gemm_smallm_max_norm_width() { return LN_MAX_K; }

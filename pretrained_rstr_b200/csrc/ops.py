@@ -84,6 +84,7 @@ def _declare(h: ctypes.CDLL) -> None:
     h.prb_host_device_address.restype = c_void_p
     h.prb_fetch_step.argtypes = [P, P, I, I, I, P, I, P, P]
     h.prb_publish_result.argtypes = [P, P, I, P]
+    h.prb_gemm_smallm_plan.argtypes = [I, I, I, I, P, P, P]
     h.prb_gemm_f32.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, I, I, P, P, P, I, I, I, I, I,
                                        P, P]
     h.prb_gemm_bf16.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, I, I, P, P]
@@ -595,6 +596,13 @@ def smallm_limits():
     if _SMALLM is None:
         _SMALLM = (lib().prb_gemm_smallm_max_rows(), lib().prb_gemm_smallm_max_norm_width())
     return _SMALLM
+
+
+def smallm_plan(m: int, norm: bool, n: int, k: int):
+    """(CTAs, pieces of K, places for a strip's sums) of a product of up to 16 rows, K a multiple of 64."""
+    got = [ctypes.c_int() for _ in range(3)]
+    _check(lib().prb_gemm_smallm_plan(m, int(norm), n, k, *(ctypes.byref(g) for g in got)), "smallm_plan")
+    return tuple(g.value for g in got)
 
 
 def gemm_smallm(out, w, a=None, norm_input=None, gamma=None, beta=None, eps=0.0, bias=None,

@@ -39,6 +39,18 @@ def test_weight_streaming_product_of_many_strips(m, n, k, norm):
     assert float((out - ref).abs().max()) <= tol * max(1.0, float(ref.abs().max()))
 
 
+@pytest.mark.parametrize("n,k", [(4800, 768), (50257, 768), (1600, 1600), (3072, 1600), (4096, 1600), (50257, 1600)])
+def test_a_second_place_for_sums_costs_no_cta_and_no_piece(n, k):
+    """16 rows without the norm: a strip in one piece, two CTAs an SM where K allows it, whatever place is left."""
+    ops = _ops()
+    ctas, pieces, sets = ops.smallm_plan(16, False, n, k)
+    strips, sms = -(-n // 16), ops.sm_count()
+    assert pieces == 1 and sets == 1
+    most = 2 * sms if k == 768 or strips <= 2 * sms else sms     # (two strips of 1,600 take one CTA an SM)
+    assert ctas == -(-strips // -(-strips // most))
+    assert ops.smallm_plan(8, False, n, k)[2] == 2 and ops.smallm_plan(16, True, n, k)[2] == 2
+
+
 @pytest.mark.parametrize("m,n,k", [(17, 1, 1), (64, 128, 32), (65, 129, 128), (129, 257, 132), (100, 300, 260),
                                    (130, 512, 768)])
 def test_float32_tiles_of_one_and_of_two_runs_a_cta_give_the_same_bits(m, n, k):
