@@ -370,8 +370,6 @@ gemm_f32_stream_kernel(Args p, StreamGeo g, const __grid_constant__ CUtensorMap 
 }
 
 // ------------------------------------------------------------------------- many rows
-int g_tile_runs = 0;                // (for measurements: 1 or 2 runs a CTA of 64 x 128; 0: the rule below)
-
 // {32 floats, rows} of a row-major [rows, k] matrix, 128-byte swizzle, zeros beyond both; x is a
 // multiple of 32 floats, so the 16-byte rule on it holds.
 int tile_map(const float* t, int rows, int k, long ld, int box_rows, CUtensorMap* out) {
@@ -682,7 +680,6 @@ int launch_tile(const Args& p, int copy, cudaStream_t stream) {
 // 768 1,465 / 1,304, 1,000 x 2,304 110 / 95, 690 x 3,072 98 / 95; 300 x 2,304 41 / 50, 1,000 x 768 41 / 50.
 // (All four runs in a CTA leave room for one an SM: 1,831.)
 int tile_runs(long tiles, int k) {
-    if (g_tile_runs > 0) return g_tile_runs;
     const int run = ((k + CH - 1) / CH + 3) / 4;
     const long sms = prb_sm_count(), slots = 2 * sms;
     auto rounds = [&](int runs) {
@@ -753,8 +750,8 @@ bool stream_geometry(const Args& p, int mb, int copy, StreamGeo* g, size_t* smem
 }
 }  // namespace
 
-// which: 0 the rule below; 1 the stream kernel where it fits, 2 / 3 tiles of 64 x 128, 64 x 64 (the
-// same bits from all of them).  settled: w was written long before (by no kernel of the step), so the
+// which: 0 the rule below; 1 the stream kernel where it fits, 2 / 3 tiles of 64 x 128, 64 x 64, 4 / 5 tiles of
+// 64 x 128 of one run and of two runs a CTA (the same bits from all of them).  settled: w was written long before (by no kernel of the step), so the
 // launch may be placed, and w read, before the kernel ahead in the stream has ended.
 // kv_width > 0 (up to 16 rows that the stream kernel takes, else refused): the product is a fused QKV
 // projection, whose key and value columns also go to the paged cache (float32, contiguous) at slots[row]: 8
@@ -802,12 +799,8 @@ PRB_API int prb_gemm_f32(float* c, const float* a, const float* w, const float* 
     // against 23, 300 x 768 x 3,072 72 against 74).
     const long big = (long)((m + 63) / 64) * ((n + 127) / 128), sms = prb_sm_count();
     const bool wide = big * 2 >= sms || (big * 8 >= 3 * sms && big * 20 <= 9 * sms);
-    if (which == 3 || (which != 2 && !wide)) return launch_tile<64, 64, 8, 4, 1>(p, tiled, stream);
-    return tile_runs(big, k) == 2 ? launch_tile<64, 128, 8, 8, 2>(p, tiled, stream)
-                                  : launch_tile<64, 128, 8, 8, 1>(p, tiled, stream);
-}
-PRB_API int prb_gemm_f32_tune(int runs) {
-    if (runs < 0 || runs > 2) return PRB_E_SIZE;
-    g_tile_runs = runs;
-    return 0;
+    const int runs = which == 4 || which == 5 ? which - 3 : tile_runs(big, k);
+    if (which == 3 || (which != 2 && which != 4 && which != 5 && !wide)) return launch_tile<64, 64, 8, 4, 1>(p, tiled, stream);
+    return runs == 2 ? launch_tile<64, 128, 8, 8, 2>(p, tiled, stream)
+                     : launch_tile<64, 128, 8, 8, 1>(p, tiled, stream);
 }

@@ -468,7 +468,7 @@ def gemm_f32(out, a, w, bias=None, resid=None, act=None, kernel: int = 0, status
     summation for every M.  ``kv_scatter`` = (k_pages, v_pages, slots, q_width): the key and value columns
     of a fused QKV product of up to 16 rows also go to the paged cache (float32, contiguous) at each row's slot.  ``settled``: ``w`` was complete before the kernel ahead in the stream
     began (a model's weights are), so it may be read while that still runs.  ``kernel`` forces one of the kernels (1 rows of weights as a
-    stream, 2 / 3 tiles of 64 x 128, 64 x 64); left at 0 the sizes choose.  All give the same bits."""
+    stream, 2 / 3 tiles of 64 x 128, 64 x 64, 4 / 5 tiles of 64 x 128 of one and of two runs a CTA); left at 0 the sizes choose.  All give the same bits."""
     what = "gemm_f32"
     for name, t in (("out", out), ("a", a), ("w", w)):
         if not t.is_cuda or t.dtype != torch.float32 or t.stride(1) != 1:

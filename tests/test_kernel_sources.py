@@ -59,3 +59,9 @@ def test_no_launch_sets_a_kernel_attribute(name):
     """cudaFuncSetAttribute costs the host as much as a launch of the small kernels of a decode step."""
     code = _code(name)
     assert "cudaFuncSetAttribute" not in code and "prb_allow_shared<" in code
+
+
+def test_float32_products_share_no_switch_between_threads():
+    """Which kernel a product takes is its call's own argument: no variable of the file that other threads' launches
+    read as well."""
+    assert not re.search(r"^(static\s+)?(int|bool|long)\s+g_\w+\s*(=|;)", _code("gemm_f32.cu"), flags=re.M)

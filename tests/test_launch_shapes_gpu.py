@@ -61,14 +61,10 @@ def test_float32_tiles_of_one_and_of_two_runs_a_cta_give_the_same_bits(m, n, k):
     wide = torch.randn(n, k + 1, device="cuda", generator=g)
     resid = torch.randn(m, n, device="cuda", generator=g)
     out = []
-    try:
-        for runs in (1, 2):
-            assert ops.lib().prb_gemm_f32_tune(runs) == 0
-            for w in (wide[:, :k].contiguous(), wide[:, :k]):
-                out.append(torch.full((m, n), float("nan"), device="cuda"))
-                ops.gemm_f32(out[-1], a, w, resid=resid, kernel=2)
-    finally:
-        ops.lib().prb_gemm_f32_tune(0)
+    for kernel in (2, 4, 5):
+        for w in (wide[:, :k].contiguous(), wide[:, :k]):
+            out.append(torch.full((m, n), float("nan"), device="cuda"))
+            ops.gemm_f32(out[-1], a, w, resid=resid, kernel=kernel)
     few = torch.full((m, n), float("nan"), device="cuda")
     for i in range(0, m, 16):
         ops.gemm_f32(few[i:i + 16], a[i:i + 16], wide[:, :k].contiguous(), resid=resid[i:i + 16].contiguous())
