@@ -472,7 +472,6 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
     }
 
     bool alive = true;
-    int asked = c0;                                           // chunks before it thread 0 has asked for
     // rows [0, BM) of a stage are A's, the next BN W's; rows outside the matrices are zeros.  A row is
     // a chunk of 128 bytes, its 16-byte pieces swizzled with the row.
     auto load_rows = [&](int c, bool weights) {
@@ -480,14 +479,10 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
         const int s = (c - c0) % TILE_STAGES;
         float* st = smem + s * Cfg::STAGE + (weights ? BM * CH : 0);
         if constexpr (COPY == COPY_TMA) {
-            // (after a wait that gave up, of whichever thread, nothing more is asked for: the stage's copy may
-            // still be on its way)
-            if (tid == 0 && !*failed) {
+            // (only after its own wait for the stage's last copy, which may else still be on its way)
+            if (tid == 0 && alive) {
                 const uint32_t bar = smem_u32(&bars[s]);
-                if (weights) {
-                    mbar_expect_tx(bar, Cfg::STAGE * 4);
-                    asked = c + 1;
-                }
+                if (weights) mbar_expect_tx(bar, Cfg::STAGE * 4);
                 asm volatile(
                     "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
                     "[%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(st)),
@@ -533,7 +528,12 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
         for (; c < end; ++c) {
             const int s = (c - c0) % TILE_STAGES;
             if constexpr (COPY == COPY_TMA) {
-                if (alive) alive = mbar_wait(smem_u32(&bars[s]), (uint32_t)((c - c0) / TILE_STAGES) & 1u, failed);
+                if (alive && !mbar_wait(smem_u32(&bars[s]), (uint32_t)((c - c0) / TILE_STAGES) & 1u, failed)) {
+                    alive = false;
+                    for (int i = c; tid == 0 && i < min(c1, c + TILE_STAGES); ++i)       // copies in flight, bounded
+                        for (uint32_t w = 0; w < tc5::WAIT_LIMIT; ++w)
+                            if (mbar_try_wait(smem_u32(&bars[(i - c0) % TILE_STAGES]), (uint32_t)((i - c0) / TILE_STAGES) & 1u)) break;
+                }
             } else {
                 cp_wait<TILE_STAGES - 1>();
                 __syncthreads();
@@ -587,9 +587,6 @@ gemm_f32_tile_kernel(Args p, const __grid_constant__ CUtensorMap map_a, const __
         cp_wait<0>();
     } else if (tid == 0 && *failed) {                         // (the last chunk's barrier is behind every wait)
         prb_set_status(p.status, PRB_S_WAIT_TIMEOUT, 41, blockIdx.x, blockIdx.y);
-        for (int i = max(c0, asked - TILE_STAGES); i < asked; ++i)       // copies in flight, bounded
-            for (uint32_t w = 0; w < tc5::WAIT_LIMIT; ++w)
-                if (mbar_try_wait(smem_u32(&bars[(i - c0) % TILE_STAGES]), (uint32_t)((i - c0) / TILE_STAGES) & 1u)) break;
     }
     __syncthreads();
 #pragma unroll

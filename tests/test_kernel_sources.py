@@ -31,16 +31,16 @@ def test_a_warp_of_the_ring_attention_has_one_answer_to_a_wait():
 
 
 def test_a_wait_that_gave_up_in_a_32_bit_tile_stops_its_whole_cluster():
-    """A bounded wait may end differently for a CTA's threads: whoever gave up, nothing more is requested into a
-    stage that may still be written, the status is recorded, and no CTA of the cluster stores sums that hold the
-    broken part."""
+    """A bounded wait may end differently for a CTA's threads: who requests copies has waited for the stage's last
+    one, whoever gave up the status is recorded, and no CTA of the cluster stores sums that hold the broken part."""
     kernel = _code("gemm_f32.cu").split("gemm_f32_tile_kernel(Args", 1)[1].split("int launch_tile_by", 1)[0]
     requests, rest = kernel.split("prb_grid_wait();", 1)
-    assert re.search(r"if \(tid == 0 && !\*failed\) \{[^}]*mbar_expect_tx", requests)
+    assert re.search(r"if \(tid == 0 && alive\) \{[^}]*mbar_expect_tx", requests)
     chunk = rest.split("mbar_wait(", 1)[1].split("load_rows(c + TILE_STAGES", 1)[0]
-    assert re.search(r"__syncthreads\(\);\s*$", chunk)             # every thread's wait is behind the next request
+    assert re.search(r"alive = false;\s*for \(int i = c; tid == 0 && i < min\(c1, c \+ TILE_STAGES\); \+\+i\)\s*"
+                     r"for \(uint32_t w = 0; w < tc5::WAIT_LIMIT", chunk)
+    assert re.search(r"__syncthreads\(\);\s*$", chunk)             # every thread's reads are behind the next request
     assert re.search(r"tid == 0 && \*failed\) \{\s*prb_set_status\(p.status, PRB_S_WAIT_TIMEOUT", rest)
-    assert re.search(r"i < asked; \+\+i\)\s*for \(uint32_t w = 0; w < tc5::WAIT_LIMIT", rest)
     before, store = rest.split("cluster_sync_all();", 1)
     assert "PRB_S_WAIT_TIMEOUT" in before and "finish(p" not in before
     assert re.search(r"any \|= ld_cluster1\(smem_u32\(&failed_word\), q\);\s*alive = any == 0;", store.split("finish(p", 1)[0])
