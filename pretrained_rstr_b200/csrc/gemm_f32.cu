@@ -671,19 +671,57 @@ int launch_tile(const Args& p, int copy, cudaStream_t stream) {
            : copy == COPY_16 ? launch_tile_by<BM, BN, TM, TN, COPY_16, 1>(p, stream)
                              : launch_tile_by<BM, BN, TM, TN, COPY_4, 1>(p, stream);
 }
-// Runs a CTA of 64 x 128 takes.  Two halve what a tile costs besides its FMAs (first copies, parts
-// through the cluster, about one and a half chunks' time) but leave half as many CTAs to deal out: the rule counts rounds
-// of two CTAs an SM, the last one cheaper where an SM has one CTA alone.  One run / two, us: 690 x 50,257 x
-// 768 1,465 / 1,304, 1,000 x 2,304 110 / 95, 690 x 3,072 98 / 95; 300 x 2,304 41 / 50, 1,000 x 768 41 / 50.
-// (All four runs in a CTA leave room for one an SM: 1,831.)
-int tile_runs(long tiles, int k) {
+// Clusters of an instance that run side by side, as the device says (asked once per device).
+template <int BM, int BN, int TM, int TN, int RUNS>
+int active_clusters() {
+    using Cfg = TileCfg<BM, BN, TM, TN, RUNS>;
+    constexpr auto kernel = gemm_f32_tile_kernel<BM, BN, TM, TN, COPY_TMA, RUNS>;
+    static std::atomic<int> known[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+    int n = known[dev].load(std::memory_order_relaxed);
+    if (n > 0) return n;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(4 / RUNS);
+    cfg.blockDim = dim3(Cfg::THREADS);
+    cfg.dynamicSmemBytes = Cfg::SMEM;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 4 / RUNS;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (prb_allow_shared<kernel>((int)Cfg::SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess)
+        cudaGetLastError();
+    n = n > 0 ? n : 1;
+    known[dev].store(n, std::memory_order_relaxed);
+    return n;
+}
+// Which tiles a product takes: 3 (64 x 64), 4 or 5 (64 x 128, one run or two a CTA).  What a launch costs is
+// counted in rounds of the clusters that the device runs side by side, a round in chunks of K: those of a CTA
+// and one and a half for its first copies and its part of the cluster's sums.  A last round that leaves the SMs
+// fewer CTAs than they hold (2 of 64 x 128, 3 of 64 x 64) is shorter; not where it is the only one, since a launch
+// that is placed early fills the SMs that the kernel ahead leaves first (logits of three texts, whose 768 columns
+// are 72 tiles: 8.19 ms with two runs there, a CTA an SM, 7.45 as it is).  A chunk of 64 x 64 takes 0.82 of one of
+// 64 x 128.  us of 3 / 4 / 5 by tiles of 64 x 128 at K = 768 (104 / 71 / 148 clusters side by side): 48 22.0 / 27.3 /
+// 32.8, 54 29.4 / 27.6 / 32.9, 70 35.9 / 27.7 / 33.1, 75 37.0 / 40.4 / 49.9, 90 41.6 / 41.0 / 50.3, 132 54.7 / 54.0 /
+// 50.7, 264 101 / 98.3 / 97.0, 4,323 1,517 / 1,474 / 1,344; at K = 3,072 90 145 / 138 / 179, 198 282 / 261 / 268.  It
+// is off most at 108 tiles (48.5 / 51.9 / 50.3: it takes 5).  (All four runs in a CTA leave room for one an SM: 1,831
+// at 4,323.)
+int tile_rule(long m, long n, int k, bool two_runs, bool only_wide) {
+    const long rows = (m + 63) / 64, big = rows * ((n + 127) / 128), small = rows * ((n + 63) / 64);
     const int run = ((k + CH - 1) / CH + 3) / 4;
-    const long sms = prb_sm_count(), slots = 2 * sms;
-    auto rounds = [&](int runs) {
-        const long ctas = tiles * (4 / runs), rest = ctas % slots;
-        return ((double)(ctas / slots) + (rest == 0 ? 0.0 : rest <= sms ? 0.6 : 1.0)) * (runs * run + 1.5);
+    auto cost = [](long clusters, int active, int held, const double* last, double chunks) {
+        const long full = clusters / active, rest = clusters % active;
+        if (full == 0) return chunks;
+        return chunks * ((double)full + (rest == 0 ? 0.0 : last[(rest * held + active - 1) / active - 1]));
     };
-    return rounds(2) < rounds(1) ? 2 : 1;
+    static const double last2[] = {0.6, 1.0}, last3[] = {0.48, 0.71, 1.0};
+    const double of3 = cost(small, active_clusters<64, 64, 8, 4, 1>(), 3, last3, 0.82 * (run + 1.5));
+    const double of4 = cost(big, active_clusters<64, 128, 8, 8, 1>(), 2, last2, run + 1.5);
+    const double of5 = two_runs ? cost(big, active_clusters<64, 128, 8, 8, 2>(), 2, last2, 2 * run + 1.5) : of4;
+    return !only_wide && of3 < of4 && of3 < of5 ? 3 : of5 < of4 ? 5 : 4;
 }
 
 constexpr size_t STREAM_SMEM = 220 * 1024;                    // the most a launch of the stream kernel takes
@@ -769,8 +807,8 @@ PRB_API int prb_gemm_f32(float* c, const float* a, const float* w, const float* 
     // 16-byte copies where every row starts on 16 bytes and K ends on them, else single floats
     const bool vec = k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)a) % 16 == 0 &&
                      ((uintptr_t)w) % 16 == 0;
-    // Up to 16 rows the stream kernel: 50,257 x 768 135 us against 146 as tiles, 768 x 768 5.5
-    // against 10.6; at 32 rows 263 against 147 and 17.5 against 15.6 (2,304 x 768).
+    // Up to 16 rows the stream kernel.  us as a stream / as tiles: 8 rows, 768 x 768 4.2 / 10.8, 2,304 x 768 6.7 / 15.0,
+    // 50,257 x 768 78 / 137; 16 rows 4.9 / 11.0, 10.2 / 15.3, 148 / 139; 32 rows 7.4 / 11.1, 18.1 / 15.3, 292 / 144.
     if (which == 1 || (which == 0 && m <= 16)) {
         StreamGeo g;
         size_t smem;
@@ -790,14 +828,17 @@ PRB_API int prb_gemm_f32(float* c, const float* a, const float* w, const float* 
     if (kv_width != 0) return PRB_E_SIZE;
     // (rows that overlap are no tensor that a copy engine's map describes)
     const int tiled = !vec ? COPY_4 : ldw >= k && lda >= k ? COPY_TMA : COPY_16;
-    // 64 x 128 where that leaves no SM without a CTA twice over, or nearly two an SM in one round of
-    // clusters (66 tiles: 690 x 768 x 768 28 us against 33, 690 x 768 x 3,072 91 against 109; 72 tiles take a
-    // second round: 137 x 3,072 x 768 39.5 against 36); else 64 x 64 (30 tiles: 300 x 768 x 768 21 us
-    // against 23, 300 x 768 x 3,072 72 against 74).
-    const long big = (long)((m + 63) / 64) * ((n + 127) / 128), sms = prb_sm_count();
-    const bool wide = big * 2 >= sms || (big * 8 >= 3 * sms && big * 20 <= 9 * sms);
-    const int runs = which == 4 || which == 5 ? which - 3 : tile_runs(big, k);
-    if (which == 3 || (which != 2 && which != 4 && which != 5 && !wide)) return launch_tile<64, 64, 8, 4, 1>(p, tiled, stream);
-    return runs == 2 ? launch_tile<64, 128, 8, 8, 2>(p, tiled, stream)
+    const int kind = which >= 3 && which <= 5 ? which : tile_rule(m, n, k, tiled == COPY_TMA, which == 2);
+    if (kind == 3) return launch_tile<64, 64, 8, 4, 1>(p, tiled, stream);
+    return kind == 5 ? launch_tile<64, 128, 8, 8, 2>(p, tiled, stream)
                      : launch_tile<64, 128, 8, 8, 1>(p, tiled, stream);
+}
+// The tiles that a product of more than 16 rows takes (3, 4 or 5, as above), and how many clusters of each kind
+// run side by side.
+PRB_API int prb_gemm_f32_tiles(int m, int n, int k, int* side_by_side) {
+    if (m <= 0 || n <= 0 || k <= 0) return 0;
+    side_by_side[0] = active_clusters<64, 64, 8, 4, 1>();
+    side_by_side[1] = active_clusters<64, 128, 8, 8, 1>();
+    side_by_side[2] = active_clusters<64, 128, 8, 8, 2>();
+    return tile_rule(m, n, k, true, false);
 }

@@ -84,6 +84,7 @@ def _declare(h: ctypes.CDLL) -> None:
     h.prb_host_device_address.restype = c_void_p
     h.prb_fetch_step.argtypes = [P, P, I, I, I, P, I, P, P]
     h.prb_publish_result.argtypes = [P, P, I, P]
+    h.prb_gemm_f32_tiles.argtypes = [I, I, I, P]
     h.prb_gemm_smallm_plan.argtypes = [I, I, I, I, P, P, P]
     h.prb_gemm_f32.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, I, I, P, P, P, I, I, I, I, I,
                                        P, P]
@@ -460,6 +461,13 @@ def copy_pages(storage, pairs, n_pairs, status) -> None:
     page_bytes = storage[0, 0].numel() * storage.element_size()
     _check(lib().prb_copy_pages(_p(storage), _p(pairs), n_pairs, page_bytes, pools, pages,
                                 _p(status), _stream()), what)
+
+
+def gemm_f32_tiles(m: int, n: int, k: int):
+    """The tiles a product of more than 16 rows takes (``kernel`` 3, 4 or 5 of :func:`gemm_f32`), and how many
+    clusters of each kind run side by side on the device."""
+    side = (c_int * 3)()
+    return int(lib().prb_gemm_f32_tiles(m, n, k, ctypes.byref(side))), tuple(side)
 
 
 def gemm_f32(out, a, w, bias=None, resid=None, act=None, kernel: int = 0, status=None,

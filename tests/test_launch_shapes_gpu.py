@@ -61,7 +61,7 @@ def test_float32_tiles_of_one_and_of_two_runs_a_cta_give_the_same_bits(m, n, k):
     wide = torch.randn(n, k + 1, device="cuda", generator=g)
     resid = torch.randn(m, n, device="cuda", generator=g)
     out = []
-    for kernel in (2, 4, 5):
+    for kernel in (0, 2, 3, 4, 5):
         for w in (wide[:, :k].contiguous(), wide[:, :k]):
             out.append(torch.full((m, n), float("nan"), device="cuda"))
             ops.gemm_f32(out[-1], a, w, resid=resid, kernel=kernel)
@@ -70,6 +70,17 @@ def test_float32_tiles_of_one_and_of_two_runs_a_cta_give_the_same_bits(m, n, k):
         ops.gemm_f32(few[i:i + 16], a[i:i + 16], wide[:, :k].contiguous(), resid=resid[i:i + 16].contiguous())
     for other in out[1:] + [few]:
         assert torch.equal(out[0], other)
+
+
+@pytest.mark.parametrize("k", [768, 1600, 3072])
+def test_float32_tiles_turn_where_a_round_of_clusters_is_full(k):
+    """Columns of 64 x 128, by the clusters that the device says run side by side: 64 x 64 while its clusters take one
+    round, then one run a CTA while those do; two runs where that saves a round."""
+    ops = _ops()
+    _kind, (small, one, two) = ops.gemm_f32_tiles(64, 128, k)
+    assert 2 * one > small and two > one
+    for tiles, kind in ((1, 3), (small // 2, 3), (small // 2 + 1, 4), (one, 4), (one + 1, 3), (two, 5), (9 * two, 5)):
+        assert ops.gemm_f32_tiles(64 * tiles, 128, k)[0] == kind, tiles
 
 
 @pytest.mark.parametrize("rows", [128, 129, 149, 2368, 2369, 5000])
