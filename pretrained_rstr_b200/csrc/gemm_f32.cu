@@ -783,12 +783,19 @@ bool stream_geometry(const Args& p, int mb, int copy, StreamGeo* g, size_t* smem
     *smem = bytes(best, g->stages);
     return true;
 }
+// The same for the most rows of A a CTA can hold; returns them, 0 where even one does not fit.
+int stream_rows(const Args& p, int copy, StreamGeo* g, size_t* smem) {
+    for (int mb = p.m == 1 ? 1 : p.m == 2 ? 2 : p.m <= 4 ? 4 : 8; mb >= 1; mb /= 2)
+        if (stream_geometry(p, mb, copy, g, smem)) return (p.m + mb - 1) / mb <= 65535 ? mb : 0;
+    return 0;
+}
+constexpr int STREAM_ROWS = 16;                               // most rows that take the stream kernel by themselves
 }  // namespace
 
 // which: 0 the rule below; 1 the stream kernel where it fits, 2 / 3 tiles of 64 x 128, 64 x 64, 4 / 5 tiles of
 // 64 x 128 of one run and of two runs a CTA (the same bits from all of them).  settled: w was written long before (by no kernel of the step), so the
 // launch may be placed, and w read, before the kernel ahead in the stream has ended.
-// kv_width > 0 (up to 16 rows that the stream kernel takes, else refused): the product is a fused QKV
+// kv_width > 0 (where prb_gemm_f32_scatters says so, else refused): the product is a fused QKV
 // projection, whose key and value columns also go to the paged cache (float32, contiguous) at slots[row]: 8
 // requests generating 24 tokens 19.2 -> 19.0 ms.  (In the tiles' epilogue it cost more than the append
 // behind them: three prompts of 301 tokens 7.36 -> 7.49 ms.)
@@ -809,20 +816,16 @@ PRB_API int prb_gemm_f32(float* c, const float* a, const float* w, const float* 
                      ((uintptr_t)w) % 16 == 0;
     // Up to 16 rows the stream kernel.  us as a stream / as tiles: 8 rows, 768 x 768 4.2 / 10.8, 2,304 x 768 6.7 / 15.0,
     // 50,257 x 768 78 / 137; 16 rows 4.9 / 11.0, 10.2 / 15.3, 148 / 139; 32 rows 7.4 / 11.1, 18.1 / 15.3, 292 / 144.
-    if (which == 1 || (which == 0 && m <= 16)) {
+    if (which == 1 || (which == 0 && m <= STREAM_ROWS)) {
         StreamGeo g;
         size_t smem;
-        int mb = m == 1 ? 1 : m == 2 ? 2 : m <= 4 ? 4 : 8;
         // (rows that overlap, an expanded row for one, are no tensor that a copy engine's map describes)
         const int copy = !vec ? COPY_4 : k % CH == 0 && k / CH <= 256 && ldw >= k ? COPY_TMA : COPY_16;
-        while (mb > 1 && !stream_geometry(p, mb, copy, &g, &smem)) mb /= 2;
-        if (stream_geometry(p, mb, copy, &g, &smem) && (m + mb - 1) / mb <= 65535) {
-            switch (mb) {
-                case 1: return launch_stream<1>(p, g, copy, smem, stream);
-                case 2: return launch_stream<2>(p, g, copy, smem, stream);
-                case 4: return launch_stream<4>(p, g, copy, smem, stream);
-                default: return launch_stream<8>(p, g, copy, smem, stream);
-            }
+        switch (stream_rows(p, copy, &g, &smem)) {
+            case 1: return launch_stream<1>(p, g, copy, smem, stream);
+            case 2: return launch_stream<2>(p, g, copy, smem, stream);
+            case 4: return launch_stream<4>(p, g, copy, smem, stream);
+            case 8: return launch_stream<8>(p, g, copy, smem, stream);
         }
     }
     if (kv_width != 0) return PRB_E_SIZE;
@@ -832,6 +835,16 @@ PRB_API int prb_gemm_f32(float* c, const float* a, const float* w, const float* 
     if (kind == 3) return launch_tile<64, 64, 8, 4, 1>(p, tiled, stream);
     return kind == 5 ? launch_tile<64, 128, 8, 8, 2>(p, tiled, stream)
                      : launch_tile<64, 128, 8, 8, 1>(p, tiled, stream);
+}
+// Whether prb_gemm_f32 brings key and value columns to the cache: whether the stream kernel takes the sizes,
+// however the rows are aligned.
+PRB_API int prb_gemm_f32_scatters(int m, int n, int k) {
+    if (m <= 0 || n <= 0 || k <= 0 || m > STREAM_ROWS) return 0;
+    Args p{};
+    p.m = m; p.n = n; p.k = k;
+    StreamGeo g;
+    size_t smem;
+    return stream_rows(p, COPY_4, &g, &smem) > 0 && stream_rows(p, COPY_TMA, &g, &smem) > 0;
 }
 // The tiles that a product of more than 16 rows takes (3, 4 or 5, as above), and how many clusters of each kind
 // run side by side.

@@ -84,6 +84,7 @@ def _declare(h: ctypes.CDLL) -> None:
     h.prb_host_device_address.restype = c_void_p
     h.prb_fetch_step.argtypes = [P, P, I, I, I, P, I, P, P]
     h.prb_publish_result.argtypes = [P, P, I, P]
+    h.prb_gemm_f32_scatters.argtypes = [I, I, I]
     h.prb_gemm_f32_tiles.argtypes = [I, I, I, P]
     h.prb_gemm_smallm_plan.argtypes = [I, I, I, I, P, P, P]
     h.prb_gemm_f32.argtypes = [P, P, P, P, P, I, I, I, L, L, L, I, I, I, P, P, P, I, I, I, I, I,
@@ -463,6 +464,11 @@ def copy_pages(storage, pairs, n_pairs, status) -> None:
                                 _p(status), _stream()), what)
 
 
+def gemm_f32_scatters(m: int, n: int, k: int) -> bool:
+    """Whether ``gemm_f32`` takes ``kv_scatter`` at these sizes."""
+    return bool(lib().prb_gemm_f32_scatters(m, n, k))
+
+
 def gemm_f32_tiles(m: int, n: int, k: int):
     """The tiles a product of more than 16 rows takes (``kernel`` 3, 4 or 5 of :func:`gemm_f32`), and how many
     clusters of each kind run side by side on the device."""
@@ -474,7 +480,7 @@ def gemm_f32(out, a, w, bias=None, resid=None, act=None, kernel: int = 0, status
              settled: bool = False, kv_scatter=None) -> None:
     """out[M,N] = act(a[M,K] . w[N,K]^T + bias) (+ resid): true 32-bit FMA, one order of
     summation for every M.  ``kv_scatter`` = (k_pages, v_pages, slots, q_width): the key and value columns
-    of a fused QKV product of up to 16 rows also go to the paged cache (float32, contiguous) at each row's slot.  ``settled``: ``w`` was complete before the kernel ahead in the stream
+    of a fused QKV product (where :func:`gemm_f32_scatters`) also go to the paged cache (float32, contiguous) at each row's slot.  ``settled``: ``w`` was complete before the kernel ahead in the stream
     began (a model's weights are), so it may be read while that still runs.  ``kernel`` forces one of the kernels (1 rows of weights as a
     stream, 2 / 3 tiles of 64 x 128, 64 x 64, 4 / 5 tiles of 64 x 128 of one and of two runs a CTA); left at 0 the sizes choose.  All give the same bits."""
     what = "gemm_f32"

@@ -80,9 +80,10 @@ class Linear:
         QKV product straight to the cache; returns True when it did."""
         m = out.shape[0]
         if self.runtime.dtype == torch.float32:
-            # (the kernel of a few rows brings keys and values to the cache; it takes every K up to 8,192)
-            if kv_scatter is not None and (m > 16 or self.n_in > 8192 or resid is not None or
-                                           not kv_scatter[0].is_contiguous() or not kv_scatter[1].is_contiguous()):
+            # (the kernel of a few rows brings keys and values to the cache)
+            if kv_scatter is not None and not (
+                    resid is None and kv_scatter[0].is_contiguous() and kv_scatter[1].is_contiguous() and
+                    ops.gemm_f32_scatters(m, self.n_out, self.n_in)):
                 kv_scatter = None
             ops.gemm_f32(out, _tensor(a), self.weight, self.bias, resid, act, status=ctx.status, settled=True,
                          kv_scatter=kv_scatter)

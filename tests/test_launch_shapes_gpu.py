@@ -135,6 +135,33 @@ def test_float32_product_scatters_keys_and_values(m, heads, kv_heads, dh, ps):
                      kv_scatter=(cache[0], cache[1], torch.zeros(17, dtype=torch.int32, device="cuda"), q_width))
 
 
+@pytest.mark.parametrize("m", [1, 5, 16])
+@pytest.mark.parametrize("k", [8192, 8224, 8225, 16384, 16640, 40000])
+def test_float32_product_says_where_it_scatters(m, k):
+    """The widest rows: where the answer is yes the product brings keys and values to the cache, however its rows
+    are aligned, and where it is no it refuses."""
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    dh, ps = 8, 16
+    a, w = torch.randn(m, k + 1, device="cuda", generator=g), torch.randn(3 * dh, k, device="cuda", generator=g)
+    slots = torch.arange(m, dtype=torch.int32, device="cuda")
+    want = ops.gemm_f32_scatters(m, 3 * dh, k)
+    assert want or k > 8225
+    for rows in (a[:, :k], a[:, :k].contiguous()):
+        keys, values = torch.zeros(2, 1, ps, dh, device="cuda"), torch.zeros(2, 1, ps, dh, device="cuda")
+        out = torch.zeros(m, 3 * dh, device="cuda")
+        if want:
+            ops.gemm_f32(out, rows, w, kv_scatter=(keys, values, slots, dh))
+            assert torch.equal(keys.view(-1, dh)[:m], out[:, dh:2 * dh])
+            assert torch.equal(values.view(-1, dh)[:m], out[:, 2 * dh:])
+            # (a sum of k products of numbers around 1, chunk by chunk)
+            assert float((out.double() - rows.double() @ w.double().t()).abs().max()) <= 1e-6 * k
+        else:
+            with pytest.raises(ops.KernelArgumentError, match="size"):
+                ops.gemm_f32(out, rows, w, kv_scatter=(keys, values, slots, dh))
+    assert not ops.gemm_f32_scatters(17, 3 * dh, 64)
+
+
 @pytest.mark.parametrize("heads", [20, 25, 32])
 def test_a_few_requests_keep_32_bit_weights(heads):
     """Fewer than 16 tokens of up to two (token, head) pairs an SM stay with the kernel that multiplies the values
