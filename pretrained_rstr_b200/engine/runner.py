@@ -353,17 +353,20 @@ class ModelRunner:
         self.last_h2d_bytes = words * 4
         if not ctx.copies:
             return
+        # (The first kernel behind the copies is launched the plain way, never early: the decode attention asks
+        # for cached pages before the kernel ahead of it has ended, and they may be pages copied here.)
         for g in range(self.n_groups):
             pairs = [(src, dst) for (gg, src, dst) in ctx.copies if gg == g]
-            host = self._pairs_hosts[ctx.staging_turn][g]
-            for i in range(0, len(pairs), host.shape[0]):
-                if i > 0:                            # the pinned buffer is used again within the step
-                    torch.cuda.current_stream().synchronize()
-                chunk = pairs[i:i + host.shape[0]]
-                host[:len(chunk)] = torch.tensor(chunk, dtype=torch.int32)
-                self._pairs_dev[:len(chunk)].copy_(host[:len(chunk)], non_blocking=True)
-                self.storage.copy_pages(g, self._pairs_dev, len(chunk), self.status)
-                self.counters["cow_copies"] += len(chunk)
+            if not pairs:
+                continue
+            # (a request copies at most the page it holds in part: one a step and group)
+            host, n = self._pairs_hosts[ctx.staging_turn][g], len(pairs)
+            if n > host.shape[0]:
+                raise StepError(f"{n} page copies in a step of at most {host.shape[0]} requests")
+            host[:n] = torch.tensor(pairs, dtype=torch.int32)
+            self._pairs_dev[:n].copy_(host[:n], non_blocking=True)
+            self.storage.copy_pages(g, self._pairs_dev, n, self.status)
+            self.counters["cow_copies"] += n
         self._host_events[ctx.staging_turn].record()     # who takes this staging buffer next waits for these too
 
     def commit(self, entries: Sequence[Entry]) -> None:

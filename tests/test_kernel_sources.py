@@ -65,3 +65,12 @@ def test_float32_products_share_no_switch_between_threads():
     """Which kernel a product takes is its call's own argument: no variable of the file that other threads' launches
     read as well."""
     assert not re.search(r"^(static\s+)?(int|bool|long)\s+g_\w+\s*(=|;)", _code("gemm_f32.cu"), flags=re.M)
+
+
+def test_the_first_kernel_behind_the_page_copies_is_launched_the_plain_way():
+    """The decode attention asks for cached pages before the kernel ahead of it has ended: all that follows the page
+    copies of a step may start early only because the embedding, and the copies themselves, do not."""
+    code = _code("elementwise.cu")
+    for entry in ("prb_embed(", "prb_copy_pages("):
+        body = code.split("PRB_API int " + entry, 1)[1].split("PRB_API", 1)[0]
+        assert "<<<" in body and "prb_launch" not in body
