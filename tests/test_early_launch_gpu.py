@@ -45,7 +45,7 @@ def test_gemm_f32_reads_weights_written_by_the_kernel_before_it(m, n, k):
     _compare(lambda src: _write(ops, w, src), lambda out: ops.gemm_f32(out, a, w), (m, n), _sources(g, n, k))
 
 
-@pytest.mark.parametrize("rows,width", [(1, 768), (100, 1024), (20, 1600), (3, 2052)])
+@pytest.mark.parametrize("rows,width", [(1, 768), (100, 1024), (20, 1600), (3, 2052), (129, 768), (2369, 1600)])
 def test_layernorm_reads_parameters_written_by_the_kernel_before_it(rows, width):
     ops = _ops()
     g = torch.Generator(device="cuda").manual_seed(rows + width)
@@ -53,6 +53,28 @@ def test_layernorm_reads_parameters_written_by_the_kernel_before_it(rows, width)
     w = torch.zeros(2, width, device="cuda")
     _compare(lambda src: _write(ops, w, src), lambda out: ops.layernorm(out, x, w[0], w[1], 1e-5), (rows, width),
              _sources(g, 2, width))
+
+
+@pytest.mark.parametrize("rows,width", [(1, 768), (128, 1024), (129, 768), (149, 1600), (2369, 1024)])
+def test_layernorm_of_settled_parameters_reads_rows_written_by_the_kernel_before_it(rows, width):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(rows + width)
+    x = torch.zeros(rows, width, device="cuda")
+    gamma, beta = torch.randn(width, device="cuda", generator=g), torch.randn(width, device="cuda", generator=g)
+    _compare(lambda src: _write(ops, x, src), lambda out: ops.layernorm(out, x, gamma, beta, 1e-5, settled=True),
+             (rows, width), _sources(g, rows, width))
+
+
+@pytest.mark.parametrize("m,n,k,kernel", [(16, 768, 768, 0), (65, 768, 768, 3), (65, 768, 3072, 4), (690, 2304, 768, 4),
+                                          (690, 2304, 768, 5), (129, 1027, 260, 5), (130, 700, 33, 0)])
+def test_gemm_f32_of_settled_weights_reads_rows_written_by_the_kernel_before_it(m, n, k, kernel):
+    """Its weights may be read while the kernel ahead still runs, its rows of A may not."""
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(n + k + kernel)
+    w = torch.randn(n, k, device="cuda", generator=g)
+    a = torch.zeros(m, k, device="cuda")
+    _compare(lambda src: _write(ops, a, src), lambda out: ops.gemm_f32(out, a, w, kernel=kernel, settled=True), (m, n),
+             _sources(g, m, k))
 
 
 @pytest.mark.parametrize("rows,width", [(1, 768), (100, 1600), (5, 4100)])
