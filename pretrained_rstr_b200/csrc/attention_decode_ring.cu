@@ -116,27 +116,22 @@ PRB_API int prb_attention_decode_ring_supports(int head_dim, int page_size) {
 PRB_API int prb_attention_decode_ring_max_list() { return MAX_LIST; }
 
 // Whether this kernel is the faster one for a launch of n_list tokens over contexts of up to
-// max_context keys; the split-key kernel of attention_decode.cu is the other.  Measured (with the
-// look-ups and the merge of both as they were) inside
-// whole decode steps, ms a step, split-key / ring, at contexts of 250, 500 and 900 tokens (n_list is
-// the capacity the step's graph was made for, so 24 requests run as 32 and 48 as 64).
-// GPT-2 small, 12 heads: 1 request 0.326 / 0.332, 0.330 / 0.334, 0.348 / 0.351; 8: 0.338 / 0.354,
-// 0.347 / 0.373, 0.390 / 0.395; 16: 0.422 / 0.453, 0.469 / 0.468, 0.537 / 0.515; 32: 0.536 / 0.523,
-// 0.607 / 0.581, 0.747 / 0.663; 64: 0.589 / 0.618, 0.782 / 0.736, 1.037 / 0.889.  Medium, 16 heads:
-// 1: 0.680 / 0.719, 0.685 / 0.724, 0.717 / 0.722; 16: 0.940 / 0.938, 1.053 / 1.071, 1.326 / 1.195; 32:
-// 1.285 / 1.181, 1.536 / 1.351, 1.696 / 1.578; 64: 1.429 / 1.303, 1.715 / 1.692, 2.246 / 2.074.  XL, 25
-// heads: 1: 1.895 / 2.029, 1.921 / 2.086, 2.068 / 2.113; 8: 1.994 / 2.161, 2.192 / 2.309, 2.493 / 2.483;
-// 16: 2.841 / 2.826, 3.190 / 3.140, 3.769 / 3.591; 32: 3.728 / 3.777, 4.479 / 4.172, 5.393 / 4.848.  An
-// engine of 320 requests, small, up to 200, 600 and 990 tokens: 65: 0.815 / 0.855, 1.120 / 1.077,
-// 1.326 / 1.213; 128: 1.209 / 1.207, 1.661 / 1.590, 1.995 / 1.837; 256: 2.434 / 2.440, 3.220 / 3.047, 3.782 /
-// 3.528.
-// The ring wins where many (token, head) pairs have long contexts (its warps stream long runs,
-// the other kernel's CTAs walk their keys one batch after the other) and in the middle range at
-// nearly every context; it loses at few requests.
-// Fewer than 16 tokens of one or two (token, head) pairs an SM stay with the split-key kernel, also where
-// this one has become the faster (8 requests of XL at 450 to 900 tokens): that one multiplies the values
-// by 32-bit weights, this one rounds the weights to bfloat16 for its matrix instructions, and the line
-// between them moves no launch from the former to the latter.
+// max_context keys, as far as precision leaves the choice; the split-key kernel of attention_decode.cu is the
+// other.  Measured inside whole decode steps, ms a step, split-key / ring, at contexts of 250, 500 and 900 tokens
+// (n_list is the capacity the step's graph was made for, so 24 requests run as 32 and 48 as 64).
+// GPT-2 small, 12 heads: 1 request 0.303 / 0.317, 0.304 / 0.318, 0.304 / 0.323; 8: 0.323 / 0.328,
+// 0.329 / 0.349, 0.378 / 0.402; 16: 0.424 / 0.431, 0.474 / 0.465, 0.531 / 0.505; 32: 0.589 / 0.579,
+// 0.660 / 0.632, 0.864 / 0.758; 64: 0.768 / 0.769, 0.985 / 0.921, 1.261 / 1.112.  Medium, 16 heads:
+// 1: 0.645 / 0.679, 0.650 / 0.681, 0.655 / 0.689; 8: 0.704 / 0.706, 0.721 / 0.752, 0.819 / 0.870; 16: 0.941 / 0.964,
+// 1.046 / 1.038, 1.287 / 1.186; 32: 1.398 / 1.260, 1.623 / 1.410, 1.859 / 1.691; 64: 1.815 / 1.643, 2.140 / 1.988,
+// 2.723 / 2.525.  XL, 25 heads: 1: 1.710 / 1.696, 1.709 / 1.713, 1.863 / 1.768; 8: 1.794 / 1.853, 2.015 / 1.989,
+// 2.236 / 2.173; 16: 2.581 / 2.445, 2.893 / 2.680, 3.588 / 3.180; 32: 3.918 / 3.855, 4.630 / 4.362, 5.615 / 5.022.
+// The ring wins where many (token, head) pairs have long contexts (its warps stream long runs, the other kernel's
+// CTAs walk their keys one batch after the other) and in the middle range at nearly every context; it loses at few
+// requests.  Two lines lie where it is the faster one by now: four pairs an SM and more at up to 512 keys (64
+// requests of small or medium, 32 of XL), and 8 requests of XL.  They stay: the split-key kernel multiplies the
+// values by 32-bit weights, this one rounds the weights to bfloat16 for its matrix instructions, and no launch is
+// moved from the former to the latter for its speed.
 PRB_API int prb_attention_decode_ring_prefers(int n_list, int n_heads, int max_context) {
     const long pairs = (long)n_list * n_heads;
     const long sms = prb_sm_count();

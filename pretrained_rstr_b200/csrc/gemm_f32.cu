@@ -16,15 +16,15 @@
 // ahead has ended); a thread keeps its chunk of up to four rows of A in registers and walks the
 // weight rows of a stage, so an FMA costs a quarter of a shared-memory operand; chunk sums meet in
 // shared memory.  The rows of A come by asynchronous copies, all at once, and what the sums are finished
-// with (quotients of run-time counts, bias, residual) is there before them: 8 rows, 2,304 x 768 7.1 -> 6.1 us,
-// 768 x 768 5.1 -> 4.3, 3,072 x 768 8.6 -> 7.6, 768 x 3,072 10.4 -> 8.3, 50,257 x 768 84 -> 77 us = 2.0 TB/s; one
+// with (quotients of run-time counts, bias, residual) is there before them: 8 rows, 2,304 x 768 7.0 -> 6.6 us,
+// 768 x 768 4.6 -> 4.2, 3,072 x 768 8.8 -> 8.4, 768 x 3,072 10.4 -> 8.1, 50,257 x 768 81 -> 78 us = 2.0 TB/s; one
 // CTA a tile of 64 x 64 (12 CTAs for 768 columns) takes 177 us on average over a model's products.
 //
 // gemm_f32_tile_kernel: more rows.  Tiles of BM x BN, the four runs of K by the CTAs of a cluster, one or
 // two each (a prompt of a few hundred tokens has too few tiles for 148 SMs otherwise), partial tiles added
 // through distributed shared memory, a part of the rows a CTA.  Stages come by TMA where the rows allow
-// it; a chunk's row is 128 bytes, its 16-byte pieces swizzled.  690 rows: 2,304 x 768 77 -> 75 us, 3,072 x 768
-// 101 -> 95, 768 x 768 31 -> 28, 768 x 3,072 106 -> 91, 50,257 x 768 1.50 -> 1.31 ms = 41 TFLOP/s; one CTA a tile
+// it; a chunk's row is 128 bytes, its 16-byte pieces swizzled.  690 rows: 2,304 x 768 77 -> 76 us, 3,072 x 768
+// 101 -> 97, 768 x 768 31 -> 28, 768 x 3,072 109 -> 91, 50,257 x 768 1.50 -> 1.34 ms = 40 TFLOP/s; one CTA a tile
 // over all of K 14 TFLOP/s.  What bounds it: the FMA loop.  fma.rn.f32x2 of operands in three registers
 // runs at 57 TFLOP/s (72 with two); 255 registers leave two warps a scheduler, which cover neither its
 // latency nor that of shared memory whole (counters at 690 x 3,072 x 768: issue slots 38 %, shared memory 59 %).
